@@ -55,8 +55,8 @@ __host__ __device__ constexpr int gbdf_rhs_bytes() {
 }
 template <class M, class JR>
 __host__ __device__ constexpr int gbdf_setup_bytes() {
-  constexpr int N = M::N, NS = M::NS, NR = M::NR;
-  return N * 8 + (N + wbdf::RXW * NR + 4 * NS) * (int)sizeof(JR);
+  constexpr int N = M::N, NS = M::NS;
+  return N * 8 + (N + wbdf::rx_len<M>() + 4 * NS) * (int)sizeof(JR);
 }
 template <class M, class JR, int G>
 __host__ __device__ constexpr int gbdf_shared_scratch_bytes() {
@@ -83,8 +83,10 @@ __device__ __forceinline__ unsigned group_mask() {
     return ((1u << G) - 1u) << (lane - lane % G);
   }
 }
+// Out of line: the kernel sums at fourteen places, and a shuffle with a run-time mask is several
+// instructions (17 KB of code inlined).
 template <int G>
-__device__ __forceinline__ double group_sum(double v, unsigned gm) {
+__device__ __noinline__ double group_sum(double v, unsigned gm) {
 #pragma unroll
   for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(gm, v, o);
   return v;
@@ -173,7 +175,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
   using namespace bdf;
   using Tab = typename M::TabG;
   static_assert(G == 4 || G == 8 || G == 16 || G == 32, "group size must divide the warp");
-  constexpr int N = M::N, NS = M::NS, NR = M::NR;
+  constexpr int N = M::N, NS = M::NS;
   constexpr int R = (N + G - 1) / G;  // vector elements per lane
   constexpr int LDA = N + 1;          // padded matrix row
   constexpr int CPW = 32 / G;         // cells per warp
@@ -208,8 +210,8 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
   const CellMem C = cell_mem(grp);
   double* const YS = reinterpret_cast<double*>(wscratch);         // [N] setup input staging
   JR* const WXS = reinterpret_cast<JR*>(YS + N);                  // [N] setup concentrations
-  JR* const WRX = WXS + N;                                        // [NR][RXW] Jacobian partials
-  JR* const WTH = WRX + wbdf::RXW * NR;                           // [4][NS] NASA-7 terms
+  JR* const WRX = WXS + N;                                        // Jacobian partials
+  JR* const WTH = WRX + wbdf::rx_len<M>();                        // [4][NS] NASA-7 terms
 
   const long long ncell = P.ncell_dev ? (long long)*P.ncell_dev : P.ncell;
   const int qmax = max(1, min(P.max_order, QMAX));
@@ -228,7 +230,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
   double del2 = 0.0, delp2 = 0.0, hg = 0.0, hub = 0.0, hlb = 0.0, rE0 = 0.0;
   int q = 1, qwait = 2, nef = 0, ncf = 0, m = 0, hin_count = 0, status = OK;
   int nst = 0, nfe = 0, nje = 0, nstlp = 0, netf = 0, ncfn = 0;  // bounded by ode.max_steps
-  bool new_step = true, need_setup = true, force_setup = true, jcur = false, setup_ok = true;
+  bool new_step = true, need_setup = true, force_setup = true, jcur = false, setup_ok = true, fresh = false;
 #pragma unroll
   for (int r = 0; r < R; ++r) { y[r] = 0.0; acor[r] = 0.0; ewt[r] = 1.0; }
 
@@ -249,6 +251,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
   };
   auto rescale = [&](double e) {
     double fac = e;
+#pragma unroll 1
     for (int j = 1; j <= q; ++j) {
 #pragma unroll
       for (int r = 0; r < R; ++r)
@@ -260,15 +263,18 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
   };
   auto predict = [&]() {
     t += h;
+#pragma unroll 1
     for (int k = 1; k <= q; ++k)
+#pragma unroll 1
       for (int j = q; j >= k; --j)
 #pragma unroll
         for (int r = 0; r < R; ++r)
           if (idx(r) < N) Z(j - 1, r) += Z(j, r);
   };
-  auto retract = [&]() {
-    t -= h;
+  auto retract = [&]() {  // t goes back where the outcome is found
+#pragma unroll 1
     for (int k = 1; k <= q; ++k)
+#pragma unroll 1
       for (int j = q; j >= k; --j)
 #pragma unroll
         for (int r = 0; r < R; ++r)
@@ -283,11 +289,13 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
     for (int i = 0; i <= QMAX; ++i) l[i] = 0.0;
     l[0] = 1.0;
     double alpha0 = 0.0;
+#pragma unroll 1
     for (int j = 1; j <= q; ++j) alpha0 -= inv_int(j);
     double hsum = h, sum_xi_inv = 0.0;
+#pragma unroll 1
     for (int i = 1; i <= q - 1; ++i) {
       if (i > 1) hsum += tau(i - 1);
-      const double xi_inv = h / hsum;
+      const double xi_inv = pgb_div64(h, hsum);
       sum_xi_inv += xi_inv;
 #pragma unroll
       for (int k = QMAX; k >= 1; --k)
@@ -298,32 +306,32 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
     for (int k = QMAX; k >= 1; --k)
       if (k <= q) l[k] += l[k - 1] * xistar_inv;
     if (q > 1) hsum += tau(q - 1);
-    const double xiq_inv = h / hsum;
+    const double xiq_inv = pgb_div64(h, hsum);
     const double alpha0_hat = -(sum_xi_inv + xiq_inv);
     const double A1 = 1.0 - alpha0_hat + alpha0;
     const double A2 = 1.0 + q * A1;
     double lq = 0.0;
 #pragma unroll
     for (int k = 0; k <= QMAX; ++k) if (k == q) lq = l[k];
-    tq2 = fabs(A1 / (alpha0 * A2));
-    tq5 = fabs(A2 * xistar_inv / (lq * xiq_inv));
+    tq2 = fabs(pgb_div64(A1, alpha0 * A2));
+    tq5 = fabs(pgb_div64(A2 * xistar_inv, lq * xiq_inv));
     if (qwait == 1) {
       if (q > 1) {
-        const double Cq = xistar_inv / lq;
+        const double Cq = pgb_div64(xistar_inv, lq);
         const double A3 = alpha0 + inv_int(q);
         const double A4 = alpha0_hat + xiq_inv;
-        tq1 = fabs(Cq * (1.0 - A4 + A3) / A3);
+        tq1 = fabs(pgb_div64(Cq * (1.0 - A4 + A3), A3));
       } else {
         tq1 = 1.0;
       }
-      const double xiq1_inv = h / (hsum + tau(q));
+      const double xiq1_inv = pgb_div64(h, hsum + tau(q));
       const double A5 = alpha0 - inv_int(q + 1);
       const double A6 = alpha0_hat - xiq1_inv;
-      const double Cpp = (1.0 - A6 + A5) / A2;
-      tq3 = fabs(Cpp / (xiq1_inv * (q + 2) * A5));
+      const double Cpp = pgb_div64(1.0 - A6 + A5, A2);
+      tq3 = fabs(pgb_div64(Cpp, xiq1_inv * (q + 2) * A5));
     }
     inv_tq4_sq = (tq2 * (1.0 / NLSCOEF)) * (tq2 * (1.0 / NLSCOEF));
-    rl1 = 1.0 / l[1];
+    rl1 = pgb_div64(1.0, l[1]);
     __syncwarp(gm);
     for (int e = sub; e <= QMAX; e += G) {
       double v = 0.0;
@@ -340,18 +348,19 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
     w[2] = 1.0;
     if (dq > 0) {
       double alpha0 = 0.0, alpha1 = 0.0, prod = 1.0, hsum = 0.0;
+#pragma unroll 1
       for (int j = 1; j <= q; ++j) {
         hsum += tau(j);
-        const double xi = hsum / hscale;
+        const double xi = pgb_div64(hsum, hscale);
         prod *= xi;
         alpha0 -= inv_int(j);
-        alpha1 += 1.0 / xi;
+        alpha1 += pgb_div64(1.0, xi);
         if (j <= q - 1)
 #pragma unroll
           for (int i = QMAX + 1; i >= 2; --i)
             if (i <= j + 2) w[i] = w[i] * xi + w[i - 1];
       }
-      const double A1 = (-alpha0 - alpha1) / prod;
+      const double A1 = pgb_div64(-alpha0 - alpha1, prod);
 #pragma unroll
       for (int r = 0; r < R; ++r)
         if (idx(r) < N) Z(q + 1, r) = A1 * Z(QMAX + 1, r);
@@ -363,9 +372,10 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
             if (idx(r) < N) Z(j, r) = fma(w[j], Z(q + 1, r), Z(j, r));
     } else {
       double hsum = 0.0;
+#pragma unroll 1
       for (int j = 1; j <= q - 2; ++j) {
         hsum += tau(j);
-        const double xi = hsum / hscale;
+        const double xi = pgb_div64(hsum, hscale);
 #pragma unroll
         for (int i = QMAX + 1; i >= 2; --i)
           if (i <= j + 2) w[i] = w[i] * xi + w[i - 1];
@@ -384,40 +394,17 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
   // (I - gamma J) x = b with the cell's factors: rows over the group's lanes, the operations and
   // their order of the warp mapping's solve
   auto solve = [&](double (&b)[R]) {
-    JR* XS = C.XS;
-    const JR* A = C.A;
+    JR x[R];
 #pragma unroll
     for (int r = 0; r < R; ++r)
-      if (idx(r) < N) XS[idx(r)] = (JR)b[r];
+      if (idx(r) < N) C.XS[idx(r)] = (JR)b[r];
     __syncwarp(gm);
-#pragma unroll 1
-    for (int k = 0; k < N; ++k) {
-      const int p = C.PIV[k];
-      if (p != k && sub == 0) { const JR tmp = XS[k]; XS[k] = XS[p]; XS[p] = tmp; }
-      __syncwarp(gm);
-      const JR bk = XS[k];
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const int i = idx(r);
-        if (i > k && i < N) XS[i] -= A[i * LDA + k] * bk;
-      }
-      __syncwarp(gm);
-    }
-#pragma unroll 1
-    for (int k = N - 1; k >= 0; --k) {
-      const JR xk = XS[k] * A[k * LDA + k];
-      __syncwarp(gm);
-      if (sub == 0) XS[k] = xk;
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const int i = idx(r);
-        if (i < k) XS[i] -= A[i * LDA + k] * xk;
-      }
-      __syncwarp(gm);
-    }
+    for (int r = 0; r < R; ++r) x[r] = idx(r) < N ? C.XS[C.PIV[idx(r)]] : JR(0);
+    lu_substitute<N, G>(C.A, gm, gbase, x);
 #pragma unroll
     for (int r = 0; r < R; ++r)
-      if (idx(r) < N) b[r] = (double)XS[idx(r)];
+      if (idx(r) < N) b[r] = (double)x[r];
     __syncwarp(gm);
   };
   // ---- cell I/O ----
@@ -456,10 +443,11 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
 #pragma unroll
     for (int r = 0; r < R; ++r)
       if (idx(r) < NS) rho_l += Z(0, r);
-    const double inv_rho = 1.0 / group_sum<G>(rho_l, gm);
+    const double inv_rho = pgb_div64(1.0, group_sum<G>(rho_l, gm));
     const double htarget = rE * inv_rho;
     double Tn = C.Z[NS];
     if (!(Tn > 90.0 && Tn < 5000.0)) Tn = 1000.0;
+#pragma unroll 1
     for (int it = 0; it < 50; ++it) {
       double hl = 0.0, cl = 0.0;
 #pragma unroll
@@ -479,7 +467,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
         }
       }
       const double hh = group_sum<G>(hl, gm), cp = group_sum<G>(cl, gm);
-      double dT = (htarget - hh) / cp;
+      double dT = pgb_div64(htarget - hh, cp);
       dT = fmax(-100.0, fmin(100.0, dT));
       Tn = fmax(90.0, fmin(5000.0, Tn + dT));
       if (fabs(dT) < 1e-10 * Tn) break;
@@ -540,7 +528,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
     tq1 = tq2 = tq3 = tq5 = tq5_saved = inv_tq4_sq = 1.0;
     q = 1; qwait = 2; nef = 0; ncf = 0; m = 0; status = OK;
     nst = 0; nfe = 0; nje = 0; nstlp = 0; netf = 0; ncfn = 0;
-    new_step = true; need_setup = true; force_setup = true; jcur = false;
+    new_step = true; need_setup = true; force_setup = true; jcur = false; fresh = false;
     __syncwarp(gm);
     return true;
   };
@@ -568,37 +556,32 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
     }
 
     // ------------------------------------------------ (B) prepare the RHS argument
+    if (phase == STEP && new_step && nst >= P.max_steps) fail_cell(MAX_STEPS);
+    if ((phase == STEP && new_step) || (phase == HIN && hin_count == 1)) set_ewt();
     if (phase == STEP) {
-      bool ok = true;
       if (new_step) {
-        if (nst >= P.max_steps) { fail_cell(MAX_STEPS); ok = false; }
-        else {
-          if ((t + h - tout) * h > 0.0) rescale((tout - t) * (1.0 - 4.0 * UROUND) / h);
-          set_ewt();
-          nef = 0; ncf = 0;
-          new_step = false;
-        }
+        nef = 0; ncf = 0;
+        new_step = false;
       }
-      if (ok) {
-        predict();
-        set_coeffs();
-        gamma = h * rl1;
-        if (nst == 0) gammap = gamma;
-        gamrat = (nst > 0) ? gamma / gammap : 1.0;
-        need_setup = force_setup || nst == 0 || nst >= nstlp + MSBP || fabs(gamrat - 1.0) > DGMAX;
-        force_setup = false;
-        jcur = false;
-        m = 0;
+      predict();
+      set_coeffs();
+      gamma = h * rl1;
+      if (nst == 0) gammap = gamma;
+      gamrat = (nst > 0) ? pgb_div64(gamma, gammap) : 1.0;
+      need_setup = force_setup || nst == 0 || nst >= nstlp + MSBP || fabs(gamrat - 1.0) > DGMAX;
+      force_setup = false;
+      jcur = false;
+      m = 0;
+      phase = NEWTON;
+      fresh = true;
+    }
+    if (fresh || phase == START || phase == RESETD) {  // from the prediction
 #pragma unroll
-        for (int r = 0; r < R; ++r) { y[r] = idx(r) < N ? Z(0, r) : 0.0; acor[r] = 0.0; }
-        phase = NEWTON;
-      }
+      for (int r = 0; r < R; ++r) { y[r] = idx(r) < N ? Z(0, r) : 0.0; acor[r] = 0.0; }
+      fresh = false;
     } else if (phase == HIN) {
 #pragma unroll
       for (int r = 0; r < R; ++r) y[r] = idx(r) < N ? fma(hg, Z(1, r), Z(0, r)) : 0.0;
-    } else if (phase == START || phase == RESETD) {
-#pragma unroll
-      for (int r = 0; r < R; ++r) y[r] = idx(r) < N ? Z(0, r) : 0.0;
     }
 
     // ------------------------------------------------ (C) one FP64 RHS per active cell
@@ -653,68 +636,58 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
     }
 
     // ------------------------------------------------ (D) consume it
-    if (phase == START) {
-      // initial step size: difference-quotient estimate of y'' (bounded)
+    // The step's vector work that more than one outcome needs (undoing the prediction, changing
+    // the order, rescaling the history) is only noted here and done once, below, for every
+    // cell that needs it: one copy of its code, and one pass of its FP64 instructions instead of
+    // one per outcome (this kernel is bound by instruction fetch as much as by the FP64 pipe).
+    bool undo = false, check_h = false, first_step = false;
+    int dq = 0;
+    double scale = 1.0;
+    if (phase == START || phase == RESETD) {
+      const double fac = phase == START ? 1.0 : h;
 #pragma unroll
       for (int r = 0; r < R; ++r)
-        if (idx(r) < N) Z(1, r) = f[r];  // f0 parked in z[1] until h is known
-      set_ewt();
+        if (idx(r) < N) Z(1, r) = fac * f[r];  // START: f0 parked until h is known
+    }
+    if (phase == START) {
+      // initial step size: difference-quotient estimate of y'' (bounded)
       const double tround = UROUND * tout;
       hlb = 100.0 * tround;
       double hub_inv = 0.0;
 #pragma unroll
       for (int r = 0; r < R; ++r)
-        if (idx(r) < N) hub_inv = fmax(hub_inv, fabs(f[r]) / fma(0.1, fabs(Z(0, r)), P.atol[idx(r)]));
+        if (idx(r) < N) hub_inv = fmax(hub_inv, pgb_div64(fabs(f[r]), fma(0.1, fabs(Z(0, r)), P.atol[idx(r)])));
       hub_inv = group_max<G>(hub_inv, gm);
       hub = 0.1 * tout;
-      if (hub * hub_inv > 1.0) hub = 1.0 / hub_inv;
+      if (hub * hub_inv > 1.0) hub = pgb_div64(1.0, hub_inv);
       hg = sqrt(hlb * hub);
       if (hub > hlb) {
         hin_count = 1;
         phase = HIN;
       } else {
         h = fmin(fmax(0.5 * hg, hlb), hub);
-        hscale = h;
-#pragma unroll
-        for (int r = 0; r < R; ++r)
-          if (idx(r) < N) Z(1, r) *= h;
-        q = 1; qwait = 2; etamax = ETAMX1;
-        __syncwarp(gm);
-        if (sub == 0) C.TAU[1] = h;
-        new_step = true;
-        phase = STEP;
+        first_step = true;
       }
     } else if (phase == HIN) {
       double d[R];
 #pragma unroll
-      for (int r = 0; r < R; ++r) d[r] = idx(r) < N ? (f[r] - Z(1, r)) / hg : 0.0;
+      for (int r = 0; r < R; ++r) d[r] = idx(r) < N ? pgb_div64(f[r] - Z(1, r), hg) : 0.0;
       const double ydd = sqrt(wms(d));
-      double hnew = (ydd * hub * hub > 2.0) ? sqrt(2.0 / ydd) : sqrt(hg * hub);
+      double hnew = sqrt((ydd * hub * hub > 2.0) ? pgb_div64(2.0, ydd) : hg * hub);
       bool done = false;
       if (hin_count == 4) {
         done = true;
       } else {
-        const double hrat = hnew / hg;
+        const double hrat = pgb_div64(hnew, hg);
         if (hrat > 0.5 && hrat < 2.0) done = true;
         else if (hin_count >= 2 && hrat > 2.0) { hnew = hg; done = true; }
         else { hg = hnew; ++hin_count; }
       }
       if (done) {
         h = fmin(fmax(0.5 * hnew, hlb), hub);
-        hscale = h;
-#pragma unroll
-        for (int r = 0; r < R; ++r)
-          if (idx(r) < N) Z(1, r) *= h;
-        q = 1; qwait = 2; etamax = ETAMX1;
-        __syncwarp(gm);
-        if (sub == 0) C.TAU[1] = h;
-        new_step = true;
-        phase = STEP;
+        first_step = true;
       }
     } else if (phase == RESETD) {
-#pragma unroll
-      for (int r = 0; r < R; ++r)
-        if (idx(r) < N) Z(1, r) = h * f[r];
       phase = STEP;
     } else if (phase == NEWTON) {
       bool singular = false;
@@ -723,7 +696,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
         need_setup = false;
         jcur = true;
       }
-      int outcome = 0;  // 0 continue, 1 converged, 2 convergence failure, 3 singular matrix
+      int outcome = 0;  // 0 continue, 1 converged, 2 convergence failure
       if (singular) {
         outcome = 3;
       } else {
@@ -732,7 +705,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
         for (int r = 0; r < R; ++r) b[r] = idx(r) < N ? fma(gamma, f[r], -fma(rl1, Z(1, r), acor[r])) : 0.0;
         solve(b);
         if (gamrat != 1.0) {
-          const double s = 2.0 / (1.0 + gamrat);
+          const double s = pgb_div64(2.0, 1.0 + gamrat);
 #pragma unroll
           for (int r = 0; r < R; ++r) b[r] *= s;
         }
@@ -740,7 +713,8 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
 #pragma unroll
         for (int r = 0; r < R; ++r)
           if (idx(r) < N) { acor[r] += b[r]; y[r] = Z(0, r) + acor[r]; }
-        if (m > 0) crate2 = fmax((CRDOWN * CRDOWN) * crate2, del2 / delp2);
+        if (m > 0) crate2 = fmax((CRDOWN * CRDOWN) * crate2, pgb_div64(del2, delp2));
+        // convergence: del * min(1, crate) / tq4 <= 1, in squares
         const double dcon2 = del2 * fmin(1.0, crate2) * inv_tq4_sq;
         if (dcon2 <= 1.0) {
           outcome = 1;
@@ -754,57 +728,55 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
         // stale Jacobian: refresh it and restart the iteration from the prediction
         need_setup = true;
         m = 0;
-#pragma unroll
-        for (int r = 0; r < R; ++r) { y[r] = idx(r) < N ? Z(0, r) : 0.0; acor[r] = 0.0; }
+        fresh = true;
       } else if (outcome >= 2) {
-        retract();
+        undo = true;
+        t -= h;
         ++ncf; ++ncfn;
         if (outcome == 3 || ncf >= MXNCF || fabs(h) <= 100.0 * UROUND * fabs(t)) {
           fail_cell(CONV);
         } else {
           force_setup = true;
           etamax = 1.0;
-          rescale(ETACF);
+          scale = ETACF;
           phase = STEP;
         }
       } else if (outcome == 1) {
         const double acnrm2 = (m == 0) ? del2 : wms(acor);
         const double dsm2 = acnrm2 * (tq2 * tq2);  // squared local error estimate
+        const double etaq = pgb_div64(1.0, pgb_pow64((BIAS2 * BIAS2) * dsm2, 0.5 * inv_int(q + 1)) + ADDON);
         if (!(dsm2 <= 1.0)) {
           // ---- local error test failed ----
-          retract();
+          undo = true;
+          t -= h;
           ++nef; ++netf;
           if (nef >= MXNEF || !isfinite(dsm2)) {
             fail_cell(isfinite(dsm2) ? ERRTEST : NONFINITE);
           } else {
+            check_h = true;
             etamax = 1.0;
+            phase = STEP;
+            scale = ETAMIN;
             if (nef <= MXNEF1) {
-              double e = 1.0 / (pgb_pow64((BIAS2 * BIAS2) * dsm2, 0.5 * inv_int(q + 1)) + ADDON);
-              e = fmax(ETAMIN, e);
-              if (nef >= SMALL_NEF) e = fmin(e, ETAMXF);
-              rescale(e);
-              phase = STEP;
+              scale = fmax(ETAMIN, etaq);
+              if (nef >= SMALL_NEF) scale = fmin(scale, ETAMXF);
             } else if (q > 1) {
-              adjust_order(-1);
-              --q;
-              qwait = q + 1;
-              rescale(ETAMIN);
-              phase = STEP;
+              dq = -1;
             } else {
-              rescale(ETAMIN);
               qwait = 10;
               phase = RESETD;
             }
-            if (phase != FINISH && fabs(h) <= 100.0 * UROUND * fabs(t)) fail_cell(HSMALL);
           }
         } else {
           // ---- step accepted: complete it ----
           ++nst;
           __syncwarp(gm);
           if (sub == 0) {
+#pragma unroll 1
             for (int i = q + 1; i >= 2; --i) C.TAU[i] = C.TAU[i - 1];
             C.TAU[1] = h;
           }
+#pragma unroll 1
           for (int j = 0; j <= q; ++j) {
             const double lj = C.LC[j];
 #pragma unroll
@@ -813,17 +785,15 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
           }
           __syncwarp(gm);
           --qwait;
+          bool save = false;
           if (qwait == 1 && q != qmax) {
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-              if (idx(r) < N) Z(QMAX + 1, r) = acor[r];
+            save = true;
             tq5_saved = tq5;
           }
           if (fabs(t - tout) <= 100.0 * UROUND * (fabs(t) + fabs(h)) || t >= tout) {
             phase = FINISH;
           } else {
             // ---- next step size and order ----
-            const double etaq = 1.0 / (pgb_pow64((BIAS2 * BIAS2) * dsm2, 0.5 * inv_int(q + 1)) + ADDON);
             int qprime = q;
             if (etamax == 1.0) {
               qwait = max(qwait, 2);
@@ -838,18 +808,19 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
 #pragma unroll
                   for (int r = 0; r < R; ++r) zq[r] = idx(r) < N ? Z(q, r) : 0.0;
                   const double ddn2 = wms(zq) * (tq1 * tq1);
-                  etaqm1 = 1.0 / (pgb_pow64((BIAS1 * BIAS1) * ddn2, 0.5 * inv_int(q)) + ADDON);
+                  etaqm1 = pgb_div64(1.0, pgb_pow64((BIAS1 * BIAS1) * ddn2, 0.5 * inv_int(q)) + ADDON);
                 }
                 if (q != qmax) {
-                  const double hr = h / tau(2);
+                  const double hr = pgb_div64(h, tau(2));
                   double hrp = hr;
+#pragma unroll 1
                   for (int k = 0; k < q; ++k) hrp *= hr;  // (h / tau2)^(q+1)
-                  const double cquot = (tq5 / tq5_saved) * hrp;
+                  const double cquot = pgb_div64(tq5, tq5_saved) * hrp;
                   double tv[R];
 #pragma unroll
                   for (int r = 0; r < R; ++r) tv[r] = idx(r) < N ? acor[r] - cquot * Z(QMAX + 1, r) : 0.0;
                   const double dup2 = wms(tv) * (tq3 * tq3);
-                  etaqp1 = 1.0 / (pgb_pow64((BIAS3 * BIAS3) * dup2, 0.5 * inv_int(q + 2)) + ADDON);
+                  etaqp1 = pgb_div64(1.0, pgb_pow64((BIAS3 * BIAS3) * dup2, 0.5 * inv_int(q + 2)) + ADDON);
                 }
                 const double etam = fmax(etaqm1, fmax(etaq, etaqp1));
                 if (etam < THRESH) {
@@ -862,9 +833,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
                 } else {
                   eta = etaqp1;
                   qprime = q + 1;
-#pragma unroll
-                  for (int r = 0; r < R; ++r)
-                    if (idx(r) < N) Z(QMAX + 1, r) = acor[r];
+                  save = true;
                 }
               } else if (eta < THRESH) {
                 eta = 1.0;
@@ -873,18 +842,46 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
               else eta = 1.0;
             }
             etamax = (nst <= SMALL_NST) ? ETAMX2 : ETAMX3;
-            if (qprime != q) {
-              adjust_order(qprime - q);
-              q = qprime;
-              qwait = q + 1;
-            }
-            if (eta != 1.0) rescale(eta);
+            dq = qprime - q;
+            scale = eta;
             new_step = true;
             phase = STEP;
+          }
+          if (save) {
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+              if (idx(r) < N) Z(QMAX + 1, r) = acor[r];
           }
         }
       }
     }
+    if (undo) retract();
+    if (dq != 0) {
+      adjust_order(dq);
+      q += dq;
+      qwait = q + 1;
+    }
+    if (first_step) {
+      hscale = h;
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (idx(r) < N) Z(1, r) *= h;
+      q = 1; qwait = 2; etamax = ETAMX1; new_step = true;
+      __syncwarp(gm);
+      if (sub == 0) C.TAU[1] = h;
+      phase = STEP;
+    }
+    // the new step size, then a cut to end at tout
+#pragma unroll 1
+    for (int pass = 0; pass < 2; ++pass) {
+      if (pass == 1) {
+        scale = 1.0;
+        if (phase == STEP && new_step && (t + h - tout) * h > 0.0)
+          scale = pgb_div64((tout - t) * (1.0 - 4.0 * UROUND), h);
+      }
+      if (scale != 1.0) rescale(scale);
+    }
+    if (check_h && fabs(h) <= 100.0 * UROUND * fabs(t)) fail_cell(HSMALL);
     // ------------------------------------------------ (F) write back a finished cell
     if (phase == FINISH) finish_cell();
     __syncwarp();

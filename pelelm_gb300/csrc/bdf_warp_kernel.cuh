@@ -37,6 +37,12 @@ namespace pgb {
 
 namespace wbdf {
 constexpr int RXW = 8;  // Jacobian scratch per reaction: dq/dT, 3 reactant partials, 3 product partials, [M] partial
+// Partials of the whole mechanism: RXW per reaction, then the [M] partials times each listed
+// collider's efficiency.
+template <class M>
+__host__ __device__ constexpr int rx_len() {
+  return RXW * M::NR + M::TabG::JAC_X;
+}
 }
 
 // Shared memory of one warp (one cell) for mechanism M and Jacobian type JR: the FP64 state
@@ -50,7 +56,7 @@ __host__ __device__ constexpr int bdf_warp_state_bytes() {
 template <class M, class JR>
 __host__ __device__ constexpr int bdf_warp_scratch_bytes() {
   constexpr int NS = M::NS, NR = M::NR;
-  constexpr int rhs = (2 * NS + NR) * 8, setup = (wbdf::RXW * NR + 4 * NS) * (int)sizeof(JR);
+  constexpr int rhs = (2 * NS + NR) * 8, setup = (wbdf::rx_len<M>() + 4 * NS) * (int)sizeof(JR);
   return ((rhs > setup ? rhs : setup) + 15) / 16 * 16;
 }
 template <class M, class JR>
@@ -218,6 +224,226 @@ __device__ __noinline__ WVec<M> warp_rhs(const WVec<M> yv, double* CS, double* G
   return fv;
 }
 
+// Sign flip by the top bit of `top`, and a test for zero, on the integer pipe (an FP64 compare
+// takes an FP64 slot).
+__device__ __forceinline__ float flip_sign(float x, unsigned top) {
+  return __uint_as_float(__float_as_uint(x) ^ (top & 0x80000000u));
+}
+__device__ __forceinline__ double flip_sign(double x, unsigned top) {
+  return __hiloint2double(__double2hiint(x) ^ (int)(top & 0x80000000u), __double2loint(x));
+}
+__device__ __forceinline__ bool not_zero(float x) { return (__float_as_uint(x) << 1) != 0u; }
+__device__ __forceinline__ bool not_zero(double x) {
+  return (((unsigned)__double2hiint(x) << 1) | (unsigned)__double2loint(x)) != 0u;
+}
+
+// Largest |a| over the warp's candidates (`ok`), NaN never: true in the slots that hold it; false
+// everywhere if no candidate is above 0. A non-negative float orders as its bit pattern, so the
+// search is warp max-reductions of integers (FP64: high words, then low words).
+template <int R>
+__device__ __forceinline__ bool warp_abs_max(const float (&a)[R], const bool (&ok)[R], bool (&is_max)[R]) {
+  unsigned bits[R], m = 0u;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const float v = fabsf(a[r]);
+    bits[r] = ok[r] && v == v ? __float_as_uint(v) : 0u;
+    m = max(m, bits[r]);
+  }
+  m = __reduce_max_sync(0xffffffffu, m);
+#pragma unroll
+  for (int r = 0; r < R; ++r) is_max[r] = m != 0u && bits[r] == m;
+  return m != 0u;
+}
+template <int R>
+__device__ __forceinline__ bool warp_abs_max(const double (&a)[R], const bool (&ok)[R], bool (&is_max)[R]) {
+  unsigned hi[R], lo[R], mh = 0u, ml = 0u;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    hi[r] = (unsigned)__double2hiint(a[r]) & 0x7fffffffu;
+    lo[r] = (unsigned)__double2loint(a[r]);
+    if (!ok[r] || hi[r] > 0x7ff00000u || (hi[r] == 0x7ff00000u && lo[r])) hi[r] = lo[r] = 0u;
+    mh = max(mh, hi[r]);
+  }
+  mh = __reduce_max_sync(0xffffffffu, mh);
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (hi[r] == mh) ml = max(ml, lo[r]);
+  ml = __reduce_max_sync(0xffffffffu, ml);
+#pragma unroll
+  for (int r = 0; r < R; ++r) is_max[r] = (mh | ml) != 0u && hi[r] == mh && lo[r] == ml;
+  return (mh | ml) != 0u;
+}
+
+// Partial-pivot LU of I - g J, J in shared memory rows of N + 1, one warp: L below the diagonal,
+// U above, reciprocal pivots on it, rows in pivot order, PIV[i] the row of J that row i came from.
+// False: singular. Each lane keeps its rows (lane + 32 r) in registers and the step loop rotates
+// them left by one, so the pivot column is always element 0 and one rolled loop body serves every
+// step; after N steps the rows are back in place. Rows are not moved between lanes: `pos` is a
+// row's place in the pivot order. The pivot row reaches the lanes by shuffles; the columns already
+// eliminated are skipped four at a time. The shared-memory form it replaces paid about a thousand
+// cycles a step in dependent loads and stores (21 species: 22k cycles a matrix).
+template <int N, class JR>
+__device__ __forceinline__ bool warp_lu_factor_regs(JR* A, int* PIV, const JR g) {
+  constexpr int R = (N + 31) / 32, LDA = N + 1;
+  const int lane = threadIdx.x & 31;
+  JR a[R][N];
+  int pos[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int i = lane + 32 * r;
+    pos[r] = i < N ? i : 2 * N;
+#pragma unroll
+    for (int j = 0; j < N; ++j) a[r][j] = i < N ? fma(-g, A[i * LDA + j], i == j ? JR(1) : JR(0)) : JR(0);
+  }
+#pragma unroll 1
+  for (int k = 0; k < N; ++k) {
+    // pivot: first row of largest |a_ik|, i >= k
+    JR head[R];
+    bool ok[R], is_max[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      head[r] = a[r][0];
+      ok[r] = pos[r] >= k && pos[r] < N;
+    }
+    if (!warp_abs_max(head, ok, is_max)) return false;
+    int p = 2 * N;
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (is_max[r]) p = min(p, pos[r]);
+    p = __reduce_min_sync(0xffffffffu, p);
+    int src = 0, slot = 0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const unsigned b = __ballot_sync(0xffffffffu, pos[r] == p);
+      if (b) { src = __ffs(b) - 1; slot = r; }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (pos[r] == p) pos[r] = k;
+      else if (pos[r] == k) pos[r] = p;
+    }
+    auto pivot_row = [&](int j) -> JR {
+      JR v = a[0][j];
+#pragma unroll
+      for (int r = 1; r < R; ++r)
+        if (slot == r) v = a[r][j];
+      return __shfl_sync(0xffffffffu, v, src);
+    };
+    const JR inv = JR(1) / pivot_row(0);
+    JR l[R];
+    bool below[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      below[r] = pos[r] > k && pos[r] < N;
+      l[r] = head[r] * inv;
+      head[r] = below[r] ? l[r] : pos[r] == k ? inv : head[r];
+    }
+    const int live = N - k;  // columns k..N-1 are elements 0..live-1
+#pragma unroll
+    for (int j0 = 1; j0 < N; j0 += 4) {
+      if (j0 < live) {
+#pragma unroll
+        for (int j = j0; j < j0 + 4 && j < N; ++j) {
+          const JR u = pivot_row(j);
+#pragma unroll
+          for (int r = 0; r < R; ++r) a[r][j - 1] = below[r] && j < live ? fma(-l[r], u, a[r][j]) : a[r][j];
+        }
+      } else {
+#pragma unroll
+        for (int j = j0; j < j0 + 4 && j < N; ++j)
+#pragma unroll
+          for (int r = 0; r < R; ++r) a[r][j - 1] = a[r][j];
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) a[r][N - 1] = head[r];
+  }
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (pos[r] < N) {
+      PIV[pos[r]] = lane + 32 * r;
+#pragma unroll
+      for (int j = 0; j < N; ++j) A[pos[r] * LDA + j] = a[r][j];
+    }
+  __syncwarp();
+  return true;
+}
+
+// The same factors for matrices whose rows do not fit registers (FP64, 53 species: 216 a lane): in
+// shared memory, the trailing block's elements dealt to the lanes one by one, so that no lane idles
+// on a row above the pivot (FP64 multiply-adds bound this: 1,670 warp instructions against 2,610
+// with a row per lane).
+template <int N, class JR>
+__device__ __forceinline__ bool warp_lu_factor_shared(JR* A, int* PIV, const JR g) {
+  constexpr int R = (N + 31) / 32, LDA = N + 1;
+  const int lane = threadIdx.x & 31;
+  for (int e = lane; e < N * LDA; e += 32) {
+    const int i = e / LDA, j = e - i * LDA;
+    if (j < N) A[e] = fma(-g, A[e], i == j ? JR(1) : JR(0));
+  }
+  for (int i = lane; i < N; i += 32) PIV[i] = i;
+  __syncwarp();
+#pragma unroll 1
+  for (int k = 0; k < N; ++k) {
+    JR col[R];
+    bool ok[R], is_max[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int i = lane + 32 * r;
+      ok[r] = i >= k && i < N;
+      col[r] = ok[r] ? A[i * LDA + k] : JR(0);
+    }
+    if (!warp_abs_max(col, ok, is_max)) return false;
+    int p = 2 * N;
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (is_max[r]) p = min(p, lane + 32 * r);
+    p = __reduce_min_sync(0xffffffffu, p);
+    __syncwarp();
+    if (p != k) {
+      for (int j = lane; j < N; j += 32) {
+        const JR tmp = A[k * LDA + j];
+        A[k * LDA + j] = A[p * LDA + j];
+        A[p * LDA + j] = tmp;
+      }
+      if (lane == 0) {
+        const int tmp = PIV[k];
+        PIV[k] = PIV[p];
+        PIV[p] = tmp;
+      }
+      __syncwarp();
+    }
+    const JR inv = JR(1) / A[k * LDA + k];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int i = lane + 32 * r;
+      if (i > k && i < N) A[i * LDA + k] *= inv;
+    }
+    __syncwarp();
+    const int m = N - 1 - k;
+    if (m > 0) {
+      int i = k + 1 + lane / m, j = k + 1 + lane % m;
+#pragma unroll 4
+      for (int e = lane; e < m * m; e += 32) {
+        A[i * LDA + j] = fma(-A[i * LDA + k], A[k * LDA + j], A[i * LDA + j]);
+        j += 32;
+        while (j >= N) { j -= m; ++i; }
+      }
+    }
+    if (lane == 0) A[k * LDA + k] = inv;
+    __syncwarp();
+  }
+  return true;
+}
+
+template <int N, class JR>
+__device__ __forceinline__ bool warp_lu_factor(JR* A, int* PIV, const JR g) {
+  // up to 128 registers of rows a lane: FP32 to N = 64, FP64 to N = 64 / 2 rows
+  if constexpr ((N + 31) / 32 * N * (int)sizeof(JR) <= 512) return warp_lu_factor_regs<N>(A, PIV, g);
+  else return warp_lu_factor_shared<N>(A, PIV, g);
+}
+
 // Jacobian (equations of jac_table, mech_tables.cuh) and partial-pivot LU of I - gamma J in
 // shared memory, one warp cooperating. False: singular. With FACTOR false it stops after the
 // Jacobian, which A then holds (the diagnostic entry point). Inlined: each kernel calls it from
@@ -343,6 +569,13 @@ __device__ __forceinline__ bool warp_setup(const WVec<M> yv, const double gamma,
       if (r.kind == 1) bm = kf * Pf - kr * Pp;
       else if (r.kind == 2) bm = dkeff_dM * (Pf - (kf > JR(0) ? kr / kf : JR(0)) * Pp);
       out[7] = bm;
+      if (r.tb >= 0) {  // the collider terms of the listed species read these
+        const TabThirdBody<JR>& t = Tab::template tb<JR>(r.tb);
+        JR* ox = RX + Tab::jac_x0(r.tb);
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          if (e < t.n) ox[e] = bm * (JR(1) + t.effm1[e]);
+      }
 #pragma unroll
       for (int row = 0; row < 6; ++row)
         if (row < r.nr + r.np) {
@@ -362,38 +595,40 @@ __device__ __forceinline__ bool warp_setup(const WVec<M> yv, const double gamma,
     // (dq/dT in the T column). The lanes' 4-byte term codes are interleaved in the table (one
     // contiguous line per warp load); each entry has one writer, so the result does not depend
     // on the lane schedule.
+    // A lane reads four terms per 16-byte load, one load ahead, and an entry's coefficient and
+    // target one entry ahead: with shared memory taking almost all of the L1, each of these loads
+    // is an L2 round trip, and a load per term made the program the setup's longest part.
     {
-      JR acc = JR(0), w = JR(0);
+      JR acc = JR(0);
+      int ent = lane;
+      TabJacEnt<JR> cur = Tab::template jac_ent<JR>(ent), ahead = Tab::template jac_ent<JR>(ent + 32);
+      uint4 quad = Tab::jac_quad(lane);
 #pragma unroll 1
-      for (int t = 0; t < Tab::JAC_TERMS; ++t) {
-        const int c = 32 * t + lane;
-        const unsigned code = Tab::jac_code(c);
-        const bool neg = (Tab::jac_neg(t) >> lane) & 1u;
-        if (code & (1u << 30)) {  // first term of an entry: its coefficient magnitude
-          const int tg = (code >> 9) & 0xfff;
-          const int i = tg / LDA, k = tg - i * LDA;
-          const JR wi = Tab::template sp<JR>(i).W;
-          w = (k == NS) ? wi : wi * Tab::template sp<JR>(k).invW;
-        }
-        const JR* pj = RX + (code & 0x1ff) * wbdf::RXW;
-        const bool tcol = (code & (1u << 21)) != 0;
-        JR v;
-        if (tcol) {
-          v = pj[0];
-        } else {
-          v = JR(0);
+      for (int q = 0; q < Tab::JAC_QUADS; ++q) {
+        const unsigned code[4] = {quad.x, quad.y, quad.z, quad.w};
+        if (q + 1 < Tab::JAC_QUADS) quad = Tab::jac_quad(32 * (q + 1) + lane);
+        JR v[4];
 #pragma unroll
-          for (int q = 0; q < 3; ++q)
-            if (code & (1u << (22 + q))) v += pj[1 + q];
+        for (int u = 0; u < 4; ++u) v[u] = RX[code[u] & 0x1fff];
 #pragma unroll
-          for (int q = 0; q < 3; ++q)
-            if (code & (1u << (25 + q))) v += pj[4 + q];
-          if (code & (1u << 28)) v += pj[7] * ((code & (1u << 31)) ? Tab::template jac_eff<JR>(c) : JR(1));
-        }
-        if (tcol || v != JR(0)) acc += (neg ? -w : w) * v;
-        if (code & (1u << 29)) {  // last term of the entry
-          A[(code >> 9) & 0xfff] = acc;
-          acc = JR(0);
+        for (int u = 0; u < 4; ++u) {
+          const unsigned c = code[u];
+          if (c & 0xfe000) {  // species on several slots of the reaction
+            const JR* pj = RX + (c & 0x1ff8);
+#pragma unroll
+            for (int s = 1; s < 7; ++s)
+              if (c & (1u << (12 + s))) v[u] += pj[s];
+            if (c & (1u << 19))
+              v[u] = fma(pj[7], (c & (1u << 22)) ? Tab::template jac_eff<JR>(32 * (4 * q + u) + lane) : JR(1), v[u]);
+          }
+          if (not_zero(v[u]) || (c & (1u << 23))) acc = fma(flip_sign(cur.w, c << 11), v[u], acc);
+          if (c & (1u << 21)) {  // last term of the entry
+            A[cur.target] = acc;
+            acc = JR(0);
+            cur = ahead;
+            ent += 32;
+            ahead = Tab::template jac_ent<JR>(min(ent + 32, 32 * (Tab::JAC_ENTS - 1) + lane));
+          }
         }
       }
     }
@@ -437,130 +672,64 @@ __device__ __forceinline__ bool warp_setup(const WVec<M> yv, const double gamma,
     __syncwarp();
   };
 
-  // ---- M = I - gamma J, partial-pivot LU in place (trailing swaps), reciprocal pivots ----
-  auto factor = [&](double gamma) -> bool {
-    const JR g = (JR)gamma;
-    for (int e = lane; e < N * LDA; e += 32) {
-      const int i = e / LDA, k = e - i * LDA;
-      if (k < N) A[e] = (i == k ? JR(1) : JR(0)) - g * A[e];
-    }
-    __syncwarp();
-#pragma unroll 1
-    for (int k = 0; k < N; ++k) {
-      // pivot: first row of largest |a_ik|, i >= k (NaN never wins; none above 0: singular)
-      int p = N;
-      if constexpr (sizeof(JR) == sizeof(float)) {
-        // a non-negative float orders as its bit pattern: one warp max-reduction, then the
-        // lowest row holding the maximum from the lane ballots (rows lane + 32 r, r ascending)
-        unsigned bits[R], m = 0u;
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const int i = idx(r);
-          unsigned b = 0u;
-          if (i >= k && i < N) {
-            const float v = fabsf(A[i * LDA + k]);
-            if (v == v) b = __float_as_uint(v);
-          }
-          bits[r] = b;
-          m = max(m, b);
-        }
-        m = __reduce_max_sync(0xffffffffu, m);
-        if (m == 0u) return false;
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const unsigned bal = __ballot_sync(0xffffffffu, bits[r] == m);
-          if (p == N && bal) p = 32 * r + __ffs(bal) - 1;
-        }
-      } else {
-        JR best = JR(-1);
-        int bi = N;
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const int i = idx(r);
-          if (i >= k && i < N) {
-            const JR v = fabs(A[i * LDA + k]);
-            if (v > best) { best = v; bi = i; }
-          }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          const JR ob = __shfl_xor_sync(0xffffffffu, best, o);
-          const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-          if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-        }
-        if (!(best > JR(0))) return false;
-        p = bi;
-      }
-      if (lane == 0) PIV[k] = p;
-      if (p != k)
-        for (int j = k + lane; j < N; j += 32) {
-          const JR tmp = A[k * LDA + j];
-          A[k * LDA + j] = A[p * LDA + j];
-          A[p * LDA + j] = tmp;
-        }
-      __syncwarp();
-      const JR inv = JR(1) / A[k * LDA + k];
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const int i = idx(r);
-        if (i > k && i < N) {
-          const JR l = A[i * LDA + k] * inv;
-          A[i * LDA + k] = l;
-#pragma unroll 4
-          for (int j = k + 1; j < N; ++j) A[i * LDA + j] -= l * A[k * LDA + j];
-        }
-      }
-      __syncwarp();
-      if (lane == 0) A[k * LDA + k] = inv;
-      __syncwarp();
-    }
-    return true;
-  };
   jacobian(yv.v);
-  if constexpr (FACTOR) return factor(gamma);
+  if constexpr (FACTOR) return warp_lu_factor<N>(A, PIV, (JR)gamma);
   else return true;
 }
 
-// (I - gamma J) x = b with the factors warp_setup left in A / PIV (trailing row swaps,
-// reciprocal pivots on the diagonal): one warp, rows over lanes, b distributed like the state
-// (element i in lane i mod 32) and overwritten with x; XS is the N-element staging vector.
+// Substitution steps of (I - gamma J) x = b, L lanes per cell with row i in lane i % L, slot i / L,
+// of the cell's lanes (mask, first lane gbase): the solution moves by shuffles, so a step costs one
+// shuffle and one multiply-add and the matrix loads run ahead of it (the staged shared-memory form
+// waited for a store, a barrier and a load at each step: 200 cycles instead of 40).
+template <int N, int L, class JR>
+__device__ __forceinline__ void lu_substitute(const JR* A, unsigned mask, int gbase, JR (&x)[(N + L - 1) / L]) {
+  constexpr int R = (N + L - 1) / L, LDA = N + 1;
+  const int sub = (threadIdx.x & 31) - gbase;
+#pragma unroll
+  for (int s = 0; s < R; ++s)
+#pragma unroll 2
+    for (int q = 0; q < (s + 1 < R ? L : N - s * L); ++q) {
+      const int k = s * L + q;
+      const JR bk = __shfl_sync(mask, x[s], gbase + q);
+#pragma unroll
+      for (int r = s; r < R; ++r) {
+        const int i = sub + L * r;
+        if (i > k && i < N) x[r] = fma(-A[i * LDA + k], bk, x[r]);
+      }
+    }
+#pragma unroll
+  for (int s = R - 1; s >= 0; --s)
+#pragma unroll 2
+    for (int q = (s + 1 < R ? L : N - s * L) - 1; q >= 0; --q) {
+      const int k = s * L + q;
+      const JR xk = __shfl_sync(mask, x[s], gbase + q) * A[k * LDA + k];
+#pragma unroll
+      for (int r = 0; r <= s; ++r) {
+        const int i = sub + L * r;
+        if (i == k) x[r] = xk;
+        else if (i < k) x[r] = fma(-A[i * LDA + k], xk, x[r]);
+      }
+    }
+}
+
+// (I - gamma J) x = b with the factors warp_setup left in A / PIV: one warp, rows over lanes, b
+// distributed like the state (element i in lane i mod 32) and overwritten with x; XS is the
+// N-element staging vector.
 template <class M, class JR>
 __device__ __forceinline__ void warp_lu_solve(const JR* A, const int* PIV, JR* XS, double (&b)[(M::N + 31) / 32]) {
-  constexpr int N = M::N, R = (N + 31) / 32, LDA = N + 1;
+  constexpr int N = M::N, R = (N + 31) / 32;
   const int lane = threadIdx.x & 31;
-  auto idx = [&](int r) { return lane + 32 * r; };
+  JR x[R];
 #pragma unroll
   for (int r = 0; r < R; ++r)
-    if (idx(r) < N) XS[idx(r)] = (JR)b[r];
+    if (lane + 32 * r < N) XS[lane + 32 * r] = (JR)b[r];
   __syncwarp();
-#pragma unroll 1
-  for (int k = 0; k < N; ++k) {
-    const int p = PIV[k];
-    if (p != k && lane == 0) { const JR tmp = XS[k]; XS[k] = XS[p]; XS[p] = tmp; }
-    __syncwarp();
-    const JR bk = XS[k];
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int i = idx(r);
-      if (i > k && i < N) XS[i] -= A[i * LDA + k] * bk;
-    }
-    __syncwarp();
-  }
-#pragma unroll 1
-  for (int k = N - 1; k >= 0; --k) {
-    const JR xk = XS[k] * A[k * LDA + k];
-    __syncwarp();
-    if (lane == 0) XS[k] = xk;
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int i = idx(r);
-      if (i < k) XS[i] -= A[i * LDA + k] * xk;
-    }
-    __syncwarp();
-  }
+  for (int r = 0; r < R; ++r) x[r] = lane + 32 * r < N ? XS[PIV[lane + 32 * r]] : JR(0);
+  lu_substitute<N, 32>(A, 0xffffffffu, 0, x);
 #pragma unroll
   for (int r = 0; r < R; ++r)
-    if (idx(r) < N) b[r] = (double)XS[idx(r)];
+    if (lane + 32 * r < N) b[r] = (double)x[r];
   __syncwarp();
 }
 
@@ -568,7 +737,7 @@ template <class M, class JR, int WPB>
 __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams P) {
   using namespace bdf;
   using Tab = typename M::TabG;
-  constexpr int N = M::N, NS = M::NS, NR = M::NR;
+  constexpr int N = M::N, NS = M::NS;
   constexpr int R = (N + 31) / 32;   // vector elements per lane
   constexpr int LDA = N + 1;         // padded matrix row
   constexpr bool MIXED = sizeof(JR) == sizeof(float);
@@ -583,8 +752,8 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
   double* CS = reinterpret_cast<double*>(scratch);  // [NS] concentrations
   double* GS = CS + NS;                          // [NS] g/RT
   double* QS = GS + NS;                          // [NR] rates of progress
-  JR* RX = reinterpret_cast<JR*>(scratch);       // [NR][RXW] Jacobian partials
-  JR* TH = RX + wbdf::RXW * NR;                  // [4][NS] NASA-7 terms of the setup
+  JR* RX = reinterpret_cast<JR*>(scratch);       // Jacobian partials
+  JR* TH = RX + wbdf::rx_len<M>();               // [4][NS] NASA-7 terms of the setup
   JR* A = reinterpret_cast<JR*>(scratch + bdf_warp_scratch_bytes<M, JR>());  // [N][LDA] Jacobian, then its LU
   JR* XS = A + N * LDA;                          // [N] solve vector
   int* PIV = reinterpret_cast<int*>(XS + N);
@@ -680,6 +849,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
 
     auto rescale = [&](double e) {
       double fac = e;
+#pragma unroll 1
       for (int j = 1; j <= q; ++j) {
 #pragma unroll
         for (int r = 0; r < R; ++r)
@@ -691,7 +861,9 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
     };
     auto predict = [&]() {
       t += h;
+#pragma unroll 1
       for (int k = 1; k <= q; ++k)
+#pragma unroll 1
         for (int j = q; j >= k; --j)
 #pragma unroll
           for (int r = 0; r < R; ++r)
@@ -699,7 +871,9 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
     };
     auto retract = [&]() {
       t -= h;
+#pragma unroll 1
       for (int k = 1; k <= q; ++k)
+#pragma unroll 1
         for (int j = q; j >= k; --j)
 #pragma unroll
           for (int r = 0; r < R; ++r)
@@ -713,8 +887,10 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
       for (int i = 0; i <= QMAX; ++i) l[i] = 0.0;
       l[0] = 1.0;
       double alpha0 = 0.0;
+#pragma unroll 1
       for (int j = 1; j <= q; ++j) alpha0 -= inv_int(j);
       double hsum = h, sum_xi_inv = 0.0;
+#pragma unroll 1
       for (int i = 1; i <= q - 1; ++i) {
         if (i > 1) hsum += TAU[i - 1];
         const double xi_inv = h / hsum;
@@ -769,6 +945,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
       w[2] = 1.0;
       if (dq > 0) {
         double alpha0 = 0.0, alpha1 = 0.0, prod = 1.0, hsum = 0.0;
+#pragma unroll 1
         for (int j = 1; j <= q; ++j) {
           hsum += TAU[j];
           const double xi = hsum / hscale;
@@ -792,6 +969,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
               if (idx(r) < N) zget(j, r) = fma(w[j], zget(q + 1, r), zget(j, r));
       } else {
         double hsum = 0.0;
+#pragma unroll 1
         for (int j = 1; j <= q - 2; ++j) {
           hsum += TAU[j];
           const double xi = hsum / hscale;
@@ -886,6 +1064,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
       if (hub * hub_inv > 1.0) hub = 1.0 / hub_inv;
       double hg = sqrt(hlb * hub), hnew = hg;
       if (hub > hlb) {
+#pragma unroll 1
         for (int count = 1; count <= 4; ++count) {
           double yy[R], fy[R];
 #pragma unroll
@@ -975,9 +1154,11 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
       ++nst;
       __syncwarp();
       if (lane == 0) {
+#pragma unroll 1
         for (int i = q + 1; i >= 2; --i) TAU[i] = TAU[i - 1];
         TAU[1] = h;
       }
+#pragma unroll 1
       for (int j = 0; j <= q; ++j) {
         const double lj = LC[j];
 #pragma unroll
@@ -1013,6 +1194,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
           if (q != qmax) {
             const double hr = h / TAU[2];
             double hrp = hr;
+#pragma unroll 1
             for (int k = 0; k < q; ++k) hrp *= hr;
             const double cquot = (tq5 / tq5_saved) * hrp;
 #pragma unroll
@@ -1075,6 +1257,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
     const double htarget = rE * inv_rho;
     double Tn = Z[NS];
     if (!(Tn > 90.0 && Tn < 5000.0)) Tn = 1000.0;
+#pragma unroll 1
     for (int it = 0; it < 50; ++it) {
       double hl = 0.0, cl = 0.0;
 #pragma unroll

@@ -28,22 +28,22 @@ struct NewtonMatrixParams {
 // Shared bytes of one block (one warp): forcing, setup scratch, matrix, solve vector, pivots.
 template <class M, class JR>
 __host__ __device__ constexpr int newton_matrix_smem() {
-  constexpr int N = M::N, NS = M::NS, NR = M::NR;
-  return (N * 8 + 15) / 16 * 16 + ((wbdf::RXW * NR + 4 * NS) * (int)sizeof(JR) + 15) / 16 * 16 +
+  constexpr int N = M::N, NS = M::NS;
+  return (N * 8 + 15) / 16 * 16 + ((wbdf::rx_len<M>() + 4 * NS) * (int)sizeof(JR) + 15) / 16 * 16 +
          ((N * (N + 1) + N) * (int)sizeof(JR) + 15) / 16 * 16 + N * 4;
 }
 
 template <class M, class JR>
 __global__ void __launch_bounds__(32) newton_matrix_kernel(const NewtonMatrixParams P) {
-  constexpr int N = M::N, NS = M::NS, NR = M::NR;
+  constexpr int N = M::N, NS = M::NS;
   constexpr int R = (N + 31) / 32, LDA = N + 1;
   extern __shared__ __align__(16) unsigned char nsmem[];
   const int lane = threadIdx.x & 31;
   double* FRC = reinterpret_cast<double*>(nsmem);
   JR* RX = reinterpret_cast<JR*>(nsmem + (N * 8 + 15) / 16 * 16);
-  JR* TH = RX + wbdf::RXW * NR;
+  JR* TH = RX + wbdf::rx_len<M>();
   JR* A = reinterpret_cast<JR*>(reinterpret_cast<unsigned char*>(RX) +
-                                ((wbdf::RXW * NR + 4 * NS) * (int)sizeof(JR) + 15) / 16 * 16);
+                                ((wbdf::rx_len<M>() + 4 * NS) * (int)sizeof(JR) + 15) / 16 * 16);
   JR* XS = A + N * LDA;
   int* PIV = reinterpret_cast<int*>(XS + N);
   for (long long c = blockIdx.x; c < P.ncell; c += gridDim.x) {

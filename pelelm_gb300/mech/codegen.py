@@ -19,6 +19,7 @@ from __future__ import annotations
 
 import math
 import os
+import struct
 from typing import Dict, List
 
 from .model import Mechanism, R_CAL, R_ERG, P_ATM
@@ -484,6 +485,79 @@ def rx_packed(rx, ns: int) -> list:
     return out
 
 
+def _f32(x: float) -> float:
+    return struct.unpack("f", struct.pack("f", x))[0]
+
+
+def jac_stream(m: Mechanism, rx, tb_rows, codes, neg, T: int, LDA: int):
+    """The contribution program (kJacC, kJacNeg) in the form the kernels stream: (quads, entries,
+    x0, nx).
+
+    quads[q][lane] holds the lane's terms 4q..4q+3, one word each: bits 0-12 the index of the term's
+    first partial (8 j + slot of reaction j, or 8 NR + x for partial x below), 13-19 further slots
+    1..7 of the same reaction to add, 20 the sign of the coefficient (1: minus), 21 last term of its
+    entry, 22 the collider slot is scaled by its efficiency, 23 T column (added even when 0).
+    entries[e][lane] = (|c| in FP64, |c| in FP32, i LDA + k) of the lane's e-th entry.
+    Partials 8 NR + x0[tb] + s: the [M] partial of third-body row tb times the efficiency of its
+    s-th listed collider, so a collider term needs no efficiency of its own."""
+    ns = m.ns
+    x0, nx = [], 0
+    for effs in tb_rows:
+        x0.append(nx)
+        nx += len(effs)
+    n_rx = len(rx)
+    assert 8 * n_rx + nx <= 8192, "partial index field too narrow for this mechanism"
+    nq = (T + 3) // 4
+    quads = [[[0, 0, 0, 0] for _ in range(32)] for _ in range(nq)]
+    ents = [[] for _ in range(32)]
+    W = [s.W for s in m.species]
+    for l_ in range(32):
+        for t in range(T):
+            c = codes[32 * t + l_]
+            if c == 0:
+                continue  # padding: adds to a sum that is never stored
+            j, tg = c & 0x1FF, (c >> 9) & 0xFFF
+            i, k = divmod(tg, LDA)
+            word = ((neg[t] >> l_) & 1) << 20 | ((c >> 29) & 1) << 21
+            if c & (1 << 21):
+                word |= (8 * j) | 1 << 23
+            else:
+                slots = [1 + b for b in range(6) if c & (1 << (22 + b))] + ([7] if c & (1 << 28) else [])
+                scaled = bool(c & (1 << 31))
+                if slots == [7] and scaled:
+                    tb = rx[j][8]
+                    word |= 8 * n_rx + x0[tb] + [sp for sp, _ in tb_rows[tb]].index(k)
+                else:
+                    word |= 8 * j + slots[0]
+                    for s_ in slots[1:]:
+                        word |= 1 << (12 + s_)
+                    if scaled:
+                        word |= 1 << 22
+            quads[t // 4][l_][t % 4] = word
+            if c & (1 << 30):
+                wd = W[i] if k == ns else W[i] * (1.0 / W[k])
+                wf = _f32(W[i]) if k == ns else _f32(_f32(W[i]) * _f32(1.0 / W[k]))
+                ents[l_].append((wd, wf, tg))
+    return quads, ents, x0, nx
+
+
+def emit_jac_stream(e: _Emitter, qual: str, m: Mechanism, rx, tb_rows, codes, neg, T: int, LDA: int):
+    quads, ents, x0, nx = jac_stream(m, rx, tb_rows, codes, neg, T, LDA)
+    ne = max(len(v) for v in ents) + 1  # one past the end: read ahead, never used
+    e(f"constexpr int NJQ = {len(quads)}, NJE = {ne}, NJX = {nx};  // quads, entries per lane; scaled partials")
+    e(f"{qual} uint4 kJacQ[32 * NJQ] = {{")
+    for q in quads:
+        e("  " + ", ".join("{" + ", ".join(f"{w}u" for w in lane) + "}" for lane in q) + ",")
+    e("};")
+    for R, suf, col in (("double", "D", 0), ("float", "F", 1)):
+        e(f"{qual} TabJacEnt<{R}> kJacEnt{suf}[32 * NJE] = {{")
+        for n_ in range(ne):
+            row = [v[n_] if n_ < len(v) else (0.0, 0.0, 0) for v in ents]
+            e("  " + ", ".join("{" + _f(v[col]) + ("f" if col else "") + f", {v[2]}}}" for v in row) + ",")
+        e("};")
+    e(f"{qual} int kJacX0[NTB] = {{{', '.join(str(8 * len(rx) + v) for v in (x0 or [0]))}}};")
+
+
 def gen_tables(m: Mechanism, space: str = "constant") -> str:
     """Mechanism tables for the table-driven kernels: per-species W, NASA-7 sets, per-reaction
     Arrhenius data, stoichiometry as species slots (a species with coefficient 2 occupies two
@@ -549,7 +623,8 @@ def gen_tables(m: Mechanism, space: str = "constant") -> str:
             return [a[0], a[1] / 2, a[2] / 3, a[3] / 4, a[4] / 5, a[5]]
 
         for sp_ in m.species:
-            arrs = [sp_.low, sp_.high, gco(sp_.low), gco(sp_.high), hco(sp_.low), hco(sp_.high)]
+            arrs = [sp_.low, sp_.high, gco(sp_.low), gco(sp_.high), hco(sp_.low), hco(sp_.high),
+                    [v / sp_.W for v in hco(sp_.low)], [v / sp_.W for v in hco(sp_.high)]]
             body = ", ".join("{" + ", ".join(cast(a_) for a_ in arr) + "}" for arr in arrs)
             e(f"  {{{cast(sp_.W)}, {cast(1.0 / sp_.W)}, {cast(sp_.Tmid)}, {body}}},")
         e("};")
@@ -657,6 +732,7 @@ def gen_tables(m: Mechanism, space: str = "constant") -> str:
         e(f"{qual} unsigned kJacNeg[NJT] = {{{', '.join(str(x) + 'u' for x in neg)}}};")
         e(f"{qual} double kJacEffD[32 * NJT] = {{{', '.join(effD)}}};")
         e(f"{qual} float kJacEffF[32 * NJT] = {{{', '.join(effF)}}};")
+        emit_jac_stream(e, qual, m, rx, tb_rows, codes, neg, T, LDA)
         # packed reaction records of the FP64 rate of progress (TabRxArr / TabRxPk)
         e(f"{qual} TabRxArr kRxArr[NR] = {{")
         for (lnA, beta, mear, *_r) in rx:
@@ -679,9 +755,12 @@ def gen_tables(m: Mechanism, space: str = "constant") -> str:
         e("  __device__ static double sprx_nu(int e) { return kSpRxNu[e]; }")
         e("  __device__ static const TabRxArr& rx_arr(int j) { return kRxArr[j]; }")
         e("  __device__ static TabRxPk rx_pk(int j) { return kRxPk[j]; }")
-        e("  static constexpr int JAC_TERMS = NJT;")
-        e("  __device__ static unsigned jac_code(int c) { return kJacC[c]; }")
-        e("  __device__ static unsigned jac_neg(int t) { return kJacNeg[t]; }")
+        e("  static constexpr int JAC_QUADS = NJQ, JAC_ENTS = NJE, JAC_X = NJX;")
+        e("  __device__ static uint4 jac_quad(int c) { return kJacQ[c]; }")
+        e("  template <class R> __device__ static const TabJacEnt<R>& jac_ent(int c) {")
+        e("    if constexpr (sizeof(R) == sizeof(double)) return kJacEntD[c]; else return kJacEntF[c];")
+        e("  }")
+        e("  __device__ static int jac_x0(int tb) { return kJacX0[tb]; }")
         e("  template <class R> __device__ static R jac_eff(int c) {")
         e("    if constexpr (sizeof(R) == sizeof(double)) return kJacEffD[c]; else return kJacEffF[c];")
         e("  }")

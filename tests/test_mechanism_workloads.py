@@ -234,6 +234,78 @@ def test_jacobian_program_replays_the_reaction_walk():
         assert max(terms) <= 1.5 * np.mean(terms) + 20, (name, terms)
 
 
+@pytest.mark.parametrize("name", ["lidryer_syn", "drm19_syn", "gri_syn"])
+def test_streamed_jacobian_program_equals_the_program(name):
+    """The form of the contribution program that the kernels stream (jac_stream: four terms a load,
+    coefficients per entry, efficiencies folded into extra partials) adds, for every entry, the same
+    products in the same order as the program it is made from."""
+    import re
+    from pelelm_gb300.mech.codegen import gen_tables
+    m = load_mechanism(name)
+    txt = gen_tables(m, "global")
+
+    def arr(nm, conv=int):
+        body = re.search(nm + r"\[[^\]]*\] = \{(.*?)\};", txt, re.S).group(1)
+        return [conv(x.strip()) for x in body.replace("{", "").replace("}", "").split(",") if x.strip()]
+
+    T, nq, ne = (int(re.search(nm + r" = (\d+)", txt).group(1)) for nm in ("NJT", "NJQ", "NJE"))
+    codes, negs = arr("kJacC", lambda x: int(x.rstrip("u"))), arr("kJacNeg", lambda x: int(x.rstrip("u")))
+    effs = arr("kJacEffD", lambda x: float(eval(x)))
+    quads = np.array(arr("kJacQ", lambda x: int(x.rstrip("u")))).reshape(nq, 32, 4)
+    ents = np.array(arr("kJacEntD", float)).reshape(ne, 32, 2)
+    entf = np.array(arr("kJacEntF", lambda x: float(x.rstrip("f")))).reshape(ne, 32, 2)
+    x0 = arr("kJacX0")
+    N, LDA = m.ns + 1, m.ns + 2
+    W = [s.W for s in m.species]
+    rng = np.random.default_rng(7)
+    P = rng.normal(size=8 * m.nr)
+    kinds = {"elementary": 0, "three_body": 1, "falloff": 2}
+    order = sorted(range(m.nr), key=lambda j: (kinds[m.reactions[j].kind], j))
+    tb_rows = [[e for e in m.reactions[j].efficiencies.values() if e != 1.0] for j in range(m.nr)
+               if m.reactions[j].kind != "elementary"]  # third-body rows in input order
+    rows = [j for j in range(m.nr) if m.reactions[j].kind != "elementary"]
+    RX = list(P) + [0.0] * sum(len(t) for t in tb_rows)
+    for row, j in enumerate(rows):
+        for s_, e in enumerate(tb_rows[row]):
+            RX[x0[row] + s_] = P[8 * order.index(j) + 7] * (1.0 + (e - 1.0))
+    for ln in range(32):
+        want, got = [], []
+        w = 0.0
+        for t in range(T):
+            c = codes[32 * t + ln]
+            if c == 0:
+                continue
+            if c & (1 << 30):
+                i, k = divmod((c >> 9) & 0xFFF, LDA)
+                w = W[i] if k == m.ns else W[i] * (1.0 / W[k])
+            pj = P[8 * (c & 0x1FF):8 * (c & 0x1FF) + 8]
+            if c & (1 << 21):
+                v = pj[0]
+            else:
+                v = sum(pj[1 + b] for b in range(6) if c & (1 << (22 + b)))
+                if c & (1 << 28):
+                    v += pj[7] * (effs[32 * t + ln] if c & (1 << 31) else 1.0)
+            want.append((-w if (negs[t] >> ln) & 1 else w, v, bool(c & (1 << 29)), (c >> 9) & 0xFFF))
+        e = 0
+        for t in range(4 * nq):
+            c = int(quads[t // 4, ln, t % 4])
+            if c == 0:
+                continue
+            v = RX[c & 0x1FFF]
+            base = (c & 0x1FFF) & ~7
+            v += sum(P[base + s_] for s_ in range(1, 7) if c & (1 << (12 + s_)))
+            if c & (1 << 19):
+                v += P[base + 7] * (effs[32 * t + ln] if c & (1 << 22) else 1.0)
+            wd, tg = ents[e, ln]
+            assert abs(entf[e, ln, 0] - wd) <= 2e-7 * wd and entf[e, ln, 1] == tg
+            assert (not c & (1 << 23)) or c & 7 == 0
+            got.append((-wd if c & (1 << 20) else wd, v, bool(c & (1 << 21)), int(tg)))
+            e += bool(c & (1 << 21))
+        assert len(want) == len(got) and e <= ne - 1
+        for a, b in zip(want, got):
+            assert a[0] == b[0] and a[2:] == b[2:] and abs(a[1] - b[1]) <= 1e-15 * (1.0 + abs(a[1]))
+
+
 def test_packed_reaction_records_match_the_reaction_table():
     """The warp and lane-group RHS read each reaction through two packed records (kRxArr,
     kRxPk); decoded, they must equal the fields of the FP64 reaction table entry by entry."""
