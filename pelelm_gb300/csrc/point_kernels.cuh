@@ -61,14 +61,12 @@ __global__ void rates_kernel(const PointParams p) {
 #pragma unroll
   for (int s = 0; s < M::NS; ++s) { Y[s] = arr_at(p.rY, i, j, k, s); rho += Y[s]; }
   const double inv_rho = 1.0 / rho;
-#pragma unroll
-  for (int s = 0; s < M::NS; ++s) Y[s] *= inv_rho;
   // MKS -> CGS: h [J/kg] * 1e4 = erg/g ; rho [kg/m^3] * 1e-3 = g/cm^3
-  const double T = hy2t_newton<M>(arr_at(p.rE, i, j, k, 0) * inv_rho * 1.0e4, Y, arr_at(p.T, i, j, k, 0),
-                                  90.0, 5000.0);
-  const double rho_cgs = rho * 1.0e-3;
+  const double T = hy2t_mixture<typename M::Tab>(arr_at(p.rE, i, j, k, 0) * inv_rho * 1.0e4,
+                                                 [&](int s) { return arr_at(p.rY, i, j, k, s); }, inv_rho,
+                                                 arr_at(p.T, i, j, k, 0), 90.0, 5000.0);
 #pragma unroll
-  for (int s = 0; s < M::NS; ++s) C[s] = rho_cgs * Y[s] / M::W(s);
+  for (int s = 0; s < M::NS; ++s) C[s] = Y[s] * (1.0e-3 / M::W(s));
   M::wdot(T, C, wd);
 #pragma unroll
   for (int s = 0; s < M::NS; ++s) arr_at(p.out, i, j, k, s) = wd[s] * M::W(s) * 1000.0;  // g/cm^3/s -> kg/m^3/s
@@ -82,15 +80,13 @@ __global__ void h2t_kernel(const PointParams p) {
   const int i = p.lo0 + (int)(c % p.len0);
   const int j = p.lo1 + (int)((c / p.len0) % p.len1);
   const int k = p.lo2 + (int)(c / ((long long)p.len0 * p.len1));
-  double Y[M::NS];
   double rho = 0.0;
-#pragma unroll
-  for (int s = 0; s < M::NS; ++s) { Y[s] = arr_at(p.rY, i, j, k, s); rho += Y[s]; }
+#pragma unroll 4
+  for (int s = 0; s < M::NS; ++s) rho += arr_at(p.rY, i, j, k, s);
   const double inv_rho = 1.0 / rho;
-#pragma unroll
-  for (int s = 0; s < M::NS; ++s) Y[s] *= inv_rho;
   double& T = arr_at(p.T, i, j, k, 0);
-  T = hy2t_newton<M>(arr_at(p.rE, i, j, k, 0) * inv_rho * 1.0e4, Y, T, p.tmin, p.tmax);
+  T = hy2t_mixture<typename M::Tab>(arr_at(p.rE, i, j, k, 0) * inv_rho * 1.0e4,
+                                    [&](int s) { return arr_at(p.rY, i, j, k, s); }, inv_rho, T, p.tmin, p.tmax);
 }
 
 // Heat release rate -sum_k rhoYdot_k h_k(T) [W/m^3] from T and the MKS reaction rates
@@ -98,7 +94,7 @@ __global__ void h2t_kernel(const PointParams p) {
 // per-cell work of the HeatRelease derive (Source/PeleLM_derive.cpp:627-650).
 template <class M>
 __global__ void heat_release_kernel(const PointParams p) {
-  using Tab = typename M::TabG;
+  using Tab = typename M::Tab;
   const long long n = (long long)p.len0 * p.len1 * p.len2;
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
@@ -106,16 +102,18 @@ __global__ void heat_release_kernel(const PointParams p) {
   const int j = p.lo1 + (int)((c / p.len0) % p.len1);
   const int k = p.lo2 + (int)(c / ((long long)p.len0 * p.len1));
   const double T = arr_at(p.T, i, j, k, 0);
-  const double invT = 1.0 / T;
   double hr = 0.0;
+#pragma unroll 3
   for (int s = 0; s < M::NS; ++s) {
     const TabSpecies<double>& sp = Tab::template sp<double>(s);
-    const double* hc = T < sp.Tmid ? sp.hlo : sp.hhi;
-    const double hRT = fma(T, fma(T, fma(T, fma(T, hc[4], hc[3]), hc[2]), hc[1]), fma(hc[5], invT, hc[0]));
-    const double h_mks = hRT * kRerg * T * sp.invW * 1.0e-4;  // erg/g -> J/kg
-    hr = fma(-arr_at(p.rY, i, j, k, s), h_mks, hr);
+    const bool lo = T < sp.Tmid;
+    double a[6];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) a[q] = lo ? sp.wlo[q] : sp.whi[q];
+    hr = fma(arr_at(p.rY, i, j, k, s),
+             fma(T, fma(T, fma(T, fma(T, fma(T, a[4], a[3]), a[2]), a[1]), a[0]), a[5]), hr);
   }
-  arr_at(p.out, i, j, k, 0) = hr;
+  arr_at(p.out, i, j, k, 0) = hr * (-kRerg * 1.0e-4);  // erg/g -> J/kg
 }
 
 // ReactorNull: rhoY += dt F, rho h += dt F_h, T from the new (h, Y), FC = 0 (CGS, in place).
