@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
   double del2 = 0.0, delp2 = 0.0, hg = 0.0, hub = 0.0, hlb = 0.0, rE0 = 0.0;
   int q = 1, qwait = 2, nef = 0, ncf = 0, m = 0, hin_count = 0, status = OK;
   long long nst = 0, nfe = 0, nje = 0, nstlp = 0, netf = 0, ncfn = 0;
-  bool new_step = true, need_setup = true, force_setup = true, jcur = false;
+  bool new_step = true, need_setup = true, force_setup = true, jcur = false, fresh = false;
 
 #pragma unroll
   for (int i = 0; i < N; ++i) { y[i] = 0.0; acor[i] = 0.0; ewt[i] = 1.0; }
@@ -165,6 +165,7 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
   };
   auto rescale = [&](double e) {
     double fac = e;
+#pragma unroll 1
     for (int j = 1; j <= q; ++j) {
 #pragma unroll
       for (int i = 0; i < N; ++i) Z(j, i) *= fac;
@@ -175,15 +176,18 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
   };
   auto predict = [&]() {
     t += h;
+#pragma unroll 1
     for (int k = 1; k <= q; ++k)
+#pragma unroll 1
       for (int j = q; j >= k; --j) {
 #pragma unroll
         for (int i = 0; i < N; ++i) Z(j - 1, i) += Z(j, i);
       }
   };
-  auto retract = [&]() {
-    t -= h;
+  auto retract = [&]() {  // t goes back where the outcome is found
+#pragma unroll 1
     for (int k = 1; k <= q; ++k)
+#pragma unroll 1
       for (int j = q; j >= k; --j) {
 #pragma unroll
         for (int i = 0; i < N; ++i) Z(j - 1, i) -= Z(j, i);
@@ -191,40 +195,43 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
   };
   // fixed-leading-coefficient BDF: Lambda(x) coefficients l[] and error constants tq1..tq5
   auto set_coeffs = [&]() {
+#pragma unroll 1
     for (int i = 0; i <= qmax; ++i) LCO(i) = 0.0;
     LCO(0) = 1.0;
     double alpha0 = 0.0;
+#pragma unroll 1
     for (int j = 1; j <= q; ++j) alpha0 -= inv_int(j);
     double hsum = h, sum_xi_inv = 0.0;
+#pragma unroll 1
     for (int i = 1; i <= q - 1; ++i) {
       if (i > 1) hsum += TAU(i - 1);
-      const double xi_inv = h / hsum;
+      const double xi_inv = pgb_div64(h, hsum);
       sum_xi_inv += xi_inv;
       for (int k = i; k >= 1; --k) LCO(k) += LCO(k - 1) * xi_inv;
     }
     const double xistar_inv = -alpha0 - sum_xi_inv;
     for (int k = q; k >= 1; --k) LCO(k) += LCO(k - 1) * xistar_inv;
     if (q > 1) hsum += TAU(q - 1);
-    const double xiq_inv = h / hsum;
+    const double xiq_inv = pgb_div64(h, hsum);
     const double alpha0_hat = -(sum_xi_inv + xiq_inv);
     const double A1 = 1.0 - alpha0_hat + alpha0;
     const double A2 = 1.0 + q * A1;
-    tq2 = fabs(A1 / (alpha0 * A2));
-    tq5 = fabs(A2 * xistar_inv / (LCO(q) * xiq_inv));
+    tq2 = fabs(pgb_div64(A1, alpha0 * A2));
+    tq5 = fabs(pgb_div64(A2 * xistar_inv, LCO(q) * xiq_inv));
     if (qwait == 1) {
       if (q > 1) {
-        const double C = xistar_inv / LCO(q);
+        const double C = pgb_div64(xistar_inv, LCO(q));
         const double A3 = alpha0 + inv_int(q);
         const double A4 = alpha0_hat + xiq_inv;
-        tq1 = fabs(C * (1.0 - A4 + A3) / A3);
+        tq1 = fabs(pgb_div64(C * (1.0 - A4 + A3), A3));
       } else {
         tq1 = 1.0;
       }
-      const double xiq1_inv = h / (hsum + TAU(q));
+      const double xiq1_inv = pgb_div64(h, hsum + TAU(q));
       const double A5 = alpha0 - inv_int(q + 1);
       const double A6 = alpha0_hat - xiq1_inv;
-      const double Cpp = (1.0 - A6 + A5) / A2;
-      tq3 = fabs(Cpp / (xiq1_inv * (q + 2) * A5));
+      const double Cpp = pgb_div64(1.0 - A6 + A5, A2);
+      tq3 = fabs(pgb_div64(Cpp, xiq1_inv * (q + 2) * A5));
     }
     inv_tq4_sq = (tq2 * (1.0 / NLSCOEF)) * (tq2 * (1.0 / NLSCOEF));
   };
@@ -234,18 +241,21 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
     w[2] = 1.0;
     if (dq > 0) {
       double alpha0 = 0.0, alpha1 = 0.0, prod = 1.0, hsum = 0.0;
+#pragma unroll 1
       for (int j = 1; j <= q; ++j) {
         hsum += TAU(j);
-        const double xi = hsum / hscale;
+        const double xi = pgb_div64(hsum, hscale);
         prod *= xi;
         alpha0 -= inv_int(j);
-        alpha1 += 1.0 / xi;
+        alpha1 += pgb_div64(1.0, xi);
         if (j <= q - 1)
+#pragma unroll 1
           for (int i = j + 2; i >= 2; --i) w[i] = w[i] * xi + w[i - 1];
       }
-      const double A1 = (-alpha0 - alpha1) / prod;
+      const double A1 = pgb_div64(-alpha0 - alpha1, prod);
 #pragma unroll
       for (int i = 0; i < N; ++i) Z(q + 1, i) = A1 * Z(QMAX + 1, i);
+#pragma unroll 1
       for (int j = 2; j <= q; ++j) {
         const double wj = w[j];
 #pragma unroll
@@ -253,11 +263,14 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
       }
     } else {
       double hsum = 0.0;
+#pragma unroll 1
       for (int j = 1; j <= q - 2; ++j) {
         hsum += TAU(j);
-        const double xi = hsum / hscale;
+        const double xi = pgb_div64(hsum, hscale);
+#pragma unroll 1
         for (int i = j + 2; i >= 2; --i) w[i] = w[i] * xi + w[i - 1];
       }
+#pragma unroll 1
       for (int j = 2; j < q; ++j) {
         const double wj = w[j];
 #pragma unroll
@@ -356,32 +369,20 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
     // rho h(t) = rho h0 + F_h t ; T from (h, Y) by Newton with the integrated T as guess
     const double rE = fma(tout, FRC(NS), rE0);
     double rho = 0.0;
-#pragma unroll
+#pragma unroll 1
     for (int k = 0; k < NS; ++k) rho += Z(0, k);
     const double inv_rho = 1.0 / rho;
-    double Yk[NS];
-#pragma unroll
-    for (int k = 0; k < NS; ++k) Yk[k] = Z(0, k) * inv_rho;
-    const double htarget = rE * inv_rho;
     double Tn = Z(0, NS);
     if (!(Tn > 90.0 && Tn < 5000.0)) Tn = 1000.0;
-    for (int it = 0; it < 50; ++it) {
-      double hh, cp;
-      M::h_cp_mix(Tn, Yk, hh, cp);
-      double dT = (htarget - hh) / cp;
-      dT = fmax(-100.0, fmin(100.0, dT));
-      Tn = fmax(90.0, fmin(5000.0, Tn + dT));
-      if (fabs(dT) < 1e-10 * Tn) break;
+    Tn = hy2t_mixture<typename M::Tab>(rE * inv_rho, [&](int k) { return Z(0, k); }, inv_rho, Tn, 90.0, 5000.0);
+    const double dt_inv = pgb_div64(1.0, tout);
+#pragma unroll 1
+    for (int k = 0; k < NS; ++k) {
+      const double rYn = __dmul_rn(Z(0, k), B.sY_out);
+      if (B.IR.p)  // separate roundings, as separate passes over arrays give
+        elem(B.IR, k) = __dsub_rn(__dmul_rn(-__dsub_rn(elem(B.rY, k), rYn), dt_inv), elem(B.rYsrc, k));
+      elem(B.rY, k) = rYn;
     }
-    if (B.IR.p) {
-      const double dt_inv = 1.0 / tout;
-#pragma unroll
-      for (int k = 0; k < NS; ++k)  // separate roundings, as separate passes over arrays give
-        elem(B.IR, k) = __dsub_rn(__dmul_rn(-__dsub_rn(elem(B.rY, k), __dmul_rn(Z(0, k), B.sY_out)), dt_inv),
-                                  elem(B.rYsrc, k));
-    }
-#pragma unroll
-    for (int k = 0; k < NS; ++k) elem(B.rY, k) = Z(0, k) * B.sY_out;
     elem(B.T, 0) = Tn;
     elem(B.rE, 0) = rE * B.sE_out;
     elem(B.FC, 0) = (status == OK) ? (double)nfe : -(double)status;
@@ -399,7 +400,7 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
   };
   auto fail_cell = [&](int st) {
     status = st;
-    finish_cell();
+    phase = FINISH;
   };
   auto load_cell = [&](long long c) {
     // box containing flat cell c (binary search over cell offsets)
@@ -422,11 +423,12 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
       if (mv < 0) {  // covered cell: no reaction, zero function count
         elem(B.FC, 0) = 0.0;
         if (B.IR.p)
+#pragma unroll 1
           for (int k = 0; k < NS; ++k) elem(B.IR, k) = -elem(B.rYsrc, k);
         return false;
       }
     }
-#pragma unroll
+#pragma unroll 3
     for (int k = 0; k < NS; ++k) {
       Z(0, k) = elem(B.rY, k) * B.sY_in;
       FRC(k) = elem(B.rYsrc, k) * B.sY_in;
@@ -434,16 +436,16 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
     Z(0, NS) = elem(B.T, 0);
     FRC(NS) = elem(B.rEsrc, 0) * B.sE_in;
     rE0 = elem(B.rE, 0) * B.sE_in;
-    for (int j = 1; j <= QMAX + 1; ++j)
-#pragma unroll
-      for (int i = 0; i < N; ++i) Z(j, i) = 0.0;
+#pragma unroll 2
+    for (int e = N; e < (QMAX + 2) * N; ++e) Z(0, e) = 0.0;  // columns 1..QMAX+1
+#pragma unroll 1
     for (int j = 0; j <= QMAX + 1; ++j) TAU(j) = 0.0;
     t = 0.0; h = 0.0; hscale = 0.0; etamax = ETAMX1; eta = 1.0;
     gamma = 0.0; gammap = 0.0; gamrat = 1.0; crate2 = 1.0; rl1 = 1.0;
     tq1 = tq2 = tq3 = tq5 = tq5_saved = inv_tq4_sq = 1.0;
     q = 1; qwait = 2; nef = 0; ncf = 0; m = 0; status = OK;
     nst = 0; nfe = 0; nje = 0; nstlp = 0; netf = 0; ncfn = 0;
-    new_step = true; need_setup = true; force_setup = true; jcur = false;
+    new_step = true; need_setup = true; force_setup = true; jcur = false; fresh = false;
     return true;
   };
 
@@ -468,38 +470,33 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
     if (__all_sync(0xffffffffu, phase == IDLE)) break;
 
     // ------------------------------------------------ (B) prepare the RHS argument
+    if (phase == STEP && new_step && nst >= P.max_steps) fail_cell(MAX_STEPS);
+    if ((phase == STEP && new_step) || (phase == HIN && hin_count == 1)) set_ewt();
     if (phase == STEP) {
-      bool ok = true;
       if (new_step) {
-        if (nst >= P.max_steps) { fail_cell(MAX_STEPS); ok = false; }
-        else {
-          if ((t + h - tout) * h > 0.0) rescale((tout - t) * (1.0 - 4.0 * UROUND) / h);
-          set_ewt();
-          nef = 0; ncf = 0;
-          new_step = false;
-        }
+        nef = 0; ncf = 0;
+        new_step = false;
       }
-      if (ok) {
-        predict();
-        set_coeffs();
-        rl1 = 1.0 / LCO(1);
-        gamma = h * rl1;
-        if (nst == 0) gammap = gamma;
-        gamrat = (nst > 0) ? gamma / gammap : 1.0;
-        need_setup = force_setup || nst == 0 || nst >= nstlp + MSBP || fabs(gamrat - 1.0) > DGMAX;
-        force_setup = false;
-        jcur = false;
-        m = 0;
+      predict();
+      set_coeffs();
+      rl1 = pgb_div64(1.0, LCO(1));
+      gamma = h * rl1;
+      if (nst == 0) gammap = gamma;
+      gamrat = (nst > 0) ? pgb_div64(gamma, gammap) : 1.0;
+      need_setup = force_setup || nst == 0 || nst >= nstlp + MSBP || fabs(gamrat - 1.0) > DGMAX;
+      force_setup = false;
+      jcur = false;
+      m = 0;
+      phase = NEWTON;
+      fresh = true;
+    }
+    if (fresh || phase == START || phase == RESETD) {  // from the prediction
 #pragma unroll
-        for (int i = 0; i < N; ++i) { y[i] = Z(0, i); acor[i] = 0.0; }
-        phase = NEWTON;
-      }
+      for (int i = 0; i < N; ++i) { y[i] = Z(0, i); acor[i] = 0.0; }
+      fresh = false;
     } else if (phase == HIN) {
 #pragma unroll
       for (int i = 0; i < N; ++i) y[i] = fma(hg, Z(1, i), Z(0, i));
-    } else if (phase == START || phase == RESETD) {
-#pragma unroll
-      for (int i = 0; i < N; ++i) y[i] = Z(0, i);
     }
 
     // ------------------------------------------------ (C) one FP64 RHS for every lane
@@ -521,57 +518,56 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
     }
 
     // ------------------------------------------------ (D) consume it
+    // The step's vector work that more than one outcome needs (undoing the prediction, changing
+    // the order, rescaling the history) is only noted here and done once, below, for every lane
+    // that needs it: one copy of its code, and one pass of its FP64 instructions instead of one
+    // per outcome (this kernel is bound by instruction fetch as much as by the FP64 pipe).
+    bool undo = false, check_h = false, first_step = false;
+    int dq = 0;
+    double scale = 1.0;
+    if (phase == START || phase == RESETD) {
+      const double fac = phase == START ? 1.0 : h;
+#pragma unroll
+      for (int i = 0; i < N; ++i) Z(1, i) = fac * f[i];  // START: f0 parked until h is known
+    }
     if (phase == START) {
       // initial step size: difference-quotient estimate of y'' (bounded)
-#pragma unroll
-      for (int i = 0; i < N; ++i) Z(1, i) = f[i];  // f0 parked in z[1] until h is known
-      set_ewt();
       const double tround = UROUND * tout;
       hlb = 100.0 * tround;
       double hub_inv = 0.0;
-#pragma unroll
+#pragma unroll 1
       for (int i = 0; i < N; ++i)
-        hub_inv = fmax(hub_inv, fabs(f[i]) / fma(0.1, fabs(Z(0, i)), P.atol[i]));
+        hub_inv = fmax(hub_inv, pgb_div64(fabs(Z(1, i)), fma(0.1, fabs(Z(0, i)), P.atol[i])));
       hub = 0.1 * tout;
-      if (hub * hub_inv > 1.0) hub = 1.0 / hub_inv;
+      if (hub * hub_inv > 1.0) hub = pgb_div64(1.0, hub_inv);
       hg = sqrt(hlb * hub);
       if (hub > hlb) {
         hin_count = 1;
         phase = HIN;
       } else {
         h = fmin(fmax(0.5 * hg, hlb), hub);
-        hscale = h;
-#pragma unroll
-        for (int i = 0; i < N; ++i) Z(1, i) *= h;
-        q = 1; qwait = 2; etamax = ETAMX1; TAU(1) = h; new_step = true;
-        phase = STEP;
+        first_step = true;
       }
     } else if (phase == HIN) {
       double d[N];
 #pragma unroll
-      for (int i = 0; i < N; ++i) d[i] = (f[i] - Z(1, i)) / hg;
+      for (int i = 0; i < N; ++i) d[i] = pgb_div64(f[i] - Z(1, i), hg);
       const double ydd = sqrt(wms(d));
-      double hnew = (ydd * hub * hub > 2.0) ? sqrt(2.0 / ydd) : sqrt(hg * hub);
+      double hnew = sqrt((ydd * hub * hub > 2.0) ? pgb_div64(2.0, ydd) : hg * hub);
       bool done = false;
       if (hin_count == 4) {
         done = true;
       } else {
-        const double hrat = hnew / hg;
+        const double hrat = pgb_div64(hnew, hg);
         if (hrat > 0.5 && hrat < 2.0) done = true;
         else if (hin_count >= 2 && hrat > 2.0) { hnew = hg; done = true; }
         else { hg = hnew; ++hin_count; }
       }
       if (done) {
         h = fmin(fmax(0.5 * hnew, hlb), hub);
-        hscale = h;
-#pragma unroll
-        for (int i = 0; i < N; ++i) Z(1, i) *= h;
-        q = 1; qwait = 2; etamax = ETAMX1; TAU(1) = h; new_step = true;
-        phase = STEP;
+        first_step = true;
       }
     } else if (phase == RESETD) {
-#pragma unroll
-      for (int i = 0; i < N; ++i) Z(1, i) = h * f[i];
       phase = STEP;
     } else if (phase == NEWTON) {
       bool singular = false;
@@ -589,14 +585,14 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
         for (int i = 0; i < N; ++i) b[i] = fma(gamma, f[i], -fma(rl1, Z(1, i), acor[i]));
         lu_solve(b);
         if (gamrat != 1.0) {
-          const double s = 2.0 / (1.0 + gamrat);
+          const double s = pgb_div64(2.0, 1.0 + gamrat);
 #pragma unroll
           for (int i = 0; i < N; ++i) b[i] *= s;
         }
         del2 = wms(b);
 #pragma unroll
         for (int i = 0; i < N; ++i) { acor[i] += b[i]; y[i] = Z(0, i) + acor[i]; }
-        if (m > 0) crate2 = fmax((CRDOWN * CRDOWN) * crate2, del2 / delp2);
+        if (m > 0) crate2 = fmax((CRDOWN * CRDOWN) * crate2, pgb_div64(del2, delp2));
         // convergence: del * min(1, crate) / tq4 <= 1, in squares
         const double dcon2 = del2 * fmin(1.0, crate2) * inv_tq4_sq;
         if (dcon2 <= 1.0) {
@@ -611,70 +607,67 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
         // stale Jacobian: refresh it and restart the iteration from the prediction
         need_setup = true;
         m = 0;
-#pragma unroll
-        for (int i = 0; i < N; ++i) { y[i] = Z(0, i); acor[i] = 0.0; }
+        fresh = true;
       } else if (outcome >= 2) {
-        retract();
+        undo = true;
+        t -= h;
         ++ncf; ++ncfn;
         if (outcome == 3 || ncf >= MXNCF || fabs(h) <= 100.0 * UROUND * fabs(t)) {
           fail_cell(CONV);
         } else {
           force_setup = true;
           etamax = 1.0;
-          rescale(ETACF);
+          scale = ETACF;
           phase = STEP;
         }
       } else if (outcome == 1) {
         const double acnrm2 = (m == 0) ? del2 : wms(acor);
         const double dsm2 = acnrm2 * (tq2 * tq2);  // squared local error estimate
+        const double etaq = pgb_div64(1.0, pgb_pow64((BIAS2 * BIAS2) * dsm2, 0.5 * inv_int(q + 1)) + ADDON);
         if (!(dsm2 <= 1.0)) {
           // ---- local error test failed ----
-          retract();
+          undo = true;
+          t -= h;
           ++nef; ++netf;
           if (nef >= MXNEF || !isfinite(dsm2)) {
             fail_cell(isfinite(dsm2) ? ERRTEST : NONFINITE);
           } else {
+            check_h = true;
             etamax = 1.0;
+            phase = STEP;
+            scale = ETAMIN;
             if (nef <= MXNEF1) {
-              double e = 1.0 / (pgb_pow64((BIAS2 * BIAS2) * dsm2, 0.5 * inv_int(q + 1)) + ADDON);
-              e = fmax(ETAMIN, e);
-              if (nef >= SMALL_NEF) e = fmin(e, ETAMXF);
-              rescale(e);
-              phase = STEP;
+              scale = fmax(ETAMIN, etaq);
+              if (nef >= SMALL_NEF) scale = fmin(scale, ETAMXF);
             } else if (q > 1) {
-              adjust_order(-1);
-              --q;
-              qwait = q + 1;
-              rescale(ETAMIN);
-              phase = STEP;
+              dq = -1;
             } else {
-              rescale(ETAMIN);
               qwait = 10;
               phase = RESETD;
             }
-            if (phase != NEED && fabs(h) <= 100.0 * UROUND * fabs(t)) fail_cell(HSMALL);
           }
         } else {
           // ---- step accepted: complete it ----
           ++nst;
+#pragma unroll 1
           for (int i = q + 1; i >= 2; --i) TAU(i) = TAU(i - 1);
           TAU(1) = h;
+#pragma unroll 1
           for (int j = 0; j <= q; ++j) {
             const double lj = LCO(j);
 #pragma unroll
             for (int i = 0; i < N; ++i) Z(j, i) = fma(lj, acor[i], Z(j, i));
           }
           --qwait;
+          bool save = false;
           if (qwait == 1 && q != qmax) {
-#pragma unroll
-            for (int i = 0; i < N; ++i) Z(QMAX + 1, i) = acor[i];
+            save = true;
             tq5_saved = tq5;
           }
           if (fabs(t - tout) <= 100.0 * UROUND * (fabs(t) + fabs(h)) || t >= tout) {
-            finish_cell();
+            phase = FINISH;
           } else {
             // ---- next step size and order ----
-            const double etaq = 1.0 / (pgb_pow64((BIAS2 * BIAS2) * dsm2, 0.5 * inv_int(q + 1)) + ADDON);
             int qprime = q;
             if (etamax == 1.0) {
               qwait = max(qwait, 2);
@@ -689,18 +682,19 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
 #pragma unroll
                   for (int i = 0; i < N; ++i) zq[i] = Z(q, i);
                   const double ddn2 = wms(zq) * (tq1 * tq1);
-                  etaqm1 = 1.0 / (pgb_pow64((BIAS1 * BIAS1) * ddn2, 0.5 * inv_int(q)) + ADDON);
+                  etaqm1 = pgb_div64(1.0, pgb_pow64((BIAS1 * BIAS1) * ddn2, 0.5 * inv_int(q)) + ADDON);
                 }
                 if (q != qmax) {
-                  const double hr = h / TAU(2);
+                  const double hr = pgb_div64(h, TAU(2));
                   double hrp = hr;
+#pragma unroll 1
                   for (int k = 0; k < q; ++k) hrp *= hr;  // (h / tau2)^(q+1)
-                  const double cquot = (tq5 / tq5_saved) * hrp;
+                  const double cquot = pgb_div64(tq5, tq5_saved) * hrp;
                   double tv[N];
 #pragma unroll
                   for (int i = 0; i < N; ++i) tv[i] = acor[i] - cquot * Z(QMAX + 1, i);
                   const double dup2 = wms(tv) * (tq3 * tq3);
-                  etaqp1 = 1.0 / (pgb_pow64((BIAS3 * BIAS3) * dup2, 0.5 * inv_int(q + 2)) + ADDON);
+                  etaqp1 = pgb_div64(1.0, pgb_pow64((BIAS3 * BIAS3) * dup2, 0.5 * inv_int(q + 2)) + ADDON);
                 }
                 const double etam = fmax(etaqm1, fmax(etaq, etaqp1));
                 if (etam < THRESH) {
@@ -713,8 +707,7 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
                 } else {
                   eta = etaqp1;
                   qprime = q + 1;
-#pragma unroll
-                  for (int i = 0; i < N; ++i) Z(QMAX + 1, i) = acor[i];
+                  save = true;
                 }
               } else if (eta < THRESH) {
                 eta = 1.0;
@@ -723,18 +716,43 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
               else eta = 1.0;
             }
             etamax = (nst <= SMALL_NST) ? ETAMX2 : ETAMX3;
-            if (qprime != q) {
-              adjust_order(qprime - q);
-              q = qprime;
-              qwait = q + 1;
-            }
-            if (eta != 1.0) rescale(eta);
+            dq = qprime - q;
+            scale = eta;
             new_step = true;
             phase = STEP;
+          }
+          if (save) {
+#pragma unroll
+            for (int i = 0; i < N; ++i) Z(QMAX + 1, i) = acor[i];
           }
         }
       }
     }
+    if (undo) retract();
+    if (dq != 0) {
+      adjust_order(dq);
+      q += dq;
+      qwait = q + 1;
+    }
+    if (first_step) {
+      hscale = h;
+#pragma unroll
+      for (int i = 0; i < N; ++i) Z(1, i) *= h;
+      q = 1; qwait = 2; etamax = ETAMX1; TAU(1) = h; new_step = true;
+      phase = STEP;
+    }
+    // the new step size, then a cut to end at tout
+#pragma unroll 1
+    for (int pass = 0; pass < 2; ++pass) {
+      if (pass == 1) {
+        scale = 1.0;
+        if (phase == STEP && new_step && (t + h - tout) * h > 0.0)
+          scale = pgb_div64((tout - t) * (1.0 - 4.0 * UROUND), h);
+      }
+      if (scale != 1.0) rescale(scale);
+    }
+    if (check_h && fabs(h) <= 100.0 * UROUND * fabs(t)) fail_cell(HSMALL);
+    if (phase == FINISH) finish_cell();
   }
 #undef Z
 #undef LCO
