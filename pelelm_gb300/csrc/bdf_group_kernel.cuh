@@ -51,11 +51,12 @@ __host__ __device__ constexpr int gbdf_cell_bytes() {
 }
 template <class M>
 __host__ __device__ constexpr int gbdf_rhs_bytes() {
-  return (2 * M::NS + M::NR) * 8;
+  return (2 * M::NS + M::NR + (M::RHS_TABLE ? 0 : M::NR)) * 8;  // unrolled: and each reaction's [M]
 }
 template <class M, class JR>
 __host__ __device__ constexpr int gbdf_setup_bytes() {
   constexpr int N = M::N, NS = M::NS;
+  if (!M::RHS_TABLE) return 0;  // unrolled: the Jacobian goes straight into the cell's matrix
   return N * 8 + (N + wbdf::rx_len<M>() + 4 * NS) * (int)sizeof(JR);
 }
 template <class M, class JR, int G>
@@ -66,6 +67,24 @@ __host__ __device__ constexpr int gbdf_shared_scratch_bytes() {
 template <class M, class JR, int G>
 __host__ __device__ constexpr int gbdf_smem_per_warp() {
   return (32 / G) * gbdf_cell_bytes<M, JR>() + gbdf_shared_scratch_bytes<M, JR, G>();
+}
+
+// J(i, k) of a row-major matrix with rows of LDA.
+template <class JR, int LDA>
+struct RowAcc {
+  JR* base;
+  __device__ __forceinline__ JR& operator()(int i, int k) const { return base[i * LDA + k]; }
+};
+
+// The unrolled Jacobian by one lane, out of line: its registers do not add to the kernel's.
+template <class M, class JR>
+__device__ __noinline__ void unrolled_jacobian(const double* y, const double* FRC, JR* A) {
+  double yl[M::N], Fl[M::NS];
+#pragma unroll
+  for (int i = 0; i < M::N; ++i) yl[i] = y[i];
+#pragma unroll
+  for (int i = 0; i < M::NS; ++i) Fl[i] = FRC[i];
+  M::template jac<JR>(yl, Fl, FRC[M::NS], RowAcc<JR, M::N + 1>{A});
 }
 
 // The group-distributed part of a length-N vector (element i in sub-lane i % G, slot i / G).
@@ -98,16 +117,114 @@ __device__ __forceinline__ double group_max(double v, unsigned gm) {
   return v;
 }
 
+// Sum over elements 0..NV-1, element i in lane i of the cell's lanes, in the order that a group of S
+// lanes adds them: sub-lane s of S takes elements s, s + S, ... in turn, then the S partial sums meet
+// by xor shuffles (S = 1: one sequential sum). Lets a wider group of lanes repeat a narrower
+// mapping's bits. lane_dot accumulates a_i b_i with multiply-adds.
+template <int NV, int S>
+__device__ __noinline__ double lane_dot(double a, double b, unsigned gm, int gbase) {
+  const int s0 = ((threadIdx.x & 31) - gbase) % S;
+  double s = 0.0;
+#pragma unroll 1
+  for (int i = s0, r = 0; r < (NV + S - 1) / S; ++r, i += S) {
+    const double x = __shfl_sync(gm, a, gbase + i), y = __shfl_sync(gm, b, gbase + i);
+    if (i < NV) s = fma(x, y, s);
+  }
+#pragma unroll
+  for (int o = S / 2; o > 0; o >>= 1) s += __shfl_xor_sync(gm, s, o);
+  return s;
+}
+
+// Rate of progress of reaction j with the operations and their order of the unrolled right-hand
+// side (mech/codegen.py): Gibbs sum over products, then reactants, then pressure; the reverse product
+// multiplied into the rate coefficient factor by factor.
+template <class Tab>
+__device__ __forceinline__ double rate_of_progress_unrolled(int j, double T, double invT, double lnT, double lnP0RT,
+                                                            double Ctot, const double* CS, const double* GS,
+                                                            double& Mthird) {
+  const TabRxArr& ar = Tab::rx_arr(j);
+  const TabRxPk pk = Tab::rx_pk(j);
+  const int kind = pk.x & 3u, nr = (pk.x >> 3) & 3u, np = (pk.x >> 5) & 3u;
+  const bool rev = (pk.x >> 2) & 1u;
+  const int dnu = (int)((pk.x >> 7) & 15u) - 8, tbi = (int)((pk.x >> 11) & 2047u) - 1;
+  const int troe = (int)(pk.x >> 22) - 1;
+  auto rs = [&](int s) { return (int)((pk.y >> (10 * s)) & 1023u); };
+  auto ps = [&](int s) { return (int)((pk.z >> (10 * s)) & 1023u); };
+  const double lnkf = fma(ar.beta, lnT, fma(ar.mEaR, invT, ar.lnA));
+  double kf = pgb_exp64(lnkf);
+  double Mc = 1.0;
+  if (tbi >= 0) {
+    const TabThirdBody<double>& tb = Tab::template tb<double>(tbi);
+    Mc = Ctot;
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+      if (e < tb.n) Mc = fma(tb.effm1[e], CS[tb.sp[e]], Mc);
+  }
+  if (kind == 2) {
+    const TabTroe<double>& fo = Tab::template troe<double>(troe);
+    const double lnk0 = fma(fo.beta0, lnT, fma(fo.mEa0R, invT, fo.lnA0));
+    const double Pr = __dmul_rn(Mc, pgb_exp64(lnk0 - lnkf));
+    double blend = pgb_div64(Pr, __dadd_rn(1.0, Pr));
+    if (fo.ntroe > 0) {
+      double Fcent = fma(fo.one_m_a, pgb_exp64(T * fo.m_invT3), __dmul_rn(fo.a, pgb_exp64(T * fo.m_invT1)));
+      if (fo.ntroe > 3) Fcent = __dadd_rn(Fcent, pgb_exp64(invT * fo.m_T2));
+      constexpr double kInvLn10 = 0.43429448190325176;  // 1 / ln 10 as the generator rounds it
+      const double lFc = __dmul_rn(pgb_log64(Fcent), kInvLn10);
+      const double cc = fma(-0.67, lFc, -0.4), nn = fma(-1.27, lFc, 0.75);
+      const double lPr = fma(pgb_log64(fmax(Pr, 1e-300)), kInvLn10, cc);
+      const double f1 = pgb_div64(lPr, fma(-0.14, lPr, nn));
+      blend = __dmul_rn(blend, pgb_exp64(pgb_div64(__dmul_rn(2.302585092994046, lFc), fma(f1, f1, 1.0))));
+    }
+    kf = __dmul_rn(kf, blend);
+  }
+  double Pf = CS[rs(0)];
+#pragma unroll
+  for (int s = 1; s < 3; ++s)
+    if (s < nr) Pf = __dmul_rn(Pf, CS[rs(s)]);
+  double q;
+  if (rev) {
+    double dG = 0.0;
+    bool first = true;
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+      const int n = side ? nr : np;
+#pragma unroll
+      for (int s = 0; s < 3; ++s) {
+        if (s >= n) continue;
+        const int k = side ? rs(s) : ps(s);
+        if (s > 0 && (side ? rs(s - 1) : ps(s - 1)) == k) continue;  // counted with its first slot
+        double nu = side ? -1.0 : 1.0;
+        if (s + 1 < n && (side ? rs(s + 1) : ps(s + 1)) == k) nu += nu;
+        dG = first ? __dmul_rn(nu, GS[k]) : fma(nu, GS[k], dG);
+        first = false;
+      }
+    }
+    if (dnu != 0) dG = fma(-(double)dnu, lnP0RT, dG);
+    double kr = -__dmul_rn(kf, pgb_exp64(fmin(dG, 700.0)));  // finite: an absent product gives 0, not NaN
+#pragma unroll
+    for (int s = 0; s < 3; ++s)
+      if (s < np) kr = __dmul_rn(kr, CS[ps(s)]);
+    q = fma(kf, Pf, kr);
+  } else {
+    q = __dmul_rn(kf, Pf);
+  }
+  Mthird = kind == 1 ? Mc : 1.0;
+  return q;
+}
+
 // Right-hand side f = [W_k wdot_k + F_k, dT/dt] at y for one cell, its group of G lanes
-// cooperating (the equations of warp_rhs with G lanes in place of 32). Inlined: the kernel calls
-// it from one place, so inlining adds no copy and removes the call's register save and restore
-// (measured: no spills left, +5 %).
-template <class M, int G>
+// cooperating (the equations of warp_rhs with G lanes in place of 32), every sum over species in the
+// order of S lanes. Inlined: the kernel calls it from one place, so inlining adds no copy and
+// removes the call's register save and restore (measured: no spills left, +5 %).
+template <class M, int G, int S>
 __device__ __forceinline__ GVec<M, G> group_rhs(const GVec<M, G> yv, double* CS, double* GS, double* QS,
                                              const double* FRC) {
   using Tab = typename M::TabG;
   constexpr int N = M::N, NS = M::NS, NR = M::NR;
   constexpr int R = (N + G - 1) / G;
+  constexpr bool UNROLLED = !M::RHS_TABLE;  // bits of the unrolled per-thread code
+  static_assert(S == G || R == 1, "another summation order needs an element per lane");
+  static_assert(!UNROLLED || S == 1, "the unrolled code sums in sequence");
   const int lane = threadIdx.x & 31, sub = lane % G, gbase = lane - sub;
   const unsigned gm = group_mask<G>();
   auto idx = [&](int r) { return sub + G * r; };
@@ -115,54 +232,104 @@ __device__ __forceinline__ GVec<M, G> group_rhs(const GVec<M, G> yv, double* CS,
   GVec<M, G> fv;
   double (&f)[R] = fv.v;
   const double T = __shfl_sync(gm, y[NS / G], gbase + NS % G);
-  const double invT = 1.0 / T;
+  const double invT = pgb_div64(1.0, T);
   const double lnT = pgb_log64(T);
   const double lnT1 = 1.0 - lnT;
   const double lnP0RT = kLnP0OverR - lnT;
-  double c_loc = 0.0;
+  double c_loc = 0.0, c_fac = 1.0;
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     const int k = idx(r);
     if (k < NS) {
-      const TabSpecies<double>& s = Tab::template sp<double>(k);
-      const double c = y[r] * s.invW;
+      double invW, Tmid;
+      bool fused = false;
+      const double* g;
+      if constexpr (UNROLLED) {
+        const TabUnrolled& s = Tab::un(k);
+        invW = s.invW;
+        Tmid = s.Tmid;
+        fused = s.only_total != 0;
+        g = T < Tmid ? s.glo : s.ghi;
+      } else {
+        const TabSpecies<double>& s = Tab::template sp<double>(k);
+        invW = s.invW;
+        Tmid = s.Tmid;
+        g = T < Tmid ? s.glo : s.ghi;
+      }
+      const double c = y[r] * invW;
       CS[k] = c;
       c_loc += c;
-      const double* g = T < s.Tmid ? s.glo : s.ghi;
+      if (fused) { c_loc = y[r]; c_fac = invW; }
       GS[k] = fma(g[0], lnT1, fma(T, fma(T, fma(T, fma(T, g[4], g[3]), g[2]), g[1]), fma(g[5], invT, g[6])));
     }
   }
-  const double Ctot = group_sum<G>(c_loc, gm);
+  double Ctot;
+  if constexpr (S == G) Ctot = group_sum<G>(c_loc, gm);
+  else Ctot = lane_dot<NS, S>(c_loc, c_fac, gm, gbase);
   __syncwarp(gm);
+#pragma unroll 1
   for (int j = sub; j < NR; j += G) {
-    QS[j] = rate_of_progress<Tab>(j, T, invT, lnT, lnP0RT, Ctot, CS, GS);
+    if constexpr (UNROLLED) QS[j] = rate_of_progress_unrolled<Tab>(j, T, invT, lnT, lnP0RT, Ctot, CS, GS, QS[NR + j]);
+    else QS[j] = rate_of_progress<Tab>(j, T, invT, lnT, lnP0RT, Ctot, CS, GS);
   }
   __syncwarp(gm);
-  double hs = 0.0, rcp = 0.0;
+  double hs = 0.0, rcp = 0.0, h_one = 0.0, cp_one = 0.0, c_one = 0.0;
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     const int k = idx(r);
     f[r] = 0.0;
     if (k < NS) {
       double wdot = 0.0;
-      const int e1 = Tab::sprx_end(k);
+      if constexpr (UNROLLED) {
+        const TabUnrolled& s = Tab::un(k);
+        const int e1 = Tab::un_begin(k + 1);
+        // the compiler fuses the product q [M] of the last reaction, if it is a third-body one, into
+        // the sums it enters
+#pragma unroll 2
+        for (int e = Tab::un_begin(k); e < e1; ++e) {
+          const int j = Tab::un_j(e);
+          const double qj = Tab::un_nu(e) * QS[j], mj = QS[NR + j];
+          wdot = Tab::un_m(e) ? fma(qj, mj, wdot) : __dadd_rn(wdot, __dmul_rn(qj, mj));
+        }
+        f[r] = fma(wdot, s.W, FRC[k]);
+        const bool lo = T < s.Tmid;
+        const double* a = lo ? s.clo : s.chi;
+        const double* hc = lo ? s.hlo : s.hhi;
+        h_one = fma(T, fma(T, fma(T, fma(T, hc[4], hc[3]), hc[2]), hc[1]), fma(hc[5], invT, hc[0]));
+        cp_one = fma(T, fma(T, fma(T, fma(T, a[4], a[3]), a[2]), a[1]), a[0]);
+        c_one = y[r];
+      } else {
+        const int e1 = Tab::sprx_end(k);
 #pragma unroll 4
-      for (int e = Tab::sprx_begin(k); e < e1; ++e) wdot = fma(Tab::sprx_nu(e), QS[Tab::sprx_j(e)], wdot);
-      const TabSpecies<double>& s = Tab::template sp<double>(k);
-      const double wm = fma(wdot, s.W, FRC[k]);
-      f[r] = wm;
-      const bool lo = T < s.Tmid;
-      const double* a = lo ? s.lo : s.hi;
-      const double* hc = lo ? s.hlo : s.hhi;
-      const double hRT = fma(T, fma(T, fma(T, fma(T, hc[4], hc[3]), hc[2]), hc[1]), fma(hc[5], invT, hc[0]));
-      const double cpR = fma(T, fma(T, fma(T, fma(T, a[4], a[3]), a[2]), a[1]), a[0]);
-      hs = fma(hRT * s.invW, wm, hs);
-      rcp = fma(y[r] * s.invW, cpR, rcp);
+        for (int e = Tab::sprx_begin(k); e < e1; ++e) wdot = fma(Tab::sprx_nu(e), QS[Tab::sprx_j(e)], wdot);
+        const TabSpecies<double>& s = Tab::template sp<double>(k);
+        const double wm = fma(wdot, s.W, FRC[k]);
+        f[r] = wm;
+        const bool lo = T < s.Tmid;
+        const double* a = lo ? s.lo : s.hi;
+        const double* hc = lo ? s.hlo : s.hhi;
+        const double hRT = fma(T, fma(T, fma(T, fma(T, hc[4], hc[3]), hc[2]), hc[1]), fma(hc[5], invT, hc[0]));
+        const double cpR = fma(T, fma(T, fma(T, fma(T, a[4], a[3]), a[2]), a[1]), a[0]);
+        if constexpr (S == G) {
+          hs = fma(hRT * s.invW, wm, hs);
+          rcp = fma(y[r] * s.invW, cpR, rcp);
+        } else {
+          h_one = hRT * s.invW;
+          cp_one = cpR;
+          c_one = y[r] * s.invW;
+        }
+      }
     }
   }
-  hs = group_sum<G>(hs, gm);
-  rcp = group_sum<G>(rcp, gm);
-  const double fT = fma(-hs, kRerg * T, FRC[NS]) / (rcp * kRerg);
+  if constexpr (S == G) {
+    hs = group_sum<G>(hs, gm);
+    rcp = group_sum<G>(rcp, gm);
+  } else {
+    hs = lane_dot<NS, S>(h_one, f[0], gm, gbase);
+    rcp = lane_dot<NS, S>(c_one, cp_one, gm, gbase);
+  }
+  if constexpr (!UNROLLED) rcp *= kRerg;
+  const double fT = pgb_div64(fma(-hs, kRerg * T, FRC[NS]), rcp);
 #pragma unroll
   for (int r = 0; r < R; ++r)
     if (idx(r) == NS) f[r] = fT;
@@ -170,7 +337,7 @@ __device__ __forceinline__ GVec<M, G> group_rhs(const GVec<M, G> yv, double* CS,
   return fv;
 }
 
-template <class M, class JR, int G, int WPB>
+template <class M, class JR, int G, int WPB, int S = G>
 __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParams P) {
   using namespace bdf;
   using Tab = typename M::TabG;
@@ -181,6 +348,10 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
   constexpr int CPW = 32 / G;         // cells per warp
   constexpr bool MIXED = sizeof(JR) == sizeof(float);
   constexpr int RW = (N + 31) / 32;   // slots of the warp-wide setup vector
+  // mechanisms whose per-thread kernel runs unrolled code: same bits here (its Jacobian evaluated by
+  // one lane, its orders of summation)
+  constexpr bool UNROLLED = !M::RHS_TABLE;
+  static_assert(!UNROLLED || (S == 1 && R == 1), "an element per lane, summed in sequence");
   extern __shared__ __align__(16) unsigned char gsmem[];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int sub = lane % G, grp = lane / G, gbase = lane - sub;
@@ -220,7 +391,8 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
   auto Z = [&](int j, int r) -> double& { return C.Z[j * N + idx(r)]; };
 
   // ---- per-group state (scalars replicated in the group's lanes; vectors distributed) ----
-  int phase = NEED;
+  // a small launch spreads its cells over the SMs: the first P.cells_per_warp groups of a warp work
+  int phase = P.cells_per_warp > 0 && grp >= P.cells_per_warp ? IDLE : NEED;
   long long cell = -1;
   int box = 0, ci = 0, cj = 0, ck = 0;
   double y[R], acor[R], ewt[R];
@@ -235,11 +407,16 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
   for (int r = 0; r < R; ++r) { y[r] = 0.0; acor[r] = 0.0; ewt[r] = 1.0; }
 
   auto wms = [&](const double (&v)[R]) -> double {  // squared WRMS norm
-    double s = 0.0;
+    if constexpr (S != G) {
+      const double x = v[0] * ewt[0];
+      return lane_dot<N, S>(x, x, gm, gbase) * (1.0 / N);
+    } else {
+      double s = 0.0;
 #pragma unroll
-    for (int r = 0; r < R; ++r)
-      if (idx(r) < N) { const double x = v[r] * ewt[r]; s = fma(x, x, s); }
-    return group_sum<G>(s, gm) * (1.0 / N);
+      for (int r = 0; r < R; ++r)
+        if (idx(r) < N) { const double x = v[r] * ewt[r]; s = fma(x, x, s); }
+      return group_sum<G>(s, gm) * (1.0 / N);
+    }
   };
   auto set_ewt = [&]() {
 #pragma unroll
@@ -401,7 +578,23 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
     __syncwarp(gm);
 #pragma unroll
     for (int r = 0; r < R; ++r) x[r] = idx(r) < N ? C.XS[C.PIV[idx(r)]] : JR(0);
-    lu_substitute<N, G>(C.A, gm, gbase, x);
+    if constexpr (UNROLLED) {
+      // the per-thread kernel's order: rows from the last up, each a sum over ascending columns
+      lu_substitute<N, G, JR, false>(C.A, gm, gbase, x);
+      if (idx(0) < N) C.XS[idx(0)] = x[0];
+      __syncwarp(gm);
+      JR xs[N];
+#pragma unroll
+      for (int k = N - 1; k >= 0; --k) {
+        JR v = C.XS[k];
+#pragma unroll
+        for (int j = k + 1; j < N; ++j) v = fma(-C.A[k * LDA + j], xs[j], v);
+        xs[k] = v * C.A[k * LDA + k];
+        if (k == idx(0)) x[0] = xs[k];
+      }
+    } else {
+      lu_substitute<N, G>(C.A, gm, gbase, x);
+    }
 #pragma unroll
     for (int r = 0; r < R; ++r)
       if (idx(r) < N) b[r] = (double)x[r];
@@ -414,20 +607,20 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
   };
   auto add_stats = [&](bool retried) {
     if (sub != 0) return;
-    ReactStats* S = P.stats;
-    atomicAdd(&S->nst, (unsigned long long)nst);
-    atomicAdd(&S->nfe, (unsigned long long)nfe);
-    atomicAdd(&S->nje, (unsigned long long)nje);
-    atomicAdd(&S->netf, (unsigned long long)netf);
-    atomicAdd(&S->ncfn, (unsigned long long)ncfn);
+    ReactStats* T = P.stats;
+    atomicAdd(&T->nst, (unsigned long long)nst);
+    atomicAdd(&T->nfe, (unsigned long long)nfe);
+    atomicAdd(&T->nje, (unsigned long long)nje);
+    atomicAdd(&T->netf, (unsigned long long)netf);
+    atomicAdd(&T->ncfn, (unsigned long long)ncfn);
     if (retried) {
-      atomicAdd(&S->nretry, 1ull);
+      atomicAdd(&T->nretry, 1ull);
       return;
     }
-    if (status != OK) atomicAdd(&S->nfail, 1ull);
-    atomicMax(&S->max_nst, (unsigned long long)nst);
+    if (status != OK) atomicAdd(&T->nfail, 1ull);
+    atomicMax(&T->max_nst, (unsigned long long)nst);
     const int bin = min(15, 31 - __clz(max(nst, 1)));
-    atomicAdd(&S->hist[bin], 1ull);
+    atomicAdd(&T->hist[bin], 1ull);
   };
   auto finish_cell = [&]() {
     const BoxDev& B = P.boxes[box];
@@ -591,7 +784,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
       GVec<M, G> yv;
 #pragma unroll
       for (int r = 0; r < R; ++r) yv.v[r] = y[r];
-      const GVec<M, G> fv = group_rhs<M, G>(yv, C.CS, C.GS, C.QS, C.FRC);
+      const GVec<M, G> fv = group_rhs<M, G, S>(yv, C.CS, C.GS, C.QS, C.FRC);
 #pragma unroll
       for (int r = 0; r < R; ++r) f[r] = fv.v[r];
       ++nfe;
@@ -604,25 +797,37 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
     // by the whole warp (cells that start a Newton iteration with a stale or missing matrix)
     __syncwarp();
     {
-      unsigned todo = __ballot_sync(0xffffffffu, sub == 0 && phase == NEWTON && m == 0 && need_setup);
+      const bool wanted = phase == NEWTON && m == 0 && need_setup;
+      unsigned todo = __ballot_sync(0xffffffffu, sub == 0 && wanted);
+      if constexpr (UNROLLED) {
+        if (wanted && idx(0) < N) C.CS[idx(0)] = y[0];  // the RHS scratch is free
+        __syncwarp();
+        if (wanted && sub == 0) unrolled_jacobian<M>(C.CS, C.FRC, C.A);
+        __syncwarp();
+      }
       while (todo) {
         const int g = (__ffs(todo) - 1) / G;
         todo &= todo - 1;
-        if (grp == g) {
-#pragma unroll
-          for (int r = 0; r < R; ++r)
-            if (idx(r) < N) YS[idx(r)] = y[r];
-        }
-        __syncwarp();
-        WVec<M> yv;
-#pragma unroll
-        for (int s = 0; s < RW; ++s) {
-          const int i = lane + 32 * s;
-          yv.v[s] = i < N ? YS[i] : 0.0;
-        }
         const double gam = __shfl_sync(0xffffffffu, gamma, g * G);
         const CellMem Cg = cell_mem(g);
-        const bool ok = warp_setup<M, JR>(yv, gam, Cg.FRC, Cg.A, WXS, WRX, WTH, Cg.PIV);
+        bool ok;
+        if constexpr (UNROLLED) {
+          ok = warp_lu_factor<N>(Cg.A, Cg.PIV, (JR)gam);
+        } else {
+          if (grp == g) {
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+              if (idx(r) < N) YS[idx(r)] = y[r];
+          }
+          __syncwarp();
+          WVec<M> yv;
+#pragma unroll
+          for (int s = 0; s < RW; ++s) {
+            const int i = lane + 32 * s;
+            yv.v[s] = i < N ? YS[i] : 0.0;
+          }
+          ok = warp_setup<M, JR>(yv, gam, Cg.FRC, Cg.A, WXS, WRX, WTH, Cg.PIV);
+        }
         __syncwarp();
         if (grp == g) {
           setup_ok = ok;
@@ -817,8 +1022,16 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
                   for (int k = 0; k < q; ++k) hrp *= hr;  // (h / tau2)^(q+1)
                   const double cquot = pgb_div64(tq5, tq5_saved) * hrp;
                   double tv[R];
+                  // the order test's difference: a group of 8 rounds the product of elements 8..15 and
+                  // fuses the others (as the compiler chose when this was one expression; kept, so
+                  // that every width of group takes the same steps)
 #pragma unroll
-                  for (int r = 0; r < R; ++r) tv[r] = idx(r) < N ? acor[r] - cquot * Z(QMAX + 1, r) : 0.0;
+                  for (int r = 0; r < R; ++r) {
+                    const double saved = idx(r) < N ? Z(QMAX + 1, r) : 0.0;
+                    if (S == 1) tv[r] = fma(-cquot, saved, acor[r]);
+                    else if (idx(r) / S == 1) tv[r] = __dsub_rn(acor[r], __dmul_rn(cquot, saved));
+                    else tv[r] = fma(-cquot, saved, acor[r]);
+                  }
                   const double dup2 = wms(tv) * (tq3 * tq3);
                   etaqp1 = pgb_div64(1.0, pgb_pow64((BIAS3 * BIAS3) * dup2, 0.5 * inv_int(q + 2)) + ADDON);
                 }

@@ -444,236 +444,238 @@ __device__ __forceinline__ bool warp_lu_factor(JR* A, int* PIV, const JR g) {
   else return warp_lu_factor_shared<N>(A, PIV, g);
 }
 
-// Jacobian (equations of jac_table, mech_tables.cuh) and partial-pivot LU of I - gamma J in
-// shared memory, one warp cooperating. False: singular. With FACTOR false it stops after the
-// Jacobian, which A then holds (the diagnostic entry point). Inlined: each kernel calls it from
-// one place, so inlining adds no copy and removes the call's register save and restore
-// (measured: lane-group kernel +5 %, warp kernel +1 %).
-template <class M, class JR, bool FACTOR = true>
-__device__ __forceinline__ bool warp_setup(const WVec<M> yv, const double gamma, const double* FRC, JR* A,
-                                        JR* XS, JR* RX, JR* TH, int* PIV) {
+// Jacobian (equations of jac_table, mech_tables.cuh) into A, one warp cooperating. Inlined: each
+// kernel calls it from one place, so inlining adds no copy and removes the call's register save and
+// restore (measured: 1 to 3 %).
+template <class M, class JR>
+__device__ __forceinline__ void warp_jacobian(const WVec<M> yv, const double* FRC, JR* A, JR* XS, JR* RX, JR* TH) {
   using Tab = typename M::TabG;
   constexpr int N = M::N, NS = M::NS, NR = M::NR;
   constexpr int R = (N + 31) / 32;
   constexpr int LDA = N + 1;
   const int lane = threadIdx.x & 31;
+  const double (&y)[R] = yv.v;
   auto idx = [&](int r) { return lane + 32 * r; };
   auto bcast = [&](const double (&v)[R], int i) -> double {
     return __shfl_sync(0xffffffffu, v[i >> 5], i & 31);
   };
-  auto jacobian = [&](const double (&y)[R]) {
-    using namespace jac_detail;
-    const JR T = (JR)bcast(y, NS);
-    const JR invT = JR(1) / T;
-    const JR lnT = pgb_logT<JR>(T);
-    const JR lnT1 = JR(1) - lnT;
-    const JR lnP0RT = JR(kLnP0OverR) - lnT;
-    const JR RT = JR(kRerg) * T;
-    // per species, once: concentration (the solve vector is free during the setup) and the
-    // NASA-7 terms g/RT, h/RT, cp/R, d(cp/R)/dT that the reaction and energy terms reuse
-    JR* TG = TH;
-    JR* TH_ = TH + NS;
-    JR* TC = TH + 2 * NS;
-    JR* TD = TH + 3 * NS;
-    JR c_loc = JR(0);
+  using namespace jac_detail;
+  const JR T = (JR)bcast(y, NS);
+  const JR invT = JR(1) / T;
+  const JR lnT = pgb_logT<JR>(T);
+  const JR lnT1 = JR(1) - lnT;
+  const JR lnP0RT = JR(kLnP0OverR) - lnT;
+  const JR RT = JR(kRerg) * T;
+  // per species, once: concentration (the solve vector is free during the setup) and the
+  // NASA-7 terms g/RT, h/RT, cp/R, d(cp/R)/dT that the reaction and energy terms reuse
+  JR* TG = TH;
+  JR* TH_ = TH + NS;
+  JR* TC = TH + 2 * NS;
+  JR* TD = TH + 3 * NS;
+  JR c_loc = JR(0);
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int k = idx(r);
-      if (k < NS) {
-        const JR c = (JR)y[r] * Tab::template sp<JR>(k).invW;
-        XS[k] = c;
-        c_loc += c;
-        JR g, h, cp, d;
-        nasa<JR>(Tab::template sp<JR>(k), T, invT, lnT1, g, h, cp, d);
-        TG[k] = g;
-        TH_[k] = h;
-        TC[k] = cp;
-        TD[k] = d;
-      }
+  for (int r = 0; r < R; ++r) {
+    const int k = idx(r);
+    if (k < NS) {
+      const JR c = (JR)y[r] * Tab::template sp<JR>(k).invW;
+      XS[k] = c;
+      c_loc += c;
+      JR g, h, cp, d;
+      nasa<JR>(Tab::template sp<JR>(k), T, invT, lnT1, g, h, cp, d);
+      TG[k] = g;
+      TH_[k] = h;
+      TC[k] = cp;
+      TD[k] = d;
     }
-    const JR Ctot = warp_sum(c_loc);
-    for (int e = lane; e < N * LDA; e += 32) A[e] = JR(0);
-    __syncwarp();
-    // (1) per-reaction partials, lanes over reactions; energy-closure sums
-    JR Qw = JR(0), cpw = JR(0);
-    for (int j = lane; j < NR; j += 32) {
-      const TabReaction<JR>& r = Tab::template rx<JR>(j);
-      const JR lnkinf = r.beta * lnT + r.mEaR * invT + r.lnA;
-      JR dlnkf = (r.beta - r.mEaR * invT) * invT;
-      JR kf = pgb_expT<JR>(lnkinf);
-      JR Mc = JR(1), alpha = JR(1), dkeff_dM = JR(0);
-      if (r.tb >= 0) {
-        const TabThirdBody<JR>& t = Tab::template tb<JR>(r.tb);
-        Mc = Ctot;
+  }
+  const JR Ctot = warp_sum(c_loc);
+  for (int e = lane; e < N * LDA; e += 32) A[e] = JR(0);
+  __syncwarp();
+  // (1) per-reaction partials, lanes over reactions; energy-closure sums
+  JR Qw = JR(0), cpw = JR(0);
+  for (int j = lane; j < NR; j += 32) {
+    const TabReaction<JR>& r = Tab::template rx<JR>(j);
+    const JR lnkinf = r.beta * lnT + r.mEaR * invT + r.lnA;
+    JR dlnkf = (r.beta - r.mEaR * invT) * invT;
+    JR kf = pgb_expT<JR>(lnkinf);
+    JR Mc = JR(1), alpha = JR(1), dkeff_dM = JR(0);
+    if (r.tb >= 0) {
+      const TabThirdBody<JR>& t = Tab::template tb<JR>(r.tb);
+      Mc = Ctot;
 #pragma unroll
-        for (int e = 0; e < 8; ++e)
-          if (e < t.n) Mc += t.effm1[e] * XS[t.sp[e]];
-        if (r.kind == 1) alpha = Mc;
-      }
-      if (r.kind == 2) {
-        const TabTroe<JR>& fo = Tab::template troe<JR>(r.troe);
-        const JR lnk0 = fo.beta0 * lnT + fo.mEa0R * invT + fo.lnA0;
-        const JR dlnk0 = (fo.beta0 - fo.mEa0R * invT) * invT;
-        const JR k0 = pgb_expT<JR>(lnk0);
-        const JR Pr = Mc * pgb_expT<JR>(lnk0 - lnkinf);
-        JR Fb = JR(1);
-        if (fo.ntroe > 0) {
-          JR Fcent = fo.one_m_a * pgb_expT<JR>(T * fo.m_invT3) + fo.a * pgb_expT<JR>(T * fo.m_invT1);
-          if (fo.ntroe > 3) Fcent += pgb_expT<JR>(fo.m_T2 * invT);
-          const JR lFc = pgb_logT<JR>(Fcent) * JR(0.4342944819032518);
-          const JR cc = JR(-0.4) - JR(0.67) * lFc, nn = JR(0.75) - JR(1.27) * lFc;
-          const JR lPr = pgb_logT<JR>(Pr > JR(1e-30) ? Pr : JR(1e-30)) * JR(0.4342944819032518) + cc;
-          const JR f1 = lPr / (nn - JR(0.14) * lPr);
-          Fb = pgb_expT<JR>(JR(2.302585092994046) * lFc / (JR(1) + f1 * f1));
-        }
-        const JR onePr = JR(1) + Pr;
-        kf = kf * Pr / onePr * Fb;
-        dkeff_dM = Fb * k0 / (onePr * onePr);
-        dlnkf = dlnkf + (dlnk0 - dlnkf) / onePr;
-      }
-      JR cr[3], cp[3];
-#pragma unroll
-      for (int s = 0; s < 3; ++s) {
-        cr[s] = s < r.nr ? XS[r.rs[s]] : JR(1);
-        cp[s] = s < r.np ? XS[r.ps[s]] : JR(1);
-      }
-      const JR Pf = cr[0] * cr[1] * cr[2];
-      const JR Pp = cp[0] * cp[1] * cp[2];
-      JR kr = JR(0), dlnkr = JR(0);
-      if (r.rev) {
-        JR dG = -(JR)r.dnu * lnP0RT, dH = JR(0);
-#pragma unroll
-        for (int s = 0; s < 3; ++s)
-          if (s < r.np) {
-            dG += TG[r.ps[s]];
-            dH += TH_[r.ps[s]];
-          }
-#pragma unroll
-        for (int s = 0; s < 3; ++s)
-          if (s < r.nr) {
-            dG -= TG[r.rs[s]];
-            dH -= TH_[r.rs[s]];
-          }
-        kr = kf * pgb_expT<JR>(fmin(dG, JR(700)));
-        dlnkr = dlnkf - (dH - (JR)r.dnu) * invT;
-      }
-      const JR q = alpha * (kf * Pf - kr * Pp);
-      JR* out = RX + j * wbdf::RXW;
-      out[0] = alpha * (kf * dlnkf * Pf - kr * dlnkr * Pp);
-#pragma unroll
-      for (int s = 0; s < 3; ++s) {
-        out[1 + s] = alpha * kf * (s == 0 ? cr[1] * cr[2] : s == 1 ? cr[0] * cr[2] : cr[0] * cr[1]);
-        out[4 + s] = -alpha * kr * (s == 0 ? cp[1] * cp[2] : s == 1 ? cp[0] * cp[2] : cp[0] * cp[1]);
-      }
-      JR bm = JR(0);
-      if (r.kind == 1) bm = kf * Pf - kr * Pp;
-      else if (r.kind == 2) bm = dkeff_dM * (Pf - (kf > JR(0) ? kr / kf : JR(0)) * Pp);
-      out[7] = bm;
-      if (r.tb >= 0) {  // the collider terms of the listed species read these
-        const TabThirdBody<JR>& t = Tab::template tb<JR>(r.tb);
-        JR* ox = RX + Tab::jac_x0(r.tb);
-#pragma unroll
-        for (int e = 0; e < 8; ++e)
-          if (e < t.n) ox[e] = bm * (JR(1) + t.effm1[e]);
-      }
-#pragma unroll
-      for (int row = 0; row < 6; ++row)
-        if (row < r.nr + r.np) {
-          const bool isr = row < r.nr;
-          const int i = isr ? r.rs[row] : r.ps[row - r.nr];
-          Qw += (isr ? -q : q) * TH_[i] * RT;
-          cpw += (isr ? -q : q) * TC[i] * JR(kRerg);
-        }
+      for (int e = 0; e < 8; ++e)
+        if (e < t.n) Mc += t.effm1[e] * XS[t.sp[e]];
+      if (r.kind == 1) alpha = Mc;
     }
-    Qw = warp_sum(Qw);
-    cpw = warp_sum(cpw);
-    __syncwarp();
-    // (2) assembly by the generated contribution program: each lane owns whole entries A[i][k]
-    // (species rows; k = NS: the T column) and sums their terms in a register, in the order of
-    // the reaction walk (reactions ascending, then row slots): a term of reaction j is c v,
-    // c = -+W_i / W_k (-+W_i in the T column) and v the partials of j that land in column k
-    // (dq/dT in the T column). The lanes' 4-byte term codes are interleaved in the table (one
-    // contiguous line per warp load); each entry has one writer, so the result does not depend
-    // on the lane schedule.
-    // A lane reads four terms per 16-byte load, one load ahead, and an entry's coefficient and
-    // target one entry ahead: with shared memory taking almost all of the L1, each of these loads
-    // is an L2 round trip, and a load per term made the program the setup's longest part.
-    {
-      JR acc = JR(0);
-      int ent = lane;
-      TabJacEnt<JR> cur = Tab::template jac_ent<JR>(ent), ahead = Tab::template jac_ent<JR>(ent + 32);
-      uint4 quad = Tab::jac_quad(lane);
+    if (r.kind == 2) {
+      const TabTroe<JR>& fo = Tab::template troe<JR>(r.troe);
+      const JR lnk0 = fo.beta0 * lnT + fo.mEa0R * invT + fo.lnA0;
+      const JR dlnk0 = (fo.beta0 - fo.mEa0R * invT) * invT;
+      const JR k0 = pgb_expT<JR>(lnk0);
+      const JR Pr = Mc * pgb_expT<JR>(lnk0 - lnkinf);
+      JR Fb = JR(1);
+      if (fo.ntroe > 0) {
+        JR Fcent = fo.one_m_a * pgb_expT<JR>(T * fo.m_invT3) + fo.a * pgb_expT<JR>(T * fo.m_invT1);
+        if (fo.ntroe > 3) Fcent += pgb_expT<JR>(fo.m_T2 * invT);
+        const JR lFc = pgb_logT<JR>(Fcent) * JR(0.4342944819032518);
+        const JR cc = JR(-0.4) - JR(0.67) * lFc, nn = JR(0.75) - JR(1.27) * lFc;
+        const JR lPr = pgb_logT<JR>(Pr > JR(1e-30) ? Pr : JR(1e-30)) * JR(0.4342944819032518) + cc;
+        const JR f1 = lPr / (nn - JR(0.14) * lPr);
+        Fb = pgb_expT<JR>(JR(2.302585092994046) * lFc / (JR(1) + f1 * f1));
+      }
+      const JR onePr = JR(1) + Pr;
+      kf = kf * Pr / onePr * Fb;
+      dkeff_dM = Fb * k0 / (onePr * onePr);
+      dlnkf = dlnkf + (dlnk0 - dlnkf) / onePr;
+    }
+    JR cr[3], cp[3];
+#pragma unroll
+    for (int s = 0; s < 3; ++s) {
+      cr[s] = s < r.nr ? XS[r.rs[s]] : JR(1);
+      cp[s] = s < r.np ? XS[r.ps[s]] : JR(1);
+    }
+    const JR Pf = cr[0] * cr[1] * cr[2];
+    const JR Pp = cp[0] * cp[1] * cp[2];
+    JR kr = JR(0), dlnkr = JR(0);
+    if (r.rev) {
+      JR dG = -(JR)r.dnu * lnP0RT, dH = JR(0);
+#pragma unroll
+      for (int s = 0; s < 3; ++s)
+        if (s < r.np) {
+          dG += TG[r.ps[s]];
+          dH += TH_[r.ps[s]];
+        }
+#pragma unroll
+      for (int s = 0; s < 3; ++s)
+        if (s < r.nr) {
+          dG -= TG[r.rs[s]];
+          dH -= TH_[r.rs[s]];
+        }
+      kr = kf * pgb_expT<JR>(fmin(dG, JR(700)));
+      dlnkr = dlnkf - (dH - (JR)r.dnu) * invT;
+    }
+    const JR q = alpha * (kf * Pf - kr * Pp);
+    JR* out = RX + j * wbdf::RXW;
+    out[0] = alpha * (kf * dlnkf * Pf - kr * dlnkr * Pp);
+#pragma unroll
+    for (int s = 0; s < 3; ++s) {
+      out[1 + s] = alpha * kf * (s == 0 ? cr[1] * cr[2] : s == 1 ? cr[0] * cr[2] : cr[0] * cr[1]);
+      out[4 + s] = -alpha * kr * (s == 0 ? cp[1] * cp[2] : s == 1 ? cp[0] * cp[2] : cp[0] * cp[1]);
+    }
+    JR bm = JR(0);
+    if (r.kind == 1) bm = kf * Pf - kr * Pp;
+    else if (r.kind == 2) bm = dkeff_dM * (Pf - (kf > JR(0) ? kr / kf : JR(0)) * Pp);
+    out[7] = bm;
+    if (r.tb >= 0) {  // the collider terms of the listed species read these
+      const TabThirdBody<JR>& t = Tab::template tb<JR>(r.tb);
+      JR* ox = RX + Tab::jac_x0(r.tb);
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        if (e < t.n) ox[e] = bm * (JR(1) + t.effm1[e]);
+    }
+#pragma unroll
+    for (int row = 0; row < 6; ++row)
+      if (row < r.nr + r.np) {
+        const bool isr = row < r.nr;
+        const int i = isr ? r.rs[row] : r.ps[row - r.nr];
+        Qw += (isr ? -q : q) * TH_[i] * RT;
+        cpw += (isr ? -q : q) * TC[i] * JR(kRerg);
+      }
+  }
+  Qw = warp_sum(Qw);
+  cpw = warp_sum(cpw);
+  __syncwarp();
+  // (2) assembly by the generated contribution program: each lane owns whole entries A[i][k]
+  // (species rows; k = NS: the T column) and sums their terms in a register, in the order of
+  // the reaction walk (reactions ascending, then row slots): a term of reaction j is c v,
+  // c = -+W_i / W_k (-+W_i in the T column) and v the partials of j that land in column k
+  // (dq/dT in the T column). The lanes' 4-byte term codes are interleaved in the table (one
+  // contiguous line per warp load); each entry has one writer, so the result does not depend
+  // on the lane schedule.
+  // A lane reads four terms per 16-byte load, one load ahead, and an entry's coefficient and
+  // target one entry ahead: with shared memory taking almost all of the L1, each of these loads
+  // is an L2 round trip, and a load per term made the program the setup's longest part.
+  {
+    JR acc = JR(0);
+    int ent = lane;
+    TabJacEnt<JR> cur = Tab::template jac_ent<JR>(ent), ahead = Tab::template jac_ent<JR>(ent + 32);
+    uint4 quad = Tab::jac_quad(lane);
 #pragma unroll 1
-      for (int q = 0; q < Tab::JAC_QUADS; ++q) {
-        const unsigned code[4] = {quad.x, quad.y, quad.z, quad.w};
-        if (q + 1 < Tab::JAC_QUADS) quad = Tab::jac_quad(32 * (q + 1) + lane);
-        JR v[4];
+    for (int q = 0; q < Tab::JAC_QUADS; ++q) {
+      const unsigned code[4] = {quad.x, quad.y, quad.z, quad.w};
+      if (q + 1 < Tab::JAC_QUADS) quad = Tab::jac_quad(32 * (q + 1) + lane);
+      JR v[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) v[u] = RX[code[u] & 0x1fff];
+      for (int u = 0; u < 4; ++u) v[u] = RX[code[u] & 0x1fff];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const unsigned c = code[u];
-          if (c & 0xfe000) {  // species on several slots of the reaction
-            const JR* pj = RX + (c & 0x1ff8);
+      for (int u = 0; u < 4; ++u) {
+        const unsigned c = code[u];
+        if (c & 0xfe000) {  // species on several slots of the reaction
+          const JR* pj = RX + (c & 0x1ff8);
 #pragma unroll
-            for (int s = 1; s < 7; ++s)
-              if (c & (1u << (12 + s))) v[u] += pj[s];
-            if (c & (1u << 19))
-              v[u] = fma(pj[7], (c & (1u << 22)) ? Tab::template jac_eff<JR>(32 * (4 * q + u) + lane) : JR(1), v[u]);
-          }
-          if (not_zero(v[u]) || (c & (1u << 23))) acc = fma(flip_sign(cur.w, c << 11), v[u], acc);
-          if (c & (1u << 21)) {  // last term of the entry
-            A[cur.target] = acc;
-            acc = JR(0);
-            cur = ahead;
-            ent += 32;
-            ahead = Tab::template jac_ent<JR>(min(ent + 32, 32 * (Tab::JAC_ENTS - 1) + lane));
-          }
+          for (int s = 1; s < 7; ++s)
+            if (c & (1u << (12 + s))) v[u] += pj[s];
+          if (c & (1u << 19))
+            v[u] = fma(pj[7], (c & (1u << 22)) ? Tab::template jac_eff<JR>(32 * (4 * q + u) + lane) : JR(1), v[u]);
+        }
+        if (not_zero(v[u]) || (c & (1u << 23))) acc = fma(flip_sign(cur.w, c << 11), v[u], acc);
+        if (c & (1u << 21)) {  // last term of the entry
+          A[cur.target] = acc;
+          acc = JR(0);
+          cur = ahead;
+          ent += 32;
+          ahead = Tab::template jac_ent<JR>(min(ent + 32, 32 * (Tab::JAC_ENTS - 1) + lane));
         }
       }
     }
-    __syncwarp();
-    // (3) constant-pressure energy row: dT/dt = (Fh - sum h_k wm_k) / (rho cp)
-    JR D = JR(0), dD = JR(0), Qf = JR(0), cpf = JR(0);
+  }
+  __syncwarp();
+  // (3) constant-pressure energy row: dT/dt = (Fh - sum h_k wm_k) / (rho cp)
+  JR D = JR(0), dD = JR(0), Qf = JR(0), cpf = JR(0);
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int k = idx(r);
-      if (k < NS) {
-        const JR h = TH_[k], c = TC[k], d = TD[k];
-        const JR iw = Tab::template sp<JR>(k).invW;
-        const JR cpm = c * JR(kRerg) * iw, hm = h * RT * iw;
-        const JR yk = (JR)y[r];
-        const JR fk = (JR)FRC[k];
-        D += yk * cpm;
-        dD += yk * d * JR(kRerg) * iw;
-        Qf -= hm * fk;
-        cpf += cpm * fk;
-      }
+  for (int r = 0; r < R; ++r) {
+    const int k = idx(r);
+    if (k < NS) {
+      const JR h = TH_[k], c = TC[k], d = TD[k];
+      const JR iw = Tab::template sp<JR>(k).invW;
+      const JR cpm = c * JR(kRerg) * iw, hm = h * RT * iw;
+      const JR yk = (JR)y[r];
+      const JR fk = (JR)FRC[k];
+      D += yk * cpm;
+      dD += yk * d * JR(kRerg) * iw;
+      Qf -= hm * fk;
+      cpf += cpm * fk;
     }
-    D = warp_sum(D);
-    dD = warp_sum(dD);
-    const JR Q = (JR)FRC[NS] - Qw + warp_sum(Qf);
-    const JR cpwm = cpw + warp_sum(cpf);
-    const JR invD = JR(1) / D;
-    const JR QD2 = Q * invD * invD;
+  }
+  D = warp_sum(D);
+  dD = warp_sum(dD);
+  const JR Q = (JR)FRC[NS] - Qw + warp_sum(Qf);
+  const JR cpwm = cpw + warp_sum(cpf);
+  const JR invD = JR(1) / D;
+  const JR QD2 = Q * invD * invD;
 #pragma unroll
-    for (int cc = 0; cc < R; ++cc) {
-      const int k = idx(cc);
-      if (k > NS) continue;
-      JR acc = JR(0);
+  for (int cc = 0; cc < R; ++cc) {
+    const int k = idx(cc);
+    if (k > NS) continue;
+    JR acc = JR(0);
 #pragma unroll 1
-      for (int i = 0; i < NS; ++i) acc += TH_[i] * RT * Tab::template sp<JR>(i).invW * A[i * LDA + k];
-      if (k < NS) {
-        A[NS * LDA + k] = -acc * invD - QD2 * TC[k] * JR(kRerg) * Tab::template sp<JR>(k).invW;
-      } else {
-        A[NS * LDA + NS] = -(acc + cpwm) * invD - QD2 * dD;
-      }
+    for (int i = 0; i < NS; ++i) acc += TH_[i] * RT * Tab::template sp<JR>(i).invW * A[i * LDA + k];
+    if (k < NS) {
+      A[NS * LDA + k] = -acc * invD - QD2 * TC[k] * JR(kRerg) * Tab::template sp<JR>(k).invW;
+    } else {
+      A[NS * LDA + NS] = -(acc + cpwm) * invD - QD2 * dD;
     }
-    __syncwarp();
-  };
+  }
+  __syncwarp();
+}
 
-  jacobian(yv.v);
-  if constexpr (FACTOR) return warp_lu_factor<N>(A, PIV, (JR)gamma);
+// The Jacobian and the LU of I - gamma J. False: singular. With FACTOR false it stops after the
+// Jacobian, which A then holds (the diagnostic entry point).
+template <class M, class JR, bool FACTOR = true>
+__device__ __forceinline__ bool warp_setup(const WVec<M> yv, const double gamma, const double* FRC, JR* A,
+                                        JR* XS, JR* RX, JR* TH, int* PIV) {
+  warp_jacobian<M, JR>(yv, FRC, A, XS, RX, TH);
+  if constexpr (FACTOR) return warp_lu_factor<M::N>(A, PIV, (JR)gamma);
   else return true;
 }
 
@@ -681,7 +683,8 @@ __device__ __forceinline__ bool warp_setup(const WVec<M> yv, const double gamma,
 // of the cell's lanes (mask, first lane gbase): the solution moves by shuffles, so a step costs one
 // shuffle and one multiply-add and the matrix loads run ahead of it (the staged shared-memory form
 // waited for a store, a barrier and a load at each step: 200 cycles instead of 40).
-template <int N, int L, class JR>
+// BACK false: the forward half alone.
+template <int N, int L, class JR, bool BACK = true>
 __device__ __forceinline__ void lu_substitute(const JR* A, unsigned mask, int gbase, JR (&x)[(N + L - 1) / L]) {
   constexpr int R = (N + L - 1) / L, LDA = N + 1;
   const int sub = (threadIdx.x & 31) - gbase;
@@ -697,6 +700,7 @@ __device__ __forceinline__ void lu_substitute(const JR* A, unsigned mask, int gb
         if (i > k && i < N) x[r] = fma(-A[i * LDA + k], bk, x[r]);
       }
     }
+  if constexpr (!BACK) return;
 #pragma unroll
   for (int s = R - 1; s >= 0; --s)
 #pragma unroll 2

@@ -60,6 +60,17 @@ struct TabTroe {
   R one_m_a, m_invT3, a, m_invT1, m_T2;
 };
 
+// Constants of one species as the unrolled right-hand side folds them: 1/W, W, Tmid, whether its
+// concentration enters the sum [M] alone (the compiler then fuses its product there), then below /
+// above Tmid g/RT (as glo / ghi), h/RT over W, and cp (erg) over W.
+struct TabUnrolled {
+  double invW, W, Tmid;
+  int only_total;
+  double glo[7], ghi[7];
+  double hlo[6], hhi[6];
+  double clo[5], chi[5];
+};
+
 // One entry of the cooperative Jacobian's contribution program: coefficient magnitude of its
 // terms, and where its sum goes (i (N + 1) + k).
 template <class R>

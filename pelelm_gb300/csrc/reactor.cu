@@ -231,6 +231,7 @@ struct pgb_reactor {
   cudaStream_t last_stream = nullptr;
   int device = 0, nsm = 0;
   SgModel sg;  // loaded when options name a surrogate file
+  bool small_ok = false;  // no option fixes the mapping or its layout: small launches choose theirs
   bool tuned = false;
   std::string tuning;  // autotuner report
 };
@@ -295,9 +296,22 @@ struct LaunchPlan {
   size_t z_bytes = 0, lu_bytes = 0;
   bool warp = false;   // warp-per-cell kernel; tpb then holds warps per block
   bool group = false;  // group-per-cell kernel; tpb then holds lanes per cell
+  bool small = false;  // small-launch kernel; tpb then holds warps per block
+  int cells_per_warp = 0;  // 0: all that the mapping holds
 };
 
 int mapping_of(const pgb_reactor* r);
+
+// Most cells of a launch that goes to the small-launch kernel. Below it the time of a launch is
+// that of its stiffest cell, one FP64 warp instruction after the other (64 cycles each on an SM
+// partition, whatever the lanes), so more lanes per cell shorten it; above it the cells in flight
+// count, and the default mappings do more cells per instruction. Measured, small against default
+// kernel, mixed precision, dt_react 1e-5 s: 9 species 512 cells 9.1 / 29.1 ms, 4096 cells 13.5 / 30.7,
+// 16384 cells 31.8 / 32.0; 21 species 512 cells 7.6 / 22.1, 4096 cells 13.2 / 22.9, 8192 cells
+// 22.6 / 22.9. At 1e-6 s, where cells differ less, the lines lie at about 7,000 and 5,800 cells.
+long long small_limit(const pgb_reactor* r) {
+  return (long long)r->nsm * (r->mech->ns <= 12 ? 48 : 40);
+}
 
 // First layout (all shared; global Nordsieck history; global history and LU) whose shared
 // footprint fits 128 threads per block (the occupancy that measures best), unless options
@@ -307,6 +321,16 @@ int mapping_of(const pgb_reactor* r);
 LaunchPlan plan_launch(const pgb_reactor* r, long long ncell, bool mixed) {
   LaunchPlan pl;
   const MechEntry& m = *r->mech;
+  if (r->small_ok && m.small_mixed && ncell <= small_limit(r)) {
+    // one block per SM, one cell per warp while the SM's twelve warps allow it
+    const int cpw = 32 / m.small_lanes;
+    pl.small = true;
+    pl.nblocks = (int)std::min<long long>(r->nsm, std::max<long long>(1, ncell));
+    const long long per_sm = (std::max<long long>(ncell, 1) + pl.nblocks - 1) / pl.nblocks;
+    pl.cells_per_warp = per_sm <= kSmallWarps ? 1 : cpw;
+    pl.tpb = (int)std::min<long long>(kSmallWarps, (per_sm + pl.cells_per_warp - 1) / pl.cells_per_warp);
+    return pl;
+  }
   if (mapping_of(r) == 2) {
     // lane groups per cell: as many warps per block as fit shared memory, one block per SM
     const int G = r->opt.group;
@@ -417,7 +441,9 @@ int enqueue_advance(pgb_reactor* r, Scratch& s, int nbox, long long ncell, doubl
   const LaunchPlan pl = plan_launch(r, ncell, r->opt.mixed);
   p.lu_scratch = pl.lu_bytes ? s.d_lu : nullptr;
   p.z_scratch = pl.z_bytes ? s.d_z : nullptr;
-  LaunchFn fn = pl.group ? (r->opt.mixed ? r->mech->group_mixed : r->mech->group_fp64)
+  p.cells_per_warp = pl.cells_per_warp;
+  LaunchFn fn = pl.small   ? (r->opt.mixed ? r->mech->small_mixed : r->mech->small_fp64)
+               : pl.group ? (r->opt.mixed ? r->mech->group_mixed : r->mech->group_fp64)
                : pl.warp ? (r->opt.mixed ? r->mech->warp_mixed : r->mech->warp_fp64)
                          : (r->opt.mixed ? r->mech->bdf_mixed : r->mech->bdf_fp64);
   // mixed precision with retry: the cells its pass fails (FP32 Newton matrices can stall where
@@ -442,7 +468,8 @@ int enqueue_advance(pgb_reactor* r, Scratch& s, int nbox, long long ncell, doubl
     q.lu_scratch = p64.lu_bytes ? s.d_lu : nullptr;
     q.z_scratch = p64.z_bytes ? s.d_z : nullptr;
     PGB_CUDA(cudaMemsetAsync(s.d_counter, 0, sizeof(unsigned long long), st));
-    const LaunchFn f64 = p64.group ? r->mech->group_fp64 : p64.warp ? r->mech->warp_fp64 : r->mech->bdf_fp64;
+    q.cells_per_warp = p64.cells_per_warp;
+    const LaunchFn f64 = p64.small ? r->mech->small_fp64 : p64.group ? r->mech->group_fp64 : p64.warp ? r->mech->warp_fp64 : r->mech->bdf_fp64;
     return f64(q, p64.tpb, st, p64.nblocks);
   };
   if (!r->sg.d_net) return run_bdf();
@@ -544,6 +571,7 @@ pgb_reactor* pgb_reactor_create(const char* name, const char* mechanism, int rea
   r->mech = m;
   r->opt = o;
   r->null_reactor = (n == "ReactorNull");
+  r->small_ok = o.mapping < 0 && o.tpb == 0 && o.wpb == 0 && o.group == 8 && o.z_global < 0 && o.lu_global < 0;
   r->device = dev;
   r->nsm = nsm;
   if (!o.surrogate.empty()) {
@@ -645,6 +673,8 @@ int run_autotune(pgb_reactor* r, const std::vector<pgb::BoxDev>& boxes, long lon
   const Options saved = r->opt;
   SgModel sg_saved = r->sg;
   r->sg.d_net = nullptr;  // time the BDF alone
+  const bool small_saved = r->small_ok;
+  r->small_ok = false;  // and the mappings of large launches
   auto fail = [&](const char* what) { rc = set_err("autotune: %s", what); };
   do {
     if (cudaMalloc(&pristine, arena_bytes) != cudaSuccess || cudaMalloc(&work, arena_bytes) != cudaSuccess ||
@@ -711,6 +741,7 @@ int run_autotune(pgb_reactor* r, const std::vector<pgb::BoxDev>& boxes, long lon
   } while (false);
   if (rc) r->opt = saved;
   r->sg = sg_saved;
+  r->small_ok = small_saved;
   cudaStreamSynchronize(st);
   if (pristine) cudaFree(pristine);
   if (work) cudaFree(work);

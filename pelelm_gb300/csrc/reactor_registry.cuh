@@ -164,6 +164,28 @@ int launch_bdf_group(const pgb::ReactParams& p, int G, cudaStream_t s, int nbloc
   return set_err("group BDF: %d lanes per cell are not compiled (4, 8)", G);
 }
 
+// The kernel of small launches: the lane-group kernel with more lanes per cell, in the summation
+// order of the mechanism's large-launch mapping (same bits). Lanes per cell: 16 of the 9-species
+// size (an element and a reaction or two a lane), 32 above.
+template <class M>
+constexpr int small_lanes() {
+  return M::RHS_TABLE ? 32 : 16;
+}
+constexpr int kSmallWarps = 12;  // 168 registers a thread, three warps per SM partition
+
+template <class M, class JR>
+int launch_bdf_small(const pgb::ReactParams& p, int warps, cudaStream_t s, int nblocks) {
+  constexpr int G = small_lanes<M>(), S = M::RHS_TABLE ? 8 : 1;
+  constexpr int per = pgb::gbdf_smem_per_warp<M, JR, G>();
+  constexpr int WPB = kMaxSmemPerBlock / per < kSmallWarps ? kMaxSmemPerBlock / per : kSmallWarps;
+  auto kern = pgb::bdf_group_kernel<M, JR, G, WPB, S>;
+  const int w = std::min(warps, WPB);
+  PGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, WPB * per));
+  kern<<<nblocks, w * 32, w * per, s>>>(p);
+  PGB_CUDA(cudaGetLastError());
+  return 0;
+}
+
 template <class M>
 int launch_null(const pgb::ReactParams& p, cudaStream_t s, int nblocks) {
   pgb::null_reactor_kernel<M><<<nblocks, 256, 0, s>>>(p);
@@ -217,6 +239,8 @@ struct MechEntry {
   LaunchFn group_mixed, group_fp64;  // group-per-cell BDF (argument: lanes per cell, 4 or 8)
   int (*group_cells_mixed)(int), (*group_cells_fp64)(int);  // cells per block for a group size
   int (*newton_fn)(const pgb::NewtonMatrixParams&, int mapping, int fp64, cudaStream_t);  // diagnostic
+  LaunchFn small_mixed, small_fp64;  // small launches (argument: warps per block), or null
+  int small_lanes;                   // their lanes per cell
 };
 
 
@@ -365,7 +389,8 @@ int h2t_entry(const pgb_box_view* v, double tmin, double tmax, cudaStream_t s) {
           ::pgb_host::warp_wpb_choice<M>(2), ::pgb_host::warp_wpb_choice<M>(3)               \
     }                                                                                        \
     , ::pgb_host::heat_release_entry<M>, nullptr, nullptr, nullptr, nullptr,                \
-        ::pgb_host::newton_matrix_entry<M, true>                                             \
+        ::pgb_host::newton_matrix_entry<M, true>, ::pgb_host::launch_bdf_small<M, float>,    \
+        ::pgb_host::launch_bdf_small<M, double>, ::pgb_host::small_lanes<M>()                \
   }
 
 // Mechanisms whose cells also run group-per-cell (the 21-species size): all of the above plus
@@ -390,7 +415,8 @@ int h2t_entry(const pgb_box_view* v, double tmin, double tmax, cudaStream_t s) {
     , ::pgb_host::heat_release_entry<M>, ::pgb_host::launch_bdf_group<M, float>,             \
         ::pgb_host::launch_bdf_group<M, double>, ::pgb_host::group_cells_per_block<M, float>, \
         ::pgb_host::group_cells_per_block<M, double>,                                        \
-        ::pgb_host::newton_matrix_entry<M, true>                                             \
+        ::pgb_host::newton_matrix_entry<M, true>, ::pgb_host::launch_bdf_small<M, float>,    \
+        ::pgb_host::launch_bdf_small<M, double>, ::pgb_host::small_lanes<M>()                \
   }
 
 // Mechanisms too large for one cell per thread: warp-per-cell BDF, ReactorNull and T(h, Y) only.
@@ -406,7 +432,7 @@ int h2t_entry(const pgb_box_view* v, double tmin, double tmax, cudaStream_t s) {
           ::pgb_host::warp_wpb_choice<M>(2), ::pgb_host::warp_wpb_choice<M>(3)               \
     }                                                                                        \
     , ::pgb_host::heat_release_entry<M>, nullptr, nullptr, nullptr, nullptr,                \
-        ::pgb_host::newton_matrix_entry<M, false>                                            \
+        ::pgb_host::newton_matrix_entry<M, false>, nullptr, nullptr, 0                       \
   }
 
 // Converts and validates one box view into its device descriptor; cell numbering of the box

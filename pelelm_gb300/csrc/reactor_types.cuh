@@ -69,6 +69,8 @@ struct ReactParams {
   // array as it found it, so a second pass (FP64 after mixed precision) can start it over.
   long long* retry_list;
   unsigned long long* retry_count;
+  // Cells that a warp works on at a time (0: all that its mapping holds).
+  int cells_per_warp;
 };
 
 }  // namespace pgb

@@ -558,6 +558,44 @@ def emit_jac_stream(e: _Emitter, qual: str, m: Mechanism, rx, tb_rows, codes, ne
     e(f"{qual} int kJacX0[NTB] = {{{', '.join(str(8 * len(rx) + v) for v in (x0 or [0]))}}};")
 
 
+def emit_unrolled_order(e: _Emitter, qual: str, m: Mechanism, order):
+    """What a lane-parallel evaluation needs to give the bits of the unrolled right-hand side
+    (gen_header): the constants as that code folds them, and each species' reactions in the order in
+    which it adds them (input order; values are positions in `order`)."""
+    e(f"{qual} TabUnrolled kUnrolled[NS] = {{")
+    for s in m.species:
+        rows = []
+        for a in (s.low, s.high):
+            rows.append([a[0] * 1.0, a[1] * -0.5, a[2] * (-1.0 / 6.0), a[3] * (-1.0 / 12.0), a[4] * -0.05, a[5] * 1.0,
+                         a[6] * -1.0])
+        for a in (s.low, s.high):
+            w = 1.0 / s.W
+            rows.append([a[0] * 1.0 * w, a[1] * 0.5 * w, a[2] * (1.0 / 3.0) * w, a[3] * 0.25 * w, a[4] * 0.2 * w,
+                         a[5] * 1.0 * w])
+        for a in (s.low, s.high):
+            w = R_ERG / s.W
+            rows.append([a[i] * w for i in range(5)])
+        used = any(s.name in r.reactants or s.name in r.products or r.efficiencies.get(s.name, 1.0) != 1.0
+                   for r in m.reactions)
+        e(f"  {{{_f(1.0 / s.W)}, {_f(s.W)}, {_f(s.Tmid)}, {0 if used else 1}, "
+          + ", ".join("{" + ", ".join(_f(v) for v in r) + "}" for r in rows) + "},")
+    e("};")
+    pos = {j: i for i, j in enumerate(order)}
+    off, jj, nu, tb = [0], [], [], []
+    for s in m.species:
+        for j, r in enumerate(m.reactions):
+            net = r.products.get(s.name, 0) - r.reactants.get(s.name, 0)
+            if net != 0:
+                jj.append(pos[j])
+                nu.append(float(net))
+                tb.append(int(r.kind == "three_body" and abs(net) == 1 and j == m.nr - 1))
+        off.append(len(jj))
+    e(f"{qual} int kUnM[{len(jj)}] = {{{', '.join(str(v) for v in tb)}}};")
+    e(f"{qual} int kUnOff[NS + 1] = {{{', '.join(str(v) for v in off)}}};")
+    e(f"{qual} int kUnJ[{len(jj)}] = {{{', '.join(str(v) for v in jj)}}};")
+    e(f"{qual} double kUnNu[{len(jj)}] = {{{', '.join(_f(v) for v in nu)}}};")
+
+
 def gen_tables(m: Mechanism, space: str = "constant") -> str:
     """Mechanism tables for the table-driven kernels: per-species W, NASA-7 sets, per-reaction
     Arrhenius data, stoichiometry as species slots (a species with coefficient 2 occupies two
@@ -742,6 +780,8 @@ def gen_tables(m: Mechanism, space: str = "constant") -> str:
         for w in rx_packed(rx, ns):
             e("  {" + ", ".join(f"{v}u" for v in w) + "},")
         e("};")
+        if kernel_family(m) == "thread":
+            emit_unrolled_order(e, qual, m, order)
         e(f"constexpr int NSPRX = {len(jj)};")
         e(f"{qual} int kSpRxOff[NS + 1] = {{{', '.join(str(x) for x in off)}}};")
         e(f"{qual} int kSpRxJ[NSPRX] = {{{', '.join(str(x) for x in jj)}}};")
@@ -749,6 +789,12 @@ def gen_tables(m: Mechanism, space: str = "constant") -> str:
     e("struct Tables {")
     e(f"  static constexpr int NS = {ns}, NR = {m.nr};")
     if glob:
+        if kernel_family(m) == "thread":
+            e("  __device__ static const TabUnrolled& un(int k) { return kUnrolled[k]; }")
+            e("  __device__ static int un_begin(int k) { return kUnOff[k]; }")
+            e("  __device__ static int un_j(int e) { return kUnJ[e]; }")
+            e("  __device__ static bool un_m(int e) { return kUnM[e] != 0; }  // the compiler fuses q [M] here")
+            e("  __device__ static double un_nu(int e) { return kUnNu[e]; }")
         e("  __device__ static int sprx_begin(int k) { return kSpRxOff[k]; }")
         e("  __device__ static int sprx_end(int k) { return kSpRxOff[k + 1]; }")
         e("  __device__ static int sprx_j(int e) { return kSpRxJ[e]; }")

@@ -1,0 +1,51 @@
+"""Small launches (the kernel with more lanes per cell that reactor.cu chooses below its limit) give
+the bits of the mechanism's large-launch mapping: states, energies and RHS counts of every cell."""
+import numpy as np
+import pytest
+
+from pelelm_gb300.reactor import BoxArrays, ReactorBase
+from pelelm_gb300.workloads import CONFIGS, make_cells
+
+
+def _advance(torch, cfg, shape, options, deck, seed, masked):
+    nx, ny, nz = shape
+    n = nx * ny * nz
+    cs = make_cells(cfg, n, seed=seed)
+    ns = cs.rY.shape[1]
+
+    def t(a, nc):
+        return torch.tensor(np.ascontiguousarray(np.asarray(a).reshape(n, nc).T.reshape(nc, nz, ny, nx)), device="cuda")
+
+    mask = None
+    if masked:
+        mask = torch.tensor(np.where(np.arange(n) % 7 == 3, -1, 1).astype(np.int32).reshape(1, nz, ny, nx), device="cuda")
+    b = BoxArrays(((0, 0, 0), (nx - 1, ny - 1, nz - 1)), t(cs.rY, ns), t(cs.rYsrc, ns), t(cs.T, 1), t(cs.rE, 1),
+                  t(cs.rEsrc, 1), t(np.zeros(n), 1), mask)
+    if deck:
+        options += " ode.atol=1e-5 peleLM.use_typ_vals_chem=1 cvode.max_order=4"
+    r = ReactorBase.create("ReactorCvode", cfg.mech, options)
+    r.init(2, 1)
+    if deck:
+        r.set_typ_vals_ode([max(1e-10, float(v)) for v in np.ptp(cs.rY, axis=0)] + [float(np.ptp(cs.T)) + 1.0])
+    nfail = r.react(b.box, b.rY, b.rY_src, b.T, b.rEner, b.rEner_src, b.FC, mask, cfg.dt, 0.0)
+    r.close()
+    return nfail, b
+
+
+# one cell; fewer cells than SMs; one cell a warp on every SM; two cells a warp (16-lane groups) and a
+# remainder that leaves half a warp idle; just below the limit of the 9-species mechanism
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(1, 1, 1), (13, 3, 2), (13, 9, 7), (17, 13, 11)])
+@pytest.mark.parametrize("cfgname,mapping", [("lidryer_amr120", "thread"), ("drm19_2M", "group")])
+@pytest.mark.parametrize("precision,deck,masked", [("mixed", False, False), ("fp64", False, True), ("mixed", True, True)])
+def test_small_launch_bits(native_lib, cuda, shape, cfgname, mapping, precision, deck, masked):
+    torch = cuda
+    cfg = CONFIGS[cfgname]
+    opts = f"gb.precision={precision}"
+    fa, a = _advance(torch, cfg, shape, opts, deck, 5, masked)
+    fb, b = _advance(torch, cfg, shape, opts + f" gb.mapping={mapping}", deck, 5, masked)
+    assert fa == fb == 0
+    assert torch.equal(a.FC, b.FC)
+    assert torch.equal(a.rY, b.rY) and torch.equal(a.rEner, b.rEner)
+    # T is one more Newton solve from (rho h, Y), by another sum over species
+    assert float(((a.T - b.T).abs() / b.T).max()) <= 1e-13
