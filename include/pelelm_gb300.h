@@ -282,6 +282,26 @@ int pgb_mlp_dup_weight_bf16(const float* W, int rows, int cols, void* out, int l
 int pgb_mlp_split_rows_bf16(const float* x, int rows, int cols, int ldx, void* out, int ldo, int off,
                             void* stream);
 
+/* One optimiser step of the MLP (forward, mean-squared error over the first n_out outputs, backward,
+ * Adam): the arithmetic of the calls above, a dozen launches on `stream`. dims[0..nlayer]: layer sizes,
+ * multiples of 32; batch a multiple of 32; at most 16 layers. k_half > 0: split input (the first
+ * layer's FP32 weight has k_half columns and its BF16 copy holds them twice, row stride dims[0]).
+ * X (batch x dims[0], row stride ldx) BF16; T (batch x dims[nlayer]) FP32; W, m and v FP32 (dims[l+1]
+ * rows), Wb BF16; *loss receives the sum of squares. workspace: pgb_mlp_train_workspace(s) bytes of
+ * device memory, 256-byte aligned, free when the work enqueued here is done. */
+typedef struct pgb_mlp_step {
+  int nlayer, batch, k_half, n_out, ldx, step;
+  int dims[17];
+  float lr, b1, b2, eps;
+  const void* X;
+  const float* T;
+  float* loss;
+  float *W[16], *b[16], *mW[16], *vW[16], *mb[16], *vb[16];
+  void* Wb[16];
+} pgb_mlp_step;
+long long pgb_mlp_train_workspace(const pgb_mlp_step* s);
+int pgb_mlp_train_step(const pgb_mlp_step* s, void* workspace, void* stream);
+
 /* Measures the device's FP64 FMA throughput in TFLOP/s (2 flops per FMA). No counterpart in
  * the reference: a measurement utility giving the roofline denominator of the FP64-bound
  * reactor kernels. */

@@ -22,7 +22,7 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVFLAGS = ["-std=c++17", "-O3", "-lineinfo", "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC",
            "-Xcompiler", "-O2"]
 # host and shared units; each mechanism adds a generated csrc/gen/unit_<name>.cu
-UNITS = ["reactor.cu", "peak.cu", "noalloc.cu", "partition.cpp", "mlp.cu", "surrogate_io.cu"]
+UNITS = ["reactor.cu", "peak.cu", "noalloc.cu", "partition.cpp", "mlp.cu", "mlp_step.cu", "surrogate_io.cu"]
 DATA = os.path.join(PKG, "data")
 
 

@@ -46,6 +46,13 @@ class SurrogateStats(C.Structure):
                [("audit_max_dT", C.c_double), ("audit_max_dY", C.c_double)]
 
 
+class MlpStep(C.Structure):
+    _fields_ = [(n, C.c_int) for n in ("nlayer", "batch", "k_half", "n_out", "ldx", "step")] + \
+               [("dims", C.c_int * 17)] + [(n, C.c_float) for n in ("lr", "b1", "b2", "eps")] + \
+               [("X", _vp), ("T", _vp), ("loss", _vp)] + \
+               [(n, _vp * 16) for n in ("W", "b", "mW", "vW", "mb", "vb", "Wb")]
+
+
 EXPORTS = {
     "pgb_version": (C.c_int, []),
     "pgb_last_error": (C.c_int, [C.c_char_p, C.c_size_t]),
@@ -77,6 +84,8 @@ EXPORTS = {
     "pgb_mlp_bias_grad": (C.c_int, [_vp, C.c_int, C.c_int, C.c_int, _vp, _vp]),
     "pgb_mlp_adam": (C.c_int, [_vp, _vp, _vp, _vp, _vp, C.c_longlong, C.c_float, C.c_float, C.c_float,
                                C.c_float, C.c_int, _vp]),
+    "pgb_mlp_train_workspace": (C.c_longlong, [C.POINTER(MlpStep)]),
+    "pgb_mlp_train_step": (C.c_int, [C.POINTER(MlpStep), _vp, _vp]),
     "pgb_mlp_f32_to_bf16": (C.c_int, [_vp, _vp, C.c_longlong, _vp]),
     "pgb_mlp_dup_weight_bf16": (C.c_int, [_vp, C.c_int, C.c_int, _vp, C.c_int, _vp]),
     "pgb_mlp_split_rows_bf16": (C.c_int, [_vp, C.c_int, C.c_int, C.c_int, _vp, C.c_int, C.c_int, _vp]),

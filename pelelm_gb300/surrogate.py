@@ -186,10 +186,35 @@ class SurrogateMLP:
             self._refresh_first_layer()
 
     def train_step(self, X, T, lr=1e-3) -> float:
+        """One Adam step on (X, T); returns the sum of squared errors (a device scalar). Forward, loss,
+        backward and update are one native call (csrc/mlp_step.cu); deeper networks than it takes
+        run the same arithmetic through the methods above."""
+        if len(self.W) <= 16:
+            return self._native_step(X, T, lr)
         Y = self.forward(X, keep=True)
         dYf, dY, loss = self.loss_grad(Y, T)
         gW, gb = self.backward(dYf, dY)
         self.adam(gW, gb, lr=lr)
+        return loss
+
+    def _native_step(self, X, T, lr, b1=0.9, b2=0.999, eps=1e-8):
+        torch = self.torch
+        s = _lib.MlpStep()
+        n = len(self.W)
+        s.nlayer, s.batch, s.n_out, s.ldx = n, X.shape[0], self.n_out, X.stride(0)
+        s.k_half = self.k_half if self.split else 0
+        s.step = self.step_count + 1
+        s.lr, s.b1, s.b2, s.eps = lr, b1, b2, eps
+        s.dims[:n + 1] = self.dims
+        loss = torch.empty(1, dtype=torch.float32, device="cuda")
+        s.X, s.T, s.loss = X.data_ptr(), T.data_ptr(), loss.data_ptr()
+        for name in ("W", "b", "mW", "vW", "mb", "vb", "Wb"):
+            getattr(s, name)[:n] = [t.data_ptr() for t in getattr(self, name)]
+        need = lib().pgb_mlp_train_workspace(C.byref(s))
+        check(min(0, need), "mlp_train_step")
+        ws = torch.empty(need, dtype=torch.uint8, device="cuda")
+        check(lib().pgb_mlp_train_step(C.byref(s), ws.data_ptr(), None), "mlp_train_step")
+        self.step_count += 1
         return loss
 
     def state_dict(self):

@@ -110,3 +110,54 @@ def test_adam_training_reduces_loss(native_lib, cuda):
     Xb = m.prepare_input(x)
     losses = [float(m.train_step(Xb, T, lr=2e-3)) for _ in range(200)]
     assert losses[-1] < 0.2 * losses[0], (losses[0], losses[-1])
+
+
+# row tiles of 128 with a remainder, output tiles with a remainder, one k step, one layer beyond the
+# input, split and plain input, the training size
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,width,depth,n_in,n_out,split", [
+    (32, 64, 1, 20, 10, True), (160, 96, 3, 44, 20, True), (288, 160, 2, 33, 40, False), (8192, 256, 4, 44, 20, True)])
+def test_native_step_equals_the_separate_kernels(native_lib, cuda, B, width, depth, n_in, n_out, split):
+    """train_step against forward, loss_grad, backward and adam on a twin: products of activations
+    keep their bits, so the gradients differ by the order in which the batch is summed alone."""
+    from pelelm_gb300.surrogate import SurrogateMLP
+    torch = cuda
+    kw = dict(width=width, depth=depth, seed=7, split_input=split)
+    a, b = (SurrogateMLP(torch, n_in, n_out, **kw) for _ in range(2))
+    g = torch.Generator(device="cuda").manual_seed(B)
+    X = a.prepare_input(torch.randn(B, n_in, device="cuda", generator=g))
+    T = torch.zeros(B, a.n_out_pad, device="cuda")
+    T[:, :n_out] = torch.randn(B, n_out, device="cuda", generator=g)
+    for step in range(2):
+        la = a.train_step(X, T, lr=1e-3)
+        Y = b.forward(X, keep=True)
+        dYf, dY, lb = b.loss_grad(Y, T)
+        b.adam(*b.backward(dYf, dY), lr=1e-3)
+        if step:
+            break
+        # sums of B terms in FP32, in two orders
+        tol = 2.0 ** -20 * B ** 0.5
+        assert abs(float(la) - float(lb)) <= tol * float(lb)
+        for x, y in zip(a.mW + a.mb, b.mW + b.mb):
+            assert float((x - y).abs().max()) <= tol * float(y.abs().max())
+    assert a.step_count == b.step_count == 2
+    for x, y in zip(a.W + a.b, b.W + b.b):
+        # an Adam step moves a parameter by lr at most; where the gradient is not small against its
+        # rounding the two agree far better
+        assert float((x - y).abs().max()) <= 2 * 2e-3 and float((x - y).abs().mean()) <= 2e-6
+    for x, y in zip(a.W[1:], a.Wb[1:]):
+        assert torch.equal(x.to(torch.bfloat16), y)
+    if split:
+        w = a.W[0].to(torch.bfloat16)
+        assert torch.equal(a.Wb[0][:, :a.k_half], w) and torch.equal(a.Wb[0][:, a.k_half:2 * a.k_half], w)
+
+
+@pytest.mark.gpu
+def test_native_step_refuses_sizes_the_products_do_not_take(native_lib, cuda):
+    from pelelm_gb300.surrogate import SurrogateMLP
+    torch = cuda
+    m = SurrogateMLP(torch, 20, 10, width=64, depth=2)
+    X, T = torch.zeros(40, m.k_in, dtype=torch.bfloat16, device="cuda"), torch.zeros(40, m.n_out_pad, device="cuda")
+    with pytest.raises(RuntimeError, match="batch"):
+        m.train_step(X, T)
+    assert m.step_count == 0
