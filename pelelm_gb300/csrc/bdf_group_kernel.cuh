@@ -179,7 +179,7 @@ __device__ __forceinline__ double rate_of_progress_unrolled(int j, double T, dou
   }
   double Pf = CS[rs(0)];
 #pragma unroll
-  for (int s = 1; s < 3; ++s)
+  for (int s = 1; s < Tab::MAXR; ++s)
     if (s < nr) Pf = __dmul_rn(Pf, CS[rs(s)]);
   double q;
   if (rev) {
@@ -189,7 +189,7 @@ __device__ __forceinline__ double rate_of_progress_unrolled(int j, double T, dou
     for (int side = 0; side < 2; ++side) {
       const int n = side ? nr : np;
 #pragma unroll
-      for (int s = 0; s < 3; ++s) {
+      for (int s = 0; s < (side ? Tab::MAXR : Tab::MAXP); ++s) {
         if (s >= n) continue;
         const int k = side ? rs(s) : ps(s);
         if (s > 0 && (side ? rs(s - 1) : ps(s - 1)) == k) continue;  // counted with its first slot
@@ -202,7 +202,7 @@ __device__ __forceinline__ double rate_of_progress_unrolled(int j, double T, dou
     if (dnu != 0) dG = fma(-(double)dnu, lnP0RT, dG);
     double kr = -__dmul_rn(kf, pgb_exp64(fmin(dG, 700.0)));  // finite: an absent product gives 0, not NaN
 #pragma unroll
-    for (int s = 0; s < 3; ++s)
+    for (int s = 0; s < Tab::MAXP; ++s)
       if (s < np) kr = __dmul_rn(kr, CS[ps(s)]);
     q = fma(kf, Pf, kr);
   } else {
@@ -249,12 +249,12 @@ __device__ __forceinline__ GVec<M, G> group_rhs(const GVec<M, G> yv, double* CS,
         invW = s.invW;
         Tmid = s.Tmid;
         fused = s.only_total != 0;
-        g = T < Tmid ? s.glo : s.ghi;
+        g = below_positive(T, Tmid) ? s.glo : s.ghi;
       } else {
         const TabSpecies<double>& s = Tab::template sp<double>(k);
         invW = s.invW;
         Tmid = s.Tmid;
-        g = T < Tmid ? s.glo : s.ghi;
+        g = below_positive(T, Tmid) ? s.glo : s.ghi;
       }
       const double c = y[r] * invW;
       CS[k] = c;
@@ -273,6 +273,19 @@ __device__ __forceinline__ GVec<M, G> group_rhs(const GVec<M, G> yv, double* CS,
     else QS[j] = rate_of_progress<Tab>(j, T, invT, lnT, lnP0RT, Ctot, CS, GS);
   }
   __syncwarp(gm);
+  if constexpr (!UNROLLED) {
+    // production rates, the longest sums together (their FP64 time is the longest lane's of a round)
+#pragma unroll 1
+    for (int i = sub; i < NS; i += G) {
+      const int k = R > 1 ? Tab::sprx_by_len(i) : i;
+      double wdot = 0.0;
+      const int e1 = Tab::sprx_end(k);
+#pragma unroll 4
+      for (int e = Tab::sprx_begin(k); e < e1; ++e) wdot = fma(Tab::sprx_nu(e), QS[Tab::sprx_j(e)], wdot);
+      CS[k] = wdot;
+    }
+    __syncwarp(gm);
+  }
   double hs = 0.0, rcp = 0.0, h_one = 0.0, cp_one = 0.0, c_one = 0.0;
 #pragma unroll
   for (int r = 0; r < R; ++r) {
@@ -292,20 +305,18 @@ __device__ __forceinline__ GVec<M, G> group_rhs(const GVec<M, G> yv, double* CS,
           wdot = Tab::un_m(e) ? fma(qj, mj, wdot) : __dadd_rn(wdot, __dmul_rn(qj, mj));
         }
         f[r] = fma(wdot, s.W, FRC[k]);
-        const bool lo = T < s.Tmid;
+        const bool lo = below_positive(T, s.Tmid);
         const double* a = lo ? s.clo : s.chi;
         const double* hc = lo ? s.hlo : s.hhi;
         h_one = fma(T, fma(T, fma(T, fma(T, hc[4], hc[3]), hc[2]), hc[1]), fma(hc[5], invT, hc[0]));
         cp_one = fma(T, fma(T, fma(T, fma(T, a[4], a[3]), a[2]), a[1]), a[0]);
         c_one = y[r];
       } else {
-        const int e1 = Tab::sprx_end(k);
-#pragma unroll 4
-        for (int e = Tab::sprx_begin(k); e < e1; ++e) wdot = fma(Tab::sprx_nu(e), QS[Tab::sprx_j(e)], wdot);
+        wdot = CS[k];
         const TabSpecies<double>& s = Tab::template sp<double>(k);
         const double wm = fma(wdot, s.W, FRC[k]);
         f[r] = wm;
-        const bool lo = T < s.Tmid;
+        const bool lo = below_positive(T, s.Tmid);
         const double* a = lo ? s.lo : s.hi;
         const double* hc = lo ? s.hlo : s.hhi;
         const double hRT = fma(T, fma(T, fma(T, fma(T, hc[4], hc[3]), hc[2]), hc[1]), fma(hc[5], invT, hc[0]));

@@ -130,18 +130,23 @@ __device__ __forceinline__ double rate_of_progress(int j, double T, double invT,
     }
     kf *= blend;
   }
-  double Pf = 1.0, Pp = 1.0;
+  // both sides hold at least one species, and no reaction more slots than MAXR / MAXP: a predicated
+  // multiply that no lane takes still costs its FP64 slot
+  double Pf = CS[rs(0)], Pp = CS[ps(0)];
 #pragma unroll
-  for (int s = 0; s < 3; ++s) if (s < nr) Pf *= CS[rs(s)];
+  for (int s = 1; s < Tab::MAXR; ++s) if (s < nr) Pf *= CS[rs(s)];
 #pragma unroll
-  for (int s = 0; s < 3; ++s) if (s < np) Pp *= CS[ps(s)];
+  for (int s = 1; s < Tab::MAXP; ++s) if (s < np) Pp *= CS[ps(s)];
   double q;
   if (rev) {
-    double dG = -dnu * lnP0RT;
+    // -dnu ln(P0/RT): a sign for dnu = -1, 0, 1
+    double dG = dnu == 0 ? 0.0 : dnu == -1 ? lnP0RT : dnu == 1 ? -lnP0RT : -dnu * lnP0RT;
+    dG += GS[ps(0)];
 #pragma unroll
-    for (int s = 0; s < 3; ++s) if (s < np) dG += GS[ps(s)];
+    for (int s = 1; s < Tab::MAXP; ++s) if (s < np) dG += GS[ps(s)];
+    dG -= GS[rs(0)];
 #pragma unroll
-    for (int s = 0; s < 3; ++s) if (s < nr) dG -= GS[rs(s)];
+    for (int s = 1; s < Tab::MAXR; ++s) if (s < nr) dG -= GS[rs(s)];
     const double kr = kf * pgb_exp64(fmin(dG, 700.0));  // finite: Pp = 0 gives 0, not NaN
     q = fma(kf, Pf, -kr * Pp);
   } else {
@@ -182,7 +187,7 @@ __device__ __noinline__ WVec<M> warp_rhs(const WVec<M> yv, double* CS, double* G
       const double c = y[r] * s.invW;
       CS[k] = c;
       c_loc += c;
-      const double* g = T < s.Tmid ? s.glo : s.ghi;
+      const double* g = below_positive(T, s.Tmid) ? s.glo : s.ghi;
       GS[k] = fma(g[0], lnT1, fma(T, fma(T, fma(T, fma(T, g[4], g[3]), g[2]), g[1]), fma(g[5], invT, g[6])));
     }
   }
@@ -192,20 +197,28 @@ __device__ __noinline__ WVec<M> warp_rhs(const WVec<M> yv, double* CS, double* G
     QS[j] = rate_of_progress<Tab>(j, T, invT, lnT, lnP0RT, Ctot, CS, GS);
   }
   __syncwarp();
+  // production rates, the longest sums together (their FP64 time is the longest lane's of a round)
+#pragma unroll 1
+  for (int i = lane; i < NS; i += 32) {
+    const int k = R > 1 ? Tab::sprx_by_len(i) : i;
+    double wdot = 0.0;
+    const int e1 = Tab::sprx_end(k);
+#pragma unroll 4
+    for (int e = Tab::sprx_begin(k); e < e1; ++e) wdot = fma(Tab::sprx_nu(e), QS[Tab::sprx_j(e)], wdot);
+    CS[k] = wdot;
+  }
+  __syncwarp();
   double hs = 0.0, rcp = 0.0;
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     const int k = idx(r);
     f[r] = 0.0;
     if (k < NS) {
-      double wdot = 0.0;
-      const int e1 = Tab::sprx_end(k);
-#pragma unroll 4
-      for (int e = Tab::sprx_begin(k); e < e1; ++e) wdot = fma(Tab::sprx_nu(e), QS[Tab::sprx_j(e)], wdot);
+      const double wdot = CS[k];
       const TabSpecies<double>& s = Tab::template sp<double>(k);
       const double wm = fma(wdot, s.W, FRC[k]);
       f[r] = wm;
-      const bool lo = T < s.Tmid;
+      const bool lo = below_positive(T, s.Tmid);
       const double* a = lo ? s.lo : s.hi;
       const double* hc = lo ? s.hlo : s.hhi;
       const double hRT = fma(T, fma(T, fma(T, fma(T, hc[4], hc[3]), hc[2]), hc[1]), fma(hc[5], invT, hc[0]));

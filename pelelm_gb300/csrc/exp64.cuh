@@ -71,6 +71,11 @@ static __device__ __noinline__ double pgb_log64(double x) {
   return fma(ed, PGB_LOG64_LN2_HI, __ldg(&kLog64LogC[j]) + fma(ed, PGB_LOG64_LN2_LO, p));
 }
 
+// a < b for b > 0, on the integer pipe (an FP64 compare takes an FP64 slot).
+__device__ __forceinline__ bool below_positive(double a, double b) {
+  return __double_as_longlong(a) < __double_as_longlong(b);
+}
+
 // a / b, one out-of-line copy for the step logic's many sites (an inlined FP64 division is about
 // 25 instructions).
 static __device__ __noinline__ double pgb_div64(double a, double b) { return a / b; }

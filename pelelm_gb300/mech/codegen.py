@@ -782,7 +782,10 @@ def gen_tables(m: Mechanism, space: str = "constant") -> str:
         e("};")
         if kernel_family(m) == "thread":
             emit_unrolled_order(e, qual, m, order)
+        lens = [off[k + 1] - off[k] for k in range(ns)]
+        by_len = sorted(range(ns), key=lambda k: (-lens[k], k))
         e(f"constexpr int NSPRX = {len(jj)};")
+        e(f"{qual} int kSpByLen[NS] = {{{', '.join(str(k) for k in by_len)}}};  // longest lists first")
         e(f"{qual} int kSpRxOff[NS + 1] = {{{', '.join(str(x) for x in off)}}};")
         e(f"{qual} int kSpRxJ[NSPRX] = {{{', '.join(str(x) for x in jj)}}};")
         e(f"{qual} double kSpRxNu[NSPRX] = {{{', '.join(_f(x) for x in nu)}}};")
@@ -796,6 +799,8 @@ def gen_tables(m: Mechanism, space: str = "constant") -> str:
             e("  __device__ static bool un_m(int e) { return kUnM[e] != 0; }  // the compiler fuses q [M] here")
             e("  __device__ static double un_nu(int e) { return kUnNu[e]; }")
         e("  __device__ static int sprx_begin(int k) { return kSpRxOff[k]; }")
+        e(f"  static constexpr int MAXR = {max(len(r[5]) for r in rx)}, MAXP = {max(len(r[6]) for r in rx)};  // slots a side")
+        e("  __device__ static int sprx_by_len(int i) { return kSpByLen[i]; }")
         e("  __device__ static int sprx_end(int k) { return kSpRxOff[k + 1]; }")
         e("  __device__ static int sprx_j(int e) { return kSpRxJ[e]; }")
         e("  __device__ static double sprx_nu(int e) { return kSpRxNu[e]; }")
