@@ -110,6 +110,22 @@ __device__ __noinline__ double group_sum(double v, unsigned gm) {
   for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(gm, v, o);
   return v;
 }
+// K quotients (K <= 8 <= G) in one division: lane i of the group forms the i-th, and all lanes get
+// all of them. The step logic is the same in every lane of a group, and an FP64 division takes ten of
+// its slots, so its quotients are formed side by side wherever they do not depend on one another.
+template <int K>
+__device__ __forceinline__ void group_div(const double (&num)[K], const double (&den)[K], double (&quot)[K],
+                                          unsigned gm, int gbase) {
+  const int sub = (threadIdx.x & 31) - gbase;
+  double a = num[0], b = den[0];
+#pragma unroll
+  for (int i = 1; i < K; ++i)
+    if (sub == i) { a = num[i]; b = den[i]; }
+  const double d = pgb_div64(a, b);
+#pragma unroll
+  for (int i = 0; i < K; ++i) quot[i] = __shfl_sync(gm, d, gbase + i);
+}
+
 template <int G>
 __device__ __forceinline__ double group_max(double v, unsigned gm) {
 #pragma unroll
@@ -471,6 +487,53 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
   auto tau = [&](int j) -> double { return C.TAU[j]; };
   // l coefficients and error constants (the arithmetic of bdf_kernel.cuh's set_coeffs); l is
   // computed in registers by every lane of the group and stored once
+  // With eight lanes or more the coefficients are spread over them (l_i in lane i) and independent
+  // quotients are formed side by side; the operations and their order are those of the form below.
+  auto set_coeffs_lanes = [&]() {
+    const double alpha0 = alpha0_of(q);
+    double hs = h;  // lane i: h + tau_1 + ... + tau_i
+#pragma unroll 1
+    for (int i = 1; i <= min(sub, QMAX); ++i) hs += tau(i);
+    const double xi = pgb_div64(h, hs);
+    double sum_xi_inv = 0.0, l = sub == 0 ? 1.0 : 0.0;
+#pragma unroll 1
+    for (int i = 1; i <= q - 1; ++i) {
+      const double xi_inv = __shfl_sync(gm, xi, gbase + i - 1);
+      sum_xi_inv += xi_inv;
+      const double below = __shfl_sync(gm, l, gbase + max(sub - 1, 0));
+      if (sub >= 1 && sub <= i) l = fma(below, xi_inv, l);
+    }
+    const double xistar_inv = -alpha0 - sum_xi_inv;
+    {
+      const double below = __shfl_sync(gm, l, gbase + max(sub - 1, 0));
+      if (sub >= 1 && sub <= q) l = fma(below, xistar_inv, l);
+    }
+    const double xiq_inv = __shfl_sync(gm, xi, gbase + q - 1), xiq1_inv = __shfl_sync(gm, xi, gbase + q);
+    const double alpha0_hat = -(sum_xi_inv + xiq_inv);
+    const double A1 = 1.0 - alpha0_hat + alpha0;
+    const double A2 = 1.0 + q * A1;
+    const double lq = __shfl_sync(gm, l, gbase + q), l1 = __shfl_sync(gm, l, gbase + 1);
+    const double A3 = alpha0 + inv_int(q), A4 = alpha0_hat + xiq_inv;
+    const double A5 = alpha0 - inv_int(q + 1), A6 = alpha0_hat - xiq1_inv;
+    double d[5];  // 1/tq2's and 1/tq5's quotients, Cq, Cpp, 1/l_1
+    group_div<5>({A1, A2 * xistar_inv, xistar_inv, 1.0 - A6 + A5, 1.0}, {alpha0 * A2, lq * xiq_inv, lq, A2, l1}, d, gm,
+                 gbase);
+    tq2 = fabs(d[0]);
+    tq5 = fabs(d[1]);
+    rl1 = d[4];
+    gamma = h * rl1;
+    double e[3];
+    group_div<3>({d[2] * (1.0 - A4 + A3), d[3], gamma}, {A3, xiq1_inv * (q + 2) * A5, gammap}, e, gm, gbase);
+    if (qwait == 1) {
+      tq1 = q > 1 ? fabs(e[0]) : 1.0;
+      tq3 = fabs(e[1]);
+    }
+    gamrat = nst > 0 ? e[2] : 1.0;
+    inv_tq4_sq = (tq2 * (1.0 / NLSCOEF)) * (tq2 * (1.0 / NLSCOEF));
+    __syncwarp(gm);
+    if (sub <= QMAX) C.LC[sub] = l;
+    __syncwarp(gm);
+  };
   auto set_coeffs = [&]() {
     double l[QMAX + 1];
 #pragma unroll
@@ -528,6 +591,42 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
       C.LC[e] = v;
     }
     __syncwarp(gm);
+  };
+  auto adjust_order_lanes = [&](int dq) {
+    double hs = 0.0;  // lane i: tau_1 + ... + tau_{i+1}
+#pragma unroll 1
+    for (int i = 0; i <= min(sub, QMAX - 1); ++i) hs += tau(i + 1);
+    const double xis = pgb_div64(hs, hscale), rxis = pgb_div64(1.0, xis);
+    double w = sub == 2 ? 1.0 : 0.0, alpha1 = 0.0, prod = 1.0;  // lane i: w_i
+    const int top = dq > 0 ? q : q - 2;
+#pragma unroll 1
+    for (int j = 1; j <= top; ++j) {
+      const double xi = __shfl_sync(gm, xis, gbase + j - 1);
+      prod *= xi;
+      alpha1 += __shfl_sync(gm, rxis, gbase + j - 1);
+      const double below = __shfl_sync(gm, w, gbase + max(sub - 1, 0));
+      if (sub >= 2 && sub <= j + 2 && (dq < 0 || j <= q - 1)) w = fma(w, xi, below);
+    }
+    if (dq > 0) {
+      const double A1 = pgb_div64(-alpha0_of(q) - alpha1, prod);
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (idx(r) < N) Z(q + 1, r) = A1 * Z(QMAX + 1, r);
+    }
+    const int from = dq > 0 ? q + 1 : q, last = dq > 0 ? q : q - 1;
+#pragma unroll 1
+    for (int j = 2; j <= last; ++j) {
+      double wj = __shfl_sync(gm, w, gbase + j);
+      if (dq < 0) wj = -wj;
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (idx(r) < N) Z(j, r) = fma(wj, Z(from, r), Z(j, r));
+    }
+    if (dq < 0) {
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (idx(r) < N) Z(q, r) = 0.0;
+    }
   };
   auto adjust_order = [&](int dq) {
     double w[QMAX + 2];
@@ -768,10 +867,14 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
         new_step = false;
       }
       predict();
-      set_coeffs();
-      gamma = h * rl1;
+      if constexpr (G >= 8) {
+        set_coeffs_lanes();
+      } else {
+        set_coeffs();
+        gamma = h * rl1;
+        gamrat = (nst > 0) ? pgb_div64(gamma, gammap) : 1.0;
+      }
       if (nst == 0) gammap = gamma;
-      gamrat = (nst > 0) ? pgb_div64(gamma, gammap) : 1.0;
       need_setup = force_setup || nst == 0 || nst >= nstlp + MSBP || fabs(gamrat - 1.0) > DGMAX;
       force_setup = false;
       jcur = false;
@@ -960,8 +1063,87 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
       } else if (outcome == 1) {
         const double acnrm2 = (m == 0) ? del2 : wms(acor);
         const double dsm2 = acnrm2 * (tq2 * tq2);  // squared local error estimate
-        const double etaq = pgb_div64(1.0, pgb_pow64((BIAS2 * BIAS2) * dsm2, 0.5 * inv_int(q + 1)) + ADDON);
-        if (!(dsm2 <= 1.0)) {
+        const bool accepted = dsm2 <= 1.0;
+        bool save = false, ended = false, orders = false;  // orders: q - 1 and q + 1 are weighed too
+        double ddn2 = 0.0, dup2 = 0.0;
+        if (accepted) {
+          // ---- step accepted: complete it ----
+          ++nst;
+          __syncwarp(gm);
+          if (sub == 0) {
+#pragma unroll 1
+            for (int i = q + 1; i >= 2; --i) C.TAU[i] = C.TAU[i - 1];
+            C.TAU[1] = h;
+          }
+#pragma unroll 1
+          for (int j = 0; j <= q; ++j) {
+            const double lj = C.LC[j];
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+              if (idx(r) < N) Z(j, r) = fma(lj, acor[r], Z(j, r));
+          }
+          __syncwarp(gm);
+          --qwait;
+          if (qwait == 1 && q != qmax) {
+            save = true;
+            tq5_saved = tq5;
+          }
+          ended = fabs(t - tout) <= 100.0 * UROUND * (fabs(t) + fabs(h)) || t >= tout;
+          orders = !ended && etamax != 1.0 && qwait == 0;
+          if (orders) {
+            if (q > 1) {
+              double zq[R];
+#pragma unroll
+              for (int r = 0; r < R; ++r) zq[r] = idx(r) < N ? Z(q, r) : 0.0;
+              ddn2 = wms(zq) * (tq1 * tq1);
+            }
+            if (q != qmax) {
+              double hr, tq;
+              if constexpr (G >= 8) {
+                double d[2];
+                group_div<2>({h, tq5}, {tau(2), tq5_saved}, d, gm, gbase);
+                hr = d[0];
+                tq = d[1];
+              } else {
+                hr = pgb_div64(h, tau(2));
+                tq = pgb_div64(tq5, tq5_saved);
+              }
+              double hrp = hr;
+#pragma unroll 1
+              for (int k = 0; k < q; ++k) hrp *= hr;  // (h / tau2)^(q+1)
+              const double cquot = tq * hrp;
+              double tv[R];
+              // the order test's difference: a group of 8 rounds the product of elements 8..15 and
+              // fuses the others (as the compiler chose when this was one expression; kept, so
+              // that every width of group takes the same steps)
+#pragma unroll
+              for (int r = 0; r < R; ++r) {
+                const double saved = idx(r) < N ? Z(QMAX + 1, r) : 0.0;
+                if (S == 1) tv[r] = fma(-cquot, saved, acor[r]);
+                else if (idx(r) / S == 1) tv[r] = __dsub_rn(acor[r], __dmul_rn(cquot, saved));
+                else tv[r] = fma(-cquot, saved, acor[r]);
+              }
+              dup2 = wms(tv) * (tq3 * tq3);
+            }
+          }
+        }
+        // step-size factors of orders q, q - 1 and q + 1
+        double etaq, etaqm1, etaqp1;
+        if constexpr (G >= 8) {  // one power and one quotient: lane 1 takes q - 1, lane 2 q + 1
+          const double x = sub == 1 ? (BIAS1 * BIAS1) * ddn2 : sub == 2 ? (BIAS3 * BIAS3) * dup2 : (BIAS2 * BIAS2) * dsm2;
+          const double a = 0.5 * inv_int(sub == 1 ? q : sub == 2 ? q + 2 : q + 1);
+          const double e = pgb_div64(1.0, pgb_pow64(x, a) + ADDON);
+          etaq = __shfl_sync(gm, e, gbase);
+          etaqm1 = __shfl_sync(gm, e, gbase + 1);
+          etaqp1 = __shfl_sync(gm, e, gbase + 2);
+        } else {
+          etaq = pgb_div64(1.0, pgb_pow64((BIAS2 * BIAS2) * dsm2, 0.5 * inv_int(q + 1)) + ADDON);
+          etaqm1 = pgb_div64(1.0, pgb_pow64((BIAS1 * BIAS1) * ddn2, 0.5 * inv_int(q)) + ADDON);
+          etaqp1 = pgb_div64(1.0, pgb_pow64((BIAS3 * BIAS3) * dup2, 0.5 * inv_int(q + 2)) + ADDON);
+        }
+        if (!orders || q == 1) etaqm1 = 0.0;
+        if (!orders || q == qmax) etaqp1 = 0.0;
+        if (!accepted) {
           // ---- local error test failed ----
           undo = true;
           t -= h;
@@ -984,29 +1166,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
             }
           }
         } else {
-          // ---- step accepted: complete it ----
-          ++nst;
-          __syncwarp(gm);
-          if (sub == 0) {
-#pragma unroll 1
-            for (int i = q + 1; i >= 2; --i) C.TAU[i] = C.TAU[i - 1];
-            C.TAU[1] = h;
-          }
-#pragma unroll 1
-          for (int j = 0; j <= q; ++j) {
-            const double lj = C.LC[j];
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-              if (idx(r) < N) Z(j, r) = fma(lj, acor[r], Z(j, r));
-          }
-          __syncwarp(gm);
-          --qwait;
-          bool save = false;
-          if (qwait == 1 && q != qmax) {
-            save = true;
-            tq5_saved = tq5;
-          }
-          if (fabs(t - tout) <= 100.0 * UROUND * (fabs(t) + fabs(h)) || t >= tout) {
+          if (ended) {
             phase = FINISH;
           } else {
             // ---- next step size and order ----
@@ -1018,34 +1178,6 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
               eta = etaq;
               if (qwait == 0) {
                 qwait = 2;
-                double etaqm1 = 0.0, etaqp1 = 0.0;
-                if (q > 1) {
-                  double zq[R];
-#pragma unroll
-                  for (int r = 0; r < R; ++r) zq[r] = idx(r) < N ? Z(q, r) : 0.0;
-                  const double ddn2 = wms(zq) * (tq1 * tq1);
-                  etaqm1 = pgb_div64(1.0, pgb_pow64((BIAS1 * BIAS1) * ddn2, 0.5 * inv_int(q)) + ADDON);
-                }
-                if (q != qmax) {
-                  const double hr = pgb_div64(h, tau(2));
-                  double hrp = hr;
-#pragma unroll 1
-                  for (int k = 0; k < q; ++k) hrp *= hr;  // (h / tau2)^(q+1)
-                  const double cquot = pgb_div64(tq5, tq5_saved) * hrp;
-                  double tv[R];
-                  // the order test's difference: a group of 8 rounds the product of elements 8..15 and
-                  // fuses the others (as the compiler chose when this was one expression; kept, so
-                  // that every width of group takes the same steps)
-#pragma unroll
-                  for (int r = 0; r < R; ++r) {
-                    const double saved = idx(r) < N ? Z(QMAX + 1, r) : 0.0;
-                    if (S == 1) tv[r] = fma(-cquot, saved, acor[r]);
-                    else if (idx(r) / S == 1) tv[r] = __dsub_rn(acor[r], __dmul_rn(cquot, saved));
-                    else tv[r] = fma(-cquot, saved, acor[r]);
-                  }
-                  const double dup2 = wms(tv) * (tq3 * tq3);
-                  etaqp1 = pgb_div64(1.0, pgb_pow64((BIAS3 * BIAS3) * dup2, 0.5 * inv_int(q + 2)) + ADDON);
-                }
                 const double etam = fmax(etaqm1, fmax(etaq, etaqp1));
                 if (etam < THRESH) {
                   eta = 1.0;
@@ -1081,7 +1213,8 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
     }
     if (undo) retract();
     if (dq != 0) {
-      adjust_order(dq);
+      if constexpr (G >= 8) adjust_order_lanes(dq);
+      else adjust_order(dq);
       q += dq;
       qwait = q + 1;
     }

@@ -53,6 +53,12 @@ __device__ __forceinline__ double inv_int(int j) {
        : j == 6 ? 1.0 / 6.0 : 1.0 / 7.0;
 }
 
+// -(1 + 1/2 + ... + 1/q), summed in that order
+__device__ __forceinline__ double alpha0_of(int q) {
+  constexpr double a1 = 0.0 - 1.0, a2 = a1 - 0.5, a3 = a2 - 1.0 / 3.0, a4 = a3 - 0.25, a5 = a4 - 0.2;
+  return q == 1 ? a1 : q == 2 ? a2 : q == 3 ? a3 : q == 4 ? a4 : a5;
+}
+
 // 1/x to ~1e-14 from an FP32 seed and one Newton step (3 FP64-pipe instructions instead of a
 // 7-8 slot IEEE division); used for error weights in mixed precision. x must lie in the
 // normal FP32 range.
