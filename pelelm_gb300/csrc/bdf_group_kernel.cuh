@@ -110,22 +110,6 @@ __device__ __noinline__ double group_sum(double v, unsigned gm) {
   for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(gm, v, o);
   return v;
 }
-// K quotients (K <= 8 <= G) in one division: lane i of the group forms the i-th, and all lanes get
-// all of them. The step logic is the same in every lane of a group, and an FP64 division takes ten of
-// its slots, so its quotients are formed side by side wherever they do not depend on one another.
-template <int K>
-__device__ __forceinline__ void group_div(const double (&num)[K], const double (&den)[K], double (&quot)[K],
-                                          unsigned gm, int gbase) {
-  const int sub = (threadIdx.x & 31) - gbase;
-  double a = num[0], b = den[0];
-#pragma unroll
-  for (int i = 1; i < K; ++i)
-    if (sub == i) { a = num[i]; b = den[i]; }
-  const double d = pgb_div64(a, b);
-#pragma unroll
-  for (int i = 0; i < K; ++i) quot[i] = __shfl_sync(gm, d, gbase + i);
-}
-
 template <int G>
 __device__ __forceinline__ double group_max(double v, unsigned gm) {
 #pragma unroll

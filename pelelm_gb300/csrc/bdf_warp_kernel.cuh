@@ -82,6 +82,22 @@ __device__ __forceinline__ double warp_max(double v) {
   return v;
 }
 
+// K quotients (K <= 8 <= G) in one division: lane i of the group forms the i-th, and all lanes get
+// all of them. The step logic is the same in every lane of a group, and an FP64 division takes ten of
+// its slots, so its quotients are formed side by side wherever they do not depend on one another.
+template <int K>
+__device__ __forceinline__ void group_div(const double (&num)[K], const double (&den)[K], double (&quot)[K],
+                                          unsigned gm, int gbase) {
+  const int sub = (threadIdx.x & 31) - gbase;
+  double a = num[0], b = den[0];
+#pragma unroll
+  for (int i = 1; i < K; ++i)
+    if (sub == i) { a = num[i]; b = den[i]; }
+  const double d = pgb_div64(a, b);
+#pragma unroll
+  for (int i = 0; i < K; ++i) quot[i] = __shfl_sync(gm, d, gbase + i);
+}
+
 // The lane-distributed part of a length-N vector (element i in lane i % 32, slot i / 32).
 template <class M>
 struct WVec {
@@ -118,15 +134,15 @@ __device__ __forceinline__ double rate_of_progress(int j, double T, double invT,
     const TabTroe<double>& fo = Tab::template troe<double>(troe);
     const double lnk0 = fma(fo.beta0, lnT, fma(fo.mEa0R, invT, fo.lnA0));
     const double Pr = Mc * pgb_exp64(lnk0 - lnkf);
-    double blend = Pr / (1.0 + Pr);
+    double blend = pgb_div64(Pr, 1.0 + Pr);
     if (fo.ntroe > 0) {
       double Fcent = fma(fo.one_m_a, pgb_exp64(T * fo.m_invT3), fo.a * pgb_exp64(T * fo.m_invT1));
       if (fo.ntroe > 3) Fcent += pgb_exp64(invT * fo.m_T2);
       const double lFc = pgb_log64(Fcent) * 0.4342944819032518;
       const double cc = fma(-0.67, lFc, -0.4), nn = fma(-1.27, lFc, 0.75);
       const double lPr = pgb_log64(fmax(Pr, 1e-300)) * 0.4342944819032518 + cc;
-      const double f1 = lPr / fma(-0.14, lPr, nn);
-      blend *= pgb_exp64(2.302585092994046 * lFc / fma(f1, f1, 1.0));
+      const double f1 = pgb_div64(lPr, fma(-0.14, lPr, nn));
+      blend *= pgb_exp64(pgb_div64(2.302585092994046 * lFc, fma(f1, f1, 1.0)));
     }
     kf *= blend;
   }
@@ -174,7 +190,7 @@ __device__ __noinline__ WVec<M> warp_rhs(const WVec<M> yv, double* CS, double* G
     return __shfl_sync(0xffffffffu, v[i >> 5], i & 31);
   };
   const double T = bcast(y, NS);
-  const double invT = 1.0 / T;
+  const double invT = pgb_div64(1.0, T);
   const double lnT = pgb_log64(T);
   const double lnT1 = 1.0 - lnT;
   const double lnP0RT = kLnP0OverR - lnT;
@@ -229,7 +245,7 @@ __device__ __noinline__ WVec<M> warp_rhs(const WVec<M> yv, double* CS, double* G
   }
   hs = warp_sum(hs);
   rcp = warp_sum(rcp);
-  const double fT = fma(-hs, kRerg * T, FRC[NS]) / (rcp * kRerg);
+  const double fT = pgb_div64(fma(-hs, kRerg * T, FRC[NS]), rcp * kRerg);
 #pragma unroll
   for (int r = 0; r < R; ++r)
     if (idx(r) == NS) f[r] = fT;
@@ -896,110 +912,85 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
           for (int r = 0; r < R; ++r)
             if (idx(r) < N) zget(j - 1, r) -= zget(j, r);
     };
-    // l coefficients and error constants (scalar, every lane; the same arithmetic as the
-    // per-thread kernel's set_coeffs)
+    // l coefficients and error constants, gamma and its ratio: the arithmetic of the per-thread kernel's
+    // set_coeffs, coefficient l_i in lane i and independent quotients formed side by side
     auto set_coeffs = [&]() {
-      double l[QMAX + 1];
-#pragma unroll
-      for (int i = 0; i <= QMAX; ++i) l[i] = 0.0;
-      l[0] = 1.0;
-      double alpha0 = 0.0;
+      const double alpha0 = alpha0_of(q);
+      double hs = h;  // lane i: h + tau_1 + ... + tau_i
 #pragma unroll 1
-      for (int j = 1; j <= q; ++j) alpha0 -= inv_int(j);
-      double hsum = h, sum_xi_inv = 0.0;
+      for (int i = 1; i <= min(lane, QMAX); ++i) hs += TAU[i];
+      const double xi = pgb_div64(h, hs);
+      double sum_xi_inv = 0.0, l = lane == 0 ? 1.0 : 0.0;
 #pragma unroll 1
       for (int i = 1; i <= q - 1; ++i) {
-        if (i > 1) hsum += TAU[i - 1];
-        const double xi_inv = h / hsum;
+        const double xi_inv = __shfl_sync(0xffffffffu, xi, i - 1);
         sum_xi_inv += xi_inv;
-#pragma unroll
-        for (int k = QMAX; k >= 1; --k)
-          if (k <= i) l[k] += l[k - 1] * xi_inv;
+        const double below = __shfl_up_sync(0xffffffffu, l, 1);
+        if (lane >= 1 && lane <= i) l = fma(below, xi_inv, l);
       }
       const double xistar_inv = -alpha0 - sum_xi_inv;
-#pragma unroll
-      for (int k = QMAX; k >= 1; --k)
-        if (k <= q) l[k] += l[k - 1] * xistar_inv;
-      if (q > 1) hsum += TAU[q - 1];
-      const double xiq_inv = h / hsum;
+      {
+        const double below = __shfl_up_sync(0xffffffffu, l, 1);
+        if (lane >= 1 && lane <= q) l = fma(below, xistar_inv, l);
+      }
+      const double xiq_inv = __shfl_sync(0xffffffffu, xi, q - 1), xiq1_inv = __shfl_sync(0xffffffffu, xi, q);
       const double alpha0_hat = -(sum_xi_inv + xiq_inv);
       const double A1 = 1.0 - alpha0_hat + alpha0;
       const double A2 = 1.0 + q * A1;
-      double lq = 0.0;
-#pragma unroll
-      for (int k = 0; k <= QMAX; ++k) if (k == q) lq = l[k];
-      tq2 = fabs(A1 / (alpha0 * A2));
-      tq5 = fabs(A2 * xistar_inv / (lq * xiq_inv));
+      const double lq = __shfl_sync(0xffffffffu, l, q), l1 = __shfl_sync(0xffffffffu, l, 1);
+      const double A3 = alpha0 + inv_int(q), A4 = alpha0_hat + xiq_inv;
+      const double A5 = alpha0 - inv_int(q + 1), A6 = alpha0_hat - xiq1_inv;
+      double d[5];
+      group_div<5>({A1, A2 * xistar_inv, xistar_inv, 1.0 - A6 + A5, 1.0}, {alpha0 * A2, lq * xiq_inv, lq, A2, l1}, d,
+                   0xffffffffu, 0);
+      tq2 = fabs(d[0]);
+      tq5 = fabs(d[1]);
+      rl1 = d[4];
+      gamma = h * rl1;
+      double e[3];
+      group_div<3>({d[2] * (1.0 - A4 + A3), d[3], gamma}, {A3, xiq1_inv * (q + 2) * A5, gammap}, e, 0xffffffffu, 0);
       if (qwait == 1) {
-        if (q > 1) {
-          const double C = xistar_inv / lq;
-          const double A3 = alpha0 + inv_int(q);
-          const double A4 = alpha0_hat + xiq_inv;
-          tq1 = fabs(C * (1.0 - A4 + A3) / A3);
-        } else {
-          tq1 = 1.0;
-        }
-        const double xiq1_inv = h / (hsum + TAU[q]);
-        const double A5 = alpha0 - inv_int(q + 1);
-        const double A6 = alpha0_hat - xiq1_inv;
-        const double Cpp = (1.0 - A6 + A5) / A2;
-        tq3 = fabs(Cpp / (xiq1_inv * (q + 2) * A5));
+        tq1 = q > 1 ? fabs(e[0]) : 1.0;
+        tq3 = fabs(e[1]);
       }
+      gamrat = nst > 0 ? e[2] : 1.0;
+      if (nst == 0) gammap = gamma;
       inv_tq4_sq = (tq2 * (1.0 / NLSCOEF)) * (tq2 * (1.0 / NLSCOEF));
       __syncwarp();
-      if (lane <= QMAX) {
-        double v = 0.0;
-#pragma unroll
-        for (int k = 0; k <= QMAX; ++k) if (k == lane) v = l[k];
-        LC[lane] = v;
-      }
+      if (lane <= QMAX) LC[lane] = l;
       __syncwarp();
     };
     auto adjust_order = [&](int dq) {
-      double w[QMAX + 2];
-#pragma unroll
-      for (int i = 0; i < QMAX + 2; ++i) w[i] = 0.0;
-      w[2] = 1.0;
-      if (dq > 0) {
-        double alpha0 = 0.0, alpha1 = 0.0, prod = 1.0, hsum = 0.0;
+      double hs = 0.0;  // lane i: tau_1 + ... + tau_{i+1}
 #pragma unroll 1
-        for (int j = 1; j <= q; ++j) {
-          hsum += TAU[j];
-          const double xi = hsum / hscale;
-          prod *= xi;
-          alpha0 -= inv_int(j);
-          alpha1 += 1.0 / xi;
-          if (j <= q - 1)
-#pragma unroll
-            for (int i = QMAX + 1; i >= 2; --i)
-              if (i <= j + 2) w[i] = w[i] * xi + w[i - 1];
-        }
-        const double A1 = (-alpha0 - alpha1) / prod;
+      for (int i = 0; i <= min(lane, QMAX - 1); ++i) hs += TAU[i + 1];
+      const double xis = pgb_div64(hs, hscale), rxis = pgb_div64(1.0, xis);
+      double w = lane == 2 ? 1.0 : 0.0, alpha1 = 0.0, prod = 1.0;  // lane i: w_i
+      const int top = dq > 0 ? q : q - 2;
+#pragma unroll 1
+      for (int j = 1; j <= top; ++j) {
+        const double xi = __shfl_sync(0xffffffffu, xis, j - 1);
+        prod *= xi;
+        alpha1 += __shfl_sync(0xffffffffu, rxis, j - 1);
+        const double below = __shfl_up_sync(0xffffffffu, w, 1);
+        if (lane >= 2 && lane <= j + 2 && (dq < 0 || j <= q - 1)) w = fma(w, xi, below);
+      }
+      if (dq > 0) {
+        const double A1 = pgb_div64(-alpha0_of(q) - alpha1, prod);
 #pragma unroll
         for (int r = 0; r < R; ++r)
           if (idx(r) < N) zget(q + 1, r) = A1 * acor_saved[r];
-#pragma unroll
-        for (int j = 2; j <= QMAX; ++j)
-          if (j <= q)
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-              if (idx(r) < N) zget(j, r) = fma(w[j], zget(q + 1, r), zget(j, r));
-      } else {
-        double hsum = 0.0;
+      }
+      const int from = dq > 0 ? q + 1 : q, last = dq > 0 ? q : q - 1;
 #pragma unroll 1
-        for (int j = 1; j <= q - 2; ++j) {
-          hsum += TAU[j];
-          const double xi = hsum / hscale;
+      for (int j = 2; j <= last; ++j) {
+        double wj = __shfl_sync(0xffffffffu, w, j);
+        if (dq < 0) wj = -wj;
 #pragma unroll
-          for (int i = QMAX + 1; i >= 2; --i)
-            if (i <= j + 2) w[i] = w[i] * xi + w[i - 1];
-        }
-#pragma unroll
-        for (int j = 2; j <= QMAX; ++j)
-          if (j < q)
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-              if (idx(r) < N) zget(j, r) = fma(-w[j], zget(q, r), zget(j, r));
+        for (int r = 0; r < R; ++r)
+          if (idx(r) < N) zget(j, r) = fma(wj, zget(from, r), zget(j, r));
+      }
+      if (dq < 0) {
 #pragma unroll
         for (int r = 0; r < R; ++r)
           if (idx(r) < N) zget(q, r) = 0.0;
@@ -1038,7 +1029,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
             tmp[r] = idx(r) < N ? fma(gamma, f[r], -fma(rl1, zget(1, r), acor[r])) : 0.0;
           solve(tmp);
           if (gamrat != 1.0) {
-            const double s = 2.0 / (1.0 + gamrat);
+            const double s = pgb_div64(2.0, 1.0 + gamrat);
 #pragma unroll
             for (int r = 0; r < R; ++r) tmp[r] *= s;
           }
@@ -1046,7 +1037,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
 #pragma unroll
           for (int r = 0; r < R; ++r)
             if (idx(r) < N) { acor[r] += tmp[r]; y[r] = zget(0, r) + acor[r]; }
-          if (mm > 0) crate2 = fmax((CRDOWN * CRDOWN) * crate2, del2 / delp2);
+          if (mm > 0) crate2 = fmax((CRDOWN * CRDOWN) * crate2, pgb_div64(del2, delp2));
           if (del2 * fmin(1.0, crate2) * inv_tq4_sq <= 1.0) {
             acnrm2 = (mm == 0) ? del2 : wms(acor);
             ok = true;
@@ -1075,10 +1066,10 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
       double hub_inv = 0.0;
 #pragma unroll
       for (int r = 0; r < R; ++r)
-        if (idx(r) < N) hub_inv = fmax(hub_inv, fabs(f[r]) / fma(0.1, fabs(zget(0, r)), P.atol[idx(r)]));
+        if (idx(r) < N) hub_inv = fmax(hub_inv, pgb_div64(fabs(f[r]), fma(0.1, fabs(zget(0, r)), P.atol[idx(r)])));
       hub_inv = warp_max(hub_inv);
       double hub = 0.1 * tout;
-      if (hub * hub_inv > 1.0) hub = 1.0 / hub_inv;
+      if (hub * hub_inv > 1.0) hub = pgb_div64(1.0, hub_inv);
       double hg = sqrt(hlb * hub), hnew = hg;
       if (hub > hlb) {
 #pragma unroll 1
@@ -1089,11 +1080,11 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
           rhs(yy, fy);
           ++nfe;
 #pragma unroll
-          for (int r = 0; r < R; ++r) tmp[r] = (fy[r] - f[r]) / hg;
+          for (int r = 0; r < R; ++r) tmp[r] = pgb_div64(fy[r] - f[r], hg);
           const double ydd = sqrt(wms(tmp));
-          hnew = (ydd * hub * hub > 2.0) ? sqrt(2.0 / ydd) : sqrt(hg * hub);
+          hnew = sqrt((ydd * hub * hub > 2.0) ? pgb_div64(2.0, ydd) : hg * hub);
           if (count == 4) break;
-          const double hrat = hnew / hg;
+          const double hrat = pgb_div64(hnew, hg);
           if (hrat > 0.5 && hrat < 2.0) break;
           if (count >= 2 && hrat > 2.0) { hnew = hg; break; }
           hg = hnew;
@@ -1112,7 +1103,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
     // ---------------------------------------------- step loop
     for (;;) {
       if (nst >= P.max_steps) { status = MAX_STEPS; break; }
-      if ((t + h - tout) * h > 0.0) rescale((tout - t) * (1.0 - 4.0 * UROUND) / h);
+      if ((t + h - tout) * h > 0.0) rescale(pgb_div64((tout - t) * (1.0 - 4.0 * UROUND), h));
       set_ewt();
       nef = 0; ncf = 0;
       double dsm2 = 0.0;
@@ -1120,10 +1111,6 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
       for (;;) {
         predict();
         set_coeffs();
-        rl1 = 1.0 / LC[1];
-        gamma = h * rl1;
-        if (nst == 0) gammap = gamma;
-        gamrat = (nst > 0) ? gamma / gammap : 1.0;
         const int nflag = newton();
         if (nflag != 0) {
           retract();
@@ -1141,7 +1128,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
           if (nef >= MXNEF || !isfinite(dsm2)) { status = isfinite(dsm2) ? ERRTEST : NONFINITE; failed = true; break; }
           etamax = 1.0;
           if (nef <= MXNEF1) {
-            double e = 1.0 / (pgb_pow64((BIAS2 * BIAS2) * dsm2, 0.5 * inv_int(q + 1)) + ADDON);
+            double e = pgb_div64(1.0, pgb_pow64((BIAS2 * BIAS2) * dsm2, 0.5 * inv_int(q + 1)) + ADDON);
             e = fmax(ETAMIN, e);
             if (nef >= SMALL_NEF) e = fmin(e, ETAMXF);
             rescale(e);
@@ -1191,7 +1178,39 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
       }
       if (fabs(t - tout) <= 100.0 * UROUND * (fabs(t) + fabs(h)) || t >= tout) break;
       // ---- next step size and order ----
-      const double etaq = 1.0 / (pgb_pow64((BIAS2 * BIAS2) * dsm2, 0.5 * inv_int(q + 1)) + ADDON);
+      // step-size factors of orders q, q - 1 and q + 1: one power and one quotient, lane 1 takes q - 1,
+      // lane 2 q + 1
+      const bool orders = etamax != 1.0 && qwait == 0;
+      double ddn2 = 0.0, dup2 = 0.0;
+      if (orders) {
+        if (q > 1) {
+          double zq[R];
+#pragma unroll
+          for (int r = 0; r < R; ++r) zq[r] = idx(r) < N ? zget(q, r) : 0.0;
+          ddn2 = wms(zq) * (tq1 * tq1);
+        }
+        if (q != qmax) {
+          double d[2];
+          group_div<2>({h, tq5}, {TAU[2], tq5_saved}, d, 0xffffffffu, 0);
+          double hrp = d[0];
+#pragma unroll 1
+          for (int k = 0; k < q; ++k) hrp *= d[0];
+          const double cquot = d[1] * hrp;
+#pragma unroll
+          for (int r = 0; r < R; ++r) tmp[r] = acor[r] - cquot * acor_saved[r];
+          dup2 = wms(tmp) * (tq3 * tq3);
+        }
+      }
+      double etaq, etaqm1 = 0.0, etaqp1 = 0.0;
+      {
+        const double x = lane == 1 ? (BIAS1 * BIAS1) * ddn2 : lane == 2 ? (BIAS3 * BIAS3) * dup2 : (BIAS2 * BIAS2) * dsm2;
+        const double a = 0.5 * inv_int(lane == 1 ? q : lane == 2 ? q + 2 : q + 1);
+        const double e = pgb_div64(1.0, pgb_pow64(x, a) + ADDON);
+        etaq = __shfl_sync(0xffffffffu, e, 0);
+        const double em = __shfl_sync(0xffffffffu, e, 1), ep = __shfl_sync(0xffffffffu, e, 2);
+        if (orders && q > 1) etaqm1 = em;
+        if (orders && q != qmax) etaqp1 = ep;
+      }
       int qprime = q;
       if (etamax == 1.0) {
         qwait = max(qwait, 2);
@@ -1200,25 +1219,6 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
         eta = etaq;
         if (qwait == 0) {
           qwait = 2;
-          double etaqm1 = 0.0, etaqp1 = 0.0;
-          if (q > 1) {
-            double zq[R];
-#pragma unroll
-            for (int r = 0; r < R; ++r) zq[r] = idx(r) < N ? zget(q, r) : 0.0;
-            const double ddn2 = wms(zq) * (tq1 * tq1);
-            etaqm1 = 1.0 / (pgb_pow64((BIAS1 * BIAS1) * ddn2, 0.5 * inv_int(q)) + ADDON);
-          }
-          if (q != qmax) {
-            const double hr = h / TAU[2];
-            double hrp = hr;
-#pragma unroll 1
-            for (int k = 0; k < q; ++k) hrp *= hr;
-            const double cquot = (tq5 / tq5_saved) * hrp;
-#pragma unroll
-            for (int r = 0; r < R; ++r) tmp[r] = acor[r] - cquot * acor_saved[r];
-            const double dup2 = wms(tmp) * (tq3 * tq3);
-            etaqp1 = 1.0 / (pgb_pow64((BIAS3 * BIAS3) * dup2, 0.5 * inv_int(q + 2)) + ADDON);
-          }
           const double etam = fmax(etaqm1, fmax(etaq, etaqp1));
           if (etam < THRESH) {
             eta = 1.0;
@@ -1270,7 +1270,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
 #pragma unroll
     for (int r = 0; r < R; ++r)
       if (idx(r) < NS) rho_l += zget(0, r);
-    const double inv_rho = 1.0 / warp_sum(rho_l);
+    const double inv_rho = pgb_div64(1.0, warp_sum(rho_l));
     const double htarget = rE * inv_rho;
     double Tn = Z[NS];
     if (!(Tn > 90.0 && Tn < 5000.0)) Tn = 1000.0;
@@ -1285,7 +1285,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
           const bool lo = Tn < s.Tmid;
           const double* a = lo ? s.lo : s.hi;
           const double* hc = lo ? s.hlo : s.hhi;
-          const double invTn = 1.0 / Tn;
+          const double invTn = pgb_div64(1.0, Tn);
           const double hRT = fma(Tn, fma(Tn, fma(Tn, fma(Tn, hc[4], hc[3]), hc[2]), hc[1]), fma(hc[5], invTn, hc[0]));
           const double cpR = fma(Tn, fma(Tn, fma(Tn, fma(Tn, a[4], a[3]), a[2]), a[1]), a[0]);
           const double Yk = zget(0, r) * inv_rho;
@@ -1294,7 +1294,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
         }
       }
       const double hh = warp_sum(hl), cp = warp_sum(cl);
-      double dT = (htarget - hh) / cp;
+      double dT = pgb_div64(htarget - hh, cp);
       dT = fmax(-100.0, fmin(100.0, dT));
       Tn = fmax(90.0, fmin(5000.0, Tn + dT));
       if (fabs(dT) < 1e-10 * Tn) break;
