@@ -375,13 +375,17 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
     }
     // rho h(t) = rho h0 + F_h t ; T from (h, Y) by Newton with the integrated T as guess
     const double rE = fma(tout, FRC(NS), rE0);
-    double rho = 0.0;
+    double rho = 0.0, hm = 0.0;
 #pragma unroll 1
-    for (int k = 0; k < NS; ++k) rho += Z(0, k);
+    for (int k = 0; k < NS; ++k) {
+      rho += Z(0, k);
+      hm = fma(Z(0, k), M::Tab::h_mid(k), hm);
+    }
     const double inv_rho = 1.0 / rho;
     double Tn = Z(0, NS);
     if (!(Tn > 90.0 && Tn < 5000.0)) Tn = 1000.0;
-    Tn = hy2t_mixture<typename M::Tab>(rE * inv_rho, [&](int k) { return Z(0, k); }, inv_rho, Tn, 90.0, 5000.0);
+    Tn = hy2t_mixture<typename M::Tab>(rE * inv_rho, [&](int k) { return Z(0, k); }, inv_rho, hm, Tn, 90.0,
+                                          5000.0);
     const double dt_inv = pgb_div64(1.0, tout);
 #pragma unroll 1
     for (int k = 0; k < NS; ++k) {

@@ -86,13 +86,24 @@ constexpr double kRerg = 8.31446261815324e7;        // erg/mol/K
 // (the iteration the CPU oracle uses), for mass densities rY(k) [any unit] of total 1 / inv_rho.
 // h(T) of a mixture is one NASA-7 polynomial whose coefficients are the species' sums, so they are
 // formed once (six multiply-adds a species) and an iteration costs a dozen FP64 operations instead
-// of eleven a species; they are formed again only when T crosses a species' Tmid. The sums carry
-// the rounding of the per-species form (1e-16 of the largest term).
-// Measured (53 species, 202,752 cells): T from rho h 685 -> 273 us.
+// of eleven a species; they are formed again only when T crosses a species' Tmid. Where all species
+// share one Tmid, hmid_sum, the sum of rY(k) h_mid(k), tells on which side the solution lies, and the
+// iteration starts there: of 32 cells one or two cross, and a warp pays for its slowest. The sums
+// carry the rounding of the per-species form (1e-16 of the largest term).
+// Measured (53 species, 202,752 cells): T from rho h 685 -> 273 us, with hmid_sum and the range of T
+// compared as integers 190 us.
 template <class Tab, class GetY>
-__device__ __forceinline__ double hy2t_mixture(double htarget, GetY rY, double inv_rho, double T, double tmin,
-                                               double tmax) {
+__device__ __forceinline__ double hy2t_mixture(double htarget, GetY rY, double inv_rho, double hmid_sum, double T,
+                                               double tmin, double tmax) {
   if (!(T > tmin && T < tmax)) T = 1000.0;
+  if constexpr (Tab::TMID > 0.0) {
+    const double hm = hmid_sum * inv_rho * kRerg;
+    if (Tab::TMID > tmin && Tab::TMID < tmax) {
+      if (htarget > hm && T < Tab::TMID) T = Tab::TMID;
+      // just below, so that the low range holds
+      if (htarget < hm && T >= Tab::TMID) T = __longlong_as_double(__double_as_longlong(Tab::TMID) - 1);
+    }
+  }
   double c[6], t_lo = 0.0, t_hi = -1.0;  // the coefficients hold for t_lo <= T < t_hi
 #pragma unroll
   for (int i = 0; i < 6; ++i) c[i] = 0.0;
@@ -103,12 +114,21 @@ __device__ __forceinline__ double hy2t_mixture(double htarget, GetY rY, double i
       t_hi = 1e300;
 #pragma unroll
       for (int i = 0; i < 6; ++i) c[i] = 0.0;
-#pragma unroll 2
+      if constexpr (Tab::TMID > 0.0) {
+        if (T < Tab::TMID) t_hi = Tab::TMID;
+        else t_lo = Tab::TMID;
+      }
+#pragma unroll 3
       for (int k = 0; k < Tab::NS; ++k) {
         const TabSpecies<double>& s = Tab::template sp<double>(k);
-        const bool lo = T < s.Tmid;
-        if (lo) t_hi = fmin(t_hi, s.Tmid);
-        else t_lo = fmax(t_lo, s.Tmid);
+        bool lo;
+        if constexpr (Tab::TMID > 0.0) {
+          lo = t_lo == 0.0;
+        } else {
+          lo = below_positive(T, s.Tmid);
+          if (lo) t_hi = fmin(t_hi, s.Tmid);
+          else t_lo = fmax(t_lo, s.Tmid);
+        }
         const double y = rY(k);
 #pragma unroll
         for (int i = 0; i < 6; ++i) c[i] = fma(y, lo ? s.wlo[i] : s.whi[i], c[i]);
@@ -118,7 +138,7 @@ __device__ __forceinline__ double hy2t_mixture(double htarget, GetY rY, double i
     }
     const double hh = fma(T, fma(T, fma(T, fma(T, fma(T, c[4], c[3]), c[2]), c[1]), c[0]), c[5]);
     const double cp = fma(T, fma(T, fma(T, fma(T, 5.0 * c[4], 4.0 * c[3]), 3.0 * c[2]), 2.0 * c[1]), c[0]);
-    double dT = (htarget - hh) / cp;
+    double dT = pgb_div64(htarget - hh, cp);
     dT = fmax(-100.0, fmin(100.0, dT));
     T = fmax(tmin, fmin(tmax, T + dT));
     if (fabs(dT) < 1e-10 * T) break;

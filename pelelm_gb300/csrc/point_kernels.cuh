@@ -61,9 +61,12 @@ __global__ void rates_kernel(const PointParams p) {
 #pragma unroll
   for (int s = 0; s < M::NS; ++s) { Y[s] = arr_at(p.rY, i, j, k, s); rho += Y[s]; }
   const double inv_rho = 1.0 / rho;
+  double hm = 0.0;
+#pragma unroll
+  for (int s = 0; s < M::NS; ++s) hm = fma(Y[s], M::Tab::h_mid(s), hm);
   // MKS -> CGS: h [J/kg] * 1e4 = erg/g ; rho [kg/m^3] * 1e-3 = g/cm^3
   const double T = hy2t_mixture<typename M::Tab>(arr_at(p.rE, i, j, k, 0) * inv_rho * 1.0e4,
-                                                 [&](int s) { return arr_at(p.rY, i, j, k, s); }, inv_rho,
+                                                 [&](int s) { return arr_at(p.rY, i, j, k, s); }, inv_rho, hm,
                                                  arr_at(p.T, i, j, k, 0), 90.0, 5000.0);
 #pragma unroll
   for (int s = 0; s < M::NS; ++s) C[s] = Y[s] * (1.0e-3 / M::W(s));
@@ -80,13 +83,18 @@ __global__ void h2t_kernel(const PointParams p) {
   const int i = p.lo0 + (int)(c % p.len0);
   const int j = p.lo1 + (int)((c / p.len0) % p.len1);
   const int k = p.lo2 + (int)(c / ((long long)p.len0 * p.len1));
-  double rho = 0.0;
-#pragma unroll 4
-  for (int s = 0; s < M::NS; ++s) rho += arr_at(p.rY, i, j, k, s);
+  double rho = 0.0, hm = 0.0;
+#pragma unroll 8
+  for (int s = 0; s < M::NS; ++s) {
+    const double v = arr_at(p.rY, i, j, k, s);
+    rho += v;
+    hm = fma(v, M::Tab::h_mid(s), hm);
+  }
   const double inv_rho = 1.0 / rho;
   double& T = arr_at(p.T, i, j, k, 0);
   T = hy2t_mixture<typename M::Tab>(arr_at(p.rE, i, j, k, 0) * inv_rho * 1.0e4,
-                                    [&](int s) { return arr_at(p.rY, i, j, k, s); }, inv_rho, T, p.tmin, p.tmax);
+                                    [&](int s) { return arr_at(p.rY, i, j, k, s); }, inv_rho, hm, T, p.tmin,
+                                    p.tmax);
 }
 
 // Heat release rate -sum_k rhoYdot_k h_k(T) [W/m^3] from T and the MKS reaction rates
@@ -106,7 +114,7 @@ __global__ void heat_release_kernel(const PointParams p) {
 #pragma unroll 3
   for (int s = 0; s < M::NS; ++s) {
     const TabSpecies<double>& sp = Tab::template sp<double>(s);
-    const bool lo = T < sp.Tmid;
+    const bool lo = below_positive(T, sp.Tmid);
     double a[6];
 #pragma unroll
     for (int q = 0; q < 6; ++q) a[q] = lo ? sp.wlo[q] : sp.whi[q];

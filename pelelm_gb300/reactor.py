@@ -32,14 +32,9 @@ def array4(t, lo=(0, 0, 0)) -> Array4:
     st = t.stride()
     if st[3] != 1:
         raise ValueError("the i direction must be contiguous")
-    a = Array4()
-    a.p = t.data_ptr()
-    a.jstride, a.kstride, a.nstride = st[2], st[1], st[0]
     nc, nz, ny, nx = t.shape
-    a.begin = (C.c_int * 3)(lo[0], lo[1], lo[2])
-    a.end = (C.c_int * 3)(lo[0] + nx, lo[1] + ny, lo[2] + nz)
-    a.ncomp = nc
-    return a
+    x, y, z = lo
+    return Array4(t.data_ptr(), st[2], st[1], st[0], (x, y, z), (x + nx, y + ny, z + nz), nc)
 
 
 @dataclass
@@ -55,18 +50,9 @@ class BoxArrays:
     mask: Optional[object] = None
 
     def view(self) -> BoxView:
-        lo = self.box[0]
-        v = BoxView()
-        v.box.lo = (C.c_int * 3)(*self.box[0])
-        v.box.hi = (C.c_int * 3)(*self.box[1])
-        v.rY = array4(self.rY, lo)
-        v.rY_src = array4(self.rY_src, lo)
-        v.T = array4(self.T, lo)
-        v.rEner = array4(self.rEner, lo)
-        v.rEner_src = array4(self.rEner_src, lo)
-        v.FC = array4(self.FC, lo)
-        v.mask = array4(self.mask, lo) if self.mask is not None else Array4()
-        return v
+        lo, hi = self.box
+        return BoxView(_lib.Box(tuple(lo), tuple(hi)), array4(self.rY, lo), array4(self.rY_src, lo), array4(self.T, lo),
+                       array4(self.rEner, lo), array4(self.rEner_src, lo), array4(self.FC, lo), array4(self.mask, lo))
 
 
 def _stream_ptr(stream) -> Optional[int]:
@@ -141,14 +127,10 @@ class ReactorGB:
         (NUM_SPECIES, nz, ny, nx) tensors, one per box) in one launch."""
         views = []
         for b, box in enumerate(boxes):
-            v = _lib.ChemView()
-            lo = box.box[0]
-            for d in range(3):
-                v.box.lo[d], v.box.hi[d] = box.box[0][d], box.box[1][d]
-            v.rhoY, v.rhoY_src, v.T = array4(box.rY, lo), array4(box.rY_src, lo), array4(box.T, lo)
-            v.rhoH, v.rhoH_src, v.FC = array4(box.rEner, lo), array4(box.rEner_src, lo), array4(box.FC, lo)
-            v.mask = array4(box.mask, lo) if box.mask is not None else _lib.Array4()
-            v.I_R = array4(I_R[b], lo) if I_R is not None else _lib.Array4()
+            lo, hi = box.box
+            v = _lib.ChemView(_lib.Box(tuple(lo), tuple(hi)), array4(box.rY, lo), array4(box.rY_src, lo),
+                              array4(box.T, lo), array4(box.rEner, lo), array4(box.rEner_src, lo), array4(box.FC, lo),
+                              array4(box.mask, lo), array4(I_R[b] if I_R is not None else None, lo))
             views.append(v)
         arr = (_lib.ChemView * len(views))(*views)
         check(lib().pgb_advance_chemistry(self._h, arr, len(views), float(dt), _stream_ptr(stream)),
@@ -229,10 +211,7 @@ def rhoh_to_temp(mechanism: str, box: Box, rhoY, rhoH, T, tmin=90.0, tmax=5000.0
 
 def heat_release(mechanism: str, box: Box, T, rhoYdot, out, stream=None) -> None:
     """HeatRelease derive over a box (MKS): out = -sum_k rhoYdot_k h_k(T) [W/m^3]."""
-    from ._lib import Box as CBox
-    b = CBox()
-    for d in range(3):
-        b.lo[d], b.hi[d] = box[0][d], box[1][d]
+    b = _lib.Box(tuple(box[0]), tuple(box[1]))
     check(lib().pgb_heat_release(mechanism.encode(), C.byref(b), C.byref(array4(T, box[0])),
                                  C.byref(array4(rhoYdot, box[0])), C.byref(array4(out, box[0])),
                                  _stream_ptr(stream)), "heat_release")
