@@ -726,38 +726,64 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
     }
     // rho h(t) = rho h0 + F_h t ; T from (h, Y) by Newton with the integrated T as guess
     const double rE = fma(tout, C.FRC[NS], rE0);
-    double rho_l = 0.0;
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-      if (idx(r) < NS) rho_l += Z(0, r);
-    const double inv_rho = pgb_div64(1.0, group_sum<G>(rho_l, gm));
-    const double htarget = rE * inv_rho;
     double Tn = C.Z[NS];
     if (!(Tn > 90.0 && Tn < 5000.0)) Tn = 1000.0;
+    if constexpr (UNROLLED) {  // as the per-thread kernel does
+      double rho = 0.0, hm = 0.0;
 #pragma unroll 1
-    for (int it = 0; it < 50; ++it) {
-      double hl = 0.0, cl = 0.0;
+      for (int k = 0; k < NS; ++k) {
+        rho += C.Z[k];
+        hm = fma(C.Z[k], M::Tab::h_mid(k), hm);
+      }
+      const double inv_rho = 1.0 / rho;
+      Tn = hy2t_mixture<typename M::Tab>(rE * inv_rho, [&](int k) { return C.Z[k]; }, inv_rho, hm, Tn, 90.0, 5000.0);
+    } else {
+      // sums over species in the order of S lanes
+      auto sum_of = [&](const double (&u)[R], const double (&v)[R]) -> double {
+        if constexpr (S == G) {
+          double x = 0.0;
+#pragma unroll
+          for (int r = 0; r < R; ++r)
+            if (idx(r) < NS) x = fma(u[r], v[r], x);
+          return group_sum<G>(x, gm);
+        } else {
+          return lane_dot<NS, S>(u[0], v[0], gm, gbase);
+        }
+      };
+      double y0[R], one[R];
 #pragma unroll
       for (int r = 0; r < R; ++r) {
-        const int k = idx(r);
-        if (k < NS) {
-          const TabSpecies<double>& s = Tab::template sp<double>(k);
-          const bool lo = Tn < s.Tmid;
-          const double* a = lo ? s.lo : s.hi;
-          const double* hc = lo ? s.hlo : s.hhi;
-          const double invTn = 1.0 / Tn;
-          const double hRT = fma(Tn, fma(Tn, fma(Tn, fma(Tn, hc[4], hc[3]), hc[2]), hc[1]), fma(hc[5], invTn, hc[0]));
-          const double cpR = fma(Tn, fma(Tn, fma(Tn, fma(Tn, a[4], a[3]), a[2]), a[1]), a[0]);
-          const double Yk = Z(0, r) * inv_rho;
-          hl = fma(Yk * s.invW, hRT * kRerg * Tn, hl);
-          cl = fma(Yk * s.invW, cpR * kRerg, cl);
-        }
+        y0[r] = idx(r) < NS ? Z(0, r) : 0.0;
+        one[r] = 1.0;
       }
-      const double hh = group_sum<G>(hl, gm), cp = group_sum<G>(cl, gm);
-      double dT = pgb_div64(htarget - hh, cp);
-      dT = fmax(-100.0, fmin(100.0, dT));
-      Tn = fmax(90.0, fmin(5000.0, Tn + dT));
-      if (fabs(dT) < 1e-10 * Tn) break;
+      const double inv_rho = pgb_div64(1.0, sum_of(y0, one));
+      const double htarget = rE * inv_rho;
+#pragma unroll 1
+      for (int it = 0; it < 50; ++it) {
+        const double invTn = pgb_div64(1.0, Tn);
+        double yw[R], hk[R], ck[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const int k = idx(r);
+          yw[r] = hk[r] = ck[r] = 0.0;
+          if (k < NS) {
+            const TabSpecies<double>& s = Tab::template sp<double>(k);
+            const bool lo = below_positive(Tn, s.Tmid);
+            const double* a = lo ? s.lo : s.hi;
+            const double* hc = lo ? s.hlo : s.hhi;
+            const double hRT = fma(Tn, fma(Tn, fma(Tn, fma(Tn, hc[4], hc[3]), hc[2]), hc[1]), fma(hc[5], invTn, hc[0]));
+            const double cpR = fma(Tn, fma(Tn, fma(Tn, fma(Tn, a[4], a[3]), a[2]), a[1]), a[0]);
+            yw[r] = y0[r] * inv_rho * s.invW;
+            hk[r] = hRT * kRerg * Tn;
+            ck[r] = cpR * kRerg;
+          }
+        }
+        const double hh = sum_of(yw, hk), cp = sum_of(yw, ck);
+        double dT = pgb_div64(htarget - hh, cp);
+        dT = fmax(-100.0, fmin(100.0, dT));
+        Tn = fmax(90.0, fmin(5000.0, Tn + dT));
+        if (fabs(dT) < 1e-10 * Tn) break;
+      }
     }
 #pragma unroll
     for (int r = 0; r < R; ++r)
@@ -820,6 +846,83 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
     return true;
   };
 
+  // hands the group's cell over at the start of a step; the group rests
+  auto hand_over = [&]() {
+    unsigned long long at = 0;
+    if (sub == 0) at = atomicAdd(P.resume_count, 1ull);
+    const ResumeRec<N, JR> rec(P.resume, __shfl_sync(gm, at, gbase));
+    if (sub == 0) {
+      ResumeHead H;
+      H.t = t; H.h = h; H.hscale = hscale; H.etamax = etamax; H.gammap = gammap; H.crate2 = crate2;
+      H.tq5_saved = tq5_saved;
+      H.cell = cell;
+      H.box = box; H.ci = ci; H.cj = cj; H.ck = ck;
+      H.q = q; H.qwait = qwait; H.nst = nst; H.nfe = nfe; H.nje = nje; H.nstlp = nstlp; H.netf = netf; H.ncfn = ncfn;
+      H.force_setup = force_setup;
+      H.full_swaps = 1;
+      *rec.head = H;
+    }
+#pragma unroll 1
+    for (int e = sub; e < (QMAX + 2) * N; e += G) rec.Z[e] = C.Z[e];
+#pragma unroll 1
+    for (int e = sub; e < QMAX + 2; e += G) rec.tau[e] = C.TAU[e];
+#pragma unroll 1
+    for (int e = sub; e < N * N; e += G) rec.lu[e] = C.A[e + e / N];  // rows of N + 1
+#pragma unroll 1
+    for (int e = sub; e < N; e += G) rec.piv[e] = C.PIV[e];
+    phase = IDLE;
+  };
+  // takes over record i
+  auto take_over = [&](unsigned long long i) {
+    const ResumeRec<N, JR> rec(P.resume, i);
+    const ResumeHead& H = *rec.head;
+    cell = H.cell;
+    box = H.box; ci = H.ci; cj = H.cj; ck = H.ck;
+    const BoxDev& B = P.boxes[box];
+#pragma unroll 1
+    for (int e = sub; e < (QMAX + 2) * N; e += G) C.Z[e] = rec.Z[e];
+#pragma unroll 1
+    for (int e = sub; e < QMAX + 2; e += G) C.TAU[e] = rec.tau[e];
+#pragma unroll 1
+    for (int e = sub; e < N * N; e += G) C.A[e + e / N] = rec.lu[e];
+#pragma unroll 1
+    for (int e = sub; e < N; e += G) {
+      C.PIV[e] = H.full_swaps ? rec.piv[e] : e;
+      C.FRC[e] = e < NS ? elem(B.rYsrc, e) * B.sY_in : elem(B.rEsrc, 0) * B.sE_in;
+    }
+    rE0 = elem(B.rE, 0) * B.sE_in;
+    t = H.t; h = H.h; hscale = H.hscale; etamax = H.etamax; eta = 1.0;
+    gamma = 0.0; gammap = H.gammap; gamrat = 1.0; crate2 = H.crate2; rl1 = 1.0;
+    tq1 = tq2 = tq3 = tq5 = inv_tq4_sq = 1.0;
+    tq5_saved = H.tq5_saved;
+    q = H.q; qwait = H.qwait; nef = 0; ncf = 0; m = 0; status = OK;
+    nst = H.nst; nfe = H.nfe; nje = H.nje; nstlp = H.nstlp; netf = H.netf; ncfn = H.ncfn;
+    new_step = true; need_setup = false; force_setup = H.force_setup != 0; jcur = false; fresh = false;
+    __syncwarp(gm);
+    if (!H.full_swaps) {
+      // the per-thread kernel exchanges rows right of the pivot: exchange the multipliers too
+      if (sub == 0) {
+#pragma unroll 1
+        for (int k = 0; k < N; ++k) {
+          const int p = rec.piv[k];
+          if (p == k) continue;
+          const int i0 = C.PIV[k];
+          C.PIV[k] = C.PIV[p];
+          C.PIV[p] = i0;
+#pragma unroll 1
+          for (int j = 0; j < k; ++j) {
+            const JR a = C.A[k * LDA + j];
+            C.A[k * LDA + j] = C.A[p * LDA + j];
+            C.A[p * LDA + j] = a;
+          }
+        }
+      }
+      __syncwarp(gm);
+    }
+    phase = STEP;
+  };
+  bool queue_empty = false;
+
   for (;;) {
     // ------------------------------------------------ (A) work stealing, one atomic per warp
     {
@@ -830,14 +933,24 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
         if (lane == leader) base = atomicAdd(P.next_cell, (unsigned long long)__popc(need));
         base = __shfl_sync(0xffffffffu, base, leader);
         const long long c = (long long)base + __popc(need & ((1u << gbase) - 1u));
+        bool past_end = false;
         if (phase == NEED) {
           if (c >= ncell) {
             phase = IDLE;
+            past_end = true;
+          } else if (S != G && P.resuming) {
+            take_over((unsigned long long)c);
           } else {
             cell = P.cell_list ? P.cell_list[c] : c;
             if (load_cell(cell)) phase = START;  // covered cells stay NEED and refetch next pass
           }
         }
+        queue_empty = __any_sync(0xffffffffu, past_end) || queue_empty;
+      }
+      if (S == G && queue_empty && P.drain > 0) {
+        const unsigned left = __ballot_sync(0xffffffffu, phase != IDLE && sub == 0);
+        if (__popc(left) <= P.drain && phase == STEP && new_step && nst < P.max_steps) hand_over();
+        __syncwarp();
       }
       if (__all_sync(0xffffffffu, phase == IDLE)) break;
     }

@@ -460,6 +460,30 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
     return true;
   };
 
+  // hands this lane's cell over at the start of a step
+  auto hand_over = [&]() {
+    const ResumeRec<N, JR> rec(P.resume, atomicAdd(P.resume_count, 1ull));
+    ResumeHead H;
+    H.t = t; H.h = h; H.hscale = hscale; H.etamax = etamax; H.gammap = gammap; H.crate2 = crate2; H.tq5_saved = tq5_saved;
+    H.cell = cell;
+    H.box = box; H.ci = ci; H.cj = cj; H.ck = ck;
+    H.q = q; H.qwait = qwait; H.nst = (int)nst; H.nfe = (int)nfe; H.nje = (int)nje; H.nstlp = (int)nstlp;
+    H.netf = (int)netf; H.ncfn = (int)ncfn;
+    H.force_setup = force_setup;
+    H.full_swaps = 0;
+    *rec.head = H;
+#pragma unroll 1
+    for (int e = 0; e < (QMAX + 2) * N; ++e) rec.Z[e] = Z(0, e);
+#pragma unroll 1
+    for (int j = 0; j < QMAX + 2; ++j) rec.tau[j] = TAU(j);
+#pragma unroll 1
+    for (int e = 0; e < N * N; ++e) rec.lu[e] = LU(0, e);
+#pragma unroll 1
+    for (int k = 0; k < N; ++k) rec.piv[k] = PIV(k);
+    phase = IDLE;
+  };
+  bool queue_empty = false;
+
   for (;;) {
     // ------------------------------------------------ (A) work stealing
     const unsigned need = __ballot_sync(0xffffffffu, phase == NEED);
@@ -468,15 +492,23 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
       unsigned long long base = 0;
       if (lane == leader) base = atomicAdd(P.next_cell, (unsigned long long)__popc(need));
       base = __shfl_sync(0xffffffffu, base, leader);
+      bool past_end = false;
       if (phase == NEED) {
         const long long c = (long long)base + __popc(need & ((1u << lane) - 1u));
         if (c >= ncell) {
           phase = IDLE;
+          past_end = true;
         } else {
           cell = P.cell_list ? P.cell_list[c] : c;
           if (load_cell(cell)) phase = START;  // masked cells stay NEED and refetch next pass
         }
       }
+      queue_empty = __any_sync(0xffffffffu, past_end) || queue_empty;
+    }
+    if (queue_empty && P.drain > 0) {
+      const unsigned left = __ballot_sync(0xffffffffu, phase != IDLE);
+      if (__popc(left) <= P.drain && phase == STEP && new_step && nst < P.max_steps) hand_over();
+      __syncwarp();
     }
     if (__all_sync(0xffffffffu, phase == IDLE)) break;
 

@@ -193,7 +193,9 @@ struct Scratch {
   pgb::BoxDev* d_boxes = nullptr;
   size_t box_cap = 0;
   pgb::BoxDev* h_boxes = nullptr;  // pinned staging
-  unsigned long long* d_counter = nullptr;
+  unsigned long long* d_counter = nullptr;  // queue head; queue head and count of handed-over cells
+  void* d_resume = nullptr;        // handed-over cells
+  size_t resume_cap = 0;
   void* d_z = nullptr;             // Nordsieck histories of the resident threads
   size_t z_cap = 0;
   void* d_lu = nullptr;            // Jacobian/LU slices of the resident threads
@@ -243,6 +245,7 @@ void free_scratch(Scratch& s) {
   if (s.d_boxes) cudaFree(s.d_boxes);
   if (s.h_boxes) cudaFreeHost(s.h_boxes);
   if (s.d_counter) cudaFree(s.d_counter);
+  if (s.d_resume) cudaFree(s.d_resume);
   if (s.d_stats) cudaFree(s.d_stats);
   if (s.d_z) cudaFree(s.d_z);
   if (s.d_lu) cudaFree(s.d_lu);
@@ -259,7 +262,7 @@ void free_scratch(Scratch& s) {
 int ensure_scratch(pgb_reactor* r, cudaStream_t st, size_t nbox, Scratch** out) {
   Scratch& s = r->scratch[st];
   if (!s.d_counter) {
-    PGB_CUDA(cudaMalloc(&s.d_counter, sizeof(unsigned long long)));
+    PGB_CUDA(cudaMalloc(&s.d_counter, 3 * sizeof(unsigned long long)));
     PGB_CUDA(cudaMalloc(&s.d_stats, sizeof(pgb::ReactStats)));
     PGB_CUDA(cudaMalloc(&s.d_retry_count, sizeof(unsigned long long)));
     PGB_CUDA(cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming));
@@ -298,6 +301,8 @@ struct LaunchPlan {
   bool group = false;  // group-per-cell kernel; tpb then holds lanes per cell
   bool small = false;  // small-launch kernel; tpb then holds warps per block
   int cells_per_warp = 0;  // 0: all that the mapping holds
+  int drain = 0;           // cells left in a warp when it hands them over (0: never)
+  size_t resume_bytes = 0;
 };
 
 int mapping_of(const pgb_reactor* r);
@@ -311,6 +316,20 @@ int mapping_of(const pgb_reactor* r);
 // 22.6 / 22.9. At 1e-6 s, where cells differ less, the lines lie at about 7,000 and 5,800 cells.
 long long small_limit(const pgb_reactor* r) {
   return (long long)r->nsm * (r->mech->ns <= 12 ? 48 : 40);
+}
+
+// A launch that chose its mapping itself hands the last cells of each warp (`left` at most) to the
+// small-launch kernel, once the queue is empty: they are its stiffest, and alone in a warp a cell is as
+// slow as a full one. The two kernels agree bit for bit, so a cell may change between them at the
+// start of any step. Callers ask for it only where they do: unrolled per-thread code, groups of 8.
+// `left` measured, mixed precision: 9 species, 18,432 cells, dt_react 1e-5 s: never 32.3 ms, 6 29.9,
+// 10 25.8, 16 22.6, 24 23.1; 32,768 cells at 1e-6 s: 8.2, 8.0, 7.8, 8.3, 9.3 (13 is between). 21
+// species, 8,000 cells: never 20.2 ms, 1 19.0, 2 18.3, 3 18.4, 4 18.9; 16,384 cells at 1e-6 s: 11.0,
+// 11.2, 11.2, 11.7.
+void set_drain(const pgb_reactor* r, LaunchPlan& pl, long long warps, bool mixed, int left) {
+  if (!r->small_ok || !r->mech->small_mixed) return;
+  pl.drain = left;
+  pl.resume_bytes = (size_t)(warps * left) * (mixed ? r->mech->resume_mixed : r->mech->resume_fp64);
 }
 
 // First layout (all shared; global Nordsieck history; global history and LU) whose shared
@@ -337,6 +356,7 @@ LaunchPlan plan_launch(const pgb_reactor* r, long long ncell, bool mixed) {
     const int per_block = (mixed ? m.group_cells_mixed : m.group_cells_fp64)(G);
     pl.group = true;
     pl.tpb = G;
+    if (G == 8) set_drain(r, pl, (long long)r->nsm * std::max(per_block * G / 32, 1), mixed, 2);
     pl.nblocks = (int)std::min<long long>(r->nsm, std::max<long long>(1, (ncell + per_block - 1) / std::max(per_block, 1)));
     return pl;
   }
@@ -373,6 +393,7 @@ LaunchPlan plan_launch(const pgb_reactor* r, long long ncell, bool mixed) {
   // persistent grid: one CTA per SM, never more CTAs than there are blocks' worth of cells
   const long long max_blocks = std::max<long long>(1, (ncell + pl.tpb - 1) / pl.tpb);
   pl.nblocks = (int)std::min<long long>(r->nsm, max_blocks);
+  if (m.small_lanes == 16) set_drain(r, pl, (long long)r->nsm * (pl.tpb / 32), mixed, 13);
   const int N = m.ns + 1;
   const size_t slots = (size_t)pl.nblocks * pl.tpb;
   if (pl.z_global) pl.z_bytes = slots * (pgb::QMAX + 2) * N * sizeof(double);
@@ -431,7 +452,7 @@ int enqueue_advance(pgb_reactor* r, Scratch& s, int nbox, long long ncell, doubl
   p.next_cell = s.d_counter;
   p.stats = s.d_stats;
   PGB_CUDA(cudaMemcpyAsync(s.d_boxes, s.h_boxes, nbox * sizeof(pgb::BoxDev), cudaMemcpyHostToDevice, st));
-  PGB_CUDA(cudaMemsetAsync(s.d_counter, 0, sizeof(unsigned long long), st));
+  PGB_CUDA(cudaMemsetAsync(s.d_counter, 0, 3 * sizeof(unsigned long long), st));
   PGB_CUDA(cudaMemsetAsync(s.d_stats, 0, sizeof(pgb::ReactStats), st));
   if (ncell == 0) return 0;
   if (r->null_reactor) {
@@ -456,8 +477,23 @@ int enqueue_advance(pgb_reactor* r, Scratch& s, int nbox, long long ncell, doubl
     p.retry_count = s.d_retry_count;
     PGB_CUDA(cudaMemsetAsync(s.d_retry_count, 0, sizeof(unsigned long long), st));
   }
+  if (pl.drain > 0 && s.d_resume && s.resume_cap >= pl.resume_bytes) {
+    p.resume = static_cast<unsigned char*>(s.d_resume);
+    p.resume_count = s.d_counter + 2;
+    p.drain = pl.drain;
+  }
   auto run_bdf = [&]() -> int {
     if (fn(p, pl.tpb, st, pl.nblocks)) return -1;
+    if (p.resume) {  // the cells it left unfinished, with more lanes each
+      pgb::ReactParams m = p;
+      m.ncell_dev = p.resume_count;
+      m.cell_list = nullptr;
+      m.next_cell = s.d_counter + 1;
+      m.drain = 0;
+      m.resuming = 1;
+      m.cells_per_warp = 0;
+      if ((r->opt.mixed ? r->mech->small_mixed : r->mech->small_fp64)(m, kSmallWarps, st, r->nsm)) return -1;
+    }
     if (!retry) return 0;
     const LaunchPlan p64 = plan_launch(r, ncell, false);
     pgb::ReactParams q = p;
@@ -465,6 +501,8 @@ int enqueue_advance(pgb_reactor* r, Scratch& s, int nbox, long long ncell, doubl
     q.ncell_dev = p.retry_count;
     q.retry_list = nullptr;
     q.retry_count = nullptr;
+    q.resume = nullptr;
+    q.drain = 0;
     q.lu_scratch = p64.lu_bytes ? s.d_lu : nullptr;
     q.z_scratch = p64.z_bytes ? s.d_z : nullptr;
     PGB_CUDA(cudaMemsetAsync(s.d_counter, 0, sizeof(unsigned long long), st));
@@ -685,7 +723,7 @@ int run_autotune(pgb_reactor* r, const std::vector<pgb::BoxDev>& boxes, long lon
     pgb_tune::gather_sample_kernel<<<(int)std::min<long long>((nsample + 255) / 256, 1024), 256, 0, st>>>(
         d_src, (int)boxes.size(), ns, nsample, stride, pristine);
     if (cudaGetLastError() != cudaSuccess) { fail("gather launch"); break; }
-    if (cudaMalloc(&sc.d_counter, sizeof(unsigned long long)) != cudaSuccess ||
+    if (cudaMalloc(&sc.d_counter, 3 * sizeof(unsigned long long)) != cudaSuccess ||
         cudaMalloc(&sc.d_stats, sizeof(pgb::ReactStats)) != cudaSuccess ||
         cudaMalloc(&sc.d_boxes, sizeof(pgb::BoxDev)) != cudaSuccess ||
         cudaMallocHost(&sc.h_boxes, sizeof(pgb::BoxDev)) != cudaSuccess) { fail("out of memory"); break; }
@@ -765,7 +803,8 @@ int advance_box_table(pgb_reactor* r, const std::vector<pgb::BoxDev>& boxes, lon
       pl.lu_bytes = std::max(pl.lu_bytes, p64.lu_bytes);
       if (ensure_buf(*s, s->d_retry, s->retry_cap, std::max<long long>(ncell, 1) * sizeof(long long))) return -1;
     }
-    if (ensure_buf(*s, s->d_z, s->z_cap, pl.z_bytes) || ensure_buf(*s, s->d_lu, s->lu_cap, pl.lu_bytes))
+    if (ensure_buf(*s, s->d_z, s->z_cap, pl.z_bytes) || ensure_buf(*s, s->d_lu, s->lu_cap, pl.lu_bytes) ||
+        ensure_buf(*s, s->d_resume, s->resume_cap, pl.resume_bytes))
       return -1;
     if (r->sg.d_net) {
       const long long acap = audit_capacity(r, ncell);

@@ -241,6 +241,7 @@ struct MechEntry {
   int (*newton_fn)(const pgb::NewtonMatrixParams&, int mapping, int fp64, cudaStream_t);  // diagnostic
   LaunchFn small_mixed, small_fp64;  // small launches (argument: warps per block), or null
   int small_lanes;                   // their lanes per cell
+  int resume_mixed, resume_fp64;     // bytes of a handed-over cell
 };
 
 
@@ -390,7 +391,8 @@ int h2t_entry(const pgb_box_view* v, double tmin, double tmax, cudaStream_t s) {
     }                                                                                        \
     , ::pgb_host::heat_release_entry<M>, nullptr, nullptr, nullptr, nullptr,                \
         ::pgb_host::newton_matrix_entry<M, true>, ::pgb_host::launch_bdf_small<M, float>,    \
-        ::pgb_host::launch_bdf_small<M, double>, ::pgb_host::small_lanes<M>()                \
+        ::pgb_host::launch_bdf_small<M, double>, ::pgb_host::small_lanes<M>(),               \
+        pgb::resume_bytes<M::N, float>(), pgb::resume_bytes<M::N, double>()                  \
   }
 
 // Mechanisms whose cells also run group-per-cell (the 21-species size): all of the above plus
@@ -416,7 +418,8 @@ int h2t_entry(const pgb_box_view* v, double tmin, double tmax, cudaStream_t s) {
         ::pgb_host::launch_bdf_group<M, double>, ::pgb_host::group_cells_per_block<M, float>, \
         ::pgb_host::group_cells_per_block<M, double>,                                        \
         ::pgb_host::newton_matrix_entry<M, true>, ::pgb_host::launch_bdf_small<M, float>,    \
-        ::pgb_host::launch_bdf_small<M, double>, ::pgb_host::small_lanes<M>()                \
+        ::pgb_host::launch_bdf_small<M, double>, ::pgb_host::small_lanes<M>(),               \
+        pgb::resume_bytes<M::N, float>(), pgb::resume_bytes<M::N, double>()                  \
   }
 
 // Mechanisms too large for one cell per thread: warp-per-cell BDF, ReactorNull and T(h, Y) only.
@@ -432,7 +435,7 @@ int h2t_entry(const pgb_box_view* v, double tmin, double tmax, cudaStream_t s) {
           ::pgb_host::warp_wpb_choice<M>(2), ::pgb_host::warp_wpb_choice<M>(3)               \
     }                                                                                        \
     , ::pgb_host::heat_release_entry<M>, nullptr, nullptr, nullptr, nullptr,                \
-        ::pgb_host::newton_matrix_entry<M, false>, nullptr, nullptr, 0                       \
+        ::pgb_host::newton_matrix_entry<M, false>, nullptr, nullptr, 0, 0, 0                 \
   }
 
 // Converts and validates one box view into its device descriptor; cell numbering of the box

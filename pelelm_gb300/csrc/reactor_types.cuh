@@ -71,6 +71,42 @@ struct ReactParams {
   unsigned long long* retry_count;
   // Cells that a warp works on at a time (0: all that its mapping holds).
   int cells_per_warp;
+  // Hand-over of unfinished cells (all null / 0: none). Once the queue is empty, a warp with at most
+  // `drain` cells left writes each of them to the next record of `resume` when it reaches the start of
+  // a step; a launch with `resuming` set takes its cells from those records.
+  unsigned char* resume;
+  unsigned long long* resume_count;
+  int drain, resuming;
+};
+
+// One handed-over cell: what a BDF integration needs at the start of a step.
+struct ResumeHead {
+  double t, h, hscale, etamax, gammap, crate2, tq5_saved;
+  long long cell;
+  int box, ci, cj, ck;
+  int q, qwait, nst, nfe, nje, nstlp, netf, ncfn;
+  int force_setup, full_swaps;  // full_swaps: rows of the factors moved whole (else: right of the pivot)
+};
+// Record: head, Nordsieck columns and the saved correction ((QMAX + 2) N), step history (QMAX + 2),
+// factors (N N, row-major, type JR), pivots (N).
+template <int N, class JR>
+__host__ __device__ constexpr int resume_bytes() {
+  return ((int)sizeof(ResumeHead) + ((QMAX + 2) * N + QMAX + 2) * 8 + N * N * (int)sizeof(JR) + N * 4 + 15) / 16 * 16;
+}
+template <int N, class JR>
+struct ResumeRec {
+  ResumeHead* head;
+  double *Z, *tau;
+  JR* lu;
+  int* piv;
+  __device__ __forceinline__ ResumeRec(unsigned char* base, unsigned long long i) {
+    unsigned char* p = base + i * resume_bytes<N, JR>();
+    head = reinterpret_cast<ResumeHead*>(p);
+    Z = reinterpret_cast<double*>(p + sizeof(ResumeHead));
+    tau = Z + (QMAX + 2) * N;
+    lu = reinterpret_cast<JR*>(tau + QMAX + 2);
+    piv = reinterpret_cast<int*>(lu + N * N);
+  }
 };
 
 }  // namespace pgb
