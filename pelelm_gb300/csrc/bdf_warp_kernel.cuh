@@ -175,11 +175,42 @@ __device__ __forceinline__ double rate_of_progress(int j, double T, double invT,
 // Right-hand side f = [W_k wdot_k + F_k, dT/dt] at y, one warp cooperating (see the kernel
 // below). One non-inlined copy serves every call site: the step loop calls it from five places
 // and inlined copies of this exp/log-heavy body overflow the instruction cache.
-template <class M>
-__device__ __noinline__ WVec<M> warp_rhs(const WVec<M> yv, double* CS, double* GS, double* QS,
-                                         const double* FRC) {
+//
+// W > 1: the warp leads a team of W warps (TP: T, 1/T, ln T, ln(P0/RT), [M] and the order, for the
+// others), which share the reactions and the species sums (team_rates).
+template <int W>
+__device__ __forceinline__ void team_sync(int id) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(32 * W) : "memory");
+}
+// Rates of progress and production rates (into CS) of one right-hand side, warp `role` of W.
+template <class M, int W>
+__device__ __forceinline__ void team_rates(int role, int id, double T, double invT, double lnT, double lnP0RT,
+                                           double Ctot, double* CS, const double* GS, double* QS) {
   using Tab = typename M::TabG;
-  constexpr int N = M::N, NS = M::NS, NR = M::NR;
+  constexpr int NS = M::NS, NR = M::NR, R = (M::N + 31) / 32;
+  const int first = 32 * role + (threadIdx.x & 31);
+  for (int j = first; j < NR; j += 32 * W) QS[j] = rate_of_progress<Tab>(j, T, invT, lnT, lnP0RT, Ctot, CS, GS);
+  if constexpr (W > 1) team_sync<W>(id);
+  else __syncwarp();
+  // production rates, the longest sums together (their FP64 time is the longest lane's of a round)
+#pragma unroll 1
+  for (int i = first; i < NS; i += 32 * W) {
+    const int k = R > 1 ? Tab::sprx_by_len(i) : i;
+    double wdot = 0.0;
+    const int e1 = Tab::sprx_end(k);
+#pragma unroll 4
+    for (int e = Tab::sprx_begin(k); e < e1; ++e) wdot = fma(Tab::sprx_nu(e), QS[Tab::sprx_j(e)], wdot);
+    CS[k] = wdot;
+  }
+  if constexpr (W > 1) team_sync<W>(id);
+  else __syncwarp();
+}
+
+template <class M, int W = 1>
+__device__ __noinline__ WVec<M> warp_rhs(const WVec<M> yv, double* CS, double* GS, double* QS,
+                                         const double* FRC, double* TP = nullptr, int id = 0) {
+  using Tab = typename M::TabG;
+  constexpr int N = M::N, NS = M::NS;
   constexpr int R = (N + 31) / 32;
   const int lane = threadIdx.x & 31;
   auto idx = [&](int r) { return lane + 32 * r; };
@@ -209,21 +240,13 @@ __device__ __noinline__ WVec<M> warp_rhs(const WVec<M> yv, double* CS, double* G
   }
   const double Ctot = warp_sum(c_loc);
   __syncwarp();
-  for (int j = lane; j < NR; j += 32) {
-    QS[j] = rate_of_progress<Tab>(j, T, invT, lnT, lnP0RT, Ctot, CS, GS);
+  if constexpr (W > 1) {
+    if (lane == 0) {
+      TP[0] = T; TP[1] = invT; TP[2] = lnT; TP[3] = lnP0RT; TP[4] = Ctot; TP[5] = 1.0;
+    }
+    team_sync<W>(id);
   }
-  __syncwarp();
-  // production rates, the longest sums together (their FP64 time is the longest lane's of a round)
-#pragma unroll 1
-  for (int i = lane; i < NS; i += 32) {
-    const int k = R > 1 ? Tab::sprx_by_len(i) : i;
-    double wdot = 0.0;
-    const int e1 = Tab::sprx_end(k);
-#pragma unroll 4
-    for (int e = Tab::sprx_begin(k); e < e1; ++e) wdot = fma(Tab::sprx_nu(e), QS[Tab::sprx_j(e)], wdot);
-    CS[k] = wdot;
-  }
-  __syncwarp();
+  team_rates<M, W>(0, id, T, invT, lnT, lnP0RT, Ctot, CS, GS, QS);
   double hs = 0.0, rcp = 0.0;
 #pragma unroll
   for (int r = 0; r < R; ++r) {
@@ -766,7 +789,8 @@ __device__ __forceinline__ void warp_lu_solve(const JR* A, const int* PIV, JR* X
   __syncwarp();
 }
 
-template <class M, class JR, int WPB>
+// W > 1: teams of W warps per cell (WPB / W cells a block), the first warp leading: for few cells.
+template <class M, class JR, int WPB, int W = 1>
 __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams P) {
   using namespace bdf;
   using Tab = typename M::TabG;
@@ -775,7 +799,9 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
   constexpr int LDA = N + 1;         // padded matrix row
   constexpr bool MIXED = sizeof(JR) == sizeof(float);
   extern __shared__ __align__(16) unsigned char wsmem[];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, wid = (threadIdx.x >> 5) / W;  // wid: the cell's place in the block
+  __shared__ double team_par[W > 1 ? WPB / W : 1][6];
+  double* const TP = team_par[W > 1 ? wid : 0];
   unsigned char* base = wsmem + (size_t)wid * bdf_warp_smem_per_warp<M, JR>();
   double* Z = reinterpret_cast<double*>(base);   // [(QMAX+2)][N]
   double* FRC = Z + (QMAX + 2) * N;              // [N] forcing (rhoY, then rho h)
@@ -791,9 +817,23 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
   JR* XS = A + N * LDA;                          // [N] solve vector
   int* PIV = reinterpret_cast<int*>(XS + N);
 
+  if constexpr (W > 1) {
+    const int role = (threadIdx.x >> 5) % W;
+    if (role > 0) {  // follow the leader's right-hand sides until it has no more cells
+      for (;;) {
+        team_sync<W>(1 + wid);
+        if (TP[5] == 0.0) return;
+        team_rates<M, W>(role, 1 + wid, TP[0], TP[1], TP[2], TP[3], TP[4], CS, GS, QS);
+      }
+    }
+  }
+
   const long long ncell = P.ncell_dev ? (long long)*P.ncell_dev : P.ncell;
   const int qmax = max(1, min(P.max_order, QMAX));
   const double tout = P.dt;
+  auto cell_done = [&]() {
+    if (P.done && lane == 0) atomicAdd(P.done, 1ull);
+  };
 
   // ---- lane-distributed vectors: element i = lane + 32 r ----
   auto idx = [&](int r) { return lane + 32 * r; };
@@ -814,7 +854,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
     WVec<M> yv;
 #pragma unroll
     for (int r = 0; r < R; ++r) yv.v[r] = y[r];
-    const WVec<M> fv = warp_rhs<M>(yv, CS, GS, QS, FRC);
+    const WVec<M> fv = warp_rhs<M, W>(yv, CS, GS, QS, FRC, TP, 1 + wid);
 #pragma unroll
     for (int r = 0; r < R; ++r) f[r] = fv.v[r];
   };
@@ -828,7 +868,9 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
     if (lane == 0) cnext = atomicAdd(P.next_cell, 1ull);
     cnext = __shfl_sync(0xffffffffu, cnext, 0);
     if ((long long)cnext >= ncell) break;
-    const long long cell = P.cell_list ? P.cell_list[cnext] : (long long)cnext;
+    const bool resuming = W > 1 && P.resuming;
+    const ResumeRec<N, JR> rec(P.resume, resuming ? cnext : 0);
+    const long long cell = resuming ? rec.head->cell : P.cell_list ? P.cell_list[cnext] : (long long)cnext;
     int lo = 0, hi = P.nbox - 1;
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
@@ -849,6 +891,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
       if (lane == 0) elem(B.FC, 0) = 0.0;
       if (B.IR.p)
         for (int k = lane; k < NS; k += 32) elem(B.IR, k) = -elem(B.rYsrc, k);
+      cell_done();
       continue;
     }
     double y[R], f[R], acor[R], tmp[R], acor_saved[R];
@@ -1057,52 +1100,106 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
     };
 
     // ---------------------------------------------- initial step size
-    rhs(y, f);
-    ++nfe;
-    set_ewt();
-    {
-      const double tround = UROUND * tout;
-      const double hlb = 100.0 * tround;
-      double hub_inv = 0.0;
+    if (!resuming) {
+      rhs(y, f);
+      ++nfe;
+      set_ewt();
+      {
+        const double tround = UROUND * tout;
+        const double hlb = 100.0 * tround;
+        double hub_inv = 0.0;
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+          if (idx(r) < N) hub_inv = fmax(hub_inv, pgb_div64(fabs(f[r]), fma(0.1, fabs(zget(0, r)), P.atol[idx(r)])));
+        hub_inv = warp_max(hub_inv);
+        double hub = 0.1 * tout;
+        if (hub * hub_inv > 1.0) hub = pgb_div64(1.0, hub_inv);
+        double hg = sqrt(hlb * hub), hnew = hg;
+        if (hub > hlb) {
+#pragma unroll 1
+          for (int count = 1; count <= 4; ++count) {
+            double yy[R], fy[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) yy[r] = idx(r) < N ? fma(hg, f[r], zget(0, r)) : 0.0;
+            rhs(yy, fy);
+            ++nfe;
+#pragma unroll
+            for (int r = 0; r < R; ++r) tmp[r] = pgb_div64(fy[r] - f[r], hg);
+            const double ydd = sqrt(wms(tmp));
+            hnew = sqrt((ydd * hub * hub > 2.0) ? pgb_div64(2.0, ydd) : hg * hub);
+            if (count == 4) break;
+            const double hrat = pgb_div64(hnew, hg);
+            if (hrat > 0.5 && hrat < 2.0) break;
+            if (count >= 2 && hrat > 2.0) { hnew = hg; break; }
+            hg = hnew;
+          }
+        }
+        h = fmin(fmax(0.5 * hnew, hlb), hub);
+      }
+      hscale = h;
 #pragma unroll
       for (int r = 0; r < R; ++r)
-        if (idx(r) < N) hub_inv = fmax(hub_inv, pgb_div64(fabs(f[r]), fma(0.1, fabs(zget(0, r)), P.atol[idx(r)])));
-      hub_inv = warp_max(hub_inv);
-      double hub = 0.1 * tout;
-      if (hub * hub_inv > 1.0) hub = pgb_div64(1.0, hub_inv);
-      double hg = sqrt(hlb * hub), hnew = hg;
-      if (hub > hlb) {
+        if (idx(r) < N) zget(1, r) = h * f[r];
+      q = 1; qwait = 2; etamax = ETAMX1;
+      if (lane == 0) TAU[1] = h;
+      __syncwarp();
+    } else {  // or the state another launch left
+      const ResumeHead& H = *rec.head;
 #pragma unroll 1
-        for (int count = 1; count <= 4; ++count) {
-          double yy[R], fy[R];
+      for (int e = lane; e < (QMAX + 1) * N; e += 32) Z[e] = rec.Z[e];
 #pragma unroll
-          for (int r = 0; r < R; ++r) yy[r] = idx(r) < N ? fma(hg, f[r], zget(0, r)) : 0.0;
-          rhs(yy, fy);
-          ++nfe;
-#pragma unroll
-          for (int r = 0; r < R; ++r) tmp[r] = pgb_div64(fy[r] - f[r], hg);
-          const double ydd = sqrt(wms(tmp));
-          hnew = sqrt((ydd * hub * hub > 2.0) ? pgb_div64(2.0, ydd) : hg * hub);
-          if (count == 4) break;
-          const double hrat = pgb_div64(hnew, hg);
-          if (hrat > 0.5 && hrat < 2.0) break;
-          if (count >= 2 && hrat > 2.0) { hnew = hg; break; }
-          hg = hnew;
-        }
-      }
-      h = fmin(fmax(0.5 * hnew, hlb), hub);
+      for (int r = 0; r < R; ++r) acor_saved[r] = idx(r) < N ? rec.Z[(QMAX + 1) * N + idx(r)] : 0.0;
+      if (lane < QMAX + 2) TAU[lane] = rec.tau[lane];
+#pragma unroll 1
+      for (int e = lane; e < N * N; e += 32) A[e + e / N] = rec.lu[e];
+#pragma unroll 1
+      for (int e = lane; e < N; e += 32) PIV[e] = rec.piv[e];
+      t = H.t; h = H.h; hscale = H.hscale; etamax = H.etamax; gammap = H.gammap; crate2 = H.crate2;
+      tq5_saved = H.tq5_saved;
+      q = H.q; qwait = H.qwait;
+      nst = H.nst; nfe = H.nfe; nje = H.nje; nstlp = H.nstlp; netf = H.netf; ncfn = H.ncfn;
+      force_setup = H.force_setup != 0;
+      __syncwarp();
     }
-    hscale = h;
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-      if (idx(r) < N) zget(1, r) = h * f[r];
-    q = 1; qwait = 2; etamax = ETAMX1;
-    if (lane == 0) TAU[1] = h;
-    __syncwarp();
 
     // ---------------------------------------------- step loop
+    bool handed_over = false;
     for (;;) {
       if (nst >= P.max_steps) { status = MAX_STEPS; break; }
+      if (W == 1 && P.drain > 0) {  // few cells left in the whole launch: leave this one to a team
+        unsigned long long done = 0;
+        if (lane == 0) done = *static_cast<volatile unsigned long long*>(P.done);
+        done = __shfl_sync(0xffffffffu, done, 0);
+        if (ncell - (long long)done <= P.drain) {
+          unsigned long long at = 0;
+          if (lane == 0) at = atomicAdd(P.resume_count, 1ull);
+          const ResumeRec<N, JR> out(P.resume, __shfl_sync(0xffffffffu, at, 0));
+          if (lane == 0) {
+            ResumeHead H;
+            H.t = t; H.h = h; H.hscale = hscale; H.etamax = etamax; H.gammap = gammap; H.crate2 = crate2;
+            H.tq5_saved = tq5_saved;
+            H.cell = cell;
+            H.box = lo; H.ci = ci; H.cj = cj; H.ck = ck;
+            H.q = q; H.qwait = qwait; H.nst = (int)nst; H.nfe = (int)nfe; H.nje = (int)nje; H.nstlp = (int)nstlp;
+            H.netf = (int)netf; H.ncfn = (int)ncfn;
+            H.force_setup = force_setup;
+            H.full_swaps = 1;
+            *out.head = H;
+          }
+#pragma unroll 1
+          for (int e = lane; e < (QMAX + 1) * N; e += 32) out.Z[e] = Z[e];
+#pragma unroll
+          for (int r = 0; r < R; ++r)
+            if (idx(r) < N) out.Z[(QMAX + 1) * N + idx(r)] = acor_saved[r];
+          if (lane < QMAX + 2) out.tau[lane] = TAU[lane];
+#pragma unroll 1
+          for (int e = lane; e < N * N; e += 32) out.lu[e] = A[e + e / N];
+#pragma unroll 1
+          for (int e = lane; e < N; e += 32) out.piv[e] = PIV[e];
+          handed_over = true;
+          break;
+        }
+      }
       if ((t + h - tout) * h > 0.0) rescale(pgb_div64((tout - t) * (1.0 - 4.0 * UROUND), h));
       set_ewt();
       nef = 0; ncf = 0;
@@ -1251,6 +1348,8 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
 
     // ---------------------------------------------- finish: rho h(t), T from (h, Y)
     __syncwarp();
+    if (handed_over) continue;
+    cell_done();
     if (status != OK && P.retry_list) {  // hand the cell to the retry pass, arrays untouched
       if (lane == 0) {
         P.retry_list[atomicAdd(P.retry_count, 1ull)] = cell;
@@ -1324,6 +1423,10 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
       atomicAdd(&S->hist[bin], 1ull);
     }
     __syncwarp();
+  }
+  if constexpr (W > 1) {  // dismiss the team
+    if (lane == 0) TP[5] = 0.0;
+    team_sync<W>(1 + wid);
   }
 }
 

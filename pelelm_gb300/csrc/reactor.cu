@@ -193,7 +193,7 @@ struct Scratch {
   pgb::BoxDev* d_boxes = nullptr;
   size_t box_cap = 0;
   pgb::BoxDev* h_boxes = nullptr;  // pinned staging
-  unsigned long long* d_counter = nullptr;  // queue head; queue head and count of handed-over cells
+  unsigned long long* d_counter = nullptr;  // queue head; queue head and count of handed-over cells; cells done
   void* d_resume = nullptr;        // handed-over cells
   size_t resume_cap = 0;
   void* d_z = nullptr;             // Nordsieck histories of the resident threads
@@ -262,7 +262,7 @@ void free_scratch(Scratch& s) {
 int ensure_scratch(pgb_reactor* r, cudaStream_t st, size_t nbox, Scratch** out) {
   Scratch& s = r->scratch[st];
   if (!s.d_counter) {
-    PGB_CUDA(cudaMalloc(&s.d_counter, 3 * sizeof(unsigned long long)));
+    PGB_CUDA(cudaMalloc(&s.d_counter, 4 * sizeof(unsigned long long)));
     PGB_CUDA(cudaMalloc(&s.d_stats, sizeof(pgb::ReactStats)));
     PGB_CUDA(cudaMalloc(&s.d_retry_count, sizeof(unsigned long long)));
     PGB_CUDA(cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming));
@@ -315,6 +315,7 @@ int mapping_of(const pgb_reactor* r);
 // 16384 cells 31.8 / 32.0; 21 species 512 cells 7.6 / 22.1, 4096 cells 13.2 / 22.9, 8192 cells
 // 22.6 / 22.9. At 1e-6 s, where cells differ less, the lines lie at about 7,000 and 5,800 cells.
 long long small_limit(const pgb_reactor* r) {
+  if (r->mech->small_lanes > 32) return (long long)r->nsm * 2;  // teams of warps: as many cells as run at once
   return (long long)r->nsm * (r->mech->ns <= 12 ? 48 : 40);
 }
 
@@ -344,6 +345,11 @@ LaunchPlan plan_launch(const pgb_reactor* r, long long ncell, bool mixed) {
     // one block per SM, one cell per warp while the SM's twelve warps allow it
     const int cpw = 32 / m.small_lanes;
     pl.small = true;
+    if (cpw == 0) {  // teams of warps
+      pl.nblocks = (int)std::min<long long>(r->nsm, std::max<long long>(1, ncell));
+      pl.tpb = ncell > r->nsm ? 2 : 1;
+      return pl;
+    }
     pl.nblocks = (int)std::min<long long>(r->nsm, std::max<long long>(1, ncell));
     const long long per_sm = (std::max<long long>(ncell, 1) + pl.nblocks - 1) / pl.nblocks;
     pl.cells_per_warp = per_sm <= kSmallWarps ? 1 : cpw;
@@ -373,6 +379,10 @@ LaunchPlan plan_launch(const pgb_reactor* r, long long ncell, bool mixed) {
     }
     pl.warp = true;
     pl.tpb = wpb;
+    if (m.small_lanes > 32 && r->small_ok) {
+      pl.drain = r->nsm * 2;  // of the whole launch: as many as the teams take at once
+      pl.resume_bytes = (size_t)pl.drain * (mixed ? m.resume_mixed : m.resume_fp64);
+    }
     pl.nblocks = (int)std::min<long long>(r->nsm, std::max<long long>(1, (ncell + wpb - 1) / wpb));
     return pl;
   }
@@ -452,7 +462,7 @@ int enqueue_advance(pgb_reactor* r, Scratch& s, int nbox, long long ncell, doubl
   p.next_cell = s.d_counter;
   p.stats = s.d_stats;
   PGB_CUDA(cudaMemcpyAsync(s.d_boxes, s.h_boxes, nbox * sizeof(pgb::BoxDev), cudaMemcpyHostToDevice, st));
-  PGB_CUDA(cudaMemsetAsync(s.d_counter, 0, 3 * sizeof(unsigned long long), st));
+  PGB_CUDA(cudaMemsetAsync(s.d_counter, 0, 4 * sizeof(unsigned long long), st));
   PGB_CUDA(cudaMemsetAsync(s.d_stats, 0, sizeof(pgb::ReactStats), st));
   if (ncell == 0) return 0;
   if (r->null_reactor) {
@@ -481,6 +491,7 @@ int enqueue_advance(pgb_reactor* r, Scratch& s, int nbox, long long ncell, doubl
     p.resume = static_cast<unsigned char*>(s.d_resume);
     p.resume_count = s.d_counter + 2;
     p.drain = pl.drain;
+    if (pl.warp) p.done = s.d_counter + 3;
   }
   auto run_bdf = [&]() -> int {
     if (fn(p, pl.tpb, st, pl.nblocks)) return -1;
@@ -492,7 +503,9 @@ int enqueue_advance(pgb_reactor* r, Scratch& s, int nbox, long long ncell, doubl
       m.drain = 0;
       m.resuming = 1;
       m.cells_per_warp = 0;
-      if ((r->opt.mixed ? r->mech->small_mixed : r->mech->small_fp64)(m, kSmallWarps, st, r->nsm)) return -1;
+      m.done = nullptr;
+      const int per_block = r->mech->small_lanes > 32 ? 2 : kSmallWarps;
+      if ((r->opt.mixed ? r->mech->small_mixed : r->mech->small_fp64)(m, per_block, st, r->nsm)) return -1;
     }
     if (!retry) return 0;
     const LaunchPlan p64 = plan_launch(r, ncell, false);
@@ -503,6 +516,12 @@ int enqueue_advance(pgb_reactor* r, Scratch& s, int nbox, long long ncell, doubl
     q.retry_count = nullptr;
     q.resume = nullptr;
     q.drain = 0;
+    q.done = nullptr;
+    if (r->small_ok && r->mech->small_lanes > 32) {  // few, and each as slow as its one warp: teams
+      q.cells_per_warp = 0;
+      PGB_CUDA(cudaMemsetAsync(s.d_counter, 0, sizeof(unsigned long long), st));
+      return r->mech->small_fp64(q, 2, st, r->nsm);
+    }
     q.lu_scratch = p64.lu_bytes ? s.d_lu : nullptr;
     q.z_scratch = p64.z_bytes ? s.d_z : nullptr;
     PGB_CUDA(cudaMemsetAsync(s.d_counter, 0, sizeof(unsigned long long), st));
@@ -723,7 +742,7 @@ int run_autotune(pgb_reactor* r, const std::vector<pgb::BoxDev>& boxes, long lon
     pgb_tune::gather_sample_kernel<<<(int)std::min<long long>((nsample + 255) / 256, 1024), 256, 0, st>>>(
         d_src, (int)boxes.size(), ns, nsample, stride, pristine);
     if (cudaGetLastError() != cudaSuccess) { fail("gather launch"); break; }
-    if (cudaMalloc(&sc.d_counter, 3 * sizeof(unsigned long long)) != cudaSuccess ||
+    if (cudaMalloc(&sc.d_counter, 4 * sizeof(unsigned long long)) != cudaSuccess ||
         cudaMalloc(&sc.d_stats, sizeof(pgb::ReactStats)) != cudaSuccess ||
         cudaMalloc(&sc.d_boxes, sizeof(pgb::BoxDev)) != cudaSuccess ||
         cudaMallocHost(&sc.h_boxes, sizeof(pgb::BoxDev)) != cudaSuccess) { fail("out of memory"); break; }

@@ -91,6 +91,18 @@ int launch_bdf_warp_wpb(const pgb::ReactParams& p, cudaStream_t s, int nblocks) 
   }
 }
 
+// Teams of four warps per cell, two cells a block (argument: cells per block).
+constexpr int kTeamWarps = 4;
+template <class M, class JR>
+int launch_bdf_team(const pgb::ReactParams& p, int cells, cudaStream_t s, int nblocks) {
+  constexpr int smem = 2 * pgb::bdf_warp_smem_per_warp<M, JR>();
+  auto kern = pgb::bdf_warp_kernel<M, JR, 2 * kTeamWarps, kTeamWarps>;
+  PGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  kern<<<nblocks, std::min(cells, 2) * kTeamWarps * 32, smem, s>>>(p);
+  PGB_CUDA(cudaGetLastError());
+  return 0;
+}
+
 // Warps per block compiled for a mechanism, most preferred first (0 ends the list): one size
 // for small mechanisms (the warp mapping is not their default), 16 for mid-sized ones (more
 // resident warps hide the latency of the lane-parallel RHS; 24 measured slower: the register
@@ -435,7 +447,9 @@ int h2t_entry(const pgb_box_view* v, double tmin, double tmax, cudaStream_t s) {
           ::pgb_host::warp_wpb_choice<M>(2), ::pgb_host::warp_wpb_choice<M>(3)               \
     }                                                                                        \
     , ::pgb_host::heat_release_entry<M>, nullptr, nullptr, nullptr, nullptr,                \
-        ::pgb_host::newton_matrix_entry<M, false>, nullptr, nullptr, 0, 0, 0                 \
+        ::pgb_host::newton_matrix_entry<M, false>, ::pgb_host::launch_bdf_team<M, float>,     \
+        ::pgb_host::launch_bdf_team<M, double>, 32 * ::pgb_host::kTeamWarps,                 \
+        pgb::resume_bytes<M::N, float>(), pgb::resume_bytes<M::N, double>()                  \
   }
 
 // Converts and validates one box view into its device descriptor; cell numbering of the box

@@ -77,6 +77,9 @@ struct ReactParams {
   unsigned char* resume;
   unsigned long long* resume_count;
   int drain, resuming;
+  // Warp kernels: cells finished so far; a warp hands its cell over when at most `drain` of the whole
+  // launch are left (null: not counted).
+  unsigned long long* done;
 };
 
 // One handed-over cell: what a BDF integration needs at the start of a step.

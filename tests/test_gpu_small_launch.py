@@ -62,3 +62,19 @@ def test_handed_over_cells_keep_their_bits(native_lib, cuda, cfgname, mapping, p
     assert fa == fb == 0
     for x, y in ((a.FC, b.FC), (a.rY, b.rY), (a.rEner, b.rEner), (a.T, b.T)):
         assert torch.equal(x, y)
+
+
+# teams of warps: one cell; fewer cells than SMs; two teams a block; above the limit, where the last
+# cells of the launch change to teams at a step; steps limited, so that cells fail and are retried
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(1, 1, 1), (7, 5, 4), (11, 5, 5), (11, 9, 5)])
+@pytest.mark.parametrize("precision,steps", [("mixed", 2000), ("fp64", 2000), ("mixed", 90)])
+def test_teams_of_warps_keep_the_bits(native_lib, cuda, shape, precision, steps):
+    torch = cuda
+    cfg = CONFIGS["gri_1M"]
+    opts = f"gb.precision={precision} ode.max_steps={steps}"
+    fa, a = _advance(torch, cfg, shape, opts, False, 3, True)
+    fb, b = _advance(torch, cfg, shape, opts + " gb.mapping=warp", False, 3, True)
+    assert fa == fb
+    for x, y in ((a.FC, b.FC), (a.rY, b.rY), (a.rEner, b.rEner), (a.T, b.T)):
+        assert torch.equal(x, y)
