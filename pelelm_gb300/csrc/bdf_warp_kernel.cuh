@@ -1,6 +1,7 @@
 // Persistent, work-stealing, warp-per-cell BDF reactor kernel for mechanisms whose per-cell state
-// no longer fits a thread: the default for drm19-sized mechanisms (21 species, 84 reactions) and
-// the only mapping for GRI-Mech-sized ones (53 species, 325 reactions, N = 54 unknowns).
+// no longer fits a thread: an option for drm19-sized mechanisms (21 species, 84 reactions) and
+// the only mapping for GRI-Mech-sized ones (53 species, 325 reactions, N = 54 unknowns), there
+// also with a team of warps per cell.
 //
 // Same contract and algorithm as bdf_kernel.cuh (the PelePhysics reactor called at
 // Source/PeleLM.cpp:5752; CVODE-class fixed-leading-coefficient variable-order Nordsieck BDF,
@@ -17,14 +18,21 @@
 //    over species again gathering their reactions (species-major lists: a deterministic order,
 //    no atomics), with warp-shuffle sums for the energy closure;
 //  * Jacobian (type JR: FP32 in mixed precision): NASA-7 terms once per species, per-reaction
-//    partials lane-parallel, then an assembly in reaction order with lanes over columns (each
-//    lane owns its columns, so the result does not depend on scheduling); constant-pressure
-//    energy row by column;
+//    partials lane-parallel, then an assembly by a generated program in reaction order with lanes
+//    over matrix entries (each entry has one owner, so the result does not depend on scheduling);
+//    constant-pressure energy row by column;
 //  * LU and triangular solves: lanes own rows; pivot search by warp arg-max (FP32: one max-
 //    reduction over the |a| bit patterns); matrix rows padded to N+1 so a column access is
 //    bank-conflict free;
 //  * per-warp state (Nordsieck history, forcing, rates, matrix) in shared memory; a warp takes
 //    the next cell index with one atomic when its cell is done (work stealing across all boxes);
+//  * with few cells a warp of its own leaves three of the four schedulers of an SM idle and a cell
+//    waits for one warp's dependent latencies: teams of W = 4 warps share its right-hand side
+//    (team_rates) and its Jacobian (partials and contribution program), the first warp leading.
+//    Used for launches of up to four cells per SM, for the last four cells per SM of a longer one
+//    (its warps hand them over) and for the FP64 pass over failed cells. Every sum keeps the order
+//    of the one-warp form, so the results are bit for bit the same. Measured (53 species, 60 cells
+//    mixed / 125 cells FP64): only the right-hand side shared 3.2 / 9.3 ms, the Jacobian too 2.5 / 7.5;
 //  * with a retry list (mixed precision), a failed cell is listed and left untouched for the
 //    FP64 pass that follows on the same stream.
 #ifndef PGB_BDF_WARP_KERNEL_CUH
@@ -499,20 +507,26 @@ __device__ __forceinline__ bool warp_lu_factor(JR* A, int* PIV, const JR g) {
 // Jacobian (equations of jac_table, mech_tables.cuh) into A, one warp cooperating. Inlined: each
 // kernel calls it from one place, so inlining adds no copy and removes the call's register save and
 // restore (measured: 1 to 3 %).
-template <class M, class JR>
-__device__ __forceinline__ void warp_jacobian(const WVec<M> yv, const double* FRC, JR* A, JR* XS, JR* RX, JR* TH) {
+// W > 1: by the warps of a team (role 0 leads and has y; TJ: four numbers it tells the others; QN: [NR]
+// the reactions' net rates, whose energy sums the leader then forms in its own order).
+template <class M, class JR, int W = 1>
+__device__ __forceinline__ void warp_jacobian(const WVec<M> yv, const double* FRC, JR* A, JR* XS, JR* RX, JR* TH,
+                                              int role = 0, int id = 0, JR* TJ = nullptr, JR* QN = nullptr) {
   using Tab = typename M::TabG;
   constexpr int N = M::N, NS = M::NS, NR = M::NR;
   constexpr int R = (N + 31) / 32;
   constexpr int LDA = N + 1;
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, first = 32 * role + lane;
   const double (&y)[R] = yv.v;
   auto idx = [&](int r) { return lane + 32 * r; };
   auto bcast = [&](const double (&v)[R], int i) -> double {
     return __shfl_sync(0xffffffffu, v[i >> 5], i & 31);
   };
   using namespace jac_detail;
-  const JR T = (JR)bcast(y, NS);
+  JR T = (JR)bcast(y, NS);
+  if constexpr (W > 1) {
+    if (role > 0) T = TJ[0];
+  }
   const JR invT = JR(1) / T;
   const JR lnT = pgb_logT<JR>(T);
   const JR lnT1 = JR(1) - lnT;
@@ -525,6 +539,7 @@ __device__ __forceinline__ void warp_jacobian(const WVec<M> yv, const double* FR
   JR* TC = TH + 2 * NS;
   JR* TD = TH + 3 * NS;
   JR c_loc = JR(0);
+  if (W == 1 || role == 0)
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     const int k = idx(r);
@@ -540,12 +555,18 @@ __device__ __forceinline__ void warp_jacobian(const WVec<M> yv, const double* FR
       TD[k] = d;
     }
   }
-  const JR Ctot = warp_sum(c_loc);
-  for (int e = lane; e < N * LDA; e += 32) A[e] = JR(0);
-  __syncwarp();
+  JR Ctot = warp_sum(c_loc);
+  for (int e = first; e < N * LDA; e += 32 * W) A[e] = JR(0);
+  if constexpr (W > 1) {
+    if (role == 0 && lane == 0) TJ[1] = Ctot;
+    team_sync<W>(id);
+    Ctot = TJ[1];
+  } else {
+    __syncwarp();
+  }
   // (1) per-reaction partials, lanes over reactions; energy-closure sums
   JR Qw = JR(0), cpw = JR(0);
-  for (int j = lane; j < NR; j += 32) {
+  for (int j = first; j < NR; j += 32 * W) {
     const TabReaction<JR>& r = Tab::template rx<JR>(j);
     const JR lnkinf = r.beta * lnT + r.mEaR * invT + r.lnA;
     JR dlnkf = (r.beta - r.mEaR * invT) * invT;
@@ -625,13 +646,33 @@ __device__ __forceinline__ void warp_jacobian(const WVec<M> yv, const double* FR
       for (int e = 0; e < 8; ++e)
         if (e < t.n) ox[e] = bm * (JR(1) + t.effm1[e]);
     }
+    if constexpr (W > 1) {
+      QN[j] = q;
+    } else {
 #pragma unroll
-    for (int row = 0; row < 6; ++row)
-      if (row < r.nr + r.np) {
-        const bool isr = row < r.nr;
-        const int i = isr ? r.rs[row] : r.ps[row - r.nr];
-        Qw += (isr ? -q : q) * TH_[i] * RT;
-        cpw += (isr ? -q : q) * TC[i] * JR(kRerg);
+      for (int row = 0; row < 6; ++row)
+        if (row < r.nr + r.np) {
+          const bool isr = row < r.nr;
+          const int i = isr ? r.rs[row] : r.ps[row - r.nr];
+          Qw += (isr ? -q : q) * TH_[i] * RT;
+          cpw += (isr ? -q : q) * TC[i] * JR(kRerg);
+        }
+    }
+  }
+  if constexpr (W > 1) {
+    team_sync<W>(id);
+    if (role == 0)
+      for (int j = lane; j < NR; j += 32) {
+        const TabReaction<JR>& r = Tab::template rx<JR>(j);
+        const JR q = QN[j];
+#pragma unroll
+        for (int row = 0; row < 6; ++row)
+          if (row < r.nr + r.np) {
+            const bool isr = row < r.nr;
+            const int i = isr ? r.rs[row] : r.ps[row - r.nr];
+            Qw += (isr ? -q : q) * TH_[i] * RT;
+            cpw += (isr ? -q : q) * TC[i] * JR(kRerg);
+          }
       }
   }
   Qw = warp_sum(Qw);
@@ -648,14 +689,38 @@ __device__ __forceinline__ void warp_jacobian(const WVec<M> yv, const double* FR
   // target one entry ahead: with shared memory taking almost all of the L1, each of these loads
   // is an L2 round trip, and a load per term made the program the setup's longest part.
   {
+    constexpr int L = 32 * W;
+    auto quad_of = [&](int c) -> uint4 {
+      if constexpr (W > 1) return Tab::team_quad(c);
+      else return Tab::jac_quad(c);
+    };
+    auto ent_of = [&](int c) -> TabJacEnt<JR> {
+      if constexpr (W > 1) return Tab::template team_ent<JR>(c);
+      else return Tab::template jac_ent<JR>(c);
+    };
+    // efficiency of a term that adds its collider slot to other partials (few do)
+    auto eff_of = [&](unsigned c, int term, int k) -> JR {
+      if constexpr (W == 1) {
+        return Tab::template jac_eff<JR>(term);
+      } else {
+        const TabThirdBody<JR>& t = Tab::template tb<JR>(Tab::template rx<JR>((c & 0x1fff) / wbdf::RXW).tb);
+        JR v = JR(1);
+        for (int e = 0; e < t.n; ++e)
+          if (t.sp[e] == k) v = JR(1) + t.effm1[e];
+        return v;
+      }
+    };
+    int quads, ents;
+    if constexpr (W > 1) { quads = Tab::TEAM_QUADS; ents = Tab::TEAM_ENTS; }
+    else { quads = Tab::JAC_QUADS; ents = Tab::JAC_ENTS; }
     JR acc = JR(0);
-    int ent = lane;
-    TabJacEnt<JR> cur = Tab::template jac_ent<JR>(ent), ahead = Tab::template jac_ent<JR>(ent + 32);
-    uint4 quad = Tab::jac_quad(lane);
+    int ent = first;
+    TabJacEnt<JR> cur = ent_of(ent), ahead = ent_of(ent + L);
+    uint4 quad = quad_of(first);
 #pragma unroll 1
-    for (int q = 0; q < Tab::JAC_QUADS; ++q) {
+    for (int q = 0; q < quads; ++q) {
       const unsigned code[4] = {quad.x, quad.y, quad.z, quad.w};
-      if (q + 1 < Tab::JAC_QUADS) quad = Tab::jac_quad(32 * (q + 1) + lane);
+      if (q + 1 < quads) quad = quad_of(L * (q + 1) + first);
       JR v[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) v[u] = RX[code[u] & 0x1fff];
@@ -668,20 +733,25 @@ __device__ __forceinline__ void warp_jacobian(const WVec<M> yv, const double* FR
           for (int s = 1; s < 7; ++s)
             if (c & (1u << (12 + s))) v[u] += pj[s];
           if (c & (1u << 19))
-            v[u] = fma(pj[7], (c & (1u << 22)) ? Tab::template jac_eff<JR>(32 * (4 * q + u) + lane) : JR(1), v[u]);
+            v[u] = fma(pj[7], (c & (1u << 22)) ? eff_of(c, L * (4 * q + u) + first, cur.target % LDA) : JR(1), v[u]);
         }
         if (not_zero(v[u]) || (c & (1u << 23))) acc = fma(flip_sign(cur.w, c << 11), v[u], acc);
         if (c & (1u << 21)) {  // last term of the entry
           A[cur.target] = acc;
           acc = JR(0);
           cur = ahead;
-          ent += 32;
-          ahead = Tab::template jac_ent<JR>(min(ent + 32, 32 * (Tab::JAC_ENTS - 1) + lane));
+          ent += L;
+          ahead = ent_of(min(ent + L, L * (ents - 1) + first));
         }
       }
     }
   }
-  __syncwarp();
+  if constexpr (W > 1) {
+    team_sync<W>(id);
+    if (role > 0) return;
+  } else {
+    __syncwarp();
+  }
   // (3) constant-pressure energy row: dT/dt = (Fh - sum h_k wm_k) / (rho cp)
   JR D = JR(0), dD = JR(0), Qf = JR(0), cpf = JR(0);
 #pragma unroll
@@ -723,10 +793,22 @@ __device__ __forceinline__ void warp_jacobian(const WVec<M> yv, const double* FR
 
 // The Jacobian and the LU of I - gamma J. False: singular. With FACTOR false it stops after the
 // Jacobian, which A then holds (the diagnostic entry point).
-template <class M, class JR, bool FACTOR = true>
+template <class M, class JR, bool FACTOR = true, int W = 1>
 __device__ __forceinline__ bool warp_setup(const WVec<M> yv, const double gamma, const double* FRC, JR* A,
-                                        JR* XS, JR* RX, JR* TH, int* PIV) {
-  warp_jacobian<M, JR>(yv, FRC, A, XS, RX, TH);
+                                        JR* XS, JR* RX, JR* TH, int* PIV, double* TP = nullptr, int id = 0,
+                                        JR* QN = nullptr) {
+  if constexpr (W > 1) {
+    JR* const TJ = reinterpret_cast<JR*>(TP);
+    const double T = __shfl_sync(0xffffffffu, yv.v[M::NS >> 5], M::NS & 31);
+    if ((threadIdx.x & 31) == 0) {
+      TJ[0] = (JR)T;
+      TP[5] = 2.0;
+    }
+    team_sync<W>(id);
+    warp_jacobian<M, JR, W>(yv, FRC, A, XS, RX, TH, 0, id, TJ, QN);
+  } else {
+    warp_jacobian<M, JR>(yv, FRC, A, XS, RX, TH);
+  }
   if constexpr (FACTOR) return warp_lu_factor<M::N>(A, PIV, (JR)gamma);
   else return true;
 }
@@ -816,6 +898,8 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
   JR* A = reinterpret_cast<JR*>(scratch + bdf_warp_scratch_bytes<M, JR>());  // [N][LDA] Jacobian, then its LU
   JR* XS = A + N * LDA;                          // [N] solve vector
   int* PIV = reinterpret_cast<int*>(XS + N);
+  // teams: [NR] net rates, after the cells' memory
+  JR* const QN = reinterpret_cast<JR*>(wsmem + (size_t)(WPB / W) * bdf_warp_smem_per_warp<M, JR>()) + (W > 1 ? wid * M::NR : 0);
 
   if constexpr (W > 1) {
     const int role = (threadIdx.x >> 5) % W;
@@ -823,6 +907,11 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
       for (;;) {
         team_sync<W>(1 + wid);
         if (TP[5] == 0.0) return;
+        if (TP[5] == 2.0) {
+          const WVec<M> none = {};
+          warp_jacobian<M, JR, W>(none, FRC, A, XS, RX, TH, role, 1 + wid, reinterpret_cast<JR*>(TP), QN);
+          continue;
+        }
         team_rates<M, W>(role, 1 + wid, TP[0], TP[1], TP[2], TP[3], TP[4], CS, GS, QS);
       }
     }
@@ -1054,7 +1143,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
 #pragma unroll
           for (int r = 0; r < R; ++r) yv.v[r] = y[r];
           ++nje;
-          const bool ok = warp_setup<M, JR>(yv, gamma, FRC, A, XS, RX, TH, PIV);
+          const bool ok = warp_setup<M, JR, true, W>(yv, gamma, FRC, A, XS, RX, TH, PIV, TP, 1 + wid, QN);
           gammap = gamma;
           gamrat = 1.0;
           crate2 = 1.0;

@@ -314,8 +314,10 @@ int mapping_of(const pgb_reactor* r);
 // kernel, mixed precision, dt_react 1e-5 s: 9 species 512 cells 9.1 / 29.1 ms, 4096 cells 13.5 / 30.7,
 // 16384 cells 31.8 / 32.0; 21 species 512 cells 7.6 / 22.1, 4096 cells 13.2 / 22.9, 8192 cells
 // 22.6 / 22.9. At 1e-6 s, where cells differ less, the lines lie at about 7,000 and 5,800 cells.
+// 53 species (teams of four warps, two at a time on an SM, against one warp a cell that hands its last
+// cells over): 448 cells 56.6 / 60.4, 576 cells 56.9 / 62.8, at 1e-6 s 6.2 / 6.1; 900 cells 7.9 / 6.4.
 long long small_limit(const pgb_reactor* r) {
-  if (r->mech->small_lanes > 32) return (long long)r->nsm * 2;  // teams of warps: as many cells as run at once
+  if (r->mech->small_lanes > 32) return (long long)r->nsm * 4;
   return (long long)r->nsm * (r->mech->ns <= 12 ? 48 : 40);
 }
 
@@ -380,7 +382,10 @@ LaunchPlan plan_launch(const pgb_reactor* r, long long ncell, bool mixed) {
     pl.warp = true;
     pl.tpb = wpb;
     if (m.small_lanes > 32 && r->small_ok) {
-      pl.drain = r->nsm * 2;  // of the whole launch: as many as the teams take at once
+      // of the whole launch. Measured with 2, 3, 4, 6 cells per SM: 3,072 cells, mixed 76.6, 76.2, 74.6,
+      // 73.5 ms (FP64, 2,048 cells: 95.8, 96.8, 93.3, 89.9); 4,096 cells at 1e-6 s 19.0, 18.7, 18.6, 19.6;
+      // 9,216 cells 126.3, 125.7, 125.4, 126.3
+      pl.drain = r->nsm * 4;
       pl.resume_bytes = (size_t)pl.drain * (mixed ? m.resume_mixed : m.resume_fp64);
     }
     pl.nblocks = (int)std::min<long long>(r->nsm, std::max<long long>(1, (ncell + wpb - 1) / wpb));

@@ -95,7 +95,8 @@ int launch_bdf_warp_wpb(const pgb::ReactParams& p, cudaStream_t s, int nblocks) 
 constexpr int kTeamWarps = 4;
 template <class M, class JR>
 int launch_bdf_team(const pgb::ReactParams& p, int cells, cudaStream_t s, int nblocks) {
-  constexpr int smem = 2 * pgb::bdf_warp_smem_per_warp<M, JR>();
+  constexpr int smem = 2 * (pgb::bdf_warp_smem_per_warp<M, JR>() + M::NR * (int)sizeof(JR));
+  static_assert(smem <= kMaxSmemPerBlock, "a block of two cells exceeds the shared memory");
   auto kern = pgb::bdf_warp_kernel<M, JR, 2 * kTeamWarps, kTeamWarps>;
   PGB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   kern<<<nblocks, std::min(cells, 2) * kTeamWarps * 32, smem, s>>>(p);

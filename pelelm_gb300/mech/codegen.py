@@ -489,7 +489,7 @@ def _f32(x: float) -> float:
     return struct.unpack("f", struct.pack("f", x))[0]
 
 
-def jac_stream(m: Mechanism, rx, tb_rows, codes, neg, T: int, LDA: int):
+def jac_stream(m: Mechanism, rx, tb_rows, codes, neg, T: int, LDA: int, L: int = 32):
     """The contribution program (kJacC, kJacNeg) in the form the kernels stream: (quads, entries,
     x0, nx).
 
@@ -508,12 +508,12 @@ def jac_stream(m: Mechanism, rx, tb_rows, codes, neg, T: int, LDA: int):
     n_rx = len(rx)
     assert 8 * n_rx + nx <= 8192, "partial index field too narrow for this mechanism"
     nq = (T + 3) // 4
-    quads = [[[0, 0, 0, 0] for _ in range(32)] for _ in range(nq)]
-    ents = [[] for _ in range(32)]
+    quads = [[[0, 0, 0, 0] for _ in range(L)] for _ in range(nq)]
+    ents = [[] for _ in range(L)]
     W = [s.W for s in m.species]
-    for l_ in range(32):
+    for l_ in range(L):
         for t in range(T):
-            c = codes[32 * t + l_]
+            c = codes[L * t + l_]
             if c == 0:
                 continue  # padding: adds to a sum that is never stored
             j, tg = c & 0x1FF, (c >> 9) & 0xFFF
@@ -539,6 +539,46 @@ def jac_stream(m: Mechanism, rx, tb_rows, codes, neg, T: int, LDA: int):
                 wf = _f32(W[i]) if k == ns else _f32(_f32(W[i]) * _f32(1.0 / W[k]))
                 ents[l_].append((wd, wf, tg))
     return quads, ents, x0, nx
+
+
+def deal_program(ents, L: int, LDA: int):
+    """The program's entries dealt to L lanes, largest first, to the lane with the fewest terms so far:
+    (terms per lane, codes, sign planes), term t of lane l at L t + l."""
+    lanes = [[] for _ in range(L)]
+    load = [0] * L
+    for key, terms in ents:
+        l_ = min(range(L), key=lambda v: (load[v], v))
+        lanes[l_].append((key, terms))
+        load[l_] += len(terms)
+    T = max(load)
+    codes, neg = [0] * (L * T), [0] * T
+    for l_ in range(L):
+        t = 0
+        for (i, k), terms in lanes[l_]:
+            for n_, (code, isr, _) in enumerate(terms):
+                flags = ((1 << 29) if n_ == len(terms) - 1 else 0) | ((1 << 30) if n_ == 0 else 0)
+                codes[L * t + l_] = (code | ((i * LDA + k) << 9) | flags) & 0xFFFFFFFF
+                neg[t] |= int(isr) << l_
+                t += 1
+    return T, codes, neg
+
+
+def emit_team_stream(e: _Emitter, qual: str, m: Mechanism, rx, tb_rows, ents, LDA: int, L: int = 128):
+    """The program once more, for the L lanes of a team of warps."""
+    T, codes, neg = deal_program(ents, L, LDA)
+    quads, lane_ents, _, _ = jac_stream(m, rx, tb_rows, codes, neg, T, LDA, L)
+    ne = max(len(v) for v in lane_ents) + 1
+    e(f"constexpr int NJQT = {len(quads)}, NJET = {ne};")
+    e(f"{qual} uint4 kJacQT[{L} * NJQT] = {{")
+    for q in quads:
+        e("  " + ", ".join("{" + ", ".join(f"{w}u" for w in lane) + "}" for lane in q) + ",")
+    e("};")
+    for R, suf, col in (("double", "D", 0), ("float", "F", 1)):
+        e(f"{qual} TabJacEnt<{R}> kJacEntT{suf}[{L} * NJET] = {{")
+        for n_ in range(ne):
+            row = [v[n_] if n_ < len(v) else (0.0, 0.0, 0) for v in lane_ents]
+            e("  " + ", ".join("{" + _f(v[col]) + ("f" if col else "") + f", {v[2]}}}" for v in row) + ",")
+        e("};")
 
 
 def emit_jac_stream(e: _Emitter, qual: str, m: Mechanism, rx, tb_rows, codes, neg, T: int, LDA: int):
@@ -771,6 +811,8 @@ def gen_tables(m: Mechanism, space: str = "constant") -> str:
         e(f"{qual} double kJacEffD[32 * NJT] = {{{', '.join(effD)}}};")
         e(f"{qual} float kJacEffF[32 * NJT] = {{{', '.join(effF)}}};")
         emit_jac_stream(e, qual, m, rx, tb_rows, codes, neg, T, LDA)
+        if kernel_family(m) == "warp":
+            emit_team_stream(e, qual, m, rx, tb_rows, ents, LDA)
         # packed reaction records of the FP64 rate of progress (TabRxArr / TabRxPk)
         e(f"{qual} TabRxArr kRxArr[NR] = {{")
         for (lnA, beta, mear, *_r) in rx:
@@ -820,6 +862,12 @@ def gen_tables(m: Mechanism, space: str = "constant") -> str:
         e("    if constexpr (sizeof(R) == sizeof(double)) return kJacEntD[c]; else return kJacEntF[c];")
         e("  }")
         e("  __device__ static int jac_x0(int tb) { return kJacX0[tb]; }")
+        if kernel_family(m) == "warp":
+            e("  static constexpr int TEAM_QUADS = NJQT, TEAM_ENTS = NJET;")
+            e("  __device__ static uint4 team_quad(int c) { return kJacQT[c]; }")
+            e("  template <class R> __device__ static const TabJacEnt<R>& team_ent(int c) {")
+            e("    if constexpr (sizeof(R) == sizeof(double)) return kJacEntTD[c]; else return kJacEntTF[c];")
+            e("  }")
         e("  template <class R> __device__ static R jac_eff(int c) {")
         e("    if constexpr (sizeof(R) == sizeof(double)) return kJacEffD[c]; else return kJacEffF[c];")
         e("  }")

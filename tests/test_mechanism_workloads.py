@@ -306,6 +306,43 @@ def test_streamed_jacobian_program_equals_the_program(name):
             assert a[0] == b[0] and a[2:] == b[2:] and abs(a[1] - b[1]) <= 1e-15 * (1.0 + abs(a[1]))
 
 
+def test_team_program_equals_the_warp_program():
+    """The contribution program dealt to the 128 lanes of a team of warps: every matrix entry has one
+    owner, which adds the same terms in the same order as the one warp of the 32-lane form, and the
+    lanes' loads are even (the longest at most the mean plus the longest entry)."""
+    import re
+    from pelelm_gb300.mech.codegen import gen_tables
+    txt = gen_tables(load_mechanism("gri_syn"), "global")
+
+    def lists(quads, ents, nq, ne, L):
+        def body(nm):
+            b = re.search(nm + r"\[[^\]]*\] = \{(.*?)\};", txt, re.S).group(1)
+            return [x.strip() for x in b.replace("{", "").replace("}", "").split(",") if x.strip()]
+
+        nq, ne = (int(re.search(nm + r" = (\d+)", txt).group(1)) for nm in (nq, ne))
+        q = np.array([int(x.rstrip("u")) for x in body(quads)]).reshape(nq, L, 4)
+        e = np.array([float(x) for x in body(ents)]).reshape(ne, L, 2)
+        out, loads = {}, []
+        for ln in range(L):
+            words = [int(w) for w in q[:, ln].reshape(-1) if w]
+            loads.append(len(words))
+            n, terms = 0, []
+            for w in words:
+                terms.append(w)
+                if w & (1 << 21):
+                    target = int(e[n, ln, 1])
+                    assert target not in out
+                    out[target] = (e[n, ln, 0], terms)
+                    n, terms = n + 1, []
+            assert not terms and n < ne
+        return out, loads
+
+    one, _ = lists("kJacQ", "kJacEntD", "NJQ", "NJE", 32)
+    team, loads = lists("kJacQT", "kJacEntTD", "NJQT", "NJET", 128)
+    assert one == team
+    assert max(loads) <= np.mean(loads) + max(len(t) for _, t in one.values())
+
+
 def test_packed_reaction_records_match_the_reaction_table():
     """The warp and lane-group RHS read each reaction through two packed records (kRxArr,
     kRxPk); decoded, they must equal the fields of the FP64 reaction table entry by entry."""
