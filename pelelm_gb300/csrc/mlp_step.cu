@@ -8,10 +8,11 @@
 //  * products read their operands as they lie (ldmatrix with or without .trans), so nothing is
 //    transposed; forward and input gradients keep the accumulation order of gemm_nt_kernel (mlp.cu),
 //    k in steps of 16 in one FP32 accumulator, so activations and gradients keep their bits;
-//  * GELU, its derivative, the loss and the bias-gradient column sums are epilogues;
-//  * the weight gradients of all layers are one launch, split along the batch so that about two CTAs
-//    per SM work, and Adam adds the splits (in order: deterministic) as it reads them.
-// Measured (batch 8192, 4 x 256): 1312 -> 170 us a step; batch 256: 370 -> 90 us (host calls).
+//  * GELU, its derivative and the loss are epilogues;
+//  * the gradients of all layers are one launch (grad_kernel), all parameters' Adam another, one block
+//    of which adds the loss's partials in FP64.
+// Measured (4 x 256): batch 8192 1310 -> 216 us a step, of it 62 us grad_kernel (the batch split over
+// more CTAs: 167 us, with other bits).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -25,18 +26,16 @@ constexpr int LD_K = TK + 8;    // operand tile [row][k]: 40 bf16 = 80 B rows
 constexpr int LD_MN = TM + 8;   // operand tile [k][row]: 136 bf16 = 272 B rows
 constexpr int kMaxLayers = 16;
 
-enum Epilogue : int { FORWARD = 0, LOSS = 1, INPUT_GRAD = 2, PARTIAL = 3 };
+enum Epilogue : int { FORWARD = 0, LOSS = 1, INPUT_GRAD = 2 };
 
 struct StepEpi {
   const float* bias;        // FORWARD, LOSS
-  float* pre;               // FORWARD: pre-activation out; INPUT_GRAD: in
+  float* pre;               // FORWARD: pre-activation out; INPUT_GRAD: in, then the FP32 dZ; LOSS: FP32 dZ
   bf16* out;                // activation, or dZ
-  float* bias_part;         // LOSS, INPUT_GRAD: [row tile][ldo] column sums of dZ
   const float* target;      // LOSS
-  float* loss;
+  float* loss_part;         // LOSS: [row tile][column tile][8] sums of the tile's warps
   float scale;
   int ldo, n_valid;
-  float* part;              // PARTIAL: C of this split
 };
 
 // Bytes of one stage of an operand whose tile is [row][k] (KMAJOR) or [k][row].
@@ -62,12 +61,13 @@ __device__ __forceinline__ void load_tile(bf16* s, const bf16* __restrict__ g, i
   }
 }
 
-// C tile (m0, n0) of A (M x K) and B (N x K) over k in [k0, k1), 8 warps as 4 x 2 of 32 x 64.
-template <bool AK, bool BK_, int EPI>
-__device__ __forceinline__ void step_tile(unsigned char* smem, const bf16* __restrict__ A, int lda, int M, int m0,
-                                          const bf16* __restrict__ B, int ldb, int N, int n0, int k0, int k1,
-                                          const StepEpi& e) {
-  constexpr int TA = tile_bytes<AK>(), TB = tile_bytes<BK_>();
+// C tile of A (M x K, [row][k]) and B (N x K, [row][k] or [k][row]), 8 warps as 4 x 2 of 32 x 64.
+template <bool BK_, int EPI>
+__global__ void __launch_bounds__(256, 2) step_gemm_kernel(const bf16* __restrict__ A, int lda, int M,
+                                                           const bf16* __restrict__ B, int ldb, int N, int K, StepEpi e) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
+  constexpr int TA = tile_bytes<true>(), TB = tile_bytes<BK_>();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wm = warp >> 1, wn = warp & 1;
   float acc[2][8][4];
@@ -79,11 +79,11 @@ __device__ __forceinline__ void step_tile(unsigned char* smem, const bf16* __res
       for (int r = 0; r < 4; ++r) acc[i][j][r] = 0.f;
   auto sa = [&](int st) { return reinterpret_cast<bf16*>(smem + st * (TA + TB)); };
   auto sb = [&](int st) { return reinterpret_cast<bf16*>(smem + st * (TA + TB) + TA); };
-  const int nk = (k1 - k0) / TK;
+  const int nk = K / TK;
   auto load = [&](int kt) {
     if (kt < nk) {
-      load_tile<AK>(sa(kt % STAGES), A, lda, m0, M, k0 + kt * TK);
-      load_tile<BK_>(sb(kt % STAGES), B, ldb, n0, N, k0 + kt * TK);
+      load_tile<true>(sa(kt % STAGES), A, lda, m0, M, kt * TK);
+      load_tile<BK_>(sb(kt % STAGES), B, ldb, n0, N, kt * TK);
     }
     cp_async_commit();
   };
@@ -101,11 +101,7 @@ __device__ __forceinline__ void step_tile(unsigned char* smem, const bf16* __res
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         const int r = wm * 32 + i * 16;
-        if constexpr (AK)
-          ldmatrix_x4(a[i][0], a[i][1], a[i][2], a[i][3], a_s + (r + (lane & 15)) * LD_K + kk + (lane >> 4) * 8);
-        else
-          ldmatrix_x4_trans(a[i][0], a[i][1], a[i][2], a[i][3],
-                            a_s + (kk + (lane & 7) + (lane >> 4) * 8) * LD_MN + r + ((lane >> 3) & 1) * 8);
+        ldmatrix_x4(a[i][0], a[i][1], a[i][2], a[i][3], a_s + (r + (lane & 15)) * LD_K + kk + (lane >> 4) * 8);
       }
 #pragma unroll
       for (int j = 0; j < 8; j += 2) {
@@ -124,12 +120,8 @@ __device__ __forceinline__ void step_tile(unsigned char* smem, const bf16* __res
     }
   }
   cp_async_wait<0>();
-  __syncthreads();  // the column sums below reuse the tiles' memory
 
-  float col[8][2];
   float sq = 0.f;
-#pragma unroll
-  for (int j = 0; j < 8; ++j) col[j][0] = col[j][1] = 0.f;
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
@@ -141,98 +133,201 @@ __device__ __forceinline__ void step_tile(unsigned char* smem, const bf16* __res
         if (m >= M || n >= N) continue;  // N is even
         float v[2] = {acc[i][j][h * 2], acc[i][j][h * 2 + 1]};
         const size_t at = (size_t)m * e.ldo + n;
-        if constexpr (EPI == PARTIAL) {
-          *reinterpret_cast<float2*>(e.part + at) = make_float2(v[0], v[1]);
-        } else {
-          if constexpr (EPI == FORWARD) {
-            v[0] += e.bias[n];
-            v[1] += e.bias[n + 1];
-            *reinterpret_cast<float2*>(e.pre + at) = make_float2(v[0], v[1]);
-            v[0] = gelu(v[0]);
-            v[1] = gelu(v[1]);
-          } else if constexpr (EPI == LOSS) {
+        if constexpr (EPI == FORWARD) {
+          v[0] += e.bias[n];
+          v[1] += e.bias[n + 1];
+          *reinterpret_cast<float2*>(e.pre + at) = make_float2(v[0], v[1]);
+          v[0] = gelu(v[0]);
+          v[1] = gelu(v[1]);
+        } else if constexpr (EPI == LOSS) {
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
-              const float y = v[c] + e.bias[n + c];
-              v[c] = 0.f;
-              if (n + c < e.n_valid) {
-                const float d = y - e.target[at + c];
-                sq += d * d;
-                v[c] = e.scale * d;
-              }
+          for (int c = 0; c < 2; ++c) {
+            const float y = v[c] + e.bias[n + c];
+            v[c] = 0.f;
+            if (n + c < e.n_valid) {
+              const float d = y - e.target[at + c];
+              sq += d * d;
+              v[c] = e.scale * d;
             }
-          } else {
-            const float2 p = *reinterpret_cast<const float2*>(e.pre + at);
-            v[0] *= gelu_grad(p.x);
-            v[1] *= gelu_grad(p.y);
           }
-          if constexpr (EPI != FORWARD) {
-            col[j][0] += v[0];
-            col[j][1] += v[1];
-          }
-          *reinterpret_cast<__nv_bfloat162*>(e.out + at) = __nv_bfloat162(__float2bfloat16(v[0]), __float2bfloat16(v[1]));
+        } else {
+          const float2 p = *reinterpret_cast<const float2*>(e.pre + at);
+          v[0] *= gelu_grad(p.x);
+          v[1] *= gelu_grad(p.y);
         }
+        if constexpr (EPI != FORWARD) *reinterpret_cast<float2*>(e.pre + at) = make_float2(v[0], v[1]);
+        *reinterpret_cast<__nv_bfloat162*>(e.out + at) = __nv_bfloat162(__float2bfloat16(v[0]), __float2bfloat16(v[1]));
       }
-  if constexpr (EPI == LOSS || EPI == INPUT_GRAD) {
-    // column sums of the tile: over a warp's 32 rows by shuffles, then over the four warp rows
-    float* cs = reinterpret_cast<float*>(smem);  // [4][TN]
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-#pragma unroll
-        for (int o = 4; o < 32; o <<= 1) col[j][c] += __shfl_xor_sync(0xffffffffu, col[j][c], o);
-        if (lane < 4) cs[wm * TN + wn * 64 + j * 8 + lane * 2 + c] = col[j][c];
-      }
-    __syncthreads();
-    if (tid < TN && n0 + tid < N)
-      e.bias_part[(size_t)(m0 / TM) * e.ldo + n0 + tid] = cs[tid] + cs[TN + tid] + cs[2 * TN + tid] + cs[3 * TN + tid];
-  }
   if constexpr (EPI == LOSS) {
 #pragma unroll
     for (int o = 16; o; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-    if (lane == 0 && sq != 0.f) atomicAdd(e.loss, sq);
+    if (lane == 0) e.loss_part[((m0 / TM) * ((N + TN - 1) / TN) + n0 / TN) * 8 + warp] = sq;
   }
 }
 
-template <bool BK_, int EPI>
-__global__ void __launch_bounds__(256, 2) step_gemm_kernel(const bf16* __restrict__ A, int lda, int M,
-                                                           const bf16* __restrict__ B, int ldb, int N, int K, StepEpi e) {
-  extern __shared__ __align__(16) unsigned char step_smem[];
-  step_tile<true, BK_, EPI>(step_smem, A, lda, M, blockIdx.y * TM, B, ldb, N, blockIdx.x * TN, 0, K, e);
-}
+// Gradients of all layers in one launch: dW (N x Kw) = dZ^T act over the batch by tiles of 32 x 64,
+// and db, the column sums of the FP32 dZ, 16 columns a block.
+//
+// Each entry of dW is one FP32 accumulator that walks the batch in steps of 16, and each column of
+// db eight chains (row mod 8) added in order: the orders of gemm_nt_kernel and bias_grad_kernel (mlp.cu),
+// so both keep their bits. Adam's first steps divide a gradient by its own size, so another order
+// shows in the parameters (measured with the batch split: 5e-5 of a bias vector).
+// What bounds it is the walk: batch / 16 dependent products an accumulator. Tiles of 64 x 64 with four,
+// eight or sixteen products a scheduler in flight and of 32 x 64 with four or eight all took 62 to 71 us at a
+// batch of 8192 and four layers of 256 (the tensor pipe a quarter busy, seven stages or ten in flight);
+// the small tile reaches most SMs at narrow layers too. A stage's fragments are read while the products
+// of the one before run. The batch split over two CTAs per SM took 20 us, but gave other sums.
+constexpr int GN = 32, GT = 64, GB = 64, GSTAGES = 7, LD_N = GN + 8, LD_G = GT + 8, GTHREADS = 256;
+constexpr int kGradSmem = GSTAGES * GB * (LD_N + LD_G) * 2;
+constexpr int kBiasCols = 16, kBiasRows = 256, kBiasStages = 6;
+static_assert(kBiasStages * kBiasRows * kBiasCols * 4 <= kGradSmem, "stage memory");
 
-// Weight gradients of all layers: layer l's dW (N x Kw) = dZ^T act over the batch, its tiles and the
-// batch's splits dealt to the grid.
-struct WGradLayer {
+struct GradLayer {
   const bf16 *dz, *act;
-  int N, Kw, lda, tiles_k, first_tile;  // first_tile: of this layer in the tile order
-  float* part;                          // [split][N][Kw]
+  const float* dzf;
+  int N, Kw, lda, tiles_k, first_tile, first_bias;  // first block of this layer's tiles, of its columns
+  float *dW, *db;
 };
-struct WGradParams {
-  WGradLayer l[kMaxLayers];
-  int nlayer, ntile, batch, chunk;  // chunk: batch rows of one split
+struct GradParams {
+  GradLayer l[kMaxLayers];
+  int nlayer, nbias, batch;  // nbias: blocks of column sums, which come first
 };
 
-__global__ void __launch_bounds__(256, 2) wgrad_kernel(const __grid_constant__ WGradParams p) {
-  extern __shared__ __align__(16) unsigned char step_smem[];
-  const int split = blockIdx.x / p.ntile;
-  int t = blockIdx.x % p.ntile, li = 0;
-  while (li + 1 < p.nlayer && p.l[li + 1].first_tile <= t) ++li;
-  const WGradLayer& L = p.l[li];
-  t -= L.first_tile;
-  StepEpi e{};
-  e.ldo = L.Kw;
-  e.part = L.part + (size_t)split * L.N * L.Kw;
-  step_tile<false, false, PARTIAL>(step_smem, L.dz, L.N, L.N, (t / L.tiles_k) * TM, L.act, L.lda, L.Kw,
-                                   (t % L.tiles_k) * TN, split * p.chunk, min(p.batch, (split + 1) * p.chunk), e);
+__device__ __forceinline__ void bias_columns(const GradLayer& L, int n0, int batch, float* smem) {
+  __shared__ float chain[8][kBiasCols];
+  const int tid = threadIdx.x, c = tid % kBiasCols, y = tid / kBiasCols;
+  const int nst = (batch + kBiasRows - 1) / kBiasRows;
+  auto load = [&](int st) {
+    if (st < nst) {
+#pragma unroll
+      for (int k = 0; k < kBiasRows * 4 / GTHREADS; ++k) {
+        const int row = (tid >> 2) + GTHREADS / 4 * k, m = st * kBiasRows + row, ch = (tid & 3) * 4;
+        cp_async16(smem + ((st % kBiasStages) * kBiasRows + row) * kBiasCols + ch,
+                   L.dzf + (size_t)min(m, batch - 1) * L.N + n0 + ch, m < batch);
+      }
+    }
+    cp_async_commit();
+  };
+  for (int st = 0; st < kBiasStages - 1; ++st) load(st);
+  float acc = 0.f;
+  for (int st = 0; st < nst; ++st) {
+    cp_async_wait<kBiasStages - 2>();
+    __syncthreads();
+    load(st + kBiasStages - 1);
+    if (y < 8) {
+      const float* p = smem + ((st % kBiasStages) * kBiasRows + y) * kBiasCols + c;
+      const int n = min(kBiasRows, batch - st * kBiasRows) / 8;  // a multiple of 4
+      for (int u = 0; u < n; u += 4) {
+        float v[4];
+#pragma unroll
+        for (int w = 0; w < 4; ++w) v[w] = p[(u + w) * 8 * kBiasCols];
+#pragma unroll
+        for (int w = 0; w < 4; ++w) acc += v[w];
+      }
+    }
+  }
+  cp_async_wait<0>();
+  if (y < 8) chain[y][c] = acc;
+  __syncthreads();
+  if (y == 0) {
+    float t = 0.f;
+    for (int k = 0; k < 8; ++k) t += chain[k][c];
+    L.db[n0 + c] = t;
+  }
 }
 
-// Adam over all parameters; a gradient is the sum of its partials in order.
+__global__ void __launch_bounds__(GTHREADS, 2) grad_kernel(const __grid_constant__ GradParams p) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  int li = 0;
+  if ((int)blockIdx.x < p.nbias) {
+    while (li + 1 < p.nlayer && p.l[li + 1].first_bias <= (int)blockIdx.x) ++li;
+    bias_columns(p.l[li], (blockIdx.x - p.l[li].first_bias) * kBiasCols, p.batch, reinterpret_cast<float*>(smem));
+    return;
+  }
+  int t = blockIdx.x - p.nbias;
+  while (li + 1 < p.nlayer && p.l[li + 1].first_tile <= t) ++li;
+  const GradLayer& L = p.l[li];
+  t -= L.first_tile;
+  const int n0 = t / L.tiles_k * GN, k0 = t % L.tiles_k * GT;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int wn = (warp >> 2) * 16, wk = (warp & 3) * 16;
+  const int nst = (p.batch + GB - 1) / GB;
+  // this thread's share of each stage: rows past the batch and columns past the matrix are zeros
+  const int rz = tid >> 2, cz = (tid & 3) * 8, rx = tid >> 3, cx = (tid & 7) * 8;
+  const bool ik = k0 + cx < L.Kw;
+  const bf16* gz = L.dz + (size_t)rz * L.N + n0 + cz;  // N is a multiple of 32
+  const bf16* gx = L.act + (size_t)rx * L.lda + (ik ? k0 + cx : 0);
+  const size_t step_z = (size_t)GB * L.N, half_x = (size_t)(GB / 2) * L.lda;
+  bf16* const s0 = reinterpret_cast<bf16*>(smem);
+  constexpr int SLOT = GB * (LD_N + LD_G);
+  int left = p.batch, wslot = 0, rslot = 0;  // left: rows of the batch from the next stage on
+  auto load = [&]() {
+    bf16* z = s0 + wslot * SLOT + rz * LD_N + cz;
+    bf16* x = s0 + wslot * SLOT + GB * LD_N + rx * LD_G + cx;
+    cp_async16(z, rz < left ? gz : L.dz, rz < left);
+    cp_async16(x, rx < left ? gx : L.act, ik && rx < left);
+    cp_async16(x + GB / 2 * LD_G, rx + GB / 2 < left ? gx + half_x : L.act, ik && rx + GB / 2 < left);
+    gz += step_z;
+    gx += 2 * half_x;
+    left -= GB;
+    wslot = wslot + 1 < GSTAGES ? wslot + 1 : 0;
+    cp_async_commit();
+  };
+  struct Fragments {
+    unsigned a[GB / 16][4], b[GB / 16][2][2];
+  };
+  float acc[2][4];
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) acc[j][r] = 0.f;
+  const bf16* const fa = s0 + ((lane & 7) + (lane >> 4) * 8) * LD_N + wn + ((lane >> 3) & 1) * 8;
+  const bf16* const fb = s0 + GB * LD_N + ((lane & 7) + ((lane >> 3) & 1) * 8) * LD_G + wk + (lane >> 4) * 8;
+  auto fetch = [&](Fragments& f) {
+    cp_async_wait<GSTAGES - 2>();
+    __syncthreads();
+    load();
+    const int at = rslot * SLOT;
+    rslot = rslot + 1 < GSTAGES ? rslot + 1 : 0;
+#pragma unroll
+    for (int q = 0; q < GB / 16; ++q) {
+      ldmatrix_x4_trans(f.a[q][0], f.a[q][1], f.a[q][2], f.a[q][3], fa + at + 16 * q * LD_N);
+      ldmatrix_x4_trans(f.b[q][0][0], f.b[q][0][1], f.b[q][1][0], f.b[q][1][1], fb + at + 16 * q * LD_G);
+    }
+  };
+  auto products = [&](const Fragments& f) {
+#pragma unroll
+    for (int q = 0; q < GB / 16; ++q)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) mma_bf16(acc[j], f.a[q], f.b[q][j]);
+  };
+  for (int st = 0; st < GSTAGES - 1; ++st) load();
+  Fragments f0, f1;
+  fetch(f0);
+#pragma unroll 1
+  for (int st = 0; st < nst; st += 2) {
+    if (st + 1 < nst) fetch(f1);
+    products(f0);
+    if (st + 1 >= nst) break;
+    if (st + 2 < nst) fetch(f0);
+    products(f1);
+  }
+  cp_async_wait<0>();
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int n = n0 + wn + (lane >> 2) + h * 8, k = k0 + wk + j * 8 + (lane & 3) * 2;
+      if (k < L.Kw)
+        *reinterpret_cast<float2*>(L.dW + (size_t)n * L.Kw + k) = make_float2(acc[j][h * 2], acc[j][h * 2 + 1]);
+    }
+}
+
+// Adam over all parameters.
 struct AdamTensor {
   float *p, *m, *v;
-  const float* part;
-  int n, npart, stride;  // partial s at part + s * stride
+  const float* grad;
+  int n;
   bf16* out;             // BF16 copy, or null
   int cols, ldo, dup;    // out row stride; dup: second copy at column dup (0: none)
   int first_block;
@@ -240,20 +335,35 @@ struct AdamTensor {
 struct AdamParams {
   AdamTensor t[2 * kMaxLayers];
   int nt;
+  float* loss;             // the last block adds the loss's partials, in order
+  const float* loss_part;
+  int nloss;
   float lr, b1, b2, eps, bc1, bc2;
 };
 
 __global__ void __launch_bounds__(256) adam_step_kernel(const __grid_constant__ AdamParams P) {
+  if (blockIdx.x == gridDim.x - 1) {
+    __shared__ double warp_part[8];
+    double sum = 0.0;
+    for (int i = threadIdx.x; i < P.nloss; i += 256) sum += (double)P.loss_part[i];
+#pragma unroll
+    for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if ((threadIdx.x & 31) == 0) warp_part[threadIdx.x >> 5] = sum;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int w = 1; w < 8; ++w) sum += warp_part[w];
+      *P.loss = (float)sum;
+    }
+    return;
+  }
   int k = 0;
   while (k + 1 < P.nt && P.t[k + 1].first_block <= (int)blockIdx.x) ++k;
   const AdamTensor& t = P.t[k];
   const int i = (blockIdx.x - t.first_block) * 256 + threadIdx.x;
   if (i >= t.n) return;
-  float g = 0.f;
-#pragma unroll 8
-  for (int s = 0; s < t.npart; ++s) g += t.part[(size_t)s * t.stride + i];
+  const float g = t.grad[i];
   const float m = P.b1 * t.m[i] + (1.f - P.b1) * g;
-  const float v = P.b2 * t.v[i] + (1.f - P.b2) * g * g;
+  const float v = __fmaf_rn(__fmul_rn(1.f - P.b2, g), g, __fmul_rn(P.b2, t.v[i]));
   t.m[i] = m;
   t.v[i] = v;
   const float w = t.p[i] - P.lr * (m / P.bc1) / (sqrtf(v / P.bc2) + P.eps);
@@ -273,14 +383,14 @@ using namespace pgb_mlp;
 namespace {
 
 constexpr int kStepSmem = STAGES * 2 * 2 * TM * LD_K;  // the larger of the layouts
-static_assert(tile_bytes<true>() >= tile_bytes<false>() && 4 * TN * 4 <= kStepSmem, "stage memory");
+static_assert(tile_bytes<true>() >= tile_bytes<false>(), "stage memory");
 
 size_t align16(size_t n) { return (n + 255) / 256 * 256; }
 
-// Workspace of a step: activations, pre-activations and dZ of the layers, gradient partials.
+// Workspace of a step: activations, pre-activations (then FP32 dZ) and dZ of the layers, gradients.
 struct Layout {
-  size_t act[kMaxLayers], pre[kMaxLayers], dz[kMaxLayers], wpart[kMaxLayers], bpart[kMaxLayers], total;
-  int split, chunk, ntile, mtiles;
+  size_t act[kMaxLayers], pre[kMaxLayers], dz[kMaxLayers], dw[kMaxLayers], db[kMaxLayers], loss, total;
+  int mtiles;
 };
 
 int weight_cols(const pgb_mlp_step& s, int l) { return l == 0 && s.k_half > 0 ? s.k_half : s.dims[l]; }
@@ -289,23 +399,16 @@ Layout layout_of(const pgb_mlp_step& s) {
   Layout y;
   size_t o = 0;
   auto take = [&](size_t n) { const size_t at = o; o += align16(n); return at; };
-  y.ntile = 0;
-  for (int l = 0; l < s.nlayer; ++l)
-    y.ntile += ((s.dims[l + 1] + TM - 1) / TM) * ((weight_cols(s, l) + TN - 1) / TN);
-  // about two CTAs per SM of a GB300, each with at least two k steps of the batch
-  const int want = std::max(1, 304 / y.ntile), most = std::max(1, s.batch / (2 * TK));
-  const int split = std::min(want, most);
-  y.chunk = ((s.batch / TK + split - 1) / split) * TK;
-  y.split = (s.batch + y.chunk - 1) / y.chunk;
   y.mtiles = (s.batch + TM - 1) / TM;
   for (int l = 0; l < s.nlayer; ++l) {
     const size_t n = (size_t)s.batch * s.dims[l + 1];
     y.act[l] = l + 1 < s.nlayer ? take(n * 2) : 0;
-    y.pre[l] = l + 1 < s.nlayer ? take(n * 4) : 0;
+    y.pre[l] = take(n * 4);
     y.dz[l] = take(n * 2);
-    y.wpart[l] = take((size_t)y.split * s.dims[l + 1] * weight_cols(s, l) * 4);
-    y.bpart[l] = take((size_t)y.mtiles * s.dims[l + 1] * 4);
+    y.dw[l] = take((size_t)s.dims[l + 1] * weight_cols(s, l) * 4);
+    y.db[l] = take((size_t)s.dims[l + 1] * 4);
   }
+  y.loss = take((size_t)y.mtiles * ((s.dims[s.nlayer] + TN - 1) / TN) * 8 * 4);
   y.total = o;
   return y;
 }
@@ -353,8 +456,7 @@ int pgb_mlp_train_step(const pgb_mlp_step* sp, void* workspace, void* stream) {
   PGB_CUDA(cudaFuncSetAttribute(step_gemm_kernel<true, FORWARD>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStepSmem));
   PGB_CUDA(cudaFuncSetAttribute(step_gemm_kernel<true, LOSS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStepSmem));
   PGB_CUDA(cudaFuncSetAttribute(step_gemm_kernel<false, INPUT_GRAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStepSmem));
-  PGB_CUDA(cudaFuncSetAttribute(wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStepSmem));
-  PGB_CUDA(cudaMemsetAsync(s.loss, 0, sizeof(float), st));
+  PGB_CUDA(cudaFuncSetAttribute(grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGradSmem));
   for (int l = 0; l < L; ++l) {
     StepEpi e{};
     e.bias = s.b[l];
@@ -366,9 +468,9 @@ int pgb_mlp_train_step(const pgb_mlp_step* sp, void* workspace, void* stream) {
                                                                           e.ldo, s.dims[l], e);
     } else {
       e.out = dz(l);
-      e.bias_part = fp(y.bpart[l]);
+      e.pre = fp(y.pre[l]);
       e.target = s.T;
-      e.loss = s.loss;
+      e.loss_part = fp(y.loss);
       e.scale = 2.f / ((float)B * (float)s.n_out);
       e.n_valid = s.n_out;
       step_gemm_kernel<true, LOSS><<<grid(e.ldo), 256, kStepSmem, st>>>(act(l - 1), ld(l - 1), B, wb(l), s.dims[l],
@@ -381,30 +483,32 @@ int pgb_mlp_train_step(const pgb_mlp_step* sp, void* workspace, void* stream) {
     e.ldo = s.dims[l];
     e.pre = fp(y.pre[l - 1]);
     e.out = dz(l - 1);
-    e.bias_part = fp(y.bpart[l - 1]);
     step_gemm_kernel<false, INPUT_GRAD><<<grid(e.ldo), 256, kStepSmem, st>>>(dz(l), s.dims[l + 1], B, wb(l), s.dims[l],
                                                                             e.ldo, s.dims[l + 1], e);
     PGB_CUDA(cudaGetLastError());
   }
-  WGradParams w;
+  GradParams w;
   w.nlayer = L;
-  w.ntile = y.ntile;
   w.batch = B;
-  w.chunk = y.chunk;
-  int first = 0;
+  int tiles = 0;
+  w.nbias = 0;
   for (int l = 0; l < L; ++l) {
-    WGradLayer& g = w.l[l];
+    GradLayer& g = w.l[l];
     g.dz = dz(l);
     g.act = act(l - 1);
+    g.dzf = fp(y.pre[l]);
     g.lda = ld(l - 1);
     g.N = s.dims[l + 1];
     g.Kw = weight_cols(s, l);
-    g.tiles_k = (g.Kw + TN - 1) / TN;
-    g.first_tile = first;
-    g.part = fp(y.wpart[l]);
-    first += ((g.N + TM - 1) / TM) * g.tiles_k;
+    g.tiles_k = (g.Kw + GT - 1) / GT;
+    g.first_tile = tiles;
+    g.first_bias = w.nbias;
+    g.dW = fp(y.dw[l]);
+    g.db = fp(y.db[l]);
+    tiles += g.N / GN * g.tiles_k;
+    w.nbias += g.N / kBiasCols;
   }
-  wgrad_kernel<<<y.ntile * y.split, 256, kStepSmem, st>>>(w);
+  grad_kernel<<<w.nbias + tiles, GTHREADS, kGradSmem, st>>>(w);
   PGB_CUDA(cudaGetLastError());
   AdamParams a;
   a.nt = 0;
@@ -412,11 +516,11 @@ int pgb_mlp_train_step(const pgb_mlp_step* sp, void* workspace, void* stream) {
   a.bc1 = 1.f - powf(s.b1, (float)s.step);
   a.bc2 = 1.f - powf(s.b2, (float)s.step);
   int blocks = 0;
-  auto add = [&](float* p, float* m, float* v, const float* part, int n, int npart, int stride, void* out, int cols,
-                 int ldo, int dup) {
+  auto add = [&](float* p, float* m, float* v, const float* grad, int n, void* out, int cols, int ldo,
+                 int dup) {
     AdamTensor& t = a.t[a.nt++];
-    t.p = p; t.m = m; t.v = v; t.part = part;
-    t.n = n; t.npart = npart; t.stride = stride;
+    t.p = p; t.m = m; t.v = v; t.grad = grad;
+    t.n = n;
     t.out = static_cast<bf16*>(out); t.cols = cols; t.ldo = ldo; t.dup = dup;
     t.first_block = blocks;
     blocks += (n + 255) / 256;
@@ -424,10 +528,13 @@ int pgb_mlp_train_step(const pgb_mlp_step* sp, void* workspace, void* stream) {
   for (int l = 0; l < L; ++l) {
     const int n = s.dims[l + 1], kw = weight_cols(s, l);
     const bool split_in = l == 0 && s.k_half > 0;
-    add(s.W[l], s.mW[l], s.vW[l], fp(y.wpart[l]), n * kw, y.split, n * kw, s.Wb[l], kw, s.dims[l], split_in ? kw : 0);
-    add(s.b[l], s.mb[l], s.vb[l], fp(y.bpart[l]), n, y.mtiles, n, nullptr, 1, 1, 0);
+    add(s.W[l], s.mW[l], s.vW[l], fp(y.dw[l]), n * kw, s.Wb[l], kw, s.dims[l], split_in ? kw : 0);
+    add(s.b[l], s.mb[l], s.vb[l], fp(y.db[l]), n, nullptr, 1, 1, 0);
   }
-  adam_step_kernel<<<blocks, 256, 0, st>>>(a);
+  a.loss = s.loss;
+  a.loss_part = fp(y.loss);
+  a.nloss = y.mtiles * ((s.dims[L] + TN - 1) / TN) * 8;
+  adam_step_kernel<<<blocks + 1, 256, 0, st>>>(a);
   PGB_CUDA(cudaGetLastError());
   return 0;
 }

@@ -112,14 +112,17 @@ def test_adam_training_reduces_loss(native_lib, cuda):
     assert losses[-1] < 0.2 * losses[0], (losses[0], losses[-1])
 
 
-# row tiles of 128 with a remainder, output tiles with a remainder, one k step, one layer beyond the
-# input, split and plain input, the training size
+# row tiles of 128 with a remainder, output tiles with a remainder, one k step, batches that are no
+# multiple of 64, of the chains of the bias gradients or of their unrolling, one layer beyond the input,
+# split and plain input, the training size
 @pytest.mark.gpu
 @pytest.mark.parametrize("B,width,depth,n_in,n_out,split", [
-    (32, 64, 1, 20, 10, True), (160, 96, 3, 44, 20, True), (288, 160, 2, 33, 40, False), (8192, 256, 4, 44, 20, True)])
+    (32, 64, 1, 20, 10, True), (160, 96, 3, 44, 20, True), (288, 160, 2, 33, 40, False),
+                                                           (1056, 64, 2, 33, 9, True), (8192, 256, 4, 44, 20, True)])
 def test_native_step_equals_the_separate_kernels(native_lib, cuda, B, width, depth, n_in, n_out, split):
-    """train_step against forward, loss_grad, backward and adam on a twin: products of activations
-    keep their bits, so the gradients differ by the order in which the batch is summed alone."""
+    """train_step against forward, loss_grad, backward and adam on a twin: every product and every sum
+    over the batch keeps its order, so parameters and moments keep their bits; the loss alone is summed
+    in another order (the separate kernels add it with atomics)."""
     from pelelm_gb300.surrogate import SurrogateMLP
     torch = cuda
     kw = dict(width=width, depth=depth, seed=7, split_input=split)
@@ -133,18 +136,10 @@ def test_native_step_equals_the_separate_kernels(native_lib, cuda, B, width, dep
         Y = b.forward(X, keep=True)
         dYf, dY, lb = b.loss_grad(Y, T)
         b.adam(*b.backward(dYf, dY), lr=1e-3)
-        if step:
-            break
-        # sums of B terms in FP32, in two orders
-        tol = 2.0 ** -20 * B ** 0.5
-        assert abs(float(la) - float(lb)) <= tol * float(lb)
-        for x, y in zip(a.mW + a.mb, b.mW + b.mb):
-            assert float((x - y).abs().max()) <= tol * float(y.abs().max())
+        assert abs(float(la) - float(lb)) <= 2.0 ** -20 * B ** 0.5 * float(lb)
     assert a.step_count == b.step_count == 2
-    for x, y in zip(a.W + a.b, b.W + b.b):
-        # an Adam step moves a parameter by lr at most; where the gradient is not small against its
-        # rounding the two agree far better
-        assert float((x - y).abs().max()) <= 2 * 2e-3 and float((x - y).abs().mean()) <= 2e-6
+    for x, y in zip(a.W + a.b + a.mW + a.mb + a.vW + a.vb, b.W + b.b + b.mW + b.mb + b.vW + b.vb):
+        assert torch.equal(x, y)
     for x, y in zip(a.W[1:], a.Wb[1:]):
         assert torch.equal(x.to(torch.bfloat16), y)
     if split:
