@@ -905,7 +905,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
 #pragma unroll 1
         for (int k = 0; k < N; ++k) {
           const int p = rec.piv[k];
-          if (p == k) continue;
+          if (p <= k || p >= N) continue;
           const int i0 = C.PIV[k];
           C.PIV[k] = C.PIV[p];
           C.PIV[p] = i0;
@@ -949,7 +949,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
       }
       if (S == G && queue_empty && P.drain > 0) {
         const unsigned left = __ballot_sync(0xffffffffu, phase != IDLE && sub == 0);
-        if (__popc(left) <= P.drain && phase == STEP && new_step && nst < P.max_steps) hand_over();
+        if (__popc(left) <= P.drain && phase == STEP && new_step && nst > 0 && nst < P.max_steps) hand_over();
         __syncwarp();
       }
       if (__all_sync(0xffffffffu, phase == IDLE)) break;

@@ -459,7 +459,8 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
     return true;
   };
 
-  // hands this lane's cell over at the start of a step
+  // hands this lane's cell over at the start of a step (not its first: there are no factors yet, and the
+  // pivots are whatever the memory holds)
   auto hand_over = [&]() {
     const ResumeRec<N, JR> rec(P.resume, atomicAdd(P.resume_count, 1ull));
     ResumeHead H;
@@ -506,7 +507,7 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
     }
     if (queue_empty && P.drain > 0) {
       const unsigned left = __ballot_sync(0xffffffffu, phase != IDLE);
-      if (__popc(left) <= P.drain && phase == STEP && new_step && nst < P.max_steps) hand_over();
+      if (__popc(left) <= P.drain && phase == STEP && new_step && nst > 0 && nst < P.max_steps) hand_over();
       __syncwarp();
     }
     if (__all_sync(0xffffffffu, phase == IDLE)) break;

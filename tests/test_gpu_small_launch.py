@@ -64,6 +64,24 @@ def test_handed_over_cells_keep_their_bits(native_lib, cuda, cfgname, mapping, p
         assert torch.equal(x, y)
 
 
+# as many cells as lanes hold at once, the last warps part full: those would hand cells over before their
+# first step, when the pivots are not yet set (they keep them until a step is done)
+@pytest.mark.gpu
+@pytest.mark.parametrize("cfgname,mapping", [("lidryer_amr120", "thread"), ("drm19_2M", "group")])
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("shape", [(25, 17, 18), (29, 27, 22)])
+def test_part_full_warps_keep_their_bits(native_lib, cuda, cfgname, mapping, precision, shape):
+    torch = cuda
+    cfg = CONFIGS[cfgname]
+    assert 0 < np.prod(shape) % 32 <= 13
+    opts = f"gb.precision={precision}"
+    fa, a = _advance(torch, cfg, shape, opts, False, 4, False)
+    fb, b = _advance(torch, cfg, shape, opts + f" gb.mapping={mapping}", False, 4, False)
+    assert fa == fb == 0
+    for x, y in ((a.FC, b.FC), (a.rY, b.rY), (a.rEner, b.rEner), (a.T, b.T)):
+        assert torch.equal(x, y)
+
+
 # teams of warps: one cell; fewer cells than SMs; two teams a block; above the limit, where the last
 # cells of the launch change to teams at a step; steps limited, so that cells fail and are retried
 @pytest.mark.gpu
