@@ -473,8 +473,8 @@ def run_gb(args, ws, rank, local, pg):
                       "nje_per_cell": st["nje"] / ncell, "max_steps_cell": st["max_nst"], "nfail": int(st["nfail"]), "nretry": int(st["nretry"]),
                       "steps_hist_log2": hist},
             "clocks": clocks,
-            # per step: [surrogate] + BDF (+ FP64 retry pass in mixed precision) + [audit]
-            "gpu_launches": args.steps * ((2 if surrogate else 0) + (2 if args.precision == "mixed" else 1)),
+            # per step: [surrogate] + BDF + its last cells (+ FP64 retry pass in mixed precision) + [audit]
+            "gpu_launches": args.steps * ((2 if surrogate else 0) + (3 if args.precision == "mixed" else 2)),
             **extra,
         }
         if cpu:

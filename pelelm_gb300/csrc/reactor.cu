@@ -827,9 +827,7 @@ int advance_box_table(pgb_reactor* r, const std::vector<pgb::BoxDev>& boxes, lon
       pl.lu_bytes = std::max(pl.lu_bytes, p64.lu_bytes);
       if (ensure_buf(*s, s->d_retry, s->retry_cap, std::max<long long>(ncell, 1) * sizeof(long long))) return -1;
     }
-    if (ensure_buf(*s, s->d_z, s->z_cap, pl.z_bytes) || ensure_buf(*s, s->d_lu, s->lu_cap, pl.lu_bytes) ||
-        ensure_buf(*s, s->d_resume, s->resume_cap, pl.resume_bytes))
-      return -1;
+    if (ensure_buf(*s, s->d_z, s->z_cap, pl.z_bytes) || ensure_buf(*s, s->d_lu, s->lu_cap, pl.lu_bytes)) return -1;
     if (r->sg.d_net) {
       const long long acap = audit_capacity(r, ncell);
       if (ensure_buf(*s, s->d_fallback, s->fallback_cap, std::max<long long>(ncell, 1) * sizeof(long long)) ||
@@ -837,6 +835,8 @@ int advance_box_table(pgb_reactor* r, const std::vector<pgb::BoxDev>& boxes, lon
                      std::max<long long>(acap, 1) * (sizeof(long long) + pgb::MAXN * sizeof(double))))
         return -1;
     }
+    // without this buffer the launch keeps its last cells: no reason to refuse the call
+    if (ensure_buf(*s, s->d_resume, s->resume_cap, pl.resume_bytes)) (void)cudaGetLastError();
   }
   PGB_CUDA(cudaEventSynchronize(s->done));  // staging buffer may still feed a previous copy
   if (nbox) std::memcpy(s->h_boxes, boxes.data(), nbox * sizeof(pgb::BoxDev));
