@@ -193,8 +193,11 @@ __device__ __forceinline__ double rate_of_progress_unrolled(int j, double T, dou
         if (s >= n) continue;
         const int k = side ? rs(s) : ps(s);
         if (s > 0 && (side ? rs(s - 1) : ps(s - 1)) == k) continue;  // counted with its first slot
-        double nu = side ? -1.0 : 1.0;
-        if (s + 1 < n && (side ? rs(s + 1) : ps(s + 1)) == k) nu += nu;
+        int same = 1;  // the coefficient: slots of one species are neighbours
+#pragma unroll
+        for (int u = s + 1; u < (side ? Tab::MAXR : Tab::MAXP); ++u)
+          if (u < n && (side ? rs(u) : ps(u)) == k) ++same;
+        const double one = side ? -1.0 : 1.0, nu = same == 1 ? one : same == 2 ? 2.0 * one : 3.0 * one;
         dG = first ? __dmul_rn(nu, GS[k]) : fma(nu, GS[k], dG);
         first = false;
       }
