@@ -69,24 +69,6 @@ __host__ __device__ constexpr int gbdf_smem_per_warp() {
   return (32 / G) * gbdf_cell_bytes<M, JR>() + gbdf_shared_scratch_bytes<M, JR, G>();
 }
 
-// J(i, k) of a row-major matrix with rows of LDA.
-template <class JR, int LDA>
-struct RowAcc {
-  JR* base;
-  __device__ __forceinline__ JR& operator()(int i, int k) const { return base[i * LDA + k]; }
-};
-
-// The unrolled Jacobian by one lane, out of line: its registers do not add to the kernel's.
-template <class M, class JR>
-__device__ __noinline__ void unrolled_jacobian(const double* y, const double* FRC, JR* A) {
-  double yl[M::N], Fl[M::NS];
-#pragma unroll
-  for (int i = 0; i < M::N; ++i) yl[i] = y[i];
-#pragma unroll
-  for (int i = 0; i < M::NS; ++i) Fl[i] = FRC[i];
-  M::template jac<JR>(yl, Fl, FRC[M::NS], RowAcc<JR, M::N + 1>{A});
-}
-
 // The group-distributed part of a length-N vector (element i in sub-lane i % G, slot i / G).
 template <class M, int G>
 struct GVec {
@@ -225,7 +207,7 @@ __device__ __forceinline__ GVec<M, G> group_rhs(const GVec<M, G> yv, double* CS,
   using Tab = typename M::TabG;
   constexpr int N = M::N, NS = M::NS, NR = M::NR;
   constexpr int R = (N + G - 1) / G;
-  constexpr bool UNROLLED = !M::RHS_TABLE;  // bits of the unrolled per-thread code
+  constexpr bool UNROLLED = !M::RHS_TABLE;  // the operations of the unrolled per-thread code
   static_assert(S == G || R == 1, "another summation order needs an element per lane");
   static_assert(!UNROLLED || S == 1, "the unrolled code sums in sequence");
   const int lane = threadIdx.x & 31, sub = lane % G, gbase = lane - sub;
@@ -259,7 +241,7 @@ __device__ __forceinline__ GVec<M, G> group_rhs(const GVec<M, G> yv, double* CS,
         Tmid = s.Tmid;
         g = below_positive(T, Tmid) ? s.glo : s.ghi;
       }
-      const double c = y[r] * invW;
+      const double c = __dmul_rn(y[r], invW);
       CS[k] = c;
       c_loc += c;
       if (fused) { c_loc = y[r]; c_fac = invW; }
@@ -299,13 +281,11 @@ __device__ __forceinline__ GVec<M, G> group_rhs(const GVec<M, G> yv, double* CS,
       if constexpr (UNROLLED) {
         const TabUnrolled& s = Tab::un(k);
         const int e1 = Tab::un_begin(k + 1);
-        // the compiler fuses the product q [M] of the last reaction, if it is a third-body one, into
-        // the sums it enters
 #pragma unroll 2
         for (int e = Tab::un_begin(k); e < e1; ++e) {
           const int j = Tab::un_j(e);
-          const double qj = Tab::un_nu(e) * QS[j], mj = QS[NR + j];
-          wdot = Tab::un_m(e) ? fma(qj, mj, wdot) : __dadd_rn(wdot, __dmul_rn(qj, mj));
+          const double nu = Tab::un_nu(e), qj = QS[j], mj = QS[NR + j];
+          wdot = Tab::un_m(e) ? fma(nu * qj, mj, wdot) : fma(nu, __dmul_rn(qj, mj), wdot);  // un_m: nu is 1 or -1
         }
         f[r] = fma(wdot, s.W, FRC[k]);
         const bool lo = below_positive(T, s.Tmid);
@@ -343,7 +323,7 @@ __device__ __forceinline__ GVec<M, G> group_rhs(const GVec<M, G> yv, double* CS,
     rcp = lane_dot<NS, S>(c_one, cp_one, gm, gbase);
   }
   if constexpr (!UNROLLED) rcp *= kRerg;
-  const double fT = pgb_div64(fma(-hs, kRerg * T, FRC[NS]), rcp);
+  const double fT = pgb_div64(fma(-hs, __dmul_rn(kRerg, T), FRC[NS]), rcp);
 #pragma unroll
   for (int r = 0; r < R; ++r)
     if (idx(r) == NS) f[r] = fT;
@@ -449,7 +429,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
         if (idx(r) < N) Z(j, r) *= fac;
       fac *= e;
     }
-    h = hscale * e;
+    h = __dmul_rn(hscale, e);
     hscale = h;
   };
   auto predict = [&]() {
@@ -498,7 +478,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
     const double xiq_inv = __shfl_sync(gm, xi, gbase + q - 1), xiq1_inv = __shfl_sync(gm, xi, gbase + q);
     const double alpha0_hat = -(sum_xi_inv + xiq_inv);
     const double A1 = 1.0 - alpha0_hat + alpha0;
-    const double A2 = 1.0 + q * A1;
+    const double A2 = fma((double)q, A1, 1.0);
     const double lq = __shfl_sync(gm, l, gbase + q), l1 = __shfl_sync(gm, l, gbase + 1);
     const double A3 = alpha0 + inv_int(q), A4 = alpha0_hat + xiq_inv;
     const double A5 = alpha0 - inv_int(q + 1), A6 = alpha0_hat - xiq1_inv;
@@ -547,7 +527,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
     const double xiq_inv = pgb_div64(h, hsum);
     const double alpha0_hat = -(sum_xi_inv + xiq_inv);
     const double A1 = 1.0 - alpha0_hat + alpha0;
-    const double A2 = 1.0 + q * A1;
+    const double A2 = fma((double)q, A1, 1.0);
     double lq = 0.0;
 #pragma unroll
     for (int k = 0; k <= QMAX; ++k) if (k == q) lq = l[k];
@@ -1016,7 +996,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
       if constexpr (UNROLLED) {
         if (wanted && idx(0) < N) C.CS[idx(0)] = y[0];  // the RHS scratch is free
         __syncwarp();
-        if (wanted && sub == 0) unrolled_jacobian<M>(C.CS, C.FRC, C.A);
+        if (wanted && sub == 0) M::template jac<JR>(C.CS, C.FRC, C.FRC[NS], C.A, LDA, 1);
         __syncwarp();
       }
       while (todo) {
@@ -1126,7 +1106,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
         if (gamrat != 1.0) {
           const double s = pgb_div64(2.0, 1.0 + gamrat);
 #pragma unroll
-          for (int r = 0; r < R; ++r) b[r] *= s;
+          for (int r = 0; r < R; ++r) b[r] = __dmul_rn(b[r], s);
         }
         del2 = wms(b);
 #pragma unroll

@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
       for (int i = 0; i < N; ++i) Z(j, i) *= fac;
       fac *= e;
     }
-    h = hscale * e;
+    h = __dmul_rn(hscale, e);
     hscale = h;
   };
   auto predict = [&]() {
@@ -213,15 +213,15 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
       if (i > 1) hsum += TAU(i - 1);
       const double xi_inv = pgb_div64(h, hsum);
       sum_xi_inv += xi_inv;
-      for (int k = i; k >= 1; --k) LCO(k) += LCO(k - 1) * xi_inv;
+      for (int k = i; k >= 1; --k) LCO(k) = fma(LCO(k - 1), xi_inv, LCO(k));
     }
     const double xistar_inv = -alpha0 - sum_xi_inv;
-    for (int k = q; k >= 1; --k) LCO(k) += LCO(k - 1) * xistar_inv;
+    for (int k = q; k >= 1; --k) LCO(k) = fma(LCO(k - 1), xistar_inv, LCO(k));
     if (q > 1) hsum += TAU(q - 1);
     const double xiq_inv = pgb_div64(h, hsum);
     const double alpha0_hat = -(sum_xi_inv + xiq_inv);
     const double A1 = 1.0 - alpha0_hat + alpha0;
-    const double A2 = 1.0 + q * A1;
+    const double A2 = fma((double)q, A1, 1.0);
     tq2 = fabs(pgb_div64(A1, alpha0 * A2));
     tq5 = fabs(pgb_div64(A2 * xistar_inv, LCO(q) * xiq_inv));
     if (qwait == 1) {
@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
         alpha1 += pgb_div64(1.0, xi);
         if (j <= q - 1)
 #pragma unroll 1
-          for (int i = j + 2; i >= 2; --i) w[i] = w[i] * xi + w[i - 1];
+          for (int i = j + 2; i >= 2; --i) w[i] = fma(w[i], xi, w[i - 1]);
       }
       const double A1 = pgb_div64(-alpha0 - alpha1, prod);
 #pragma unroll
@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
         hsum += TAU(j);
         const double xi = pgb_div64(hsum, hscale);
 #pragma unroll 1
-        for (int i = j + 2; i >= 2; --i) w[i] = w[i] * xi + w[i - 1];
+        for (int i = j + 2; i >= 2; --i) w[i] = fma(w[i], xi, w[i - 1]);
       }
 #pragma unroll 1
       for (int j = 2; j < q; ++j) {
@@ -288,8 +288,8 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
   };
   // M = I - gamma J in the LU slice, factor with partial pivoting (trailing swaps)
   auto setup_matrix = [&]() -> bool {
-    LuAcc<JR> acc{LUb, N, lu_stride};
     if constexpr (M::JAC_TABLE) {
+      LuAcc<JR> acc{LUb, N, lu_stride};
       // concentrations go to the solve vector (free during the setup); forcing read in place
       jac_table<typename M::Tab, JR>(y, [&](int k) -> double { return FRC(k); }, FRC(NS), acc,
                                      [&](int k) -> JR& { return XS(k); });
@@ -297,12 +297,12 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
       double Fl[NS];
 #pragma unroll
       for (int i = 0; i < NS; ++i) Fl[i] = FRC(i);
-      M::template jac<JR>(y, Fl, FRC(NS), acc);
+      M::template jac<JR>(y, Fl, FRC(NS), LUb, N * (int)lu_stride, (int)lu_stride);
     }
     const JR g = (JR)gamma;
 #pragma unroll 1
     for (int i = 0; i < N; ++i)
-      for (int k = 0; k < N; ++k) LU(i, k) = (i == k ? JR(1) : JR(0)) - g * LU(i, k);
+      for (int k = 0; k < N; ++k) LU(i, k) = fma(-g, LU(i, k), i == k ? JR(1) : JR(0));
     bool ok = true;
     // partial-pivot LU; the diagonal keeps the reciprocal pivot for the solve
 #pragma unroll 1
@@ -320,9 +320,9 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
       const JR inv = JR(1) / LU(k, k);
       LU(k, k) = inv;
       for (int i = k + 1; i < N; ++i) {
-        const JR l = LU(i, k) * inv;
+        const JR l = pgb_mul(LU(i, k), inv);
         LU(i, k) = l;
-        for (int j = k + 1; j < N; ++j) LU(i, j) -= l * LU(k, j);
+        for (int j = k + 1; j < N; ++j) LU(i, j) = fma(-l, LU(k, j), LU(i, j));
       }
     }
     ++nje;
@@ -342,13 +342,13 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
       const int p = PIV(k);
       if (p != k) { const JR tmp = XS(k); XS(k) = XS(p); XS(p) = tmp; }
       const JR bk = XS(k);
-      for (int i = k + 1; i < N; ++i) XS(i) -= LU(i, k) * bk;
+      for (int i = k + 1; i < N; ++i) XS(i) = fma(-LU(i, k), bk, XS(i));
     }
 #pragma unroll 1
     for (int k = N - 1; k >= 0; --k) {
       JR sacc = XS(k);
-      for (int j = k + 1; j < N; ++j) sacc -= LU(k, j) * XS(j);
-      XS(k) = sacc * LU(k, k);
+      for (int j = k + 1; j < N; ++j) sacc = fma(-LU(k, j), XS(j), sacc);
+      XS(k) = pgb_mul(sacc, LU(k, k));
     }
 #pragma unroll
     for (int i = 0; i < N; ++i) b[i] = (double)XS(i);
@@ -630,7 +630,7 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
         if (gamrat != 1.0) {
           const double s = pgb_div64(2.0, 1.0 + gamrat);
 #pragma unroll
-          for (int i = 0; i < N; ++i) b[i] *= s;
+          for (int i = 0; i < N; ++i) b[i] = __dmul_rn(b[i], s);
         }
         del2 = wms(b);
 #pragma unroll
@@ -735,7 +735,7 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
                   const double cquot = pgb_div64(tq5, tq5_saved) * hrp;
                   double tv[N];
 #pragma unroll
-                  for (int i = 0; i < N; ++i) tv[i] = acor[i] - cquot * Z(QMAX + 1, i);
+                  for (int i = 0; i < N; ++i) tv[i] = fma(-cquot, Z(QMAX + 1, i), acor[i]);
                   const double dup2 = wms(tv) * (tq3 * tq3);
                   etaqp1 = pgb_div64(1.0, pgb_pow64((BIAS3 * BIAS3) * dup2, 0.5 * inv_int(q + 2)) + ADDON);
                 }

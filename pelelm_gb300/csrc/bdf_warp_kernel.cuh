@@ -141,14 +141,14 @@ __device__ __forceinline__ double rate_of_progress(int j, double T, double invT,
   if (kind == 2) {
     const TabTroe<double>& fo = Tab::template troe<double>(troe);
     const double lnk0 = fma(fo.beta0, lnT, fma(fo.mEa0R, invT, fo.lnA0));
-    const double Pr = Mc * pgb_exp64(lnk0 - lnkf);
-    double blend = pgb_div64(Pr, 1.0 + Pr);
+    const double Pr = __dmul_rn(Mc, pgb_exp64(lnk0 - lnkf));
+    double blend = pgb_div64(Pr, __dadd_rn(1.0, Pr));
     if (fo.ntroe > 0) {
       double Fcent = fma(fo.one_m_a, pgb_exp64(T * fo.m_invT3), fo.a * pgb_exp64(T * fo.m_invT1));
       if (fo.ntroe > 3) Fcent += pgb_exp64(invT * fo.m_T2);
       const double lFc = pgb_log64(Fcent) * 0.4342944819032518;
       const double cc = fma(-0.67, lFc, -0.4), nn = fma(-1.27, lFc, 0.75);
-      const double lPr = pgb_log64(fmax(Pr, 1e-300)) * 0.4342944819032518 + cc;
+      const double lPr = fma(pgb_log64(fmax(Pr, 1e-300)), 0.4342944819032518, cc);
       const double f1 = pgb_div64(lPr, fma(-0.14, lPr, nn));
       blend *= pgb_exp64(pgb_div64(2.302585092994046 * lFc, fma(f1, f1, 1.0)));
     }
@@ -1021,7 +1021,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
           if (idx(r) < N) zget(j, r) *= fac;
         fac *= e;
       }
-      h = hscale * e;
+      h = __dmul_rn(hscale, e);
       hscale = h;
     };
     auto predict = [&]() {
@@ -1068,7 +1068,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
       const double xiq_inv = __shfl_sync(0xffffffffu, xi, q - 1), xiq1_inv = __shfl_sync(0xffffffffu, xi, q);
       const double alpha0_hat = -(sum_xi_inv + xiq_inv);
       const double A1 = 1.0 - alpha0_hat + alpha0;
-      const double A2 = 1.0 + q * A1;
+      const double A2 = fma((double)q, A1, 1.0);
       const double lq = __shfl_sync(0xffffffffu, l, q), l1 = __shfl_sync(0xffffffffu, l, 1);
       const double A3 = alpha0 + inv_int(q), A4 = alpha0_hat + xiq_inv;
       const double A5 = alpha0 - inv_int(q + 1), A6 = alpha0_hat - xiq1_inv;
@@ -1163,7 +1163,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
           if (gamrat != 1.0) {
             const double s = pgb_div64(2.0, 1.0 + gamrat);
 #pragma unroll
-            for (int r = 0; r < R; ++r) tmp[r] *= s;
+            for (int r = 0; r < R; ++r) tmp[r] = __dmul_rn(tmp[r], s);
           }
           del2 = wms(tmp);
 #pragma unroll
@@ -1383,7 +1383,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
           for (int k = 0; k < q; ++k) hrp *= d[0];
           const double cquot = d[1] * hrp;
 #pragma unroll
-          for (int r = 0; r < R; ++r) tmp[r] = acor[r] - cquot * acor_saved[r];
+          for (int r = 0; r < R; ++r) tmp[r] = fma(-cquot, acor_saved[r], acor[r]);
           dup2 = wms(tmp) * (tq3 * tq3);
         }
       }

@@ -61,7 +61,7 @@ struct TabTroe {
 };
 
 // Constants of one species as the unrolled right-hand side folds them: 1/W, W, Tmid, whether its
-// concentration enters the sum [M] alone (the compiler then fuses its product there), then below /
+// concentration enters the sum [M] alone (its product is then fused there), then below /
 // above Tmid g/RT (as glo / ghi), h/RT over W, and cp (erg) over W.
 struct TabUnrolled {
   double invW, W, Tmid;

@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(32) newton_matrix_thread_kernel(const NewtonMa
       double Fl[NS];
 #pragma unroll
       for (int i = 0; i < NS; ++i) Fl[i] = F[i];
-      M::template jac<JR>(y, Fl, P.Fh[c], acc);
+      M::template jac<JR>(y, Fl, P.Fh[c], Jt, 32 * N, 32);
     }
     for (int i = 0; i < N; ++i)
       for (int k = 0; k < N; ++k) P.J[c * N * N + i * N + k] = (double)acc(i, k);

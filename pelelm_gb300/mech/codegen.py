@@ -9,8 +9,8 @@ mechanism-specific generated rate/thermo code), written from scratch for sm_103a
 * rates evaluate ln k in FP64 FMAs and take one exponential per coefficient;
 * the Jacobian is a template on its arithmetic type: ``float`` recomputes every rate
   coefficient in FP32 (the inexact-Newton preconditioner), ``double`` gives the plain
-  FP64 Jacobian. It writes J(i,k) through an accessor so the caller decides where the
-  matrix lives (shared memory per thread).
+  FP64 Jacobian. It writes J(i,k) at strides the caller gives, so the caller decides where the
+  matrix lives (shared memory per thread or per cell).
 
 The formulas are those of the CPU oracle (``oracle/chem_oracle.cpp``), which is the
 equation-level restatement of Model.rst:227-296.
@@ -95,6 +95,20 @@ def check_supported(m: Mechanism) -> None:
         if r.rev is not None:
             raise ValueError(f"{m.name}: reaction {j} ({r.equation()}) has explicit reverse parameters "
                              "(REV), which the rate kernels do not evaluate")
+
+
+def total_only(m: Mechanism) -> set:
+    """Species whose concentration enters the sum [M] alone; the exact form fuses its product there."""
+    return {k for k, s in enumerate(m.species)
+            if not any(s.name in r.reactants or s.name in r.products or r.efficiencies.get(s.name, 1.0) != 1.0
+                       for r in m.reactions)}
+
+
+def fused_third_body(m: Mechanism) -> int:
+    """The reaction whose product q [M] the exact form fuses into the production rates: the last one, if
+    it is a third-body reaction (-1: none). With total_only the contractions that the built-in mechanism's
+    code had before its roundings were written out."""
+    return m.nr - 1 if m.nr and m.reactions[-1].kind == "three_body" else -1
 
 
 def gen_header(m: Mechanism) -> str:
@@ -238,6 +252,97 @@ def gen_header(m: Mechanism) -> str:
                             (f"{expr} - q{j}" if nu == -1 else f"fma({_f(nu)}, q{j}, {expr})"))
             e(f"const double wd{k} = {expr};")
 
+    def emit_rates_exact():
+        """The same from y, C{k} and g{k} with every rounding written out: the lane-parallel evaluation
+        (rate_of_progress_unrolled and group_rhs, csrc/bdf_group_kernel.cuh) performs these operations in
+        this order, so the two agree bit for bit whatever the compiler would contract."""
+        alone = total_only(m)
+        if any(r.kind != "elementary" for r in m.reactions):
+            tot = "C0"
+            for k in range(1, ns):
+                tot = f"fma(y[{k}], {_f(1.0 / W[k])}, {tot})" if k in alone else f"__dadd_rn({tot}, C{k})"
+            e(f"const double Ctot = {tot};")
+        e(f"const double lnP0RT = {_f(lnP0_R)} - lnT;")
+
+        def product(first, names):
+            for n_ in names:
+                first = f"__dmul_rn({first}, {n_})" if first else n_
+            return first
+
+        for j, r in enumerate(m.reactions):
+            e(f"// R{j}: {r.equation()}")
+            e(f"double q{j};")
+            if j == fused_third_body(m):
+                e(f"double qu{j}, M{j};  // q{j} = qu{j} M{j}")
+            e("{")
+            e.ind += 1
+            e(f"const double lnkf = fma({_f(r.rate.beta)}, lnT, fma({_f(-r.rate.Ea / R_CAL)}, invT, {_f(math.log(r.rate.A))}));")
+            if r.kind != "elementary":
+                terms = "Ctot"
+                for sname, eff in r.efficiencies.items():
+                    if eff != 1.0:
+                        terms = f"fma({_f(eff - 1.0)}, C{idx[sname]}, {terms})"
+                e(f"const double M = {terms};")
+            if r.kind == "falloff":
+                e(f"const double lnk0 = fma({_f(r.low.beta)}, lnT, fma({_f(-r.low.Ea / R_CAL)}, invT, {_f(math.log(r.low.A))}));")
+                e("const double Pr = __dmul_rn(M, pgb_exp(lnk0 - lnkf));")
+                e("double blend = Pr / __dadd_rn(1.0, Pr);")
+                if r.troe:
+                    a, T3, T1 = r.troe[:3]
+                    fc = f"fma({_f(1.0 - a)}, pgb_exp(T * {_f(-1.0 / T3)}), __dmul_rn({_f(a)}, pgb_exp(T * {_f(-1.0 / T1)})))"
+                    if len(r.troe) > 3:
+                        fc = f"__dadd_rn({fc}, pgb_exp(invT * {_f(-r.troe[3])}))"
+                    e(f"const double lFc = __dmul_rn(pgb_log({fc}), {_f(1.0 / LN10)});")
+                    e("const double cc = fma(-0.67, lFc, -0.4), nn = fma(-1.27, lFc, 0.75);")
+                    e(f"const double lPr = fma(pgb_log(fmax(Pr, 1e-300)), {_f(1.0 / LN10)}, cc);")
+                    e("const double f1 = lPr / fma(-0.14, lPr, nn);")
+                    e(f"blend = __dmul_rn(blend, pgb_exp(__dmul_rn({_f(LN10)}, lFc) / fma(f1, f1, 1.0)));")
+                e("const double kf = __dmul_rn(pgb_exp(lnkf), blend);")
+            else:
+                e("const double kf = pgb_exp(lnkf);")
+            pf = product("", [f"C{idx[s]}" for s, nu in r.reactants.items() for _ in range(nu)])
+            if r.reversible:
+                dg = ""
+                for side, sign in ((r.products, 1), (r.reactants, -1)):
+                    for s, nu in side.items():
+                        g = f"g{idx[s]}"
+                        if not dg:
+                            dg = g if nu == 1 else f"__dmul_rn({nu}.0, {g})"
+                        elif nu == 1:
+                            dg = f"__d{'add' if sign > 0 else 'sub'}_rn({dg}, {g})"
+                        else:
+                            dg = f"fma({sign * nu}.0, {g}, {dg})"
+                dnu = sum(r.products.values()) - sum(r.reactants.values())
+                if dnu != 0:
+                    dg = f"fma({_f(-dnu)}, lnP0RT, {dg})"
+                # exponent capped at 700: exp stays finite, so an absent product (Pp = 0)
+                # gives a zero reverse term instead of inf * 0 = NaN
+                e(f"const double kr = -__dmul_rn(kf, pgb_exp(fmin({dg}, 700.0)));")
+                pr = product("kr", [f"C{idx[s]}" for s, nu in r.products.items() for _ in range(nu)])
+                e(f"q{j} = fma(kf, {pf}, {pr});")
+            else:
+                e(f"q{j} = __dmul_rn(kf, {pf});")
+            if j == fused_third_body(m):
+                e(f"qu{j} = q{j};")
+                e(f"M{j} = M;")
+            if r.kind == "three_body":
+                e(f"q{j} = __dmul_rn(q{j}, M);")
+            e.ind -= 1
+            e("}")
+        for k in range(ns):
+            expr = ""
+            for j, r in enumerate(m.reactions):
+                nu = r.products.get(m.species[k].name, 0) - r.reactants.get(m.species[k].name, 0)
+                if nu == 0:
+                    continue
+                if expr and abs(nu) == 1 and j == fused_third_body(m):
+                    expr = f"fma({'-' if nu < 0 else ''}qu{j}, M{j}, {expr})"
+                elif abs(nu) == 1:
+                    expr = f"__d{'add' if nu > 0 else 'sub'}_rn({expr}, q{j})" if expr else ("q" if nu > 0 else "-q") + str(j)
+                else:
+                    expr = f"fma({_f(nu)}, q{j}, {expr})" if expr else f"__dmul_rn({_f(nu)}, q{j})"
+            e(f"const double wd{k} = {expr or '0.0'};")
+
     def emit_gibbs():
         for t in sorted({s.Tmid for s in m.species}):
             e(f"const bool lo_{int(t)} = T < {_f(t)};")
@@ -266,32 +371,45 @@ def gen_header(m: Mechanism) -> str:
     e(f"const double T = y[{ns}];")
     e("const double invT = 1.0 / T;")
     e("const double lnT = pgb_log(T);")
+    exact = kernel_family(m) == "thread"  # another kernel repeats the bits of this function
     for k in range(ns):
-        e(f"const double C{k} = y[{k}] * {_f(1.0 / W[k])};")
+        c = _f(1.0 / W[k])
+        e(f"const double C{k} = " + (f"__dmul_rn(y[{k}], {c});" if exact else f"y[{k}] * {c};"))
     emit_gibbs()
-    emit_rates_fp64(True)
+    if exact:
+        emit_rates_exact()
+    else:
+        emit_rates_fp64(True)
     e("double hs = 0.0, rcp = 0.0;")
     for k, sp in enumerate(m.species):
         lf = f"lo_{int(sp.Tmid)}"
         e(f"{{ const double wm = fma(wd{k}, {_f(W[k])}, F[{k}]); ydot[{k}] = wm;")
         e(f"  hs = fma({_hW_expr(sp, lf, 1.0 / W[k])}, wm, hs);")
         e(f"  rcp = fma(y[{k}], {_cpW_expr(sp, lf, R_ERG / W[k])}, rcp); }}")
-    e(f"ydot[{ns}] = fma(-hs, {_f(R_ERG)} * T, Fh) / rcp;")
+    e(f"ydot[{ns}] = fma(-hs, __dmul_rn({_f(R_ERG)}, T), Fh) / rcp;")
     e.ind -= 1
     e("}")
     e()
     # ---------------------------------------------------------------- Jacobian template
-    e("// Analytic Jacobian d ydot / d y in arithmetic type R, written through J(i, k).")
-    e("// Falloff blending factors are held frozen in the [M] and T derivatives.")
-    e("template <class R, class Acc>")
-    e("__device__ __forceinline__ static void jac(const double* __restrict__ y, const double* __restrict__ Fd, const double Fhd, Acc J) {")
+    e("// Analytic Jacobian d ydot / d y in arithmetic type R: entry (i, k) to A[i rs + k cs].")
+    e("// Falloff blending factors are held frozen in the [M] and T derivatives. Every rounding is written")
+    e("// out (fma, pgb_mul, pgb_add), so the kernels that inline it get the same bits.")
+    e("template <class R>")
+    e("__device__ __forceinline__ static void jac(const double* __restrict__ y, const double* __restrict__ Fd, const double Fhd, R* A, const int rs, const int cs) {")
     e.ind += 1
+    mul = lambda *v: v[0] if len(v) == 1 else f"pgb_mul({mul(*v[:-1])}, {v[-1]})"
+    add = lambda x, y_: f"pgb_add({x}, {y_})"
+    neg = lambda x: x[1:] if x.startswith("-") else "-" + x
+    fma = lambda x, y_, z: f"fma({x}, {y_}, {z})"
+
+    def scaled(nu, x, acc):  # acc + nu x
+        return add(acc, x if nu > 0 else neg(x)) if abs(nu) == 1 else fma(f"R({_f(nu)})", x, acc)
+
     e(f"const R T = (R)y[{ns}];")
     e("const R invT = R(1) / T;")
     e("const R lnT = pgb_logT<R>(T);")
-    e("const R T2 = T * T, T3 = T2 * T;")
     for k in range(ns):
-        e(f"const R C{k} = (R)(y[{k}] * {_f(1.0 / W[k])});")
+        e(f"const R C{k} = (R)__dmul_rn(y[{k}], {_f(1.0 / W[k])});")
     # thermo in R
     tmids = sorted({s.Tmid for s in m.species})
     for t in tmids:
@@ -300,16 +418,33 @@ def gen_header(m: Mechanism) -> str:
         for i in range(7):
             e(f"const R a{k}_{i} = lo_{int(s.Tmid)} ? R({_f(s.low[i])}) : R({_f(s.high[i])});")
     e("const R lnT1 = R(1) - lnT;")
+    unused = {k for k in range(ns) if not any(m.species[k].name in r.reactants or m.species[k].name in r.products
+                                              for r in m.reactions)}
     for k in range(ns):
-        e(f"const R g{k} = a{k}_0 * lnT1 + T * (a{k}_1 * R(-0.5) + T * (a{k}_2 * R(-1.0 / 6.0) + T * (a{k}_3 * R(-1.0 / 12.0) + T * a{k}_4 * R(-0.05)))) + a{k}_5 * invT - a{k}_6;")
-        e(f"const R h{k} = a{k}_0 + T * (a{k}_1 * R(0.5) + T * (a{k}_2 * R(1.0 / 3.0) + T * (a{k}_3 * R(0.25) + T * a{k}_4 * R(0.2)))) + a{k}_5 * invT;")
-        e(f"const R cp{k} = a{k}_0 + T * (a{k}_1 + T * (a{k}_2 + T * (a{k}_3 + T * a{k}_4)));")
-        e(f"const R dcp{k} = a{k}_1 + T * (R(2) * a{k}_2 + T * (R(3) * a{k}_3 + T * R(4) * a{k}_4));")
+        c = [f"a{k}_{i}" for i in range(7)]
+        e(f"const R Ta{k} = {mul('T', c[4])};")
+        g = fma(c[3], "R(-1.0 / 12.0)", mul(f"Ta{k}", "R(-0.05)"))
+        g = fma("T", g, mul(c[2], "R(-1.0 / 6.0)"))
+        g = fma("T", g, mul(c[1], "R(-0.5)"))
+        g = fma(c[5], "invT", fma(c[0], "lnT1", mul("T", g)))
+        e(f"const R g{k} = {g} - {c[6]};")
+        h = fma(c[3], "R(0.25)", mul(f"Ta{k}", "R(0.2)"))
+        h = fma(c[2], "R(1.0 / 3.0)", mul("T", h))
+        h = fma(c[1], "R(0.5)", mul("T", h)) if k in unused else fma("T", h, mul(c[1], "R(0.5)"))
+        e(f"const R h{k} = {fma(c[5], 'invT', fma('T', h, c[0]))};")
+        e(f"const R cp{k} = {fma('T', fma('T', fma('T', add(c[3], f'Ta{k}'), c[2]), c[1]), c[0])};")
+        d = fma("R(3)", c[3], mul("T", "R(4)", c[4]))
+        e(f"const R dcp{k} = {fma('T', fma('R(2)', c[2], mul('T', d)), c[1])};")
+    e("R J[N][N];")
+    e("#pragma unroll")
     e("for (int i = 0; i < N; ++i)")
-    e("  for (int k = 0; k < N; ++k) J(i, k) = R(0);")
-    needM = any(r.kind != "elementary" for r in m.reactions)
-    if needM:
-        e("const R Ctot = " + " + ".join(f"C{k}" for k in range(ns)) + ";")
+    e("#pragma unroll")
+    e("  for (int k = 0; k < N; ++k) J[i][k] = R(0);")
+    if any(r.kind != "elementary" for r in m.reactions):
+        tot = "C0"
+        for k in range(1, ns):
+            tot = f"pgb_add_scaled<R>({tot}, y[{k}], {_f(1.0 / W[k])})" if k in total_only(m) else add(tot, f"C{k}")
+        e(f"const R Ctot = {tot};")
     e(f"const R lnP0RT = R({_f(lnP0_R)}) - lnT;")
     for k in range(ns):
         e(f"R wd{k} = R(0);")
@@ -321,124 +456,145 @@ def gen_header(m: Mechanism) -> str:
         e.ind += 1
         lnA = math.log(r.rate.A)
         ear = r.rate.Ea / R_CAL
-        e(f"const R lnkf_inf = R({_f(r.rate.beta)}) * lnT + R({_f(-ear)}) * invT + R({_f(lnA)});")
-        e(f"R dlnkf = (R({_f(r.rate.beta)}) + R({_f(ear)}) * invT) * invT;")
+        e(f"const R eT = {mul(f'R({_f(ear)})', 'invT')};")
+        e(f"const R lnkf_inf = {add(fma(f'R({_f(r.rate.beta)})', 'lnT', '-eT'), f'R({_f(lnA)})')};")
+        e(f"R dlnkf = {mul(add(f'R({_f(r.rate.beta)})', 'eT'), 'invT')};")
         if r.kind != "elementary":
             terms = "Ctot"
             for sname, eff in r.efficiencies.items():
                 if eff != 1.0:
-                    terms = f"{terms} + R({_f(eff - 1.0)}) * C{idx[sname]}"
+                    terms = fma(f"R({_f(eff - 1.0)})", f"C{idx[sname]}", terms)
             e(f"const R M = {terms};")
         if r.kind == "falloff":
             lnA0 = math.log(r.low.A)
             ear0 = r.low.Ea / R_CAL
-            e(f"const R lnk0 = R({_f(r.low.beta)}) * lnT + R({_f(-ear0)}) * invT + R({_f(lnA0)});")
-            e(f"const R dlnk0 = (R({_f(r.low.beta)}) + R({_f(ear0)}) * invT) * invT;")
+            e(f"const R eT0 = {mul(f'R({_f(ear0)})', 'invT')};")
+            e(f"const R lnk0 = {add(fma(f'R({_f(r.low.beta)})', 'lnT', '-eT0'), f'R({_f(lnA0)})')};")
+            e(f"const R dlnk0 = {mul(add(f'R({_f(r.low.beta)})', 'eT0'), 'invT')};")
             e("const R k0 = pgb_expT<R>(lnk0);")
             e("const R kinf = pgb_expT<R>(lnkf_inf);")
-            e("const R Pr = M * pgb_expT<R>(lnk0 - lnkf_inf);")
+            e("const R Pr = pgb_mul(M, pgb_expT<R>(lnk0 - lnkf_inf));")
             if r.troe:
                 a, T3, T1 = r.troe[:3]
-                fc = f"R({_f(1.0 - a)}) * pgb_expT<R>(T * R({_f(-1.0 / T3)})) + R({_f(a)}) * pgb_expT<R>(T * R({_f(-1.0 / T1)}))"
+                fc = fma(f"R({_f(1.0 - a)})", f"pgb_expT<R>(T * R({_f(-1.0 / T3)}))",
+                         mul(f"R({_f(a)})", f"pgb_expT<R>(T * R({_f(-1.0 / T1)}))"))
                 if len(r.troe) > 3:
-                    fc += f" + pgb_expT<R>(invT * R({_f(-r.troe[3])}))"
-                e(f"const R Fcent = {fc};")
-                e(f"const R lFc = pgb_logT<R>(Fcent) * R({_f(1.0 / LN10)});")
-                e("const R cc = R(-0.4) - R(0.67) * lFc, nn = R(0.75) - R(1.27) * lFc;")
-                e(f"const R lPr = pgb_logT<R>(Pr > R(1e-30) ? Pr : R(1e-30)) * R({_f(1.0 / LN10)}) + cc;")
-                e("const R f1 = lPr / (nn - R(0.14) * lPr);")
-                e(f"const R Fb = pgb_expT<R>(R({_f(LN10)}) * lFc / (R(1) + f1 * f1));")
+                    fc = add(fc, f"pgb_expT<R>(invT * R({_f(-r.troe[3])}))")
+                e(f"const R lFc = {mul(f'pgb_logT<R>({fc})', f'R({_f(1.0 / LN10)})')};")
+                e("const R cc = fma(R(-0.67), lFc, R(-0.4)), nn = fma(R(-1.27), lFc, R(0.75));")
+                e(f"const R lPr = fma(pgb_logT<R>(Pr > R(1e-30) ? Pr : R(1e-30)), R({_f(1.0 / LN10)}), cc);")
+                e("const R f1 = lPr / fma(R(-0.14), lPr, nn);")
+                e(f"const R Fb = pgb_expT<R>({mul(f'R({_f(LN10)})', 'lFc')} / fma(f1, f1, R(1)));")
             else:
                 e("const R Fb = R(1);")
-            e("const R onePr = R(1) + Pr;")
-            e("const R kf = kinf * Pr / onePr * Fb;")
-            e("const R dkeff_dM = Fb * k0 / (onePr * onePr);")
-            e("dlnkf = dlnkf + (dlnk0 - dlnkf) / onePr;")
+            e("const R onePr = pgb_add(R(1), Pr);")
+            e("const R kf = pgb_mul(pgb_mul(kinf, Pr) / onePr, Fb);")
+            e("const R dkeff_dM = pgb_mul(Fb, k0) / pgb_mul(onePr, onePr);")
+            e("dlnkf = pgb_add(dlnkf, (dlnk0 - dlnkf) / onePr);")
         else:
             e("const R kf = pgb_expT<R>(lnkf_inf);")
         pf_f = [idx[s] for s, nu in r.reactants.items() for _ in range(nu)]
         pr_f = [idx[s] for s, nu in r.products.items() for _ in range(nu)]
-        e("const R Pf = " + " * ".join(f"C{k}" for k in pf_f) + ";")
-        e("const R Pp = " + " * ".join(f"C{k}" for k in pr_f) + ";")
+        e("const R Pf = " + mul(*[f"C{k}" for k in pf_f]) + ";")
         dnu = sum(r.products.values()) - sum(r.reactants.values())
+        third = r.kind == "three_body"
         if r.reversible:
-            dg, dh = [], []
-            for s, nu in r.products.items():
-                dg.append(f"+ R({nu}) * g{idx[s]}")
-                dh.append(f"+ R({nu}) * h{idx[s]}")
-            for s, nu in r.reactants.items():
-                dg.append(f"- R({nu}) * g{idx[s]}")
-                dh.append(f"- R({nu}) * h{idx[s]}")
-            dgs = " ".join(dg)
+            e("const R Pp = " + mul(*[f"C{k}" for k in pr_f]) + ";")
+            dg = dh = "R(0)"
+            for side, sign in ((r.products, 1), (r.reactants, -1)):
+                for s, nu in side.items():
+                    dg = scaled(sign * nu, f"g{idx[s]}", dg)
+                    dh = scaled(sign * nu, f"h{idx[s]}", dh)
             if dnu != 0:
-                dgs += f" - R({dnu}) * lnP0RT"
-            e(f"const R kr = kf * pgb_expT<R>(fmin(R(0) {dgs}, R(700)));")
-            e(f"const R dlnkr = dlnkf - (R(0) {' '.join(dh)} - R({dnu})) * invT;")
+                dg = scaled(-dnu, "lnP0RT", dg)
+            e(f"const R kr = pgb_mul(kf, pgb_expT<R>(fmin({dg}, R(700))));")
+            e(f"const R dlnkr = fma(-({dh} - R({dnu})), invT, dlnkf);")
+            e("const R net = fma(kf, Pf, -pgb_mul(kr, Pp));")
+            e(f"const R net_T = {fma(mul('kf', 'dlnkf'), 'Pf', neg(mul('kr', 'dlnkr', 'Pp')))};")
         else:
-            e("const R kr = R(0);")
-            e("const R dlnkr = R(0);")
-        alpha = "M" if r.kind == "three_body" else "R(1)"
-        e(f"const R alpha = {alpha};")
-        e("const R q = alpha * (kf * Pf - kr * Pp);")
-        e("const R dqdT = alpha * (kf * dlnkf * Pf - kr * dlnkr * Pp);")
-        # partials dq/dC_k
-        dq: Dict[int, List[str]] = {}
+            e("const R net = pgb_mul(kf, Pf);")
+            e(f"const R net_T = {mul('kf', 'dlnkf', 'Pf')};")
+        # partials dq/dC_k, each a list of products
+        dq: Dict[int, List[List[str]]] = {}
 
         def partials(side_list, coef):
-            uniq = sorted(set(side_list))
-            for k in uniq:
+            for k in sorted(set(side_list)):
                 nu = side_list.count(k)
                 others = list(side_list)
                 others.remove(k)
-                term = f"{coef}" + (f" * R({nu})" if nu > 1 else "") + "".join(f" * C{o}" for o in others)
-                dq.setdefault(k, []).append(term)
+                dq.setdefault(k, []).append(coef + ([f"R({nu})"] if nu > 1 else []) + [f"C{o}" for o in others])
 
-        partials(pf_f, "alpha * kf")
+        partials(pf_f, ["M", "kf"] if third else ["kf"])
         if r.reversible:
-            partials(pr_f, "-alpha * kr")
-        if r.kind == "three_body":
-            e("const R base = kf * Pf - kr * Pp;")
-        elif r.kind == "falloff":
-            e("const R base = dkeff_dM * (Pf - (kf > R(0) ? kr / kf : R(0)) * Pp);")
-        for k, terms in dq.items():
-            e(f"const R dq{k} = " + " + ".join(terms) + ";")
+            partials(pr_f, ["-M", "kr"] if third else ["-kr"])
+        if r.kind == "falloff":
+            rev = "fma(-(kf > R(0) ? kr / kf : R(0)), Pp, Pf)" if r.reversible else "Pf"
+            e(f"const R base = pgb_mul(dkeff_dM, {rev});")
         nus = {}
         for s, nu in r.reactants.items():
             nus[idx[s]] = nus.get(idx[s], 0) - nu
         for s, nu in r.products.items():
             nus[idx[s]] = nus.get(idx[s], 0) + nu
-        for i, nu in nus.items():
-            if nu == 0:
+        nus = {i: nu for i, nu in nus.items() if nu != 0}
+        # a product that is only ever added (coefficients 1 and -1) goes into the sums' multiply-adds
+        whole = {k for k in dq if len(dq[k]) == 1 and len(dq[k][0]) > 1 and all(abs(nu * W[i] / W[k]) == 1.0
+                                                                              for i, nu in nus.items())}
+        for k, terms in dq.items():
+            if k in whole:
                 continue
-            e(f"wd{i} += R({nu}) * q;")
-            e(f"dT{i} += R({nu}) * dqdT;")
+            v = mul(*terms[0])
+            for t in terms[1:]:
+                v = fma(mul(*t[:-1]), t[-1], v) if len(t) > 1 else add(v, t[0])
+            e(f"const R dq{k} = {v};")
+        split = third and all(abs(nu) == 1 for nu in nus.values())
+        if third and not split:
+            e("const R q = pgb_mul(M, net), q_T = pgb_mul(M, net_T);")
+        for i, nu in nus.items():
+            for acc, v in ((f"wd{i}", "net"), (f"dT{i}", "net_T")):
+                if split:
+                    e(f"{acc} = {fma('M' if nu > 0 else '-M', v, acc)};")
+                else:
+                    e(f"{acc} = {scaled(nu, v.replace('net', 'q') if third else v, acc)};")
             for k in dq:
-                e(f"J({i}, {k}) += R({_f(nu * W[i] / W[k])}) * dq{k};")
+                co, at = nu * W[i] / W[k], f"J[{i}][{k}]"
+                if k in whole:
+                    t = dq[k][0]
+                    e(f"{at} = {fma(mul(*t[:-1]) if co > 0 else neg(mul(*t[:-1])), t[-1], at)};")
+                else:
+                    e(f"{at} = {scaled(co, f'dq{k}', at)};")
             if r.kind != "elementary":
                 effs = {idx[s]: eff for s, eff in r.efficiencies.items()}
                 for k in range(ns):
                     eff = effs.get(k, 1.0)
                     if eff != 0.0:
-                        e(f"J({i}, {k}) += R({_f(nu * W[i] / W[k] * eff)}) * base;")
+                        e(f"J[{i}][{k}] = {scaled(nu * W[i] / W[k] * eff, 'net' if third else 'base', f'J[{i}][{k}]')};")
         e.ind -= 1
         e("}")
     # temperature column and energy row
     e("R Dm = R(0), dDm = R(0), Q = (R)Fhd;")
     for k in range(ns):
-        e(f"const R wm{k} = wd{k} * R({_f(W[k])}) + (R)Fd[{k}];")
-        e(f"const R hm{k} = h{k} * R({_f(R_ERG / W[k])}) * T;")
-        e(f"const R cpm{k} = cp{k} * R({_f(R_ERG / W[k])});")
-        e(f"Dm += (R)y[{k}] * cpm{k};")
-        e(f"dDm += (R)y[{k}] * dcp{k} * R({_f(R_ERG / W[k])});")
-        e(f"Q -= hm{k} * wm{k};")
-        e(f"J({k}, {ns}) = R({_f(W[k])}) * dT{k};")
+        e(f"const R wm{k} = fma(wd{k}, R({_f(W[k])}), (R)Fd[{k}]);")
+        e(f"const R hm{k} = {mul(f'h{k}', f'R({_f(R_ERG / W[k])})', 'T')};")
+        e(f"const R cpm{k} = {mul(f'cp{k}', f'R({_f(R_ERG / W[k])})')};")
+        e(f"Dm = fma((R)y[{k}], cpm{k}, Dm);")
+        e(f"dDm = fma({mul(f'(R)y[{k}]', f'dcp{k}')}, R({_f(R_ERG / W[k])}), dDm);")
+        e(f"Q = fma(-hm{k}, wm{k}, Q);")
+        e(f"J[{k}][{ns}] = {mul(f'R({_f(W[k])})', f'dT{k}')};")
     e("const R invD = R(1) / Dm;")
-    e("const R QD2 = Q * invD * invD;")
+    e(f"const R QD2 = {mul('Q', 'invD', 'invD')};")
     for k in range(ns):
-        terms = " + ".join(f"hm{i} * J({i}, {k})" for i in range(ns))
-        e(f"J({ns}, {k}) = -({terms}) * invD - QD2 * cpm{k};")
-    terms = " + ".join(f"cpm{i} * wm{i} + hm{i} * J({i}, {ns})" for i in range(ns))
-    e(f"J({ns}, {ns}) = -({terms}) * invD - QD2 * dDm;")
+        sum_ = mul("hm0", f"J[0][{k}]") if ns == 1 else fma("hm0", f"J[0][{k}]", mul("hm1", f"J[1][{k}]"))
+        for i in range(2, ns):
+            sum_ = fma(f"hm{i}", f"J[{i}][{k}]", sum_)
+        e(f"J[{ns}][{k}] = fma(-({sum_}), invD, -pgb_mul(QD2, cpm{k}));")
+    sum_ = fma("cpm0", "wm0", mul("hm0", f"J[0][{ns}]"))
+    for i in range(1, ns):
+        sum_ = fma(f"hm{i}", f"J[{i}][{ns}]", fma(f"cpm{i}", f"wm{i}", sum_))
+    e(f"J[{ns}][{ns}] = fma(-({sum_}), invD, -pgb_mul(QD2, dDm));")
+    e("#pragma unroll")
+    e("for (int i = 0; i < N; ++i)")
+    e("#pragma unroll")
+    e("  for (int k = 0; k < N; ++k) A[i * rs + k * cs] = J[i][k];")
     e.ind -= 1
     e("}")
     e.ind -= 1
@@ -599,9 +755,9 @@ def emit_jac_stream(e: _Emitter, qual: str, m: Mechanism, rx, tb_rows, codes, ne
 
 
 def emit_unrolled_order(e: _Emitter, qual: str, m: Mechanism, order):
-    """What a lane-parallel evaluation needs to give the bits of the unrolled right-hand side
-    (gen_header): the constants as that code folds them, and each species' reactions in the order in
-    which it adds them (input order; values are positions in `order`)."""
+    """What a lane-parallel evaluation needs to repeat the unrolled right-hand side (gen_header,
+    emit_rates_exact): the constants as that code folds them, and each species' reactions in the order
+    in which it adds them (input order; values are positions in `order`)."""
     e(f"{qual} TabUnrolled kUnrolled[NS] = {{")
     for s in m.species:
         rows = []
@@ -615,9 +771,7 @@ def emit_unrolled_order(e: _Emitter, qual: str, m: Mechanism, order):
         for a in (s.low, s.high):
             w = R_ERG / s.W
             rows.append([a[i] * w for i in range(5)])
-        used = any(s.name in r.reactants or s.name in r.products or r.efficiencies.get(s.name, 1.0) != 1.0
-                   for r in m.reactions)
-        e(f"  {{{_f(1.0 / s.W)}, {_f(s.W)}, {_f(s.Tmid)}, {0 if used else 1}, "
+        e(f"  {{{_f(1.0 / s.W)}, {_f(s.W)}, {_f(s.Tmid)}, {int(m.index(s.name) in total_only(m))}, "
           + ", ".join("{" + ", ".join(_f(v) for v in r) + "}" for r in rows) + "},")
     e("};")
     pos = {j: i for i, j in enumerate(order)}
@@ -628,7 +782,7 @@ def emit_unrolled_order(e: _Emitter, qual: str, m: Mechanism, order):
             if net != 0:
                 jj.append(pos[j])
                 nu.append(float(net))
-                tb.append(int(r.kind == "three_body" and abs(net) == 1 and j == m.nr - 1))
+                tb.append(int(abs(net) == 1 and j == fused_third_body(m)))
         off.append(len(jj))
     e(f"{qual} int kUnM[{len(jj)}] = {{{', '.join(str(v) for v in tb)}}};")
     e(f"{qual} int kUnOff[NS + 1] = {{{', '.join(str(v) for v in off)}}};")
@@ -846,7 +1000,7 @@ def gen_tables(m: Mechanism, space: str = "constant") -> str:
             e("  __device__ static const TabUnrolled& un(int k) { return kUnrolled[k]; }")
             e("  __device__ static int un_begin(int k) { return kUnOff[k]; }")
             e("  __device__ static int un_j(int e) { return kUnJ[e]; }")
-            e("  __device__ static bool un_m(int e) { return kUnM[e] != 0; }  // the compiler fuses q [M] here")
+            e("  __device__ static bool un_m(int e) { return kUnM[e] != 0; }  // q [M] is fused here")
             e("  __device__ static double un_nu(int e) { return kUnNu[e]; }")
         e("  __device__ static int sprx_begin(int k) { return kSpRxOff[k]; }")
         e(f"  static constexpr int MAXR = {max(len(r[5]) for r in rx)}, MAXP = {max(len(r[6]) for r in rx)};  // slots a side")

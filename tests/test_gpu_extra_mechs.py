@@ -45,3 +45,19 @@ def test_coefficients_of_three_match_the_oracle(extra, oracle_mod, cuda, shape, 
     assert within.mean() >= 0.999
     out = np.nonzero(~within)[0]
     outliers_within_global_error(om, cs, out, (rYg[out], Tg[out]), (rYo[out], To[out]), cfg.dt, cfg.rtol)
+
+
+# one warp; two cells a warp; just above the small-launch limit, where the last cells of each warp change
+# kernels; the roundings of both kernels are written out, so no compiler choice can tell them apart
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(5, 1, 1), (13, 9, 7), (17, 13, 11), (23, 21, 19)])
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_kernels_agree_bit_for_bit(extra, cuda, shape, precision):
+    cfg = CONFIGS["lidryer_amr120"]
+    cs = make_cells(cfg, int(np.prod(shape)), seed=8)
+    with extra_mechs.library(extra[0]):
+        a, fa = _advance(cuda, cfg, cs, shape, "trio_syn", f"gb.precision={precision}")
+        b, fb = _advance(cuda, cfg, cs, shape, "trio_syn", f"gb.precision={precision} gb.mapping=thread")
+    assert fa == fb == 0
+    for x, y in zip(a, b):
+        np.testing.assert_array_equal(x, y)
