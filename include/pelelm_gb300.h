@@ -121,6 +121,11 @@ int pgb_reactor_tuning(pgb_reactor* r, char* buf, size_t n);
 /* Waits for the last advance on its stream and returns its counters. */
 int pgb_reactor_get_stats(pgb_reactor* r, pgb_stats* out);
 
+/* How the last advance ran (waits for it): *small_launch 1 if all cells went to the kernel with more
+ * lanes per cell, else 0; *handed_over the cells that changed to that kernel at one of their steps. No
+ * counterpart in the reference. */
+int pgb_reactor_last_route(pgb_reactor* r, int* small_launch, unsigned long long* handed_over);
+
 /* Counters of the learned surrogate in the last advance (reactor created with gb.surrogate).
  * No counterpart in the reference. ncell: unmasked cells; accept: cells written by the
  * surrogate; fallback: cells advanced by the BDF (rejected + audited); ood/mis/cons/ens/neg:

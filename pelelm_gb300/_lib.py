@@ -84,6 +84,7 @@ EXPORTS = {
     "pgb_mlp_bias_grad": (C.c_int, [_vp, C.c_int, C.c_int, C.c_int, _vp, _vp]),
     "pgb_mlp_adam": (C.c_int, [_vp, _vp, _vp, _vp, _vp, C.c_longlong, C.c_float, C.c_float, C.c_float,
                                C.c_float, C.c_int, _vp]),
+    "pgb_reactor_last_route": (C.c_int, [_vp, C.POINTER(C.c_int), C.POINTER(C.c_ulonglong)]),
     "pgb_mlp_train_workspace": (C.c_longlong, [C.POINTER(MlpStep)]),
     "pgb_mlp_train_step": (C.c_int, [C.POINTER(MlpStep), _vp, _vp]),
     "pgb_mlp_f32_to_bf16": (C.c_int, [_vp, _vp, C.c_longlong, _vp]),

@@ -214,6 +214,7 @@ struct Scratch {
   unsigned long long* d_retry_count = nullptr;
   cudaEvent_t done = nullptr;
   long long last_ncell = 0;
+  int last_small = 0;              // the last advance was a small launch
   // graph cache
   cudaGraphExec_t gexec = nullptr;
   std::vector<pgb::BoxDev> gkey;
@@ -821,6 +822,7 @@ int advance_box_table(pgb_reactor* r, const std::vector<pgb::BoxDev>& boxes, lon
   if (ensure_scratch(r, st, std::max(nbox, 1), &s)) return -1;
   if (!r->null_reactor) {
     LaunchPlan pl = plan_launch(r, ncell, r->opt.mixed);
+    s->last_small = pl.small;
     if (r->opt.mixed && r->opt.retry) {  // the FP64 retry pass shares the global scratch
       const LaunchPlan p64 = plan_launch(r, ncell, false);
       pl.z_bytes = std::max(pl.z_bytes, p64.z_bytes);
@@ -941,6 +943,18 @@ int pgb_reactor_get_stats(pgb_reactor* r, pgb_stats* out) {
   out->nfail = h.nfail; out->max_nst = h.max_nst;
   for (int i = 0; i < 16; ++i) out->hist[i] = h.hist[i];
   out->nretry = h.nretry;
+  return 0;
+}
+
+int pgb_reactor_last_route(pgb_reactor* r, int* small_launch, unsigned long long* handed_over) {
+  if (!r || !small_launch || !handed_over) return set_err("null argument");
+  std::lock_guard<std::mutex> g(r->mu);
+  auto it = r->scratch.find(r->last_stream);
+  if (it == r->scratch.end()) return set_err("no advance has run yet");
+  Scratch& s = it->second;
+  PGB_CUDA(cudaEventSynchronize(s.done));
+  PGB_CUDA(cudaMemcpy(handed_over, s.d_counter + 2, sizeof(*handed_over), cudaMemcpyDeviceToHost));
+  *small_launch = s.last_small;
   return 0;
 }
 

@@ -109,6 +109,13 @@ class ReactorGB:
                 "ncfn": s.ncfn, "nfail": s.nfail, "max_nst": s.max_nst, "hist": list(s.hist),
                 "nretry": s.nretry}
 
+    def last_route(self):
+        """(small launch, cells handed over) of the last advance: whether all cells went to the kernel
+        with more lanes per cell, and how many changed to it at one of their steps."""
+        small, n = C.c_int(), C.c_ulonglong()
+        check(lib().pgb_reactor_last_route(self._h, C.byref(small), C.byref(n)), "last_route")
+        return bool(small.value), n.value
+
     def tuning(self) -> str:
         """The autotuner's report (gb.autotune=1), empty before the first advance."""
         buf = C.create_string_buffer(4096)
