@@ -58,6 +58,7 @@ struct Options {
   int lu_global = -1;      // gb.lu = shared | global (L2-resident Jacobian/LU); -1 = auto
   int mapping = -1;        // gb.mapping = thread | warp | group (cell per thread / warp / lane group); -1 = auto
   int group = 8;           // gb.group: lanes per cell of the group mapping (4 or 8)
+  bool group_given = false;
   int wpb = 0;             // gb.wpb: warps per block of the warp mapping (0 = most that fit)
   bool autotune = false;   // gb.autotune: time the compiled mappings on the first advance's cells
   bool retry = true;       // gb.retry: cells the mixed-precision pass fails are integrated again in FP64
@@ -100,6 +101,7 @@ int parse_options(const char* s, Options& o) {
         else return set_err("gb.mapping must be thread, warp or group, got '%s'", v.c_str());
       } else if (k == "gb.group") {
         o.group = std::stoi(v);
+        o.group_given = true;
         if (o.group != 4 && o.group != 8) return set_err("gb.group must be 4 or 8, got '%s'", v.c_str());
       } else if (k == "gb.wpb") o.wpb = std::stoi(v);
       else if (k == "gb.autotune") o.autotune = std::stoi(v) != 0;
@@ -234,7 +236,7 @@ struct pgb_reactor {
   cudaStream_t last_stream = nullptr;
   int device = 0, nsm = 0;
   SgModel sg;  // loaded when options name a surrogate file
-  bool small_ok = false;  // no option fixes the mapping or its layout: small launches choose theirs
+  bool small_ok = false;  // no option or tuning fixes the mapping or its layout: small launches choose theirs
   bool tuned = false;
   std::string tuning;  // autotuner report
 };
@@ -634,7 +636,7 @@ pgb_reactor* pgb_reactor_create(const char* name, const char* mechanism, int rea
   r->mech = m;
   r->opt = o;
   r->null_reactor = (n == "ReactorNull");
-  r->small_ok = o.mapping < 0 && o.tpb == 0 && o.wpb == 0 && o.group == 8 && o.z_global < 0 && o.lu_global < 0;
+  r->small_ok = o.mapping < 0 && o.tpb == 0 && o.wpb == 0 && !o.group_given && o.z_global < 0 && o.lu_global < 0;
   r->device = dev;
   r->nsm = nsm;
   if (!o.surrogate.empty()) {
@@ -738,6 +740,7 @@ int run_autotune(pgb_reactor* r, const std::vector<pgb::BoxDev>& boxes, long lon
   r->sg.d_net = nullptr;  // time the BDF alone
   const bool small_saved = r->small_ok;
   r->small_ok = false;  // and the mappings of large launches
+  bool keep_small = true;
   auto fail = [&](const char* what) { rc = set_err("autotune: %s", what); };
   do {
     if (cudaMalloc(&pristine, arena_bytes) != cudaSuccess || cudaMalloc(&work, arena_bytes) != cudaSuccess ||
@@ -801,10 +804,16 @@ int run_autotune(pgb_reactor* r, const std::vector<pgb::BoxDev>& boxes, long lon
     if (pick.mapping == 2) r->opt.group = pick.wpb; else r->opt.wpb = pick.wpb;
     rep << "on " << nsample << " sample cells -> " << name(pick);
     r->tuning = rep.str();
+    // the pick stays in force for every call: another mapping than the default sums in another order
+    // than the kernel of small launches and last cells
+    const int chosen = r->opt.mapping;
+    r->opt.mapping = -1;
+    keep_small = chosen == mapping_of(r) && (chosen != 2 || pick.wpb == 8);
+    r->opt.mapping = chosen;
   } while (false);
   if (rc) r->opt = saved;
   r->sg = sg_saved;
-  r->small_ok = small_saved;
+  r->small_ok = small_saved && keep_small;
   cudaStreamSynchronize(st);
   if (pristine) cudaFree(pristine);
   if (work) cudaFree(work);
