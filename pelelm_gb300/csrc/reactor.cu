@@ -17,6 +17,7 @@
 #include <string>
 #include <vector>
 
+#include "optional_buffer.h"
 #include "reactor_registry.cuh"
 #include "surrogate_host.h"
 
@@ -196,8 +197,7 @@ struct Scratch {
   size_t box_cap = 0;
   pgb::BoxDev* h_boxes = nullptr;  // pinned staging
   unsigned long long* d_counter = nullptr;  // queue head; queue head and count of handed-over cells; cells done
-  void* d_resume = nullptr;        // handed-over cells
-  size_t resume_cap = 0;
+  OptionalBuffer resume;           // handed-over cells
   void* d_z = nullptr;             // Nordsieck histories of the resident threads
   size_t z_cap = 0;
   void* d_lu = nullptr;            // Jacobian/LU slices of the resident threads
@@ -248,7 +248,7 @@ void free_scratch(Scratch& s) {
   if (s.d_boxes) cudaFree(s.d_boxes);
   if (s.h_boxes) cudaFreeHost(s.h_boxes);
   if (s.d_counter) cudaFree(s.d_counter);
-  if (s.d_resume) cudaFree(s.d_resume);
+  if (s.resume.p) cudaFree(s.resume.p);
   if (s.d_stats) cudaFree(s.d_stats);
   if (s.d_z) cudaFree(s.d_z);
   if (s.d_lu) cudaFree(s.d_lu);
@@ -433,6 +433,25 @@ int ensure_buf(Scratch& s, void*& buf, size_t& cap, size_t bytes) {
   return 0;
 }
 
+// Room for handed-over cells. Without it the launch keeps its last cells, so a failed allocation is no
+// reason to refuse the call, and leaves no error behind.
+void ensure_resume(Scratch& s, size_t bytes) {
+  s.resume.ensure(
+      bytes,
+      [](size_t n) -> void* {
+        void* q = nullptr;
+        if (cudaMalloc(&q, n) == cudaSuccess) return q;
+        (void)cudaGetLastError();
+        return nullptr;
+      },
+      [&](void* old) {
+        if (s.gexec) { cudaGraphExecDestroy(s.gexec); s.gexec = nullptr; s.gkey.clear(); }
+        if (!old) return;
+        cudaEventSynchronize(s.done);  // an advance in flight may use it
+        cudaFree(old);
+      });
+}
+
 // Kernel mapping: 0 cell per thread, 1 cell per warp, 2 cell per lane group. Cell-per-thread
 // kernels exist for mechanisms whose per-cell state fits a thread, group kernels for the
 // 21-species size; gb.mapping overrides the default below.
@@ -495,8 +514,8 @@ int enqueue_advance(pgb_reactor* r, Scratch& s, int nbox, long long ncell, doubl
     p.retry_count = s.d_retry_count;
     PGB_CUDA(cudaMemsetAsync(s.d_retry_count, 0, sizeof(unsigned long long), st));
   }
-  if (pl.drain > 0 && s.d_resume && s.resume_cap >= pl.resume_bytes) {
-    p.resume = static_cast<unsigned char*>(s.d_resume);
+  if (pl.drain > 0 && s.resume.p && s.resume.cap >= pl.resume_bytes) {
+    p.resume = static_cast<unsigned char*>(s.resume.p);
     p.resume_count = s.d_counter + 2;
     p.drain = pl.drain;
     if (pl.warp) p.done = s.d_counter + 3;
@@ -846,8 +865,7 @@ int advance_box_table(pgb_reactor* r, const std::vector<pgb::BoxDev>& boxes, lon
                      std::max<long long>(acap, 1) * (sizeof(long long) + pgb::MAXN * sizeof(double))))
         return -1;
     }
-    // without this buffer the launch keeps its last cells: no reason to refuse the call
-    if (ensure_buf(*s, s->d_resume, s->resume_cap, pl.resume_bytes)) (void)cudaGetLastError();
+    ensure_resume(*s, pl.resume_bytes);
   }
   PGB_CUDA(cudaEventSynchronize(s->done));  // staging buffer may still feed a previous copy
   if (nbox) std::memcpy(s->h_boxes, boxes.data(), nbox * sizeof(pgb::BoxDev));
