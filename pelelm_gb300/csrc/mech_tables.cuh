@@ -87,8 +87,10 @@ constexpr double kRerg = 8.31446261815324e7;        // erg/mol/K
 // h(T) of a mixture is one NASA-7 polynomial whose coefficients are the species' sums, so they are
 // formed once (six multiply-adds a species) and an iteration costs a dozen FP64 operations instead
 // of eleven a species; they are formed again only when T crosses a species' Tmid. Where all species
-// share one Tmid, hmid_sum, the sum of rY(k) h_mid(k), tells on which side the solution lies, and the
-// iteration starts there: of 32 cells one or two cross, and a warp pays for its slowest. The sums
+// share one Tmid and no h jumps there, hmid_sum, the sum of rY(k) h_mid(k), tells on which side the
+// solution lies, and the iteration starts there: of 32 cells one or two cross, and a warp pays for its
+// slowest. (Where an h jumps, as fitted polynomials do, a target may have a root on either side or none,
+// and the guess decides: the iteration then starts at it.) The sums
 // carry the rounding of the per-species form (1e-16 of the largest term).
 // Measured (53 species, 202,752 cells): T from rho h 685 -> 273 us, with hmid_sum and the range of T
 // compared as integers 226 us.
@@ -96,7 +98,7 @@ template <class Tab, class GetY>
 __device__ __forceinline__ double hy2t_mixture(double htarget, GetY rY, double inv_rho, double hmid_sum, double T,
                                                double tmin, double tmax) {
   if (!(T > tmin && T < tmax)) T = 1000.0;
-  if constexpr (Tab::TMID > 0.0) {
+  if constexpr (Tab::TMID > 0.0 && Tab::JOINED) {
     const double hm = hmid_sum * inv_rho * kRerg;
     if (Tab::TMID > tmin && Tab::TMID < tmax) {
       if (htarget > hm && T < Tab::TMID) T = Tab::TMID;

@@ -987,12 +987,16 @@ def gen_tables(m: Mechanism, space: str = "constant") -> str:
         e(f"{qual} double kSpRxNu[NSPRX] = {{{', '.join(_f(x) for x in nu)}}};")
     tmids = sorted({s.Tmid for s in m.species})
     hmid = []  # h/R per gram of every species at the common Tmid (low-range polynomial)
+    joined = len(tmids) == 1  # every h continuous there, but for rounding
     for s in m.species:
-        a, t = s.low, tmids[0]
-        hmid.append((a[5] + t * (a[0] + t * (a[1] / 2 + t * (a[2] / 3 + t * (a[3] / 4 + t * a[4] / 5))))) / s.W)
+        t = tmids[0]
+        lo, hi = (a[5] + t * (a[0] + t * (a[1] / 2 + t * (a[2] / 3 + t * (a[3] / 4 + t * a[4] / 5)))) for a in (s.low, s.high))
+        joined = joined and abs(lo - hi) <= 1e-12 * (abs(lo) + t)
+        hmid.append(lo / s.W)
     e(f"{qual} double kHMid[NS] = {{{', '.join(_f(v) for v in hmid)}}};")
     e("struct Tables {")
     e(f"  static constexpr double TMID = {_f(tmids[0]) if len(tmids) == 1 else '-1.0'};  // common Tmid, or -1")
+    e(f"  static constexpr bool JOINED = {'true' if joined else 'false'};  // no jump of any h at that Tmid")
     e("  __device__ static double h_mid(int k) { return kHMid[k]; }")
     e(f"  static constexpr int NS = {ns}, NR = {m.nr};")
     if glob:

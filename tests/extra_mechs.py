@@ -29,6 +29,17 @@ def trio():
     return m
 
 
+def jump():
+    """H2, H and N2, whose enthalpies fall by 20 K R at the common Tmid."""
+    m = workloads.load_mechanism("lidryer_syn")
+    m.name = "jump_syn"
+    m.species = [s for s in m.species if s.name in ("H2", "H", "N2")]
+    for s in m.species:
+        s.high[5] -= 20.0
+    m.reactions = [Reaction("three_body", {"H": 2}, {"H2": 1}, True, Arrhenius(1e18, -1.0, 0.0))]
+    return m
+
+
 def build(outdir, mechs):
     """Library of `mechs` alone in outdir; returns its path. Units that hold no mechanism are the
     product's objects."""

@@ -4,7 +4,7 @@ import pytest
 
 import extra_mechs
 from helpers import boxes_from_cells, gather, outliers_within_global_error, tol_ratio
-from pelelm_gb300.reactor import ReactorBase
+from pelelm_gb300.reactor import ReactorBase, rhoh_to_temp
 from pelelm_gb300.workloads import CONFIGS, make_cells
 
 
@@ -12,7 +12,7 @@ from pelelm_gb300.workloads import CONFIGS, make_cells
 def extra(native_lib, tmp_path_factory):
     """(library, folder) of the extra mechanisms."""
     d = str(tmp_path_factory.mktemp("extra"))
-    return extra_mechs.build(d, [extra_mechs.trio()]), d
+    return extra_mechs.build(d, [extra_mechs.trio(), extra_mechs.jump()]), d
 
 
 def _advance(torch, cfg, cs, shape, mech, options):
@@ -61,3 +61,31 @@ def test_kernels_agree_bit_for_bit(extra, cuda, shape, precision):
     assert fa == fb == 0
     for x, y in zip(a, b):
         np.testing.assert_array_equal(x, y)
+
+
+# enthalpies that jump at Tmid: targets between the two branches have a root on either side (a 5 K overlap),
+# and the guess decides, as in the oracle's iteration from that guess
+@pytest.mark.gpu
+def test_the_guess_decides_where_enthalpy_jumps(extra, oracle_mod, cuda):
+    torch = cuda
+    so, d = extra
+    om = oracle_mod.OracleMech(f"{d}/jump_syn.mech")
+    rng = np.random.default_rng(2)
+    n, ns = 256, 3
+    Y = rng.uniform(0.1, 1.0, (n, ns))
+    Y /= Y.sum(1, keepdims=True)
+    T = np.where(np.arange(n) % 2 == 0, rng.uniform(1000.2, 1004.0, n), rng.uniform(996.0, 999.8, n))
+    guess = T + np.where(T > 1000.0, 0.5, -0.5)
+    h = np.array([om.mixture_h(t, y) for t, y in zip(T, Y)])
+    rho = rng.uniform(0.2, 2.0, n)
+
+    def t3(a, nc):
+        return torch.tensor(np.ascontiguousarray(np.asarray(a).reshape(n, nc).T.reshape(nc, 1, 1, n)), device="cuda")
+
+    Tg = t3(guess, 1)
+    with extra_mechs.library(so):
+        rhoh_to_temp("jump_syn", ((0, 0, 0), (n - 1, 0, 0)), t3(Y * rho[:, None], ns), t3(rho * h * 1e-4, 1), Tg)
+        torch.cuda.synchronize()
+    To = om.hy2t(h, Y, guess)
+    np.testing.assert_allclose(To, T, rtol=1e-9)  # both sides have cells whose root is the guess's
+    np.testing.assert_allclose(Tg.cpu().numpy().reshape(n), To, rtol=1e-9)
