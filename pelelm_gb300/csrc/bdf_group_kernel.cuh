@@ -718,8 +718,8 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
         rho += C.Z[k];
         hm = fma(C.Z[k], M::Tab::h_mid(k), hm);
       }
-      const double inv_rho = 1.0 / rho;
-      Tn = hy2t_mixture<typename M::Tab>(rE * inv_rho, [&](int k) { return C.Z[k]; }, inv_rho, hm, Tn, 90.0, 5000.0);
+      Tn = hy2t_mixture<typename M::Tab>(__dmul_rn(rE, 1.0 / kRerg), [&](int k) { return C.Z[k]; }, rho, hm, Tn, 90.0,
+                                         5000.0);
     } else {
       // sums over species in the order of S lanes
       auto sum_of = [&](const double (&u)[R], const double (&v)[R]) -> double {

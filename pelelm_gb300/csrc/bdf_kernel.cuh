@@ -380,11 +380,10 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
       rho += Z(0, k);
       hm = fma(Z(0, k), M::Tab::h_mid(k), hm);
     }
-    const double inv_rho = 1.0 / rho;
     double Tn = Z(0, NS);
     if (!(Tn > 90.0 && Tn < 5000.0)) Tn = 1000.0;
-    Tn = hy2t_mixture<typename M::Tab>(rE * inv_rho, [&](int k) { return Z(0, k); }, inv_rho, hm, Tn, 90.0,
-                                          5000.0);
+    Tn = hy2t_mixture<typename M::Tab>(__dmul_rn(rE, 1.0 / kRerg), [&](int k) { return Z(0, k); }, rho, hm, Tn, 90.0,
+                                       5000.0);
     const double dt_inv = pgb_div64(1.0, tout);
 #pragma unroll 1
     for (int k = 0; k < NS; ++k) {

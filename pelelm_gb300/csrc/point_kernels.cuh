@@ -60,13 +60,12 @@ __global__ void rates_kernel(const PointParams p) {
   double rho = 0.0;
 #pragma unroll
   for (int s = 0; s < M::NS; ++s) { Y[s] = arr_at(p.rY, i, j, k, s); rho += Y[s]; }
-  const double inv_rho = 1.0 / rho;
   double hm = 0.0;
 #pragma unroll
   for (int s = 0; s < M::NS; ++s) hm = fma(Y[s], M::Tab::h_mid(s), hm);
-  // MKS -> CGS: h [J/kg] * 1e4 = erg/g ; rho [kg/m^3] * 1e-3 = g/cm^3
-  const double T = hy2t_mixture<typename M::Tab>(arr_at(p.rE, i, j, k, 0) * inv_rho * 1.0e4,
-                                                 [&](int s) { return arr_at(p.rY, i, j, k, s); }, inv_rho, hm,
+  // rho h [J/m^3] over R in the unit of rho [kg/m^3]: h [J/kg] * 1e4 = erg/g
+  const double T = hy2t_mixture<typename M::Tab>(__dmul_rn(arr_at(p.rE, i, j, k, 0), 1.0e4 / kRerg),
+                                                 [&](int s) { return arr_at(p.rY, i, j, k, s); }, rho, hm,
                                                  arr_at(p.T, i, j, k, 0), 90.0, 5000.0);
 #pragma unroll
   for (int s = 0; s < M::NS; ++s) C[s] = Y[s] * (1.0e-3 / M::W(s));
@@ -90,11 +89,9 @@ __global__ void h2t_kernel(const PointParams p) {
     rho += v;
     hm = fma(v, M::Tab::h_mid(s), hm);
   }
-  const double inv_rho = 1.0 / rho;
   double& T = arr_at(p.T, i, j, k, 0);
-  T = hy2t_mixture<typename M::Tab>(arr_at(p.rE, i, j, k, 0) * inv_rho * 1.0e4,
-                                    [&](int s) { return arr_at(p.rY, i, j, k, s); }, inv_rho, hm, T, p.tmin,
-                                    p.tmax);
+  T = hy2t_mixture<typename M::Tab>(__dmul_rn(arr_at(p.rE, i, j, k, 0), 1.0e4 / kRerg),
+                                    [&](int s) { return arr_at(p.rY, i, j, k, s); }, rho, hm, T, p.tmin, p.tmax);
 }
 
 // Heat release rate -sum_k rhoYdot_k h_k(T) [W/m^3] from T and the MKS reaction rates

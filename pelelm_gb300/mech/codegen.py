@@ -20,6 +20,7 @@ from __future__ import annotations
 import math
 import os
 import struct
+from fractions import Fraction
 from typing import Dict, List
 
 from .model import Mechanism, R_CAL, R_ERG, P_ATM
@@ -645,6 +646,16 @@ def _f32(x: float) -> float:
     return struct.unpack("f", struct.pack("f", x))[0]
 
 
+def enthalpy_about(a, W: float, tref: float) -> list:
+    """h/R per gram of NASA-7 coefficients `a` as a polynomial in x = T - tref, [d1..d5, d0] with
+    h = d0 + x (d1 + x (d2 + ...)); each rounded once."""
+    t, w = Fraction(tref), Fraction(W)
+    cp = [Fraction(v) / w for v in a[:5]]
+    d = [sum(cp[j] * math.comb(j, i) * t ** (j - i) for j in range(i, 5)) / (i + 1) for i in range(5)]
+    d0 = Fraction(a[5]) / w + sum(cp[i] * t ** (i + 1) / (i + 1) for i in range(5))
+    return [float(v) for v in d] + [float(d0)]
+
+
 def jac_stream(m: Mechanism, rx, tb_rows, codes, neg, T: int, LDA: int, L: int = 32):
     """The contribution program (kJacC, kJacNeg) in the form the kernels stream: (quads, entries,
     x0, nx).
@@ -837,6 +848,11 @@ def gen_tables(m: Mechanism, space: str = "constant") -> str:
         order = sorted(range(len(rx)), key=lambda j: (rx[j][3], j))
         rx = [rx[j] for j in order]
     maxeff = max([len(t) for t in tb_rows] + [1])
+    tmids = sorted({s.Tmid for s in m.species})
+    # where the mixture's enthalpy polynomial is expanded: mid-range below and above a common Tmid
+    # (errors of T from rho h against 64 bits on the workloads' states, 2-norm: expanded about 0 K 1.0 to
+    # 1.4e-16, about 1000 K 0.7 to 1.1e-16, so 0.6 to 0.8e-16), else one point, as ranges mix
+    tref = (600.0, 1800.0) if len(tmids) == 1 else (1000.0, 1000.0)
     e = _Emitter()
     e(f"// GENERATED by pelelm_gb300/mech/codegen.py (tables, {space} memory) from pelelm_gb300/data/{m.name}.json.")
     guard = f"PGB_{nsname.upper()}_CUH"
@@ -985,7 +1001,6 @@ def gen_tables(m: Mechanism, space: str = "constant") -> str:
         e(f"{qual} int kSpRxOff[NS + 1] = {{{', '.join(str(x) for x in off)}}};")
         e(f"{qual} int kSpRxJ[NSPRX] = {{{', '.join(str(x) for x in jj)}}};")
         e(f"{qual} double kSpRxNu[NSPRX] = {{{', '.join(_f(x) for x in nu)}}};")
-    tmids = sorted({s.Tmid for s in m.species})
     hmid = []  # h/R per gram of every species at the common Tmid (low-range polynomial)
     joined = len(tmids) == 1  # every h continuous there, but for rounding
     for s in m.species:
@@ -993,10 +1008,17 @@ def gen_tables(m: Mechanism, space: str = "constant") -> str:
         lo, hi = (a[5] + t * (a[0] + t * (a[1] / 2 + t * (a[2] / 3 + t * (a[3] / 4 + t * a[4] / 5)))) for a in (s.low, s.high))
         joined = joined and abs(lo - hi) <= 1e-12 * (abs(lo) + t)
         hmid.append(lo / s.W)
+    e(f"{qual} TabEnthalpy kEnthalpy[NS] = {{")
+    for s in m.species:
+        e("  {" + ", ".join("{" + ", ".join(_f(v) for v in enthalpy_about(a, s.W, t)) + "}"
+                            for a, t in zip((s.low, s.high), tref)) + "},")
+    e("};")
     e(f"{qual} double kHMid[NS] = {{{', '.join(_f(v) for v in hmid)}}};")
     e("struct Tables {")
     e(f"  static constexpr double TMID = {_f(tmids[0]) if len(tmids) == 1 else '-1.0'};  // common Tmid, or -1")
+    e(f"  static constexpr double TREF_LO = {_f(tref[0])}, TREF_HI = {_f(tref[1])};  // of the mixture polynomial")
     e(f"  static constexpr bool JOINED = {'true' if joined else 'false'};  // no jump of any h at that Tmid")
+    e("  __device__ static const TabEnthalpy& enthalpy(int k) { return kEnthalpy[k]; }")
     e("  __device__ static double h_mid(int k) { return kHMid[k]; }")
     e(f"  static constexpr int NS = {ns}, NR = {m.nr};")
     if glob:
