@@ -29,7 +29,7 @@
 //  * with few cells a warp of its own leaves three of the four schedulers of an SM idle and a cell
 //    waits for one warp's dependent latencies: teams of W = 4 warps share its right-hand side
 //    (team_rates) and its Jacobian (partials and contribution program), the first warp leading.
-//    Used for launches of up to four cells per SM, for the last four cells per SM of a longer one
+//    Used for launches of up to two cells per SM, for the last four cells per SM of a longer one
 //    (its warps hand them over) and for the FP64 pass over failed cells. Every sum keeps the order
 //    of the one-warp form, so the results are bit for bit the same. Measured (53 species, 60 cells
 //    mixed / 125 cells FP64): only the right-hand side shared 3.2 / 9.3 ms, the Jacobian too 2.5 / 7.5;

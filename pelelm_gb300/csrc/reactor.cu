@@ -313,15 +313,21 @@ int mapping_of(const pgb_reactor* r);
 // Most cells of a launch that goes to the small-launch kernel. Below it the time of a launch is
 // that of its stiffest cell, one FP64 warp instruction after the other (64 cycles each on an SM
 // partition, whatever the lanes), so more lanes per cell shorten it; above it the cells in flight
-// count, and the default mappings do more cells per instruction. Measured, small against default
-// kernel, mixed precision, dt_react 1e-5 s: 9 species 512 cells 9.1 / 29.1 ms, 4096 cells 13.5 / 30.7,
-// 16384 cells 31.8 / 32.0; 21 species 512 cells 7.6 / 22.1, 4096 cells 13.2 / 22.9, 8192 cells
-// 22.6 / 22.9. At 1e-6 s, where cells differ less, the lines lie at about 7,000 and 5,800 cells.
-// 53 species (teams of four warps, two at a time on an SM, against one warp a cell that hands its last
-// cells over): 448 cells 56.6 / 60.4, 576 cells 56.9 / 62.8, at 1e-6 s 6.2 / 6.1; 900 cells 7.9 / 6.4.
-long long small_limit(const pgb_reactor* r) {
-  if (r->mech->small_lanes > 32) return (long long)r->nsm * 4;
-  return (long long)r->nsm * (r->mech->ns <= 12 ? 48 : 40);
+// count, and the default mappings do more cells per instruction. Cells differ less over a short
+// dt_react, so the line lies lower there. Measured, small against default kernel (which hands its last
+// cells over), ms at cells per SM, dt_react 1e-6 and 1e-5 s:
+//   9 species, mixed  36: 3.4 / 3.9, 13.8 / 21.7   40: 4.1 / 4.1, 15.3 / 21.0   48: 4.3 / 4.1, 16.8 / 20.5
+//   9 species, FP64   28: 7.8 / 7.8, 25.6 / 37.7   36: 10.2 / 8.2, 29.5 / 38.6  48: 12.9 / 7.9, 36.0 / 36.9
+//  21 species, mixed  32: 4.8 / 5.2, 13.4 / 15.9   36: 5.3 / 5.2, 15.1 / 16.3   40: 5.8 / 5.3, 16.3 / 16.8
+//  21 species, FP64   28: 8.2 / 8.0, 21.2 / 21.3   36: 10.1 / 11.8, 23.7 / 24.8  40: 11.2 / 12.6, 26.1 / 27.0
+// 53 species (teams of four warps, two at a time on an SM, against one warp a cell)
+//   mixed  2: 5.8 / 5.9, 17.3 / 17.7   3: 7.0 / 6.4, 21.1 / 21.0      FP64  2: 8.6 / 8.7, 29.2 / 29.4   3: 14.1 / 12.3, 35.5 / 34.1
+long long small_limit(const pgb_reactor* r, double dt) {
+  const bool brief = dt < 3e-6;
+  const int per_sm = r->mech->small_lanes > 32 ? 2
+                     : r->mech->ns <= 12       ? (!brief ? 48 : r->opt.mixed ? 40 : 28)
+                                               : (brief && r->opt.mixed ? 34 : 40);
+  return (long long)r->nsm * per_sm;
 }
 
 // A launch that chose its mapping itself hands the last cells of each warp (`left` at most) to the
@@ -343,10 +349,10 @@ void set_drain(const pgb_reactor* r, LaunchPlan& pl, long long warps, bool mixed
 // force the layout or the block size. `mixed` selects the precision planned for (the FP64
 // retry pass plans FP64 whatever gb.precision says, and then ignores a gb.wpb that does not
 // fit FP64's shared memory).
-LaunchPlan plan_launch(const pgb_reactor* r, long long ncell, bool mixed) {
+LaunchPlan plan_launch(const pgb_reactor* r, long long ncell, bool mixed, double dt) {
   LaunchPlan pl;
   const MechEntry& m = *r->mech;
-  if (r->small_ok && m.small_mixed && ncell <= small_limit(r)) {
+  if (r->small_ok && m.small_mixed && ncell <= small_limit(r, dt)) {
     // one block per SM, one cell per warp while the SM's twelve warps allow it
     const int cpw = 32 / m.small_lanes;
     pl.small = true;
@@ -496,7 +502,7 @@ int enqueue_advance(pgb_reactor* r, Scratch& s, int nbox, long long ncell, doubl
     const long long nb = std::min<long long>((ncell + 255) / 256, (long long)r->nsm * 8);
     return r->mech->null_fn(p, st, (int)nb);
   }
-  const LaunchPlan pl = plan_launch(r, ncell, r->opt.mixed);
+  const LaunchPlan pl = plan_launch(r, ncell, r->opt.mixed, dt);
   p.lu_scratch = pl.lu_bytes ? s.d_lu : nullptr;
   p.z_scratch = pl.z_bytes ? s.d_z : nullptr;
   p.cells_per_warp = pl.cells_per_warp;
@@ -535,7 +541,7 @@ int enqueue_advance(pgb_reactor* r, Scratch& s, int nbox, long long ncell, doubl
       if ((r->opt.mixed ? r->mech->small_mixed : r->mech->small_fp64)(m, per_block, st, r->nsm)) return -1;
     }
     if (!retry) return 0;
-    const LaunchPlan p64 = plan_launch(r, ncell, false);
+    const LaunchPlan p64 = plan_launch(r, ncell, false, dt);
     pgb::ReactParams q = p;
     q.cell_list = p.retry_list;
     q.ncell_dev = p.retry_count;
@@ -544,7 +550,9 @@ int enqueue_advance(pgb_reactor* r, Scratch& s, int nbox, long long ncell, doubl
     q.resume = nullptr;
     q.drain = 0;
     q.done = nullptr;
-    if (r->small_ok && r->mech->small_lanes > 32) {  // few, and each as slow as its one warp: teams
+    // few, as a rule, and each as slow as its one warp: teams. (Where most cells fail one warp a cell is faster:
+    // 484 retried 41.0 / 40.2 ms, 1,252 51.5 / 48.8, 5,023 175 / 150; without teams in either pass 58.2, 69.1, 208.)
+    if (r->small_ok && r->mech->small_lanes > 32) {
       q.cells_per_warp = 0;
       PGB_CUDA(cudaMemsetAsync(s.d_counter, 0, sizeof(unsigned long long), st));
       return r->mech->small_fp64(q, 2, st, r->nsm);
@@ -800,7 +808,7 @@ int run_autotune(pgb_reactor* r, const std::vector<pgb::BoxDev>& boxes, long lon
     for (const Cand& c : cands) {
       r->opt.mapping = c.mapping;
       if (c.mapping == 2) r->opt.group = c.wpb; else r->opt.wpb = c.wpb;
-      const LaunchPlan pl = plan_launch(r, nsample, r->opt.mixed);
+      const LaunchPlan pl = plan_launch(r, nsample, r->opt.mixed, dt);
       if (ensure_buf(sc, sc.d_z, sc.z_cap, pl.z_bytes) || ensure_buf(sc, sc.d_lu, sc.lu_cap, pl.lu_bytes)) { rc = -1; break; }
       float ms = 0.f;
       for (int rep_i = 0; rep_i < 2 && !rc; ++rep_i) {  // warm-up launch, then the timed one
@@ -849,10 +857,10 @@ int advance_box_table(pgb_reactor* r, const std::vector<pgb::BoxDev>& boxes, lon
   Scratch* s = nullptr;
   if (ensure_scratch(r, st, std::max(nbox, 1), &s)) return -1;
   if (!r->null_reactor) {
-    LaunchPlan pl = plan_launch(r, ncell, r->opt.mixed);
+    LaunchPlan pl = plan_launch(r, ncell, r->opt.mixed, dt_react);
     s->last_small = pl.small;
     if (r->opt.mixed && r->opt.retry) {  // the FP64 retry pass shares the global scratch
-      const LaunchPlan p64 = plan_launch(r, ncell, false);
+      const LaunchPlan p64 = plan_launch(r, ncell, false, dt_react);
       pl.z_bytes = std::max(pl.z_bytes, p64.z_bytes);
       pl.lu_bytes = std::max(pl.lu_bytes, p64.lu_bytes);
       if (ensure_buf(*s, s->d_retry, s->retry_cap, std::max<long long>(ncell, 1) * sizeof(long long))) return -1;

@@ -49,3 +49,22 @@ def test_layout_keys_fix_the_kernel(native_lib, cuda, key):
     r = _reactor(cfg, key)
     assert _advance(cuda, r, cfg, (13, 9, 7), 3)[1] == (False, 0)
     r.close()
+
+
+# cells per SM on either side of the lines, short and long advances, both precisions
+@pytest.mark.gpu
+@pytest.mark.parametrize("cfgname,precision,dt,below,above", [
+    ("lidryer_amr120", "mixed", 1e-6, 40, 41), ("lidryer_amr120", "mixed", 1e-5, 48, 49),
+    ("lidryer_amr120", "fp64", 1e-6, 28, 29), ("lidryer_amr120", "fp64", 1e-5, 48, 49),
+    ("drm19_2M", "mixed", 1e-6, 34, 35), ("drm19_2M", "mixed", 1e-5, 40, 41), ("drm19_2M", "fp64", 1e-6, 40, 41),
+    ("gri_1M", "mixed", 1e-6, 2, 3)])
+def test_the_line_of_small_launches(native_lib, cuda, cfgname, precision, dt, below, above):
+    cfg = CONFIGS[cfgname]
+    sms = cuda.cuda.get_device_properties(0).multi_processor_count
+    r = _reactor(cfg, f"gb.precision={precision} ode.max_steps=2000")
+    for per_sm, small in ((below, True), (above, False)):
+        n = sms * per_sm
+        boxes = boxes_from_cells(cuda, make_cells(cfg, n, seed=6), [(n, 1, 1)])
+        r.react_boxes(boxes, dt, 0.0)
+        assert r.last_route()[0] == small
+    r.close()
