@@ -135,8 +135,7 @@ __global__ void __launch_bounds__(TPB, 1) bdf_reactor_kernel(const ReactParams P
   const double tout = P.dt;
 
   // ---- per-lane state ----
-  // a small launch spreads its cells over the SMs: the first P.cells_per_warp lanes of a warp work
-  int phase = P.cells_per_warp > 0 && lane >= P.cells_per_warp ? IDLE : NEED;
+  int phase = NEED;
   long long cell = -1;
   const long long ncell = P.ncell_dev ? (long long)*P.ncell_dev : P.ncell;
   int box = 0, ci = 0, cj = 0, ck = 0;

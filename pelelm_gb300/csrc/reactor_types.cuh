@@ -69,7 +69,7 @@ struct ReactParams {
   // array as it found it, so a second pass (FP64 after mixed precision) can start it over.
   long long* retry_list;
   unsigned long long* retry_count;
-  // Cells that a warp works on at a time (0: all that its mapping holds).
+  // Small-launch kernel: cells that a warp works on at a time (0: all that it holds).
   int cells_per_warp;
   // Hand-over of unfinished cells (all null / 0: none). Once the queue is empty, a warp with at most
   // `drain` cells left writes each of them to the next record of `resume` when it reaches the start of

@@ -915,10 +915,8 @@ def gen_tables(m: Mechanism, space: str = "constant") -> str:
         # stored partials of j that its code selects. Terms keep the order of the reaction walk
         # they replace: reactions ascending, then the row slots of the reaction. Entries go to
         # the 32 lanes largest first, to the lane with the fewest terms so far; each lane's terms
-        # are stored interleaved (term t of lane l at 32 t + l, lanes padded with empty terms to
-        # the longest) so a warp reads one contiguous line per load. Only the 4-byte codes are
-        # streamed per setup: W_i / W_k comes from the species table at an entry's first term,
-        # and a collider efficiency is read only where it differs from 1.
+        # are interleaved (term t of lane l at 32 t + l, lanes padded with empty terms to the
+        # longest). The kernels read it in the form that jac_stream makes of it.
         # code bits: 0-8 reaction (table order), 9-20 entry i * (N + 1) + k, 21 dq/dT (T column),
         # 22-24 / 25-27 the reactant / product slots of j holding species k, 28 the collider
         # term dq/d[M] times the efficiency of k, 29 last term of its entry (store the sum), 30
@@ -976,8 +974,10 @@ def gen_tables(m: Mechanism, space: str = "constant") -> str:
                         effF[pos] = f"(1.0f + {_f(em1)}f)"
                     t += 1
         e(f"constexpr int NJT = {T};  // program terms per lane (padded)")
+        e("#if 0  // the program that the streamed form below is made from: no kernel reads it")
         e(f"{qual} unsigned kJacC[32 * NJT] = {{{', '.join(str(x) + 'u' for x in codes)}}};")
         e(f"{qual} unsigned kJacNeg[NJT] = {{{', '.join(str(x) + 'u' for x in neg)}}};")
+        e("#endif")
         e(f"{qual} double kJacEffD[32 * NJT] = {{{', '.join(effD)}}};")
         e(f"{qual} float kJacEffF[32 * NJT] = {{{', '.join(effF)}}};")
         emit_jac_stream(e, qual, m, rx, tb_rows, codes, neg, T, LDA)
