@@ -172,11 +172,14 @@ __global__ void __launch_bounds__(256, 2) step_gemm_kernel(const bf16* __restric
 // db eight chains (row mod 8) added in order: the orders of gemm_nt_kernel and bias_grad_kernel (mlp.cu),
 // so both keep their bits. Adam's first steps divide a gradient by its own size, so another order
 // shows in the parameters (measured with the batch split: 5e-5 of a bias vector).
-// What bounds it is the walk: batch / 16 dependent products an accumulator. Tiles of 64 x 64 with four,
-// eight or sixteen products a scheduler in flight and of 32 x 64 with four or eight all took 62 to 71 us at a
-// batch of 8192 and four layers of 256 (the tensor pipe a quarter busy, seven stages or ten in flight);
-// the small tile reaches most SMs at narrow layers too. A stage's fragments are read while the products
-// of the one before run. The batch split over two CTAs per SM took 20 us, but gave other sums.
+// What bounds it is a stage's turn-round: a tile walks the batch in 128 stages of 64 rows at 1,100 cycles each
+// (batch 8192, four layers of 256: 62 us; 174 CTAs, issue slots of a busy SM 26 % used), and of these the four
+// dependent products of an accumulator are some 130; the rest is the wait for the copies, the block's barrier, and
+// each thread's three copies and eight fragment loads. The tiles are the long part (a step without them takes
+// 156 us, without the column sums 212, with both 214). Tiles of 64 x 64 with four, eight or sixteen products a
+// scheduler in flight and of 32 x 64 with four or eight all took 62 to 71 us (seven stages or ten in flight); the
+// small tile reaches most SMs at narrow layers too. A stage's fragments are read while the products of the one
+// before run. The batch split over two CTAs per SM took 20 us, but gave other sums.
 constexpr int GN = 32, GT = 64, GB = 64, GSTAGES = 7, LD_N = GN + 8, LD_G = GT + 8, GTHREADS = 256;
 constexpr int kGradSmem = GSTAGES * GB * (LD_N + LD_G) * 2;
 constexpr int kBiasCols = 16, kBiasRows = 256, kBiasStages = 6;
