@@ -740,7 +740,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_group_kernel(const ReactParam
         one[r] = 1.0;
       }
       const double inv_rho = pgb_div64(1.0, sum_of(y0, one));
-      const double htarget = rE * inv_rho;
+      const double htarget = __dmul_rn(rE, inv_rho);
 #pragma unroll 1
       for (int it = 0; it < 50; ++it) {
         const double invTn = pgb_div64(1.0, Tn);

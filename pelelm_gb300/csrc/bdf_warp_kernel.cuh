@@ -239,7 +239,7 @@ __device__ __noinline__ WVec<M> warp_rhs(const WVec<M> yv, double* CS, double* G
     const int k = idx(r);
     if (k < NS) {
       const TabSpecies<double>& s = Tab::template sp<double>(k);
-      const double c = y[r] * s.invW;
+      const double c = __dmul_rn(y[r], s.invW);
       CS[k] = c;
       c_loc += c;
       const double* g = below_positive(T, s.Tmid) ? s.glo : s.ghi;
@@ -507,6 +507,7 @@ __device__ __forceinline__ bool warp_lu_factor(JR* A, int* PIV, const JR g) {
 // Jacobian (equations of jac_table, mech_tables.cuh) into A, one warp cooperating. Inlined: each
 // kernel calls it from one place, so inlining adds no copy and removes the call's register save and
 // restore (measured: 1 to 3 %).
+// Every rounding is written out (fma, pgb_mul, pgb_add): kernels of different widths hand cells to one another.
 // W > 1: by the warps of a team (role 0 leads and has y; TJ: four numbers it tells the others; QN: [NR]
 // the reactions' net rates, whose energy sums the leader then forms in its own order).
 template <class M, class JR, int W = 1>
@@ -544,11 +545,11 @@ __device__ __forceinline__ void warp_jacobian(const WVec<M> yv, const double* FR
   for (int r = 0; r < R; ++r) {
     const int k = idx(r);
     if (k < NS) {
-      const JR c = (JR)y[r] * Tab::template sp<JR>(k).invW;
+      const JR c = pgb_mul((JR)y[r], Tab::template sp<JR>(k).invW);
       XS[k] = c;
       c_loc += c;
       JR g, h, cp, d;
-      nasa<JR>(Tab::template sp<JR>(k), T, invT, lnT1, g, h, cp, d);
+      nasa_exact<JR>(Tab::template sp<JR>(k), T, invT, lnT1, g, h, cp, d);
       TG[k] = g;
       TH_[k] = h;
       TC[k] = cp;
@@ -568,8 +569,9 @@ __device__ __forceinline__ void warp_jacobian(const WVec<M> yv, const double* FR
   JR Qw = JR(0), cpw = JR(0);
   for (int j = first; j < NR; j += 32 * W) {
     const TabReaction<JR>& r = Tab::template rx<JR>(j);
-    const JR lnkinf = r.beta * lnT + r.mEaR * invT + r.lnA;
-    JR dlnkf = (r.beta - r.mEaR * invT) * invT;
+    const JR eT = pgb_mul(r.mEaR, invT);
+    const JR lnkinf = pgb_add(fma(r.beta, lnT, eT), r.lnA);
+    JR dlnkf = pgb_mul(pgb_add(r.beta, -eT), invT);
     JR kf = pgb_expT<JR>(lnkinf);
     JR Mc = JR(1), alpha = JR(1), dkeff_dM = JR(0);
     if (r.tb >= 0) {
@@ -577,29 +579,32 @@ __device__ __forceinline__ void warp_jacobian(const WVec<M> yv, const double* FR
       Mc = Ctot;
 #pragma unroll
       for (int e = 0; e < 8; ++e)
-        if (e < t.n) Mc += t.effm1[e] * XS[t.sp[e]];
+        if (e < t.n) Mc = fma(t.effm1[e], XS[t.sp[e]], Mc);
       if (r.kind == 1) alpha = Mc;
     }
     if (r.kind == 2) {
       const TabTroe<JR>& fo = Tab::template troe<JR>(r.troe);
-      const JR lnk0 = fo.beta0 * lnT + fo.mEa0R * invT + fo.lnA0;
-      const JR dlnk0 = (fo.beta0 - fo.mEa0R * invT) * invT;
+      const JR eT0 = pgb_mul(fo.mEa0R, invT);
+      const JR lnk0 = pgb_add(fma(fo.beta0, lnT, eT0), fo.lnA0);
+      const JR dlnk0_T = pgb_add(fo.beta0, -eT0);  // times 1/T: d ln k0 / dT
       const JR k0 = pgb_expT<JR>(lnk0);
-      const JR Pr = Mc * pgb_expT<JR>(lnk0 - lnkinf);
+      const JR Pr = pgb_mul(Mc, pgb_expT<JR>(lnk0 - lnkinf));
       JR Fb = JR(1);
       if (fo.ntroe > 0) {
-        JR Fcent = fo.one_m_a * pgb_expT<JR>(T * fo.m_invT3) + fo.a * pgb_expT<JR>(T * fo.m_invT1);
-        if (fo.ntroe > 3) Fcent += pgb_expT<JR>(fo.m_T2 * invT);
-        const JR lFc = pgb_logT<JR>(Fcent) * JR(0.4342944819032518);
-        const JR cc = JR(-0.4) - JR(0.67) * lFc, nn = JR(0.75) - JR(1.27) * lFc;
-        const JR lPr = pgb_logT<JR>(Pr > JR(1e-30) ? Pr : JR(1e-30)) * JR(0.4342944819032518) + cc;
-        const JR f1 = lPr / (nn - JR(0.14) * lPr);
-        Fb = pgb_expT<JR>(JR(2.302585092994046) * lFc / (JR(1) + f1 * f1));
+        JR Fcent = fma(fo.one_m_a, pgb_expT<JR>(T * fo.m_invT3), pgb_mul(fo.a, pgb_expT<JR>(T * fo.m_invT1)));
+        if (fo.ntroe > 3) Fcent = pgb_add(Fcent, pgb_expT<JR>(fo.m_T2 * invT));
+        const JR lFc = pgb_mul(pgb_logT<JR>(Fcent), JR(0.4342944819032518));
+        const JR cc = fma(JR(-0.67), lFc, JR(-0.4)), nn = fma(JR(-1.27), lFc, JR(0.75));
+        const JR lPr = fma(pgb_logT<JR>(Pr > JR(1e-30) ? Pr : JR(1e-30)), JR(0.4342944819032518), cc);
+        const JR f1 = lPr / fma(JR(-0.14), lPr, nn);
+        Fb = pgb_expT<JR>(pgb_mul(JR(2.302585092994046), lFc) / fma(f1, f1, JR(1)));
       }
-      const JR onePr = JR(1) + Pr;
-      kf = kf * Pr / onePr * Fb;
-      dkeff_dM = Fb * k0 / (onePr * onePr);
-      dlnkf = dlnkf + (dlnk0 - dlnkf) / onePr;
+      const JR onePr = pgb_add(JR(1), Pr);
+      kf = pgb_mul(pgb_mul(kf, Pr) / onePr, Fb);
+      dkeff_dM = pgb_mul(Fb, k0) / pgb_mul(onePr, onePr);
+      // (the FP64 form fuses the difference: what each type's code did before its roundings were written out)
+      const JR dln = sizeof(JR) == sizeof(double) ? fma(dlnk0_T, invT, -dlnkf) : pgb_add(pgb_mul(dlnk0_T, invT), -dlnkf);
+      dlnkf = pgb_add(dlnkf, dln / onePr);
     }
     JR cr[3], cp[3];
 #pragma unroll
@@ -625,19 +630,20 @@ __device__ __forceinline__ void warp_jacobian(const WVec<M> yv, const double* FR
           dH -= TH_[r.rs[s]];
         }
       kr = kf * pgb_expT<JR>(fmin(dG, JR(700)));
-      dlnkr = dlnkf - (dH - (JR)r.dnu) * invT;
+      dlnkr = fma(-(dH - (JR)r.dnu), invT, dlnkf);
     }
-    const JR q = alpha * (kf * Pf - kr * Pp);
+    const JR net = fma(kf, Pf, -pgb_mul(kr, Pp));
+    const JR q = pgb_mul(alpha, net);
     JR* out = RX + j * wbdf::RXW;
-    out[0] = alpha * (kf * dlnkf * Pf - kr * dlnkr * Pp);
+    out[0] = pgb_mul(alpha, fma(pgb_mul(kf, dlnkf), Pf, -pgb_mul(pgb_mul(kr, dlnkr), Pp)));
 #pragma unroll
     for (int s = 0; s < 3; ++s) {
       out[1 + s] = alpha * kf * (s == 0 ? cr[1] * cr[2] : s == 1 ? cr[0] * cr[2] : cr[0] * cr[1]);
       out[4 + s] = -alpha * kr * (s == 0 ? cp[1] * cp[2] : s == 1 ? cp[0] * cp[2] : cp[0] * cp[1]);
     }
     JR bm = JR(0);
-    if (r.kind == 1) bm = kf * Pf - kr * Pp;
-    else if (r.kind == 2) bm = dkeff_dM * (Pf - (kf > JR(0) ? kr / kf : JR(0)) * Pp);
+    if (r.kind == 1) bm = net;
+    else if (r.kind == 2) bm = pgb_mul(dkeff_dM, fma(-(kf > JR(0) ? kr / kf : JR(0)), Pp, Pf));
     out[7] = bm;
     if (r.tb >= 0) {  // the collider terms of the listed species read these
       const TabThirdBody<JR>& t = Tab::template tb<JR>(r.tb);
@@ -654,8 +660,8 @@ __device__ __forceinline__ void warp_jacobian(const WVec<M> yv, const double* FR
         if (row < r.nr + r.np) {
           const bool isr = row < r.nr;
           const int i = isr ? r.rs[row] : r.ps[row - r.nr];
-          Qw += (isr ? -q : q) * TH_[i] * RT;
-          cpw += (isr ? -q : q) * TC[i] * JR(kRerg);
+          Qw = fma(pgb_mul(isr ? -q : q, TH_[i]), RT, Qw);
+          cpw = fma(pgb_mul(isr ? -q : q, TC[i]), JR(kRerg), cpw);
         }
     }
   }
@@ -670,8 +676,8 @@ __device__ __forceinline__ void warp_jacobian(const WVec<M> yv, const double* FR
           if (row < r.nr + r.np) {
             const bool isr = row < r.nr;
             const int i = isr ? r.rs[row] : r.ps[row - r.nr];
-            Qw += (isr ? -q : q) * TH_[i] * RT;
-            cpw += (isr ? -q : q) * TC[i] * JR(kRerg);
+            Qw = fma(pgb_mul(isr ? -q : q, TH_[i]), RT, Qw);
+            cpw = fma(pgb_mul(isr ? -q : q, TC[i]), JR(kRerg), cpw);
           }
       }
   }
@@ -763,10 +769,10 @@ __device__ __forceinline__ void warp_jacobian(const WVec<M> yv, const double* FR
       const JR cpm = c * JR(kRerg) * iw, hm = h * RT * iw;
       const JR yk = (JR)y[r];
       const JR fk = (JR)FRC[k];
-      D += yk * cpm;
-      dD += yk * d * JR(kRerg) * iw;
-      Qf -= hm * fk;
-      cpf += cpm * fk;
+      D = fma(yk, cpm, D);
+      dD = fma(pgb_mul(pgb_mul(yk, d), JR(kRerg)), iw, dD);
+      Qf = fma(-hm, fk, Qf);
+      cpf = fma(cpm, fk, cpf);
     }
   }
   D = warp_sum(D);
@@ -781,11 +787,11 @@ __device__ __forceinline__ void warp_jacobian(const WVec<M> yv, const double* FR
     if (k > NS) continue;
     JR acc = JR(0);
 #pragma unroll 1
-    for (int i = 0; i < NS; ++i) acc += TH_[i] * RT * Tab::template sp<JR>(i).invW * A[i * LDA + k];
+    for (int i = 0; i < NS; ++i) acc = fma(pgb_mul(pgb_mul(TH_[i], RT), Tab::template sp<JR>(i).invW), A[i * LDA + k], acc);
     if (k < NS) {
-      A[NS * LDA + k] = -acc * invD - QD2 * TC[k] * JR(kRerg) * Tab::template sp<JR>(k).invW;
+      A[NS * LDA + k] = fma(-pgb_mul(pgb_mul(QD2, TC[k]), JR(kRerg)), Tab::template sp<JR>(k).invW, pgb_mul(-acc, invD));
     } else {
-      A[NS * LDA + NS] = -(acc + cpwm) * invD - QD2 * dD;
+      A[NS * LDA + NS] = fma(-(acc + cpwm), invD, -pgb_mul(QD2, dD));
     }
   }
   __syncwarp();
@@ -1459,7 +1465,7 @@ __global__ void __launch_bounds__(WPB * 32, 1) bdf_warp_kernel(const ReactParams
     for (int r = 0; r < R; ++r)
       if (idx(r) < NS) rho_l += zget(0, r);
     const double inv_rho = pgb_div64(1.0, warp_sum(rho_l));
-    const double htarget = rE * inv_rho;
+    const double htarget = __dmul_rn(rE, inv_rho);
     double Tn = Z[NS];
     if (!(Tn > 90.0 && Tn < 5000.0)) Tn = 1000.0;
 #pragma unroll 1

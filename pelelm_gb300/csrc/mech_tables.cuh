@@ -174,6 +174,21 @@ __device__ __forceinline__ void nasa(const TabSpecies<R>& s, R T, R invT, R lnT1
   gRT = a[0] * lnT1 + T * (a[1] * R(-0.5) + T * (a[2] * R(-1.0 / 6.0) + T * (a[3] * R(-1.0 / 12.0) + T * a[4] * R(-0.05)))) +
         a[5] * invT - a[6];
 }
+// The same with its roundings written out (warp_jacobian, whose callers have to agree bit for bit).
+template <class R>
+__device__ __forceinline__ void nasa_exact(const TabSpecies<R>& s, R T, R invT, R lnT1, R& gRT, R& hRT, R& cpR, R& dcpR) {
+  const bool lo = T < s.Tmid;
+  R a[7];
+#pragma unroll
+  for (int i = 0; i < 7; ++i) a[i] = lo ? s.lo[i] : s.hi[i];
+  const R Ta = pgb_mul(T, a[4]);
+  cpR = fma(T, fma(T, fma(T, pgb_add(a[3], Ta), a[2]), a[1]), a[0]);
+  dcpR = fma(T, fma(R(2), a[2], pgb_mul(T, fma(R(3), a[3], pgb_mul(pgb_mul(T, R(4)), a[4])))), a[1]);
+  const R h2 = fma(a[2], R(1.0 / 3.0), pgb_mul(T, fma(a[3], R(0.25), pgb_mul(Ta, R(0.2)))));
+  hRT = fma(a[5], invT, fma(T, fma(T, h2, pgb_mul(a[1], R(0.5))), a[0]));
+  const R g2 = fma(T, fma(a[3], R(-1.0 / 12.0), pgb_mul(Ta, R(-0.05))), pgb_mul(a[2], R(-1.0 / 6.0)));
+  gRT = fma(a[5], invT, fma(a[0], lnT1, pgb_mul(T, fma(T, g2, pgb_mul(a[1], R(-0.5)))))) - a[6];
+}
 }  // namespace jac_detail
 
 // J(i,k) = d ydot_i / d y_k in type R. y: state (FP64, registers); Fr(k): rhoY forcing; Fh: rho h

@@ -40,6 +40,33 @@ def jump():
     return m
 
 
+def reduced(base, name, ns):
+    """`base` with ns species (CH4, its products and air among them), the least connected ones left out,
+    and the reactions of those alone."""
+    m = workloads.load_mechanism(base)
+    m.name = name
+    held = {"CH4", "O2", "N2", "H", "O", "OH", "CO2", "H2O"}
+    keep = [s.name for s in m.species]
+    while len(keep) > ns:
+        uses = {s: sum(s in r.reactants or s in r.products for r in m.reactions) for s in keep if s not in held}
+        keep.remove(min(uses, key=uses.get))
+        m.reactions = [r for r in m.reactions if all(s in keep for s in [*r.reactants, *r.products])]
+    m.species = [s for s in m.species if s.name in keep]
+    for r in m.reactions:
+        r.efficiencies = {s: e for s, e in r.efficiencies.items() if s in keep}
+    return m
+
+
+def reduced_cells(cs, base, m):
+    """The states of `base` on the species of `m`."""
+    cols = [base.index(s.name) for s in m.species]
+    cs = copy.deepcopy(cs)
+    cs.rY, cs.rYsrc = cs.rY[:, cols].copy(), cs.rYsrc[:, cols].copy()
+    rho = cs.rY.sum(1)
+    cs.rE = rho * workloads.mixture_h(m, cs.T, cs.rY / rho[:, None])
+    return cs
+
+
 def build(outdir, mechs):
     """Library of `mechs` alone in outdir; returns its path. Units that hold no mechanism are the
     product's objects."""

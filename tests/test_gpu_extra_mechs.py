@@ -5,23 +5,29 @@ import pytest
 import extra_mechs
 from helpers import boxes_from_cells, gather, outliers_within_global_error, tol_ratio
 from pelelm_gb300.reactor import ReactorBase, rhoh_to_temp
-from pelelm_gb300.workloads import CONFIGS, make_cells
+from pelelm_gb300.workloads import CONFIGS, load_mechanism, make_cells
+
+
+REDUCED = {"mid_syn": extra_mechs.reduced("drm19_syn", "mid_syn", 14), "wide_syn": extra_mechs.reduced("gri_syn", "wide_syn", 33)}
 
 
 @pytest.fixture(scope="session")
 def extra(native_lib, tmp_path_factory):
     """(library, folder) of the extra mechanisms."""
     d = str(tmp_path_factory.mktemp("extra"))
-    return extra_mechs.build(d, [extra_mechs.trio(), extra_mechs.jump()]), d
+    return extra_mechs.build(d, [extra_mechs.trio(), extra_mechs.jump(), *REDUCED.values()]), d
 
 
-def _advance(torch, cfg, cs, shape, mech, options):
+def _advance(torch, cfg, cs, shape, mech, options, small=None):
     boxes = boxes_from_cells(torch, cs, [shape])
     r = ReactorBase.create("ReactorCvode", mech, f"ode.rtol={cfg.rtol} ode.atol={cfg.atol} {options}")
     r.init(2, 1)
     r.react_boxes(boxes, cfg.dt, 0.0)
     torch.cuda.synchronize()
     nfail = r.stats()["nfail"]
+    if small is not None:  # a small launch, or cells handed over
+        route = r.last_route()
+        assert route[0] if small else route[1] > 0
     r.close()
     return gather(boxes, cs.rY.shape[1]), nfail
 
@@ -61,6 +67,24 @@ def test_kernels_agree_bit_for_bit(extra, cuda, shape, precision):
     assert fa == fb == 0
     for x, y in zip(a, b):
         np.testing.assert_array_equal(x, y)
+
+
+# the same of a group of lanes (14 species) and a warp (33) a cell: a small launch and one that hands cells over
+@pytest.mark.gpu
+@pytest.mark.parametrize("mech,cfgname,mapping,shapes", [("mid_syn", "drm19_2M", "group", [(13, 9, 7), (23, 21, 19)]),
+                                                        ("wide_syn", "gri_1M", "warp", [(13, 9, 2), (13, 9, 7)])])
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_larger_mechanisms_agree_bit_for_bit(extra, cuda, mech, cfgname, mapping, shapes, precision):
+    cfg = CONFIGS[cfgname]
+    for shape, small in zip(shapes, (True, False)):
+        cs = extra_mechs.reduced_cells(make_cells(cfg, int(np.prod(shape)), seed=8), load_mechanism(cfg.mech), REDUCED[mech])
+        opts = f"gb.precision={precision} ode.max_steps=2000"
+        with extra_mechs.library(extra[0]):
+            a, fa = _advance(cuda, cfg, cs, shape, mech, opts, small)
+            b, fb = _advance(cuda, cfg, cs, shape, mech, opts + f" gb.mapping={mapping}", None)
+        assert fa == fb
+        for x, y in zip(a, b):
+            np.testing.assert_array_equal(x, y)
 
 
 # enthalpies that jump at Tmid: targets between the two branches have a root on either side (a 5 K overlap),
