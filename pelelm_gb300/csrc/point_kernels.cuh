@@ -71,7 +71,7 @@ __global__ void rates_kernel(const PointParams p) {
   for (int s = 0; s < M::NS; ++s) C[s] = Y[s] * (1.0e-3 / M::W(s));
   M::wdot(T, C, wd);
 #pragma unroll
-  for (int s = 0; s < M::NS; ++s) arr_at(p.out, i, j, k, s) = wd[s] * M::W(s) * 1000.0;  // g/cm^3/s -> kg/m^3/s
+  for (int s = 0; s < M::NS; ++s) arr_at(p.out, i, j, k, s) = wd[s] * (M::W(s) * 1000.0);  // g/cm^3/s -> kg/m^3/s
 }
 
 template <class M>

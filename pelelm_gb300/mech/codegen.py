@@ -168,6 +168,9 @@ def gen_header(m: Mechanism) -> str:
     e("}")
     e()
     # ---------------------------------------------------------------- FP64 rates core
+    def plus_EaRT(ear, lnA):
+        return f"fma({_f(-ear)}, invT, {_f(lnA)})" if ear != 0 else _f(lnA)
+
     def emit_rates_fp64(with_energy: bool):
         """Emit body computing q{j} from T, lnT, invT, C{k}, g{k} (FP64)."""
         # third-body concentrations
@@ -182,7 +185,12 @@ def gen_header(m: Mechanism) -> str:
             e(f"double q{j};")
             e("{")
             e.ind += 1
-            e(f"const double lnkf = fma({_f(r.rate.beta)}, lnT, fma({_f(-ear)}, invT, {_f(lnA)}));")
+            # A as a factor: added to the exponent (near 30) it would cost the rate ten roundings
+            if r.kind == "falloff":
+                e(f"const double lnkf = fma({_f(r.rate.beta)}, lnT, {plus_EaRT(ear, lnA)});")
+            else:
+                beta, ear_T = _f(r.rate.beta), f"{_f(-ear)} * invT"
+                e("const double lnkfA = " + (f"{beta} * lnT;" if ear == 0 else f"fma({beta}, lnT, {ear_T});"))
             if r.kind != "elementary":
                 terms = "Ctot"
                 for sname, eff in r.efficiencies.items():
@@ -192,7 +200,7 @@ def gen_header(m: Mechanism) -> str:
             if r.kind == "falloff":
                 lnA0 = math.log(r.low.A)
                 ear0 = r.low.Ea / R_CAL
-                e(f"const double lnk0 = fma({_f(r.low.beta)}, lnT, fma({_f(-ear0)}, invT, {_f(lnA0)}));")
+                e(f"const double lnk0 = fma({_f(r.low.beta)}, lnT, {plus_EaRT(ear0, lnA0)});")
                 # Pr = k0 M / kinf
                 e("const double Pr = M * pgb_exp(lnk0 - lnkf);")
                 if r.troe:
@@ -211,7 +219,7 @@ def gen_header(m: Mechanism) -> str:
                     e("const double blend = Pr / (1.0 + Pr);")
                 e("const double kf = pgb_exp(lnkf) * blend;")
             else:
-                e("const double kf = pgb_exp(lnkf);")
+                e(f"const double kf = {_f(r.rate.A)} * pgb_exp(lnkfA);")
             pf = " * ".join(f"C{idx[s]}" for s, nu in r.reactants.items() for _ in range(nu))
             pr = " * ".join(f"C{idx[s]}" for s, nu in r.products.items() for _ in range(nu))
             if r.reversible:
