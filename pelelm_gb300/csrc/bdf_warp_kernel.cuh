@@ -530,8 +530,8 @@ __device__ __forceinline__ void warp_jacobian(const WVec<M> yv, const double* FR
   }
   const JR invT = JR(1) / T;
   const JR lnT = pgb_logT<JR>(T);
-  const JR lnT1 = JR(1) - lnT;
-  const JR lnP0RT = JR(kLnP0OverR) - lnT;
+  const JR lnT1 = pgb_add(JR(1), -lnT);
+  const JR lnP0RT = pgb_add(JR(kLnP0OverR), -lnT);
   const JR RT = JR(kRerg) * T;
   // per species, once: concentration (the solve vector is free during the setup) and the
   // NASA-7 terms g/RT, h/RT, cp/R, d(cp/R)/dT that the reaction and energy terms reuse

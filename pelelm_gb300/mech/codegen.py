@@ -426,7 +426,7 @@ def gen_header(m: Mechanism) -> str:
     for k, s in enumerate(m.species):
         for i in range(7):
             e(f"const R a{k}_{i} = lo_{int(s.Tmid)} ? R({_f(s.low[i])}) : R({_f(s.high[i])});")
-    e("const R lnT1 = R(1) - lnT;")
+    e("const R lnT1 = pgb_add(R(1), -lnT);")
     unused = {k for k in range(ns) if not any(m.species[k].name in r.reactants or m.species[k].name in r.products
                                               for r in m.reactions)}
     for k in range(ns):
@@ -454,7 +454,7 @@ def gen_header(m: Mechanism) -> str:
         for k in range(1, ns):
             tot = f"pgb_add_scaled<R>({tot}, y[{k}], {_f(1.0 / W[k])})" if k in total_only(m) else add(tot, f"C{k}")
         e(f"const R Ctot = {tot};")
-    e(f"const R lnP0RT = R({_f(lnP0_R)}) - lnT;")
+    e(f"const R lnP0RT = pgb_add(R({_f(lnP0_R)}), -lnT);")
     for k in range(ns):
         e(f"R wd{k} = R(0);")
     for k in range(ns):
