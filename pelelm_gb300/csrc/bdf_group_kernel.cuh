@@ -241,9 +241,9 @@ __device__ __forceinline__ GVec<M, G> group_rhs(const GVec<M, G> yv, double* CS,
         Tmid = s.Tmid;
         g = below_positive(T, Tmid) ? s.glo : s.ghi;
       }
-      const double c = __dmul_rn(y[r], invW);
+      const double c = y[r] * invW;
       CS[k] = c;
-      c_loc += c;
+      c_loc = __dadd_rn(c_loc, c);
       if (fused) { c_loc = y[r]; c_fac = invW; }
       GS[k] = fma(g[0], lnT1, fma(T, fma(T, fma(T, fma(T, g[4], g[3]), g[2]), g[1]), fma(g[5], invT, g[6])));
     }
@@ -323,7 +323,7 @@ __device__ __forceinline__ GVec<M, G> group_rhs(const GVec<M, G> yv, double* CS,
     rcp = lane_dot<NS, S>(c_one, cp_one, gm, gbase);
   }
   if constexpr (!UNROLLED) rcp *= kRerg;
-  const double fT = pgb_div64(fma(-hs, __dmul_rn(kRerg, T), FRC[NS]), rcp);
+  const double fT = pgb_div64(fma(-hs, kRerg * T, FRC[NS]), rcp);
 #pragma unroll
   for (int r = 0; r < R; ++r)
     if (idx(r) == NS) f[r] = fT;
